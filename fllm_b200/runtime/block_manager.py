@@ -284,6 +284,7 @@ class BlockManager:
         keep = self.blocks_needed(new_total)
         while len(sb.table) > keep:
             b = sb.table.pop()
+            sb._np_dirty = True               # the mirror may not keep what later appends put in these places
             if b >= 0:
                 self._release(b)
         sb.num_tokens = min(sb.num_tokens, new_total)

@@ -375,3 +375,18 @@ def test_preempted_victim_gives_back_rows_budget_and_cow_pairs():
     assert step.seqs == [] and step.cow == [] and step.cow_owner == []
     assert sch._take_refund() == 3 and sch._take_refund() == 0
     assert dropped == [b] and b in sch.waiting
+
+
+def test_table_mirror_follows_a_rollback_and_growth():
+    """Blocks that a rollback gave back and other sequences took must not stay in the array that batches are built from."""
+    from fllm_b200.runtime.block_manager import BlockManager
+    bm = BlockManager(16, 16, enable_prefix_caching=False)
+    for s in (0, 1):
+        bm.allocate(s, [])
+        assert bm.ensure_capacity(s, 33)
+        assert bm.np_table(s).tolist() == bm.table(s)
+    bm.truncate(0, 32)
+    bm.truncate(1, 32)
+    assert bm.ensure_capacity(0, 33) and bm.ensure_capacity(1, 33)
+    for s in (0, 1):
+        assert bm.np_table(s).tolist() == bm.table(s)
