@@ -123,7 +123,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a,
   volatile int* last_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   __nv_bfloat16* stage_out = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<uint8_t*>(bars) + S::kBarBytes);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp();
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -161,27 +161,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a,
   const int total = grouped ? *p.g_num_tiles * p.m_tiles : tiles * p.k_splits;
 
   if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
+    // ------------------------------------------------------------ TMA producer (the whole warp, one elected lane issues: uniform_warp)
     int pre = 0;                 // leading k-blocks of the first item whose weight tile is already in flight
-    if (lane == 0 && !grouped) {
+    if (!grouped && (int)blockIdx.x < total) {
       const int w = blockIdx.x;
-      if (w < total) {
-        const int split = p.cluster_red ? w % p.k_splits : w / tiles;
-        const int t = p.cluster_red ? w / p.k_splits : w - split * tiles;
-        const int n_idx = t / p.m_tiles;
-        const int m_idx = t - n_idx * p.m_tiles;
-        const int kb0 = split * p.kb_per_split;
-        const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
-        pre = min(kb1 - kb0, STAGES);
+      const int split = p.cluster_red ? w % p.k_splits : w / tiles;
+      const int t = p.cluster_red ? w / p.k_splits : w - split * tiles;
+      const int n_idx = t / p.m_tiles;
+      const int m_idx = t - n_idx * p.m_tiles;
+      const int kb0 = split * p.kb_per_split;
+      const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+      pre = min(kb1 - kb0, STAGES);
+      if (elect_one()) {
         for (int i = 0; i < pre; ++i) {
           mbar_expect_tx(&full_bar[i], S::kStageBytes);
           if (p.transposed) tma_load_2d(sA + i * S::kABytes, &tma_a, &full_bar[i], (kb0 + i) * BK, m_idx * BM);
           else tma_load_2d(sB + i * S::kBBytes, &tma_b, &full_bar[i], (kb0 + i) * BK, n_idx * BN);
         }
       }
+      __syncwarp();
     }
     if (!grouped) pdl_wait();
     uint32_t arrived = 0;        // bit s: rank s delivered all of its rows of the gathered operand
+    bool ok = true;
     if (p.ag_flags && p.transposed) {
       // decode orientation: every tile needs every rank's rows, so the whole warp polls the
       // arrival counters at once (one lane per source rank) instead of one after the other
@@ -195,92 +197,94 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a,
           if (p.status) atomicCAS(p.status, FLLM_OK, FLLM_ERR_PEER_TIMEOUT);
           *abort_flag = 1;
         }
+        ok = false;
       }
       arrived = 0xffffffffu;
       asm volatile("fence.proxy.async;" ::: "memory");
       __syncwarp();
     }
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = *abort_flag == 0;
-      for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-        const int split = p.cluster_red ? w % p.k_splits : w / tiles;
-        const int t = p.cluster_red ? w / p.k_splits : w - split * tiles;
-        const int n_idx = t / p.m_tiles;
-        const int m_idx = t - n_idx * p.m_tiles;
-        const int kb0 = split * p.kb_per_split;
-        const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
-        if (p.ag_flags) {
-          // token rows this tile reads: all of them when tokens sit in the N dimension
-          const int t_lo = p.transposed ? n_idx * BN : m_idx * BM;
-          const int t_hi = min(p.ag_tokens, t_lo + (p.transposed ? BN : BM));
-          if (t_hi > t_lo) {
-            for (int s = t_lo / p.rows_per; s <= (t_hi - 1) / p.rows_per && ok; ++s) {
-              if (arrived & (1u << s)) continue;
-              const uint32_t target = p.ag_consumed[s] + (uint32_t)rows_owned(p.ag_tokens, p.rows_per, s);
-              if (!wait_flag_ge(p.ag_flags + s, target, kPeerWaitPolls)) {
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
+      const int split = p.cluster_red ? w % p.k_splits : w / tiles;
+      const int t = p.cluster_red ? w / p.k_splits : w - split * tiles;
+      const int n_idx = t / p.m_tiles;
+      const int m_idx = t - n_idx * p.m_tiles;
+      const int kb0 = split * p.kb_per_split;
+      const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+      if (p.ag_flags) {
+        // token rows this tile reads: all of them when tokens sit in the N dimension
+        const int t_lo = p.transposed ? n_idx * BN : m_idx * BM;
+        const int t_hi = min(p.ag_tokens, t_lo + (p.transposed ? BN : BM));
+        if (t_hi > t_lo) {
+          for (int s = t_lo / p.rows_per; s <= (t_hi - 1) / p.rows_per && ok; ++s) {
+            if (arrived & (1u << s)) continue;
+            const uint32_t target = p.ag_consumed[s] + (uint32_t)rows_owned(p.ag_tokens, p.rows_per, s);
+            if (!__all_sync(0xffffffffu, wait_flag_ge(p.ag_flags + s, target, kPeerWaitPolls))) {
+              if (lane == 0) {
                 if (p.status) atomicExch(p.status, FLLM_ERR_PEER_TIMEOUT);
                 *abort_flag = 1;
-                ok = false;
               }
-              arrived |= 1u << s;
+              ok = false;
             }
-            // rows were written by peers through the generic proxy; TMA reads them through the async proxy
-            asm volatile("fence.proxy.async;" ::: "memory");
+            arrived |= 1u << s;
           }
-          if (!ok) break;
+          // rows were written by peers through the generic proxy; TMA reads them through the async proxy
+          asm volatile("fence.proxy.async;" ::: "memory");
+          __syncwarp();
         }
-        for (int kb = kb0; kb < kb1; ++kb) {
-          const bool prefetched = w == (int)blockIdx.x && kb - kb0 < pre;   // weight half already requested
-          if (!prefetched) {
-            if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-            mbar_expect_tx(&full_bar[stage], S::kStageBytes);
-          }
-          const int a_row = grouped ? p.g_tile_expert[n_idx] * p.g_rows + m_idx * BM : m_idx * BM;
-          const int b_row = grouped ? p.g_tile_row0[n_idx] : n_idx * BN;
+        if (!ok) break;
+      }
+      const int a_row = grouped ? p.g_tile_expert[n_idx] * p.g_rows + m_idx * BM : m_idx * BM;
+      const int b_row = grouped ? p.g_tile_row0[n_idx] : n_idx * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const bool prefetched = w == (int)blockIdx.x && kb - kb0 < pre;   // weight half already requested
+        if (!prefetched && !mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+        if (elect_one()) {
+          if (!prefetched) mbar_expect_tx(&full_bar[stage], S::kStageBytes);
           if (!(prefetched && p.transposed))
             tma_load_2d(sA + stage * S::kABytes, &tma_a, &full_bar[stage], kb * BK, a_row);
           if (!(prefetched && !p.transposed))
             tma_load_2d(sB + stage * S::kBBytes, &tma_b, &full_bar[stage], kb * BK, b_row);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, BN, 1, 1);
-      int stage = 0;
-      uint32_t phase = 0;
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-        const int split = p.cluster_red ? w % p.k_splits : w / tiles;
-        const int kb0 = split * p.kb_per_split;
-        const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+    constexpr uint32_t idesc = make_idesc(BM, BN, 1, 1);
+    const uint64_t da0 = make_smem_desc_sw128(smem_u32(sA)), db0 = make_smem_desc_sw128(smem_u32(sB));
+    int stage = 0;
+    uint32_t phase = 0;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
+      const int split = p.cluster_red ? w % p.k_splits : w / tiles;
+      const int kb0 = split * p.kb_per_split;
+      const int kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+      if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) break;
+      tc_fence_after_sync();
+      const uint32_t d_tmem = tmem_base + acc * BN;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint64_t da = make_smem_desc_sw128(smem_u32(sA + stage * S::kABytes));
-          const uint64_t db = make_smem_desc_sw128(smem_u32(sB + stage * S::kBBytes));
+        if (elect_one()) {
+          const uint64_t da = da0 + (uint64_t)(stage * (S::kABytes >> 4)), db = db0 + (uint64_t)(stage * (S::kBBytes >> 4));
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // advancing 16 bf16 = 32 bytes inside the swizzle row: +2 in 16-byte units
             tc_mma_bf16(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           tc_commit(&empty_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (kb + 1 == kb1) tc_commit(&tfull_bar[acc]);
         }
-        if (!ok) break;
-        tc_commit(&tfull_bar[acc]);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1;
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
     }
   } else {
     // ------------------------------------------------------------ epilogue
@@ -647,6 +651,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a,
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, int rows, int cols,
                                      long long ldc, const __nv_bfloat16* __restrict__ bias,
                                      __nv_bfloat16* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
@@ -844,10 +850,25 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
   if ((K & 7) || (N & 7) || (ldx & 7) || (ldw & 7) || (ldy & 1))
     throw std::runtime_error("linear_bf16: K, N and the row pitches must be multiples of 8");
   const int sms = sm_count();
-  // Large local products go to the CTA-pair kernel (cta_group::2, 256 x 256 tiles) once its tiles fill the machine.
-  if (!tpa && force_splits <= 0 && (ldy & 7) == 0 && linear_bf16_pair_supported(T, N, K) &&
-      (long long)((T + 255) / 256) * ((N + 255) / 256) >= sms / 2)
-    return linear_bf16_pair(x, ldx, w, ldw, bias, y, ldy, T, N, K, status, stream, glu ? ex : nullptr);
+  constexpr size_t kCounterBytes = 64 * 1024;
+  // Local products of more tokens than one swap-AB tile holds go to the CTA-pair kernel (cta_group::2, 256 x 256 tiles), over splits of K
+  // while its tiles do not fill the machine (200 tokens, 6144 x 4096: 25.4 us on one-CTA tiles, which read every weight twice).
+  if (!tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && T > 128 && N >= 256 && K >= BK) {
+    int splits = 1;
+    if ((long long)((T + 255) / 256) * ((N + 255) / 256) < sms / 2)
+      splits = linear_bf16_pair_splits(T, N, K, workspace && workspace_bytes > kCounterBytes && (!glu || defer) ? workspace_bytes - kCounterBytes : 0);
+    float* partials = splits > 1 ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + kCounterBytes) : nullptr;
+    splits = linear_bf16_pair(x, ldx, w, ldw, bias, y, ldy, T, N, K, status, stream, glu && splits <= 1 ? ex : nullptr, max(splits, 1), partials);
+    if (splits == 1) return 1;
+    if (defer) {
+      ex->deferred_splits = splits;
+      return 1;
+    }
+    const size_t n = (size_t)T * N;
+    launch_pdl(splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float*)partials, splits, T, N, ldy,
+               reinterpret_cast<const __nv_bfloat16*>(bias), reinterpret_cast<__nv_bfloat16*>(y));
+    return 2;
+  }
   GemmArgs a{};
   a.K = K;
   a.k_blocks = (K + BK - 1) / BK;
@@ -900,7 +921,6 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
     splits = min(min(slots / tiles, a.k_blocks / 4), 16);
   }
   // workspace = [tile counters (kCounterBytes, zero between launches)] [fp32 partial tiles]
-  constexpr size_t kCounterBytes = 64 * 1024;
   if (splits > 1 && (!workspace || workspace_bytes <= kCounterBytes || (size_t)tiles * 4 > kCounterBytes || bn > 128))
     splits = 1;
   while (splits > 1 && kCounterBytes + (size_t)splits * tiles * BM * bn * sizeof(float) > workspace_bytes) --splits;
@@ -972,10 +992,7 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
   if (a.k_splits > 1 && !a.fixup) {
     // dense [token][feature] partials in both orientations
     const size_t n = (size_t)T * N;
-    const int threads = 256;
-    const int blocks = (int)((n / 4 + threads - 1) / threads);
-    splitk_reduce_kernel<<<blocks, threads, 0, stream>>>(a.ws, a.k_splits, T, N, ldy, a.bias, a.out);
-    cuda_check(cudaGetLastError(), "splitk_reduce_kernel launch");
+    launch_pdl(splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float*)a.ws, a.k_splits, T, N, ldy, a.bias, a.out);
     return 2;
   }
   return 1;

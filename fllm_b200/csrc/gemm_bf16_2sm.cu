@@ -37,6 +37,8 @@ constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;                // shared-window a
 struct Gemm2Args {
   int M, N, K;                               // M = tokens, N = features
   int m_tiles, n_tiles, k_blocks;
+  int k_splits, kb_per_split;                // items are (split, tile); more than one split: fp32 partial sums in ws, [split][token][feature]
+  float* ws;
   long long ldc;
   __nv_bfloat16* out;
   const __nv_bfloat16* bias;
@@ -110,7 +112,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
   uint64_t* tempty_bar = bars + 2 * P2_STAGES + 2;   // used in the even CTA: both epilogues drained the buffer
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * P2_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
 
@@ -132,49 +134,53 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
   // columns. The next kernel starts when the whole grid is done, and for the same reason this one does not start before
   // the kernels ahead of it are done: pairs and single CTAs never hold tensor memory at the same time.
 
-  const int tiles = p.m_tiles * p.n_tiles;
+  const int tiles = p.m_tiles * p.n_tiles, items = tiles * p.k_splits;
   const int n_clusters = gridDim.x >> 1, cluster_id = blockIdx.x >> 1;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int t = cluster_id; t < tiles && ok; t += n_clusters) {
-        const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int w = cluster_id; w < items && ok; w += n_clusters) {
+      const int split = w / tiles, t = w - split * tiles;
+      const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
+      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+        if (elect_one()) {
           if (leader) mbar_expect_tx(&full_bar[stage], 2 * kP2StageBytes);
-          tma_load_2d_pair(sX + stage * kP2OperandBytes, &tma_x, &full_bar[stage], kb * P2_BK,
-                           m_idx * P2_TILE + (int)rank * P2_ROWS);
-          tma_load_2d_pair(sW + stage * kP2OperandBytes, &tma_w, &full_bar[stage], kb * P2_BK,
-                           n_idx * P2_TILE + (int)rank * P2_ROWS);
-          if (++stage == P2_STAGES) { stage = 0; phase ^= 1; }
+          tma_load_2d_pair(sX + stage * kP2OperandBytes, &tma_x, &full_bar[stage], kb * P2_BK, m_idx * P2_TILE + (int)rank * P2_ROWS);
+          tma_load_2d_pair(sW + stage * kP2OperandBytes, &tma_w, &full_bar[stage], kb * P2_BK, n_idx * P2_TILE + (int)rank * P2_ROWS);
         }
+        __syncwarp();
+        if (++stage == P2_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader) {
       constexpr uint32_t idesc = make_idesc(P2_TILE, P2_TILE, 1, 1);       // bf16 x bf16, M = 256 over the pair, N = 256
+      const uint64_t da0 = make_smem_desc_sw128(smem_u32(sX)), db0 = make_smem_desc_sw128(smem_u32(sW));
       int stage = 0, buf = 0;
       uint32_t phase = 0, buf_phase = 0;
       bool ok = true;
-      for (int t = cluster_id; t < tiles && ok; t += n_clusters) {
-        if (!mbar_wait(&tempty_bar[buf], buf_phase ^ 1, abort_flag)) break;
+      for (int w = cluster_id; w < items && ok; w += n_clusters) {
+        const int kb0 = w / tiles * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+        if (!mbar_wait_warp(&tempty_bar[buf], buf_phase ^ 1, abort_flag)) break;
         tc_fence_after_sync();
-        for (int kb = 0; kb < p.k_blocks; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint64_t da = make_smem_desc_sw128(smem_u32(sX + stage * kP2OperandBytes));
-          const uint64_t db = make_smem_desc_sw128(smem_u32(sW + stage * kP2OperandBytes));
+          if (elect_one()) {
+            const uint64_t off = (uint64_t)(stage * (kP2OperandBytes >> 4));
 #pragma unroll
-          for (int k = 0; k < P2_BK / 16; ++k)
-            tc_mma_bf16_pair(tmem_base + buf * P2_TILE, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          tc_commit_pair(&empty_bar[stage]);
+            for (int k = 0; k < P2_BK / 16; ++k)
+              tc_mma_bf16_pair(tmem_base + buf * P2_TILE, da0 + off + 2 * k, db0 + off + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            tc_commit_pair(&empty_bar[stage]);
+            if (kb + 1 == kb1) tc_commit_pair(&tfull_bar[buf]);
+          }
+          __syncwarp();
           if (++stage == P2_STAGES) { stage = 0; phase ^= 1; }
         }
-        if (!ok) break;
-        tc_commit_pair(&tfull_bar[buf]);
         buf ^= 1;
         if (buf == 0) buf_phase ^= 1;
       }
@@ -183,7 +189,8 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
     const int q = warp & 3;
     int buf = 0;
     uint32_t buf_phase = 0;
-    for (int t = cluster_id; t < tiles; t += n_clusters) {
+    for (int w = cluster_id; w < items; w += n_clusters) {
+      const int split = w / tiles, t = w - split * tiles;
       const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
       if (!mbar_wait(&tfull_bar[buf], buf_phase, abort_flag)) break;
       tc_fence_after_sync();
@@ -206,7 +213,14 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
         uint32_t r[32];
         tmem_ld_32x32(t_row + c0, r);
         tmem_ld_wait();
-        if (p.glu) {
+        if (p.k_splits > 1) {
+          float* part = p.ws + ((size_t)split * p.M + m) * p.N + n_base + c0;
+          if (m < p.M) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 4)
+              if (n_base + c0 + c < p.N) *reinterpret_cast<uint4*>(part + c) = make_uint4(r[c], r[c + 1], r[c + 2], r[c + 3]);
+          }
+        } else if (p.glu) {
           // features run along the columns: a 32-column chunk holds 16 (gate, up) pairs of this token
           const int n0 = n_base + c0;
           if (m < p.M && n0 < p.N) {
@@ -262,11 +276,28 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
 
 bool linear_bf16_pair_supported(int T, int N, int K) { return T >= 256 && N % 8 == 0 && N >= 256 && K % 8 == 0 && K >= P2_BK; }
 
+// K splits with which pairs finish a product of more than 128 tokens that has fewer tiles than pairs, or 0 when `workspace_bytes` holds
+// no split. In units of 10 ns: a K block of a tile takes 37, its share of the HBM bandwidth (27 for its products), an item 300 to start and
+// drain, a partial sum is written and read at 5 TB/s; a round of items is as long as one.
+int linear_bf16_pair_splits(int T, int N, int K, size_t workspace_bytes) {
+  const int pairs = sm_count() / 2, kbs = (K + P2_BK - 1) / P2_BK;
+  const long long tiles = (long long)((T + P2_TILE - 1) / P2_TILE) * ((N + P2_TILE - 1) / P2_TILE);
+  long long best = -1;
+  int splits = 0;
+  for (int s = 1; s <= 8 && s * 4 <= kbs; ++s) {
+    if (s > 1 && (size_t)s * T * N * sizeof(float) > workspace_bytes) break;
+    const long long cost = (tiles * s + pairs - 1) / pairs * ((kbs + s - 1) / s * 37 + 300) + (s > 1 ? (long long)(s * (double)T * N * 8 / 50000.0) : 0);
+    if (best < 0 || cost < best) { best = cost; splits = s; }
+  }
+  return splits;
+}
+
 // y[T, N] = x[T, K] * w[N, K]^T (+ bias[N]); row pitches in elements. With ex->glu the gated activation runs in the
-// epilogue and y is [T, N / 2] (N a multiple of 32).
+// epilogue and y is [T, N / 2] (N a multiple of 32). splits > 1: fp32 partial sums [splits][T][N] go to `partials` instead
+// (without bias or activation); returns the number of them.
 int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* y, long long ldy,
-                     int T, int N, int K, int* status, cudaStream_t stream, const LinearExtras* ex) {
-  if (!linear_bf16_pair_supported(T, N, K)) throw std::runtime_error("linear_bf16_pair: needs >= 256 tokens, N >= 256, N % 8 == 0, K % 8 == 0");
+                     int T, int N, int K, int* status, cudaStream_t stream, const LinearExtras* ex, int splits, float* partials) {
+  if (T <= 128 || N < 256 || N % 8 || K % 8 || K < P2_BK) throw std::runtime_error("linear_bf16_pair: needs more than 128 tokens, N >= 256, N % 8 == 0, K % 8 == 0");
   if ((ldy & 7)) throw std::runtime_error("linear_bf16_pair: output rows must be 16-byte aligned");
   const int glu = ex ? ex->glu : 0;
   if (glu && ((N & 31) || (ex->glu_pd != 16 && ex->glu_pd != 1))) throw std::runtime_error("linear_bf16_pair: GLU needs N % 32 == 0 and a pair distance of 16 or 1");
@@ -274,6 +305,9 @@ int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw,
   if (glu) { a.glu = glu; a.glu_pd = ex->glu_pd; a.glu_alpha = ex->glu_alpha; a.glu_limit = ex->glu_limit; }
   a.M = T; a.N = N; a.K = K;
   a.m_tiles = (T + P2_TILE - 1) / P2_TILE; a.n_tiles = (N + P2_TILE - 1) / P2_TILE; a.k_blocks = (K + P2_BK - 1) / P2_BK;
+  a.kb_per_split = (a.k_blocks + splits - 1) / splits;
+  a.k_splits = (a.k_blocks + a.kb_per_split - 1) / a.kb_per_split;
+  a.ws = partials;
   a.ldc = ldy; a.out = reinterpret_cast<__nv_bfloat16*>(y); a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.status = status;
   const CUtensorMap tx = make_tmap_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, K, ldx * 2, P2_ROWS, P2_BK, true);
   const CUtensorMap tw = make_tmap_2d(w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldw * 2, P2_ROWS, P2_BK, true);
@@ -281,9 +315,9 @@ int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw,
   if (first_call_on_device(configured))
     cuda_check(cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2Smem),
                "cudaFuncSetAttribute(gemm_bf16_pair_kernel)");
-  const int clusters = std::min(a.m_tiles * a.n_tiles, sm_count() / 2);
+  const int clusters = std::min(a.m_tiles * a.n_tiles * a.k_splits, sm_count() / 2);
   launch_cluster(false, gemm_bf16_pair_kernel, dim3(2 * clusters), dim3(kP2Threads), (size_t)kP2Smem, stream, 2u, tx, tw, a);
-  return 1;
+  return a.k_splits;
 }
 
 }  // namespace fllm

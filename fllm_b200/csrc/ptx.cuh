@@ -52,6 +52,12 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Index of the warp as a value the compiler knows to be the same in all lanes: branches on it stay convergent, and what they compute
+// can live in uniform registers. TMA and tcgen05.mma take their addresses and descriptors from those. Issued by `if (lane == 0)` in divergent
+// code every operand moves there first: 86 clocks per tcgen05.mma measured (a product of 128 x 16 x 16 values needs 8), and more per
+// box of TMA. So the whole warp walks the loop of a producer or MMA role, votes on its waits, and one elected lane issues.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // ----------------------------------------------------------------------------
 // mbarrier
 // ----------------------------------------------------------------------------
@@ -118,6 +124,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
   *abort_flag = 1;
   return false;
+}
+
+// The same by all lanes of a warp, which go on together.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
 }
 
 // ----------------------------------------------------------------------------
