@@ -32,6 +32,53 @@ int64_t moe_grouped_linear_w4(const Tensor& xp, const Tensor& codes, const Tenso
                                      st, cur_stream());
 }
 
+// x bf16 [tokens, k] -> xp fp16 [rows, k] times a power of two per row, factor fp32 [rows] (csrc/gemm_w4a16.cu: rows_f16)
+void moe_rows_f16(const Tensor& x, const optional<Tensor>& token_of, Tensor xp, Tensor factor, const optional<Tensor>& row_weight) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1, "x: bf16 rows");
+  TORCH_CHECK(xp.scalar_type() == at::kHalf && xp.dim() == 2 && xp.is_contiguous() && xp.size(1) == x.size(1), "xp: contiguous [rows, k] fp16");
+  TORCH_CHECK(factor.scalar_type() == at::kFloat && factor.is_contiguous() && factor.numel() >= xp.size(0), "factor: fp32 [rows]");
+  const int* t = nullptr;
+  if (token_of.has_value() && token_of->defined()) {
+    TORCH_CHECK(token_of->scalar_type() == at::kInt && token_of->is_contiguous() && token_of->numel() >= xp.size(0), "token_of: int32 [rows]");
+    t = token_of->data_ptr<int>();
+  } else {
+    TORCH_CHECK(xp.size(0) <= x.size(0), "xp: as many rows as x");
+  }
+  const float* w = nullptr;
+  if (row_weight.has_value() && row_weight->defined()) {
+    TORCH_CHECK(row_weight->scalar_type() == at::kFloat && row_weight->is_contiguous() && row_weight->numel() >= xp.size(0), "row_weight: fp32 [rows]");
+    w = row_weight->data_ptr<float>();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  fllm::rows_f16(x.data_ptr(), x.stride(0), t, w, xp.data_ptr(), factor.data_ptr<float>(), (int)xp.size(0), (int)x.size(1), cur_stream());
+}
+
+// The same on fp16 rows; factor: per row, or none (folded into alpha). glu_scale > 0: clamped SwiGLU-OAI in the epilogue, y fp16 [rows, n / 2] times it.
+int64_t moe_grouped_linear_w4_f16(const Tensor& xp, const optional<Tensor>& factor, const Tensor& codes, const Tensor& scales, int64_t fmt, double alpha,
+                                  const optional<Tensor>& bias_stack, Tensor y, const Tensor& tile_expert, const Tensor& tile_row0, const Tensor& num_tiles,
+                                  int64_t bn, const optional<Tensor>& status, double glu_alpha, double glu_limit, double glu_scale) {
+  const bool glu = glu_scale > 0;
+  TORCH_CHECK(codes.dim() == 3 && codes.is_contiguous() && codes.element_size() == 1, "codes: contiguous [E, n, k/2] bytes");
+  TORCH_CHECK(scales.is_contiguous() && scales.is_cuda() && scales.element_size() == 1 &&
+              scales.numel() == codes.numel() * 2 / (fmt == 0 ? 16 : 32), "scales: one byte per block");
+  TORCH_CHECK(xp.dim() == 2 && xp.stride(1) == 1 && xp.size(1) == codes.size(2) * 2 && xp.scalar_type() == at::kHalf, "xp: [rows, k] fp16");
+  TORCH_CHECK(y.dim() == 2 && y.stride(1) == 1 && y.size(0) == xp.size(0) && y.size(1) == codes.size(1) / (glu ? 2 : 1) &&
+              y.scalar_type() == (glu ? at::kHalf : at::kBFloat16), "y: [rows, n] bf16, or [rows, n / 2] fp16 behind an activation");
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(y.data_ptr()) & 15) == 0, "y: 16-byte aligned");
+  fllm::W4Rows r{nullptr, (float)glu_alpha, (float)glu_limit, (float)glu_scale};
+  if (factor.has_value() && factor->defined()) {
+    TORCH_CHECK(factor->scalar_type() == at::kFloat && factor->is_contiguous() && factor->numel() >= xp.size(0), "factor: fp32 [rows]");
+    r.factor = factor->data_ptr<float>();
+  }
+  c10::cuda::CUDAGuard guard(xp.device());
+  int* st = status.has_value() && status->defined() ? status->data_ptr<int>() : nullptr;
+  return fllm::moe_grouped_linear_w4(xp.data_ptr(), xp.stride(0), codes.data_ptr(), scales.data_ptr(), (int)fmt, (float)alpha,
+                                     optp(bias_stack), y.data_ptr(), y.stride(0), (int)xp.size(0), (int)codes.size(1),
+                                     (int)codes.size(2) * 2, (int)codes.size(0), tile_expert.data_ptr<int>(),
+                                     tile_row0.data_ptr<int>(), num_tiles.data_ptr<int>(), (int)tile_expert.numel(), (int)bn,
+                                     st, cur_stream(), &r);
+}
+
 // ---- expert-parallel all-to-all: a context of every rank's buffer addresses, then the four steps
 std::vector<fllm::EpArgs> g_ep;
 
@@ -104,6 +151,8 @@ void ep_wait_returns(int64_t h, int64_t epoch, const Tensor& status, const optio
 
 TORCH_LIBRARY_FRAGMENT(fllm_b200, m) {
   m.def("moe_grouped_linear_w4(Tensor xp, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status) -> int", &moe_grouped_linear_w4);
+  m.def("moe_rows_f16(Tensor x, Tensor? token_of, Tensor(a!) xp, Tensor(b!) factor, Tensor? row_weight=None) -> ()", &moe_rows_f16);
+  m.def("moe_grouped_linear_w4_f16(Tensor xp, Tensor? factor, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status, float glu_alpha=1.0, float glu_limit=0.0, float glu_scale=0.0) -> int", &moe_grouped_linear_w4_f16);
   m.def("ep_ctx_create(int ranks, int my_rank, int cap, int hidden, int experts_per_rank, int[] recv_x, int[] recv_meta, int[] ctrl, int[] comb_y) -> int", &ep_ctx_create);
   m.def("ep_dispatch(int ctx, Tensor x, Tensor ids, int epoch, Tensor? status, Tensor(a!)? call_ctr=None) -> ()", &ep_dispatch);
   m.def("ep_ingest(int ctx, int epoch, Tensor(a!) ids_out, Tensor(b!) count_out, Tensor? status, Tensor? call_ctr=None) -> ()", &ep_ingest);

@@ -41,9 +41,23 @@ int64_t linear_fp8_block(const Tensor& xq, const Tensor& sx, const Tensor& wq, c
                                 y.stride(0), (int)T, (int)N, (int)K, st, cur_stream(), ws, ws_bytes);
 }
 
+// y = x w^T (+ bias) on block-scaled e4m3 weights: quantise the activations, multiply; returns (y, kernels launched)
+std::tuple<Tensor, int64_t> fp8_block_apply(const Tensor& x, const Tensor& wq, const Tensor& sw, const optional<Tensor>& bias,
+                                            const optional<Tensor>& status, const optional<Tensor>& workspace) {
+  TORCH_CHECK(x.is_cuda() && x.dim() == 2 && wq.dim() == 2 && x.size(1) == wq.size(1), "x: [T, K], wq: [N, K]");
+  c10::cuda::CUDAGuard guard(x.device());
+  const Tensor xc = x.contiguous();
+  const int64_t T = x.size(0), K = x.size(1);
+  Tensor xq = at::empty({T, K}, x.options().dtype(at::kByte)), sx = at::empty({T, K / 128}, x.options().dtype(at::kFloat));
+  Tensor y = at::empty({T, wq.size(0)}, x.options().dtype(at::kBFloat16));
+  quant_fp8_1x128(xc, xq, sx);
+  const int64_t n = linear_fp8_block(xq, sx, wq, sw, bias, y, status, workspace);
+  return {y, 1 + n};
+}
+
 // codes uint8 [N, K/2]; scales uint8 [N, K/16] e4m3 (fmt 0), [N, K/32] e8m0 (fmt 1) or bf16 [N, K/32, 2] = {scale, min} (fmt 2)
 int64_t linear_w4a16(const Tensor& x, const Tensor& codes, const Tensor& scales, int64_t fmt, double alpha,
-                     const optional<Tensor>& bias, Tensor y, const optional<Tensor>& workspace, const optional<Tensor>& status) {
+                     const optional<Tensor>& bias, Tensor y, const optional<Tensor>& workspace, const optional<Tensor>& status, bool f16) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1, "x: bf16 rows");
   TORCH_CHECK(codes.is_contiguous() && codes.element_size() == 1 && codes.dim() == 2 && codes.size(1) * 2 == x.size(1), "codes: [N, K/2] bytes");
   const int64_t T = x.size(0), N = codes.size(0), K = x.size(1);
@@ -210,7 +224,8 @@ void w4_dequant(const Tensor& codes, const Tensor& scales, int64_t fmt, double a
 TORCH_LIBRARY_FRAGMENT(fllm_b200, m) {
   m.def("quant_fp8_1x128(Tensor x, Tensor(a!) xq, Tensor(b!) sx) -> ()", &quant_fp8_1x128);
   m.def("linear_fp8_block(Tensor xq, Tensor sx, Tensor wq, Tensor sw, Tensor? bias, Tensor(a!) y, Tensor? status, Tensor? workspace=None) -> int", &linear_fp8_block);
-  m.def("linear_w4a16(Tensor x, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status) -> int", &linear_w4a16);
+  m.def("fp8_block_apply(Tensor x, Tensor wq, Tensor sw, Tensor? bias, Tensor? status, Tensor? workspace) -> (Tensor, int)", &fp8_block_apply);
+  m.def("linear_w4a16(Tensor x, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status, bool f16=False) -> int", &linear_w4a16);
   m.def("quant_mx(Tensor x, Tensor(a!) xq, Tensor(b!) sf) -> ()", &quant_mx);
   m.def("quant_rows_8bit(Tensor x, Tensor(a!) xq, Tensor(b!) tok_scale, bool is_int8) -> ()", &quant_rows_8bit);
   m.def("linear_w8a8(Tensor xq, Tensor tok_scale, Tensor wq, Tensor feat_scale, bool is_int8, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status) -> int", &linear_w8a8);

@@ -135,14 +135,22 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
                      long long ldy, int T, int N, int K, int* status, cudaStream_t stream, void* workspace = nullptr,
                      size_t workspace_bytes = 0);   // workspace: fp32 split-K partials (few tiles, or K above 8192)
 
-// ---- packed 4-bit weights x bf16 activations (fmt 0 = NVFP4: e4m3 scale per 16; 1 = MXFP4: e8m0 per 32)
+void widen_rows(const void* x, long long ldx, float* out, int rows, int cols, cudaStream_t s);   // bf16 rows -> fp32
+
+// ---- packed 4-bit weights x 16-bit activations (fmt 0 = NVFP4: e4m3 scale per 16; 1 = MXFP4: e8m0 per 32)
 int linear_w4a16(const void* x, long long ldx, const void* codes, const void* scales, int fmt, float alpha,
                  const void* bias, void* y, long long ldy, int T, int N, int K, void* workspace, size_t workspace_bytes,
-                 int* status, cudaStream_t stream);
+                 int* status, cudaStream_t stream, bool f16 = false);
+// bf16 rows -> fp16 rows times 2^-e and factor[row] = 2^e; row r reads x[token_of[r]] (null: x[r]; -1: zeros)
+void rows_f16(const void* x, long long ldx, const int* token_of, const float* row_weight, void* out, float* factor, int rows, int K, cudaStream_t s);
+struct W4Rows {               // fp16 activation rows of a grouped product
+  const float* factor;        // per row (null: folded into alpha)
+  float glu_alpha, glu_limit, glu_scale;   // glu_scale > 0: clamped SwiGLU-OAI in the epilogue, fp16 output times glu_scale
+};
 int moe_grouped_linear_w4(const void* xp, long long ldx, const void* codes_stack, const void* scales_stack, int fmt,
                           float alpha, const void* bias_stack, void* y, long long ldy, int rows_cap, int n_out, int K,
                           int experts, const int* tile_expert, const int* tile_row0, const int* num_tiles, int max_tiles,
-                          int bn, int* status, cudaStream_t stream);
+                          int bn, int* status, cudaStream_t stream, const W4Rows* rows = nullptr);
 void w4_dequant_bf16(const void* codes, const void* scales, int fmt, float alpha, void* out, long long rows, int K,
                      cudaStream_t s);
 

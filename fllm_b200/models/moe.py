@@ -9,6 +9,7 @@ a partial sum that the caller reduces like a dense FFN output.
 """
 from __future__ import annotations
 
+import math
 from typing import Optional
 
 import torch
@@ -145,6 +146,46 @@ def _grouped(k_ops, ops, x, w, bias, y, tile_e, tile_r, ntiles, bn):
         k_ops.moe_grouped_linear(x, w, bias, y, tile_e, tile_r, ntiles, bn, ops.status)
 
 
+def _fp16_experts(lw) -> bool:
+    """Packed expert stacks that multiply as fp16 (ops.fp4.fp16_form)."""
+    return all(getattr(w, "f16", False) for w in (lw.exp_gate_up, lw.exp_down))
+
+
+def _oai_scale(alpha: float, limit: float) -> float:
+    """Power of two that brings the largest value of the clamped SwiGLU-OAI, limit (limit + 1), below the largest fp16 value; 0 where the
+    activation has no such bound. (The gate is not clamped from below: x sigmoid(alpha x) >= -0.279 / alpha.)"""
+    if not (alpha > 0 and limit > 0):
+        return 0.0
+    top = max(limit, 0.279 / alpha) * (limit + 1)
+    return 2.0 ** min(12, math.floor(math.log2(60000 / top))) if top < 60000 else 0.0
+
+
+def _packed_ffn(cfg, ops, spec: MoeSpec, lw, x: torch.Tensor, token_of, row_w, tile_e, tile_r, ntiles, bn: int, rows: int) -> torch.Tensor:
+    """Expert networks on packed stacks in fp16: rows gathered and converted in one kernel, the activation in the epilogue of the first
+    product where it is bounded (its fp16 values times a constant need no factor per row), else on rows converted again."""
+    H, k_ops = x.shape[1], ops.k
+    gu, dn = lw.exp_gate_up, lw.exp_down
+    where = (tile_e, tile_r, ntiles, bn, ops.status)
+    new = lambda n, dtype: torch.empty(rows, n, dtype=dtype, device=x.device)
+    xp, factor = new(H, torch.float16), torch.empty(rows, dtype=torch.float32, device=x.device)
+    k_ops.moe_rows_f16(x, token_of, xp, factor, row_w)
+    limit = cfg.swiglu_limit if spec.limit is None else spec.limit
+    scale = _oai_scale(cfg.swiglu_alpha, limit) if spec.act == "swiglu_oai" and cfg.mlp_kind != "plain" and gu.shape[1] % 16 == 0 else 0.0
+    if scale > 0:
+        act = new(gu.shape[1] // 2, torch.float16)
+        k_ops.moe_grouped_linear_w4_f16(xp, factor, gu.codes, gu.scales, gu.fmt, gu.alpha, lw.exp_gate_up_b, act, *where, cfg.swiglu_alpha, limit, scale)
+        factor = None
+    else:
+        u = new(gu.shape[1], torch.bfloat16)
+        k_ops.moe_grouped_linear_w4_f16(xp, factor, gu.codes, gu.scales, gu.fmt, gu.alpha, lw.exp_gate_up_b, u, *where)
+        u = ops.act_(u, spec.act) if cfg.mlp_kind == "plain" else ops.glu(u, ACT_KIND.get(spec.act, 0), cfg.swiglu_alpha, limit)
+        act, scale = new(u.shape[1], torch.float16), 1.0
+        k_ops.moe_rows_f16(u, None, act, factor)
+    y = new(H, torch.bfloat16)
+    k_ops.moe_grouped_linear_w4_f16(act, factor, dn.codes, dn.scales, dn.fmt, dn.alpha / scale, lw.exp_down_b, y, *where)
+    return y
+
+
 def _padded_router(lw, gate=None):
     """Router weight and bias with the expert count padded to a multiple of 8 (e.g. 60 experts); ``gate`` [.., H]: its first row follows
     the experts'."""
@@ -227,7 +268,10 @@ def moe_ffn(dec, lw, h: torch.Tensor, xe: Optional[torch.Tensor] = None, add: Op
         else:
             k_ops.moe_route(logits, None, k, spec.router != "softmax_topk", ids, wts)
     share = e_local / spec.experts
-    bn = 64 if h.dtype == torch.float32 else _token_tile(T * k * share / max(e_local, 1))
+    fp16 = h.dtype == torch.bfloat16 and _fp16_experts(lw)
+    per_expert = T * k * share / max(e_local, 1)
+    # packed weights are expanded once per tile: a tile that most experts fit into saves more than its padding costs
+    bn = 64 if h.dtype == torch.float32 else _token_tile(per_expert * (1.5 if fp16 else 1.0))
     rows_cap = -(-(T * k + e_local * (bn - 1)) // bn) * bn
     max_tiles = rows_cap // bn
     i32 = dict(dtype=torch.int32, device=h.device)
@@ -237,14 +281,17 @@ def moe_ffn(dec, lw, h: torch.Tensor, xe: Optional[torch.Tensor] = None, add: Op
     ntiles = torch.zeros(2, **i32)
     row_w = torch.empty(rows_cap, dtype=torch.float32, device=h.device) if spec.weigh_input else None
     k_ops.moe_align(ids, spec.experts, lo, lo + e_local, bn, row_of, token_of, tile_e, tile_r, ntiles, wts if spec.weigh_input else None, row_w)
-    xp = torch.empty(rows_cap, H, dtype=h.dtype, device=h.device)
-    k_ops.moe_gather(h if xe is None else xe, token_of, xp, row_w)
-    gu = torch.empty(rows_cap, lw.exp_gate_up.shape[1], dtype=h.dtype, device=h.device)
-    _grouped(k_ops, ops, xp, lw.exp_gate_up, lw.exp_gate_up_b, gu, tile_e, tile_r, ntiles, bn)
-    act = ops.act_(gu, spec.act) if cfg.mlp_kind == "plain" else \
-        ops.glu(gu, ACT_KIND.get(spec.act, 0), cfg.swiglu_alpha, cfg.swiglu_limit if spec.limit is None else spec.limit)
-    y = torch.empty(rows_cap, H, dtype=h.dtype, device=h.device)
-    _grouped(k_ops, ops, act, lw.exp_down, lw.exp_down_b, y, tile_e, tile_r, ntiles, bn)
+    if fp16:
+        y = _packed_ffn(cfg, ops, spec, lw, h if xe is None else xe, token_of, row_w, tile_e, tile_r, ntiles, bn, rows_cap)
+    else:
+        xp = torch.empty(rows_cap, H, dtype=h.dtype, device=h.device)
+        k_ops.moe_gather(h if xe is None else xe, token_of, xp, row_w)
+        gu = torch.empty(rows_cap, lw.exp_gate_up.shape[1], dtype=h.dtype, device=h.device)
+        _grouped(k_ops, ops, xp, lw.exp_gate_up, lw.exp_gate_up_b, gu, tile_e, tile_r, ntiles, bn)
+        act = ops.act_(gu, spec.act) if cfg.mlp_kind == "plain" else \
+            ops.glu(gu, ACT_KIND.get(spec.act, 0), cfg.swiglu_alpha, cfg.swiglu_limit if spec.limit is None else spec.limit)
+        y = torch.empty(rows_cap, H, dtype=h.dtype, device=h.device)
+        _grouped(k_ops, ops, act, lw.exp_down, lw.exp_down_b, y, tile_e, tile_r, ntiles, bn)
     out = torch.empty(T, H, dtype=h.dtype, device=h.device)
     k_ops.moe_combine(y, row_of, None if spec.weigh_input else wts, out, add, gate)
     ops.launches += 6

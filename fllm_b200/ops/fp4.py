@@ -80,6 +80,19 @@ def dequantize_fp4(codes: torch.Tensor, scales: torch.Tensor, fmt: int, alpha: f
     return v.view(N, K) * alpha
 
 
+def fp16_form(codes: torch.Tensor, scales: torch.Tensor, fmt: int) -> bool:
+    """Whether every value of a packed matrix is exact in fp16: NVFP4 always; MXFP4 when the scale byte of every block that holds
+    something else than zeros lies in [104, 140] (0.5 x 2^-23 .. 6 x 2^13; scale 0 counts as a factor of 0). Looked at once, when the
+    weight is laid out: the packed GEMM then multiplies fp16 values, otherwise bf16 ones."""
+    if fmt == NVFP4 or scales.numel() == 0:
+        return True
+    out = (scales > 140) | ((scales < 104) & (scales != 0))
+    if not bool(out.any()):
+        return True
+    rows = (codes.reshape(-1, 16)[out.reshape(-1)] & 0x77) != 0
+    return not bool(rows.any())
+
+
 class Fp4Weight:
     """A [N, K] matrix held as packed FP4 codes + block scales (+ tensor scale)."""
 
@@ -87,6 +100,7 @@ class Fp4Weight:
         self.codes, self.scales, self.fmt, self.alpha = codes, scales, int(fmt), float(alpha)
         self.shape = (codes.shape[0], codes.shape[1] * 2)
         self.device = codes.device
+        self.f16 = fp16_form(codes, scales, self.fmt)
 
     @classmethod
     def from_dense(cls, w: torch.Tensor, fmt="nvfp4") -> "Fp4Weight":
@@ -114,7 +128,7 @@ class Fp4Weight:
         if T <= 128:
             y = out if out is not None else torch.empty(T, N, dtype=torch.bfloat16, device=x.device)
             ops.launches += ops.k.linear_w4a16(x, self.codes, self.scales, self.fmt, self.alpha, bias, y,
-                                               ops.workspace, ops.status)
+                                               ops.workspace, ops.status, self.f16)
             return y
         dense = ops.scratch_bf16(N * K).view(N, K)
         ops.k.w4_dequant(self.codes, self.scales, self.fmt, self.alpha, dense)
@@ -131,6 +145,7 @@ class Fp4ExpertStack:
         self.codes, self.scales, self.fmt, self.alpha = codes.contiguous(), scales.contiguous(), int(fmt), float(alpha)
         self.shape = (codes.shape[0], codes.shape[1], codes.shape[2] * 2)
         self.device = codes.device
+        self.f16 = fp16_form(self.codes, self.scales, self.fmt)
 
     @classmethod
     def from_dense(cls, stack: torch.Tensor, fmt="mxfp4") -> "Fp4ExpertStack":

@@ -1,0 +1,115 @@
+"""Packed FP4 weights on the fp16 form: row conversion, dense and grouped products at the edges of tiles, and which weights take it."""
+import pytest
+import torch
+
+from fllm_b200.ops.fp4 import Fp4ExpertStack, Fp4Weight, dequantize_fp4, fp16_form
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from fllm_b200.ops import get_ops
+    return get_ops(torch.device("cuda:0"))
+
+
+def _rand(shape, seed, std=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * std).to(torch.bfloat16)
+
+
+def _rel(y, ref):
+    return ((y.double() - ref).norm() / ref.norm()).item()
+
+
+def test_which_weights_are_exact_in_fp16():
+    codes = torch.full((2, 32), 0x77, dtype=torch.uint8)
+    scales = torch.full((2, 2), 120, dtype=torch.uint8)
+    assert fp16_form(codes, scales, 1) and fp16_form(codes, scales, 0)
+    for s, ok in ((104, True), (103, False), (140, True), (141, False), (0, True), (255, False)):
+        scales[1, 1] = s
+        assert fp16_form(codes, scales, 1) == ok
+    codes[1, 16:] = 0x88                       # zeros (of either sign) need no scale, unless it is not a number
+    for s, ok in ((1, True), (103, True)):
+        scales[1, 1] = s
+        assert fp16_form(codes, scales, 1) == ok
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [64, 320, 2880, 28672])
+def test_rows_keep_every_value(ops, K):
+    """fp16 rows times their factor are the bf16 rows again, over the whole exponent range and next to values that are not finite. A value
+    below 2^-31 of the row's largest, whose 8 bits reach under the smallest fp16 step of 2^-24, may be off by half of that step."""
+    x = _rand((9, K), 1)
+    x[0] *= 2.0 ** 100
+    x[1] *= 2.0 ** -110
+    x[2] = 0
+    x[3, 1::2] *= 2.0 ** -20
+    x[4, 5], x[5, 6], x[5, 7] = float("nan"), float("inf"), -float("inf")
+    x[6] = torch.finfo(torch.bfloat16).max
+    xh, f = torch.empty(11, K, dtype=torch.float16, device="cuda"), torch.empty(11, device="cuda")
+    token_of = torch.tensor([0, -1, 1, 2, 3, 4, 5, 6, 7, 8, -1], dtype=torch.int32, device="cuda")
+    ops.k.moe_rows_f16(x.cuda(), token_of, xh, f)
+    back = (xh.double() * f.double()[:, None]).cpu()
+    rows = [i for i in range(11) if token_of[i] >= 0]
+    xd = x.double()
+    finite = xd.isfinite()
+    assert torch.equal(back[rows][~finite].nan_to_num(5.0), xd[~finite].nan_to_num(5.0))
+    off = torch.where(finite, (back[rows] - xd).abs(), 0)
+    top = torch.where(finite, xd.abs(), 0).amax(1, keepdim=True)
+    assert (off <= f.double().cpu()[rows][:, None] * 2.0 ** -25).all() and (off[finite & (xd.abs() >= top * 2.0 ** -31)] == 0).all()
+    assert (back[[1, 10]] == 0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fmt", ["nvfp4", "mxfp4"])
+@pytest.mark.parametrize("T,N,K", [(5, 128, 64), (17, 136, 192), (64, 256, 1088), (65, 1000, 320), (128, 40960, 256), (128, 512, 12288)])
+def test_dense_against_64_bits(ops, fmt, T, N, K):
+    """One rounding to bf16 (2^-9 of a value at most, 0.17 % in the mean square) is all that a correct product is off."""
+    x, q = _rand((T, K), 1).cuda(), Fp4Weight.from_dense(_rand((N, K), 2, 0.05).cuda(), fmt)
+    assert q.f16
+    x[0] *= 2.0 ** 40
+    y = ops.linear(x, q)
+    ref = x.double() @ dequantize_fp4(q.codes, q.scales, q.fmt, 1.0).double().t() * q.alpha
+    assert _rel(y[:1], ref[:1]) < 2.5e-3 and _rel(y[1:], ref[1:]) < 2.5e-3
+    assert ops.check_status() == 0
+
+
+@pytest.mark.gpu
+def test_scales_beyond_fp16_take_the_bf16_form(ops):
+    q = Fp4Weight.from_dense(_rand((256, 512), 2, 0.05).cuda(), "mxfp4")
+    q = Fp4Weight(q.codes, q.scales - 60, 1)
+    assert not q.f16
+    x = _rand((24, 512), 1).cuda()
+    assert _rel(ops.linear(x, q), x.double() @ dequantize_fp4(q.codes, q.scales, 1).double().t()) < 2.5e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bn", [16, 32, 64, 128])
+@pytest.mark.parametrize("n,k", [(32, 64), (304, 192), (5760, 2880)])
+@pytest.mark.parametrize("glu", [False, True])
+def test_grouped(ops, bn, n, k, glu):
+    """Experts with no row, one row, a full tile and one more than that; the clamped activation in the epilogue."""
+    counts = [0, 1, bn, bn + 1, 7]
+    E = len(counts)
+    q = Fp4ExpertStack.from_dense(_rand((E, n, k), 3, 0.05).cuda())
+    bias = _rand((E, n), 4, 0.1).cuda()
+    tiles = [(e, j) for e, c in enumerate(counts) for j in range(-(-c // bn))]
+    rows = len(tiles) * bn
+    tile_e = torch.tensor([e for e, _ in tiles] + [0] * 3, dtype=torch.int32, device="cuda")
+    tile_r = torch.arange(len(tiles) + 3, dtype=torch.int32, device="cuda") * bn
+    real = torch.cat([torch.arange(bn) + j * bn < counts[e] for e, j in tiles]).cuda()
+    x = _rand((rows, k), 5).cuda()
+    token_of = torch.where(real, torch.arange(rows, device="cuda"), -1).int()
+    xh, f = torch.empty(rows, k, dtype=torch.float16, device="cuda"), torch.empty(rows, device="cuda")
+    ops.k.moe_rows_f16(x, token_of, xh, f)
+    y = torch.empty(rows, n // 2 if glu else n, dtype=torch.float16 if glu else torch.bfloat16, device="cuda")
+    num = torch.tensor([len(tiles), rows], dtype=torch.int32, device="cuda")
+    ops.k.moe_grouped_linear_w4_f16(xh, f, q.codes, q.scales, 1, 1.0, bias, y, tile_e, tile_r, num, bn, ops.status, *((1.702, 7.0, 512.0) if glu else ()))
+    dense = q.dense().double()
+    for i, (e, _) in enumerate(tiles):
+        s = slice(i * bn, (i + 1) * bn)
+        ref = x[s].double() @ dense[e].t() + bias[e].double()
+        if glu:
+            g, u = ref[:, 0::2].clamp(max=7.0), ref[:, 1::2].clamp(-7.0, 7.0)
+            ref = g * torch.sigmoid(1.702 * g) * (u + 1) * 512.0
+        # 0.05 x sqrt(k) in front of the activation; its fp16 result is rounded to 2^-11
+        assert _rel(y[s][real[s]], ref[real[s]]) < 2.5e-3
+    assert ops.check_status() == 0
