@@ -19,6 +19,8 @@
 // 128-element boundaries.
 #include <cuda_fp8.h>
 
+#include <algorithm>
+
 #include "fllm_ops.h"
 #include "ptx.cuh"
 #include "tma_host.h"
@@ -28,7 +30,7 @@ namespace fllm {
 constexpr int F8_BM = 128;
 constexpr int F8_BK = 128;      // e4m3 elements = bytes per swizzle row = scale block depth
 constexpr int F8_UMMA_K = 32;
-constexpr int kF8Threads = 192;
+constexpr int kF8Threads = 64 + 256;      // TMA warp, MMA warp, eight promoting warps
 
 struct Fp8GemmArgs {
   int M, N, K;              // MMA orientation: D[M][N] = A[M][K] B[N][K]^T
@@ -49,18 +51,29 @@ struct Fp8Smem {
   static constexpr int kABytes = F8_BM * F8_BK;
   static constexpr int kBBytes = BN * F8_BK;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = (BN <= 64 ? 80 * 1024 : 160 * 1024) / kStageBytes;
-  static constexpr int kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;
-  static constexpr int kScaleFloats = 64 * BN;            // token scales of a swap-AB tile, up to 64 K blocks
+  static constexpr int kScaleFloats = BN <= 64 ? 64 * BN : 0;       // token scales of a swap-AB tile, up to 64 K blocks
+  static constexpr int kStages = (196 * 1024 - kScaleFloats * 4) / kStageBytes > 10 ? 10 : (196 * 1024 - kScaleFloats * 4) / kStageBytes;
+  // A K block's product stays in its buffer until the promoting warps have added it up: the tensor core runs ahead by the other buffers.
+  static constexpr int kBuffers = BN == 256 ? 2 : 4;
+  static constexpr int kTmemCols = kBuffers * BN < 128 ? (kBuffers * BN < 64 ? 64 : kBuffers * BN) : kBuffers * BN;
+  static constexpr int kHalves = BN >= 64 ? 2 : 1;                  // warps that share a lane quarter split the columns
+  static constexpr int kCols = BN / kHalves;                        // columns of a promoting thread
+  static constexpr int kPromote = 128 * kHalves;                    // promoting threads with columns
   static constexpr int kTotal = kStages * kStageBytes + kScaleFloats * 4 + 256 + 1024;
+  static_assert((2 * kStages + 2 * kBuffers) * 8 + 8 <= 256, "barrier block");
 };
 
+// What bounds it: a 128 x 256 x 128 block is 512 clocks of the tensor core; promoting it is 32768 multiply-adds, 256 issue slots of each
+// scheduler over eight warps, so the products bound it as long as a thread's share costs one multiply-add per value: one factor per row
+// and K block (activation scale x weight scale, read ahead), one accumulator register per column. 128 x 128 tiles read and write shared memory
+// twice as often per product; they remain for few tiles.
 template <int BN>
 __global__ void __launch_bounds__(kF8Threads, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const Fp8GemmArgs p) {
   using S = Fp8Smem<BN>;
-  constexpr int STAGES = S::kStages;
+  constexpr int STAGES = S::kStages, NBUF = S::kBuffers, COLS = S::kCols;
+  constexpr bool SWAP = BN <= 64;          // tokens in the N dimension
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
@@ -70,14 +83,14 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + STAGES;
   uint64_t* tfull_bar = bars + 2 * STAGES;
-  uint64_t* tempty_bar = bars + 2 * STAGES + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint64_t* tempty_bar = tfull_bar + NBUF;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + NBUF);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 128); }
+    for (int a = 0; a < NBUF; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 4 * S::kHalves); }
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -87,56 +100,75 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();
   const int tiles = p.m_tiles * p.n_tiles * p.k_splits;      // work items: the split is the fastest index
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
-        const int split = w % p.k_splits, t = w / p.k_splits;
-        const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
-        const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-          mbar_expect_tx(&full_bar[stage], S::kStageBytes);
-          tma_load_2d(sA + stage * S::kABytes, &tma_a, &full_bar[stage], kb * F8_BK, m_idx * F8_BM);
-          tma_load_2d(sB + stage * S::kBBytes, &tma_b, &full_bar[stage], kb * F8_BK, n_idx * BN);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+    int stage = 0, pre = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    {                                    // weights are static: the first stages' are requested before waiting for the quantiser
+      const int split = blockIdx.x % p.k_splits, t = blockIdx.x / p.k_splits;
+      const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
+      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+      pre = min(kb1 - kb0, STAGES);
+      if (elect_one()) {
+        for (int i = 0; i < pre; ++i) {
+          mbar_expect_tx(&full_bar[i], S::kStageBytes);
+          if (SWAP) tma_load_2d(sA + i * S::kABytes, &tma_a, &full_bar[i], (kb0 + i) * F8_BK, m_idx * F8_BM);
+          else tma_load_2d(sB + i * S::kBBytes, &tma_b, &full_bar[i], (kb0 + i) * F8_BK, n_idx * BN);
         }
+      }
+      __syncwarp();
+    }
+    pdl_wait();
+    for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
+      const int split = w % p.k_splits, t = w / p.k_splits;
+      const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
+      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const bool requested = pre > 0;
+        if (requested) --pre;
+        else if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+        if (elect_one()) {
+          if (!requested) mbar_expect_tx(&full_bar[stage], S::kStageBytes);
+          if (!requested || !SWAP) tma_load_2d(sA + stage * S::kABytes, &tma_a, &full_bar[stage], kb * F8_BK, m_idx * F8_BM);
+          if (!requested || SWAP) tma_load_2d(sB + stage * S::kBBytes, &tma_b, &full_bar[stage], kb * F8_BK, n_idx * BN);
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(F8_BM, BN, 0, 0);      // e4m3 x e4m3
-      int stage = 0, buf = 0;
-      uint32_t phase = 0, buf_phase = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
-        const int split = w % p.k_splits;
-        const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-        for (int kb = kb0; kb < kb1; ++kb) {
-          // each K block gets its own accumulator: wait until the epilogue drained this buffer
-          if (!mbar_wait(&tempty_bar[buf], buf_phase ^ 1, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint64_t da = make_smem_desc_sw128(smem_u32(sA + stage * S::kABytes));
-          const uint64_t db = make_smem_desc_sw128(smem_u32(sB + stage * S::kBBytes));
+    constexpr uint32_t idesc = make_idesc(F8_BM, BN, 0, 0);      // e4m3 x e4m3
+    const uint64_t da0 = make_smem_desc_sw128(smem_u32(sA)), db0 = make_smem_desc_sw128(smem_u32(sB));
+    int stage = 0, buf = 0;
+    uint32_t phase = 0, buf_phase = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
+      const int split = w % p.k_splits;
+      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        // each K block gets its own accumulator: wait until the promoting warps drained this buffer
+        if (!mbar_wait_warp(&tempty_bar[buf], buf_phase ^ 1, abort_flag) || !mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+        tc_fence_after_sync();
+        if (elect_one()) {
+          const uint64_t da = da0 + (uint64_t)(stage * (S::kABytes >> 4)), db = db0 + (uint64_t)(stage * (S::kBBytes >> 4));
 #pragma unroll
           for (int k = 0; k < F8_BK / F8_UMMA_K; ++k)
             tc_mma_f8f6f4(tmem_base + buf * BN, da + 2 * k, db + 2 * k, idesc, k > 0 ? 1u : 0u);
           tc_commit(&empty_bar[stage]);
           tc_commit(&tfull_bar[buf]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-          buf ^= 1;
-          if (buf == 0) buf_phase ^= 1;
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        if (++buf == NBUF) { buf = 0; buf_phase ^= 1; }
       }
     }
-  } else {
-    const int q = warp & 3;
-    const int etid = (warp - 2) * 32 + lane;                        // 0..127 among epilogue threads
+  } else if (threadIdx.x - 64 < S::kPromote) {
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int etid = threadIdx.x - 64;
+    pdl_wait();                            // scales of the activations; outputs may still be in use by the predecessor
     int buf = 0;
     uint32_t buf_phase = 0;
     bool ok = true;
@@ -145,75 +177,67 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
       const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
       const int m = m_idx * F8_BM + q * 32 + lane;
-      const int n_base = n_idx * BN;
-      if (p.transposed) {
-        // token scales of the tile: s_scale[kb][c] = sx[n_base + c][kb]
-        asm volatile("bar.sync 1, 128;" ::: "memory");              // previous tile finished reading
-        for (int i = etid; i < (kb1 - kb0) * BN; i += 128) {
+      const int n_base = n_idx * BN + half * COLS;
+      if (SWAP) {
+        // token scales of the tile: s_scale[kb][c] = sx[n + c][kb]
+        asm volatile("bar.sync 1, %0;" ::"n"(S::kPromote) : "memory");              // previous tile finished reading
+        for (int i = etid; i < (kb1 - kb0) * BN; i += S::kPromote) {
           const int kb = kb0 + i / BN, c = i % BN;
-          const int tok = n_base + c;
+          const int tok = n_idx * BN + c;
           s_scale[i] = tok < p.N ? p.sx[(size_t)tok * p.k_blocks + kb] : 0.f;
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(S::kPromote) : "memory");
       }
-      float acc[BN];
+      // scale of the weights: features lie along the rows (one block of 128 per tile), or along the columns (one per thread: COLS divides 128)
+      const float* wrow = p.sw + (size_t)(SWAP ? m_idx : min(n_base, p.N - 1) >> 7) * p.k_blocks;
+      const float* xrow = p.sx + (size_t)(SWAP ? 0 : min(m, p.M - 1)) * p.k_blocks;
+      auto factor = [&](int kb) { return kb < kb1 ? (SWAP ? wrow[kb] : xrow[kb] * wrow[kb]) : 0.f; };
+      float acc[COLS];
 #pragma unroll
-      for (int c = 0; c < BN; ++c) acc[c] = 0.f;
-      for (int kb = kb0; kb < kb1 && ok; ++kb) {
+      for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
+      float f0 = factor(kb0), f1 = factor(kb0 + 1);
+      for (int kb = kb0; kb < kb1; ++kb) {
+        const float f = f0;
+        f0 = f1; f1 = factor(kb + 2);
         if (!mbar_wait(&tfull_bar[buf], buf_phase, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t t_row = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
-        float row_scale;                                            // constant along the thread's row
-        if (p.transposed) row_scale = p.sw[(size_t)m_idx * p.k_blocks + kb];          // 128 features = 1 block
-        else row_scale = m < p.M ? p.sx[(size_t)m * p.k_blocks + kb] : 0.f;
-        constexpr int CH = BN < 32 ? 16 : 32;
+        const uint32_t t_row = tmem_base + buf * BN + half * COLS + ((uint32_t)(q * 32) << 16);
+        constexpr int CH = COLS < 32 ? 16 : 32;
 #pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += CH) {
-          uint32_t r[32];
-          if constexpr (CH == 32) {
-            tmem_ld_32x32(t_row + c0, r);
-          } else {
-            uint32_t r16[16];
-            tmem_ld_32x16(t_row + c0, r16);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) r[i] = r16[i];
-          }
+        for (int c0 = 0; c0 < COLS; c0 += CH) {
+          uint32_t r[CH];
+          if constexpr (CH == 32) tmem_ld_32x32(t_row + c0, r);
+          else tmem_ld_32x16(t_row + c0, r);
           tmem_ld_wait();
-          if (p.transposed) {
 #pragma unroll
-            for (int c = 0; c < CH; ++c) acc[c0 + c] += __uint_as_float(r[c]) * (row_scale * s_scale[(kb - kb0) * BN + c0 + c]);
-          } else {
-#pragma unroll
-            for (int c = 0; c < CH; ++c) {
-              // columns are features: one weight scale per 128 columns
-              const float cs = p.sw[(size_t)((n_base + c0 + c) >> 7) * p.k_blocks + kb];
-              acc[c0 + c] += __uint_as_float(r[c]) * (row_scale * cs);
-            }
+          for (int c = 0; c < CH; ++c) {
+            if (SWAP) acc[c0 + c] += __uint_as_float(r[c]) * (f * s_scale[(kb - kb0) * BN + half * COLS + c0 + c]);
+            else acc[c0 + c] += __uint_as_float(r[c]) * f;
           }
         }
         tc_fence_before_sync();
-        mbar_arrive(&tempty_bar[buf]);
-        buf ^= 1;
-        if (buf == 0) buf_phase ^= 1;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+        if (++buf == NBUF) { buf = 0; buf_phase ^= 1; }
       }
       if (!ok) break;
       // store
       if (p.k_splits > 1) {                                   // fp32 partial sums [split][token][feature]; bias in the reduction
-        float* wsp = p.ws + (size_t)split * (p.transposed ? (size_t)p.N * p.M : (size_t)p.M * p.N);
-        if (p.transposed) {                                   // lanes run along features: coalesced
+        float* wsp = p.ws + (size_t)split * (size_t)p.N * p.M;
+        if (SWAP) {                                           // lanes run along features: coalesced
 #pragma unroll
-          for (int c = 0; c < BN; ++c)
+          for (int c = 0; c < COLS; ++c)
             if (n_base + c < p.N && m < p.M) wsp[(size_t)(n_base + c) * p.M + m] = acc[c];
         } else if (m < p.M) {
 #pragma unroll
-          for (int c = 0; c < BN; c += 4)
+          for (int c = 0; c < COLS; c += 4)
             if (n_base + c < p.N) *reinterpret_cast<float4*>(wsp + (size_t)m * p.N + n_base + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
         }
-      } else if (!p.transposed) {
+      } else if (!SWAP) {
         if (m < p.M) {
           __nv_bfloat16* dst = p.out + (size_t)m * p.ldc + n_base;
 #pragma unroll
-          for (int c = 0; c < BN; c += 8) {
+          for (int c = 0; c < COLS; c += 8) {
             if (n_base + c < p.N) {
               float v[8];
 #pragma unroll
@@ -229,7 +253,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         const float bias_m = (p.bias && m < p.M) ? __bfloat162float(p.bias[m]) : 0.f;
         const bool odd = lane & 1;
 #pragma unroll
-        for (int c = 0; c < BN; c += 2) {
+        for (int c = 0; c < COLS; c += 2) {
           const float own0 = acc[c] + bias_m, own1 = acc[c + 1] + bias_m;
           const float recv = __shfl_xor_sync(0xffffffffu, odd ? own0 : own1, 1);
           const int n = n_base + c + (odd ? 1 : 0);
@@ -249,6 +273,8 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 // out[t][n] = bf16(sum_s ws[s][t][n] + bias[n])
 __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ ws, int splits, int rows, int cols, long long ldc,
                                          const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
@@ -267,29 +293,43 @@ __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ ws, int split
   *reinterpret_cast<uint2*>(out + (size_t)r * ldc + c) = o;
 }
 
-// x bf16 [T][K] -> e4m3 [T][K] and scales [T][K/128] (amax / 448 per 128 values). One warp per group.
-__global__ void quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ xq,
-                                       float* __restrict__ sx, int tokens, int K) {
+// x bf16 [T][K] -> e4m3 [T][K] and scales [T][K/128] (amax / 448 per 128 values). Half a warp per group, 16 bytes per lane (one warp per
+// group with 8 bytes per lane moved 2.3 TB/s at 1965 x 8192).
+__global__ void __launch_bounds__(256) quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ xq,
+                                                              float* __restrict__ sx, int tokens, int K) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int kb_n = K / 128;
-  const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (gw >= (long long)tokens * kb_n) return;
-  const int t = (int)(gw / kb_n), kb = (int)(gw - (long long)t * kb_n), lane = threadIdx.x & 31;
-  const uint2 raw = *reinterpret_cast<const uint2*>(x + (size_t)t * ldx + kb * 128 + lane * 4);
-  const float2 a = unpack_bf16x2(raw.x), b = unpack_bf16x2(raw.y);
-  float amax = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y)));
-  amax = warp_max(amax);
+  const long long g = ((long long)blockIdx.x * 256 + threadIdx.x) >> 4;
+  const int l = threadIdx.x & 15;
+  const bool in = g < (long long)tokens * kb_n;
+  const int t = in ? (int)(g / kb_n) : 0, kb = in ? (int)(g - (long long)t * kb_n) : 0;
+  uint4 raw = make_uint4(0, 0, 0, 0);
+  if (in) {
+    const __nv_bfloat16* src = x + (size_t)t * ldx + kb * 128 + l * 8;
+    if ((ldx & 7) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+      raw = *reinterpret_cast<const uint4*>(src);
+    } else {
+      const uint2 a = reinterpret_cast<const uint2*>(src)[0], b = reinterpret_cast<const uint2*>(src)[1];
+      raw = make_uint4(a.x, a.y, b.x, b.y);
+    }
+  }
+  const float2 a = unpack_bf16x2(raw.x), b = unpack_bf16x2(raw.y), c = unpack_bf16x2(raw.z), d = unpack_bf16x2(raw.w);
+  float amax = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))), fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (!in) return;
   const float scale = fmaxf(amax, 1e-10f) / 448.f, inv = 1.f / scale;
-  __nv_fp8x4_e4m3 q(make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv));
-  *reinterpret_cast<uint32_t*>(xq + (size_t)t * K + kb * 128 + lane * 4) = *reinterpret_cast<uint32_t*>(&q);
-  if (lane == 0) sx[(size_t)t * kb_n + kb] = scale;
+  __nv_fp8x4_e4m3 q0(make_float4(a.x * inv, a.y * inv, b.x * inv, b.y * inv)), q1(make_float4(c.x * inv, c.y * inv, d.x * inv, d.y * inv));
+  *reinterpret_cast<uint2*>(xq + (size_t)t * K + kb * 128 + l * 8) = make_uint2(*reinterpret_cast<uint32_t*>(&q0), *reinterpret_cast<uint32_t*>(&q1));
+  if (l == 0) sx[(size_t)t * kb_n + kb] = scale;
 }
 
 void quant_fp8_1x128(const void* x, long long ldx, void* xq, float* sx, int tokens, int K, cudaStream_t s) {
   if (tokens <= 0) return;
   if (K % 128) throw std::runtime_error("quant_fp8_1x128: K must be a multiple of 128");
   const long long groups = (long long)tokens * (K / 128);
-  quant_fp8_1x128_kernel<<<(int)((groups + 7) / 8), 256, 0, s>>>((const __nv_bfloat16*)x, ldx, (uint8_t*)xq, sx, tokens, K);
-  cuda_check(cudaGetLastError(), "quant_fp8_1x128_kernel");
+  launch_pdl(quant_fp8_1x128_kernel, dim3((unsigned)((groups + 15) / 16)), dim3(256), 0, s, (const __nv_bfloat16*)x, ldx, (uint8_t*)xq, sx, tokens, K);
 }
 
 template <int BN>
@@ -300,8 +340,7 @@ static void launch_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const Fp8Ge
     cuda_check(cudaFuncSetAttribute(gemm_fp8_block_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
                "cudaFuncSetAttribute(gemm_fp8_block_kernel)");
   }
-  gemm_fp8_block_kernel<BN><<<grid, kF8Threads, S::kTotal, s>>>(ta, tb, a);
-  cuda_check(cudaGetLastError(), "gemm_fp8_block_kernel launch");
+  launch_pdl(gemm_fp8_block_kernel<BN>, dim3(grid), dim3(kF8Threads), S::kTotal, s, ta, tb, a);
 }
 
 // y[T][N] = dequant(xq, sx) * dequant(wq, sw)^T (+ bias)
@@ -316,45 +355,47 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   a.out = reinterpret_cast<__nv_bfloat16*>(y); a.ldc = ldy;
   a.sx = sx; a.sw = sw; a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.status = status;
   const bool swap = T <= 64;                          // decode: features fill the 128-row MMA dimension
-  int bn;
-  CUtensorMap ta, tb;
-  if (swap) {
-    bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64);
-    a.M = N; a.N = T; a.transposed = 1;
-    ta = make_tmap_2d(wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, F8_BM, F8_BK, true);
-    tb = make_tmap_2d(xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, T, K, K, bn, F8_BK, true);
-  } else {
-    bn = 128;
-    a.M = T; a.N = N; a.transposed = 0;
-    ta = make_tmap_2d(xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, T, K, K, F8_BM, F8_BK, true);
-    tb = make_tmap_2d(wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, bn, F8_BK, true);
-  }
+  const int sms = sm_count();
+  a.M = swap ? N : T; a.N = swap ? T : N; a.transposed = swap;
   a.m_tiles = (a.M + F8_BM - 1) / F8_BM;
+  // Tile width and K splits by the rounds of items over the SMs, in units of 1/100 us. A K block takes what its products take, or the
+  // time in which an SM's share of the HBM bandwidth brings its weights (37 per 128 features) when no other tile of the step reads
+  // them, too. 128-wide blocks take 18 and not 14, half of a 256-wide one: they move twice the shared memory per product. Partial sums
+  // are written and read once, and cost a launch.
+  int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1;
+  const int least = (a.k_blocks + 63) / 64;           // the token scales of a split fit their shared-memory block
+  const bool can_split = workspace && (N & 3) == 0;
+  long long best = -1;
+  for (int w : {swap ? bn : 256, swap ? 0 : 128}) {
+    if (w == 0 || (w == 256 && N % 256)) continue;
+    const int n_tiles = (a.N + w - 1) / w;
+    const long long block = std::max(swap ? 14 : (w == 256 ? 28 : 18), a.m_tiles == 1 || swap ? (w == 256 ? 74 : 37) : 0);
+    for (int s = least; s <= 16 * least && s <= a.k_blocks; ++s) {
+      if (s > 1 && (!can_split || (size_t)s * T * N * 4 > workspace_bytes)) break;
+      const long long rounds = ((long long)a.m_tiles * n_tiles * s + sms - 1) / sms;
+      const long long cost = rounds * ((a.k_blocks + s - 1) / s * block + 100) + (s > 1 ? 250 + (long long)((double)s * T * N * 8 / 60000.0) : 0);
+      if (best < 0 || cost < best) { best = cost; bn = w; splits = s; }
+    }
+  }
+  if (best < 0) throw std::runtime_error("linear_fp8_block: K above 8192 needs a split-K workspace");
   a.n_tiles = (a.N + bn - 1) / bn;
-  // Few tiles cannot pull the whole HBM bandwidth: split K until the machine is full. A split's token scales must
-  // also fit their shared-memory block (64 K blocks).
-  const int slots = sm_count() * (bn <= 64 ? 2 : 1);
-  const int tiles = a.m_tiles * a.n_tiles;
-  int splits = 1;
-  if (tiles * 2 <= slots && a.k_blocks >= 8) splits = std::min(std::min(slots / tiles, a.k_blocks / 4), 16);
-  splits = std::max(splits, (a.k_blocks + 63) / 64);
-  while (splits > (a.k_blocks + 63) / 64 && (!workspace || (size_t)splits * T * N * 4 > workspace_bytes || (N & 3))) --splits;
-  if (splits > 1 && (!workspace || (size_t)splits * T * N * 4 > workspace_bytes || (N & 3)))
-    throw std::runtime_error("linear_fp8_block: K above 8192 needs a split-K workspace");
+  const CUtensorMap tw = make_tmap_2d(wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, swap ? F8_BM : bn, F8_BK, true);
+  const CUtensorMap tx = make_tmap_2d(xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, T, K, K, swap ? bn : F8_BM, F8_BK, true);
+  const CUtensorMap &ta = swap ? tw : tx, &tb = swap ? tx : tw;
   a.kb_per_split = (a.k_blocks + splits - 1) / splits;
   a.k_splits = (a.k_blocks + a.kb_per_split - 1) / a.kb_per_split;
   a.ws = reinterpret_cast<float*>(workspace);
-  const int grid = std::min(tiles * a.k_splits, slots);
+  const int grid = std::min(a.m_tiles * a.n_tiles * a.k_splits, sms);
   switch (bn) {
     case 16: launch_fp8<16>(ta, tb, a, grid, stream); break;
     case 32: launch_fp8<32>(ta, tb, a, grid, stream); break;
     case 64: launch_fp8<64>(ta, tb, a, grid, stream); break;
-    default: launch_fp8<128>(ta, tb, a, grid, stream); break;
+    case 128: launch_fp8<128>(ta, tb, a, grid, stream); break;
+    default: launch_fp8<256>(ta, tb, a, grid, stream); break;
   }
   if (a.k_splits > 1) {
     const size_t n = (size_t)T * N;
-    fp8_splitk_reduce_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, stream>>>(a.ws, a.k_splits, T, N, ldy, a.bias, a.out);
-    cuda_check(cudaGetLastError(), "fp8_splitk_reduce_kernel");
+    launch_pdl(fp8_splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float*)a.ws, a.k_splits, T, N, ldy, a.bias, a.out);
     return 2;
   }
   return 1;
