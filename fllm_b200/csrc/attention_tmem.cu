@@ -54,7 +54,6 @@ struct FaTmemParams {
   int window;
   int min_q;             // sequences with fewer query rows are not this kernel's
   float scale_log2, softcap, scale;
-  int pv_wide;           // one N=128 MMA per 16 tokens instead of two N=64 ones
   int tile_variant;      // 0: pick by shape; 1 / 2: force one / two query tiles per CTA
   int bidir;             // 1: no causal mask, every query row sees all kv_len tokens (encoders)
 };
@@ -244,7 +243,7 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int qt = gridDim.x - 1 - blockIdx.x;      // the tiles with the longest KV range start first
   const int kvh = blockIdx.y, seq = blockIdx.z;
   const int G = p.group;
@@ -291,71 +290,69 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
   const uint32_t t_o = tmem_base + 128;
 
   if (warp == 0) {
-    if (lane == 0) {
-      const int* table = p.block_tables + (size_t)seq * p.max_blocks;
-      const int last_page = (kv_len + kPageT - 1) / kPageT - 1;
-      // first cache row of the tile's pages; pages past the sequence repeat its last page (finite values).
-      // The next tile's table entries are requested before this tile's waits, so their latency is hidden.
-      int rows[kTileT / kPageT], nxt[kTileT / kPageT];
+    const int* table = p.block_tables + (size_t)seq * p.max_blocks;
+    const int last_page = (kv_len + kPageT - 1) / kPageT - 1;
+    // first cache row of the tile's pages; pages past the sequence repeat its last page (finite values).
+    // The next tile's table entries are requested before this tile's waits, so their latency is hidden.
+    int rows[kTileT / kPageT], nxt[kTileT / kPageT];
 #pragma unroll
-      for (int pg = 0; pg < kTileT / kPageT; ++pg)
-        nxt[pg] = table[min(tile_lo * (kTileT / kPageT) + pg, last_page)];
-      for (int it = 0; it < n_tiles; ++it) {
-        const int page1 = (tile_lo + it + 1) * (kTileT / kPageT);
+    for (int pg = 0; pg < kTileT / kPageT; ++pg)
+      nxt[pg] = table[min(tile_lo * (kTileT / kPageT) + pg, last_page)];
+    for (int it = 0; it < n_tiles; ++it) {
+      const int page1 = (tile_lo + it + 1) * (kTileT / kPageT);
 #pragma unroll
-        for (int pg = 0; pg < kTileT / kPageT; ++pg) {
-          rows[pg] = (nxt[pg] * p.hkv + kvh) * kPageT;
-          nxt[pg] = table[min(page1 + pg, last_page)];
-        }
-        if (it > 0 && !mbar_wait(k_empty, (it - 1) & 1, abort_flag)) break;
+      for (int pg = 0; pg < kTileT / kPageT; ++pg) {
+        rows[pg] = (nxt[pg] * p.hkv + kvh) * kPageT;
+        nxt[pg] = table[min(page1 + pg, last_page)];
+      }
+      if (it > 0 && !mbar_wait_warp(k_empty, (it - 1) & 1, abort_flag)) break;
+      if (elect_one()) {
         mbar_expect_tx(k_full, TB);
 #pragma unroll
         for (int pg = 0; pg < kTileT / kPageT; ++pg) {
 #pragma unroll
           for (int h = 0; h < D / 64; ++h) tma_load_2d(sk + h * kHalfBytes + pg * 2048, &tma_k, k_full, 64 * h, rows[pg]);
         }
-        if (it > 0 && !mbar_wait(v_empty, (it - 1) & 1, abort_flag)) break;
+      }
+      __syncwarp();
+      if (it > 0 && !mbar_wait_warp(v_empty, (it - 1) & 1, abort_flag)) break;
+      if (elect_one()) {
         mbar_expect_tx(v_full, TB);
 #pragma unroll
-        for (int pg = 0; pg < kTileT / kPageT; ++pg) {
-#pragma unroll
-          for (int h = 0; h < D / 64; ++h) tma_load_2d(sv + h * kHalfBytes + pg * 2048, &tma_v, v_full, 64 * h, rows[pg]);
-        }
+        for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_3d(sv + pg * (D / 64) * 2048, &tma_v, v_full, 0, rows[pg], 0);
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc(128, 128, 1, 1);
-      constexpr uint32_t idesc_pv = make_idesc(128, 64, 1, 1) | (1u << 16);     // B is MN-major
-      constexpr uint32_t idesc_pv_wide = make_idesc(128, 128, 1, 1) | (1u << 16);
-      const uint32_t q_addr = smem_u32(sq), k_addr = smem_u32(sk), v_addr = smem_u32(sv);
-      for (int it = 0; it < n_tiles; ++it) {
-        const uint32_t ph = it & 1;
-        if (!mbar_wait(k_full, ph, abort_flag)) break;
-        tc_fence_after_sync();
+    constexpr uint32_t idesc_s = make_idesc(128, 128, 1, 1);
+    constexpr uint32_t idesc_pv = make_idesc(128, D, 1, 1) | (1u << 16);     // B is MN-major
+    const uint64_t dq = make_smem_desc_sw128(smem_u32(sq)), dk = make_smem_desc_sw128(smem_u32(sk));
+    const uint64_t dv = smem_desc_sw128_1k(smem_u32(sv), D == 128 ? 2048 : 1024);     // V lands by pages: [page][D / 64][16][64]
+    for (int it = 0; it < n_tiles; ++it) {
+      const uint32_t ph = it & 1;
+      if (!mbar_wait_warp(k_full, ph, abort_flag)) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * kHalfBytes + (k & 3) * 32;
-          tc_mma_bf16(t_s, make_smem_desc_sw128(q_addr + off), make_smem_desc_sw128(k_addr + off), idesc_s, k > 0);
+          const uint32_t off = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
+          tc_mma_bf16(t_s, dq + off, dk + off, idesc_s, k > 0);
         }
         tc_commit(s_full);
         tc_commit(k_empty);
-        if (!mbar_wait(p_ready, ph, abort_flag) || !mbar_wait(v_full, ph, abort_flag)) break;
-        tc_fence_after_sync();
+      }
+      __syncwarp();
+      if (!mbar_wait_warp(p_ready, ph, abort_flag) || !mbar_wait_warp(v_full, ph, abort_flag)) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        // at D = 128 the second 64-wide atom of V's rows lies half a page further: the leading offset
 #pragma unroll
-        for (int k = 0; k < kTileT / 16; ++k) {
-          const uint32_t acc = (it > 0 || k > 0) ? 1u : 0u;
-          if (D == 128 && p.pv_wide) {      // the second 64-wide atom of V's rows lies one half tile further: the leading offset
-            tc_mma_bf16_ts(t_o, t_s + 8 * k, smem_desc_sw128_1k(v_addr + k * 2048, kHalfBytes), idesc_pv_wide, acc);
-          } else {
-            tc_mma_bf16_ts(t_o, t_s + 8 * k, smem_desc_sw128_1k(v_addr + k * 2048), idesc_pv, acc);
-            if (D == 128)
-              tc_mma_bf16_ts(t_o + 64, t_s + 8 * k, smem_desc_sw128_1k(v_addr + kHalfBytes + k * 2048), idesc_pv, acc);
-          }
-        }
+        for (int k = 0; k < kTileT / 16; ++k)
+          tc_mma_bf16_ts(t_o, t_s + 8 * k, dv + (uint64_t)(k * (D / 64) * (2048 >> 4)), idesc_pv, (it > 0 || k > 0) ? 1u : 0u);
         tc_commit(v_empty);
         if (it == n_tiles - 1) tc_commit(o_done);
       }
+      __syncwarp();
     }
   } else {
     const int quarter = warp & 3;                       // the lane quarter this warp may touch
@@ -392,11 +389,11 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
 }
 
 // The same pipeline with two 128-row query tiles per CTA sharing every K/V tile (half the K/V traffic per
-// FLOP, which is what bounds the one-tile kernel: its 64 KB per 8.4 MFLOP tile saturates L2 first). Ten warps:
-// producer, issuer, and one softmax group of four warps per query tile. The issuer interleaves the two tiles
+// FLOP, which is what bounds the one-tile kernel: its 64 KB per 8.4 MFLOP tile saturates L2 first). Twelve warps:
+// three producers, issuer, and one softmax group of four warps per query tile. The issuer interleaves the two tiles
 // (PV0, next S0, PV1, next S1) so that one group's softmax runs under the other tile's MMAs; K and V are
 // double buffered. Tensor memory: S0 S1 O0 O1 = 512 columns, one CTA per SM.
-constexpr int kThreadsT2 = 320;
+constexpr int kThreadsT2 = 384;
 template <int D> constexpr int smem_two() { return 6 * tile_bytes<D>() + 256 + 1024; }
 
 template <int D>
@@ -420,7 +417,7 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int qt = gridDim.x - 1 - blockIdx.x;
   const int kvh = blockIdx.y, seq = blockIdx.z;
   const int G = p.group;
@@ -442,7 +439,7 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
+      mbar_init(&k_full[i], D / 64); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4);
     }
     mbar_init(o_done, 1);
@@ -467,94 +464,90 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      const int* table = p.block_tables + (size_t)seq * p.max_blocks;
-      const int last_page = (kv_len + kPageT - 1) / kPageT - 1;
-      int rows[kTileT / kPageT], nxt[kTileT / kPageT];
+  if (warp == 0 || warp >= 10) {
+    // Three warps ask for the pages, one box of theirs after the other: warp 0 for the first 64 columns of K, warp 10 for the
+    // others, warp 11 for V. (One warp for all 32 boxes of a tile needed longer than the products of the tile.)
+    const bool is_v = warp == 11;
+    const int half = warp == 10 ? 1 : 0;
+    uint64_t *full = is_v ? v_full : k_full, *empty = is_v ? v_empty : k_empty;
+    const int* table = p.block_tables + (size_t)seq * p.max_blocks;
+    const int last_page = (kv_len + kPageT - 1) / kPageT - 1;
+    int rows[kTileT / kPageT], nxt[kTileT / kPageT];
 #pragma unroll
-      for (int pg = 0; pg < kTileT / kPageT; ++pg)
-        nxt[pg] = table[min(tile_lo * (kTileT / kPageT) + pg, last_page)];
-      for (int it = 0; it < n_tiles; ++it) {
-        const int b = it & 1;
-        const uint32_t prev = ((it >> 1) - 1) & 1;       // phase of the stage's previous use
-        const int page1 = (tile_lo + it + 1) * (kTileT / kPageT);
+    for (int pg = 0; pg < kTileT / kPageT; ++pg)
+      nxt[pg] = table[min(tile_lo * (kTileT / kPageT) + pg, last_page)];
+    for (int it = 0; it < n_tiles && (half == 0 || D == 128); ++it) {
+      const int b = it & 1;
+      const int page1 = (tile_lo + it + 1) * (kTileT / kPageT);
 #pragma unroll
-        for (int pg = 0; pg < kTileT / kPageT; ++pg) {
-          rows[pg] = (nxt[pg] * p.hkv + kvh) * kPageT;
-          nxt[pg] = table[min(page1 + pg, last_page)];
-        }
-        if (it >= 2 && !mbar_wait(&k_empty[b], prev, abort_flag)) break;
-        mbar_expect_tx(&k_full[b], TB);
-        uint8_t* kd = sk + b * TB;
+      for (int pg = 0; pg < kTileT / kPageT; ++pg) {
+        rows[pg] = (nxt[pg] * p.hkv + kvh) * kPageT;
+        nxt[pg] = table[min(page1 + pg, last_page)];
+      }
+      if (it >= 2 && !mbar_wait_warp(&empty[b], ((it >> 1) - 1) & 1, abort_flag)) break;      // phase of the stage's previous use
+      if (elect_one()) {
+        if (is_v) {
+          mbar_expect_tx(&full[b], TB);
 #pragma unroll
-        for (int pg = 0; pg < kTileT / kPageT; ++pg) {
+          for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_3d(sv + b * TB + pg * (D / 64) * 2048, &tma_v, &full[b], 0, rows[pg], 0);
+        } else {
+          mbar_expect_tx(&full[b], kHalfBytes);
 #pragma unroll
-          for (int h = 0; h < D / 64; ++h) tma_load_2d(kd + h * kHalfBytes + pg * 2048, &tma_k, &k_full[b], 64 * h, rows[pg]);
-        }
-        if (it >= 2 && !mbar_wait(&v_empty[b], prev, abort_flag)) break;
-        mbar_expect_tx(&v_full[b], TB);
-        uint8_t* vd = sv + b * TB;
-#pragma unroll
-        for (int pg = 0; pg < kTileT / kPageT; ++pg) {
-#pragma unroll
-          for (int h = 0; h < D / 64; ++h) tma_load_2d(vd + h * kHalfBytes + pg * 2048, &tma_v, &v_full[b], 64 * h, rows[pg]);
+          for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_2d(sk + b * TB + half * kHalfBytes + pg * 2048, &tma_k, &full[b], 64 * half, rows[pg]);
         }
       }
+      __syncwarp();
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc(128, 128, 1, 1);
-      constexpr uint32_t idesc_pv = make_idesc(128, 64, 1, 1) | (1u << 16);     // B is MN-major
-      constexpr uint32_t idesc_pv_wide = make_idesc(128, 128, 1, 1) | (1u << 16);
-      const uint32_t q_addr = smem_u32(sq), k_addr = smem_u32(sk), v_addr = smem_u32(sv);
-      auto issue_s = [&](int g, int stage) {
+    constexpr uint32_t idesc_s = make_idesc(128, 128, 1, 1);
+    constexpr uint32_t idesc_pv = make_idesc(128, D, 1, 1) | (1u << 16);     // B is MN-major
+    const uint64_t dq = make_smem_desc_sw128(smem_u32(sq)), dk = make_smem_desc_sw128(smem_u32(sk));
+    const uint64_t dv = smem_desc_sw128_1k(smem_u32(sv), D == 128 ? 2048 : 1024);     // V lands by pages: [page][D / 64][16][64]
+    auto issue_s = [&](int g, int stage) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * kHalfBytes + (k & 3) * 32;
-          tc_mma_bf16(tmem_base + 128 * g, make_smem_desc_sw128(q_addr + g * TB + off),
-                      make_smem_desc_sw128(k_addr + stage * TB + off), idesc_s, k > 0);
-        }
-      };
-      auto issue_pv = [&](int g, int stage, bool first) {
-        const uint32_t t_p = tmem_base + 128 * g, t_o = tmem_base + 256 + 128 * g;
-        const uint32_t vb = v_addr + stage * TB;
+      for (int k = 0; k < D / 16; ++k) {
+        const uint32_t off = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
+        tc_mma_bf16(tmem_base + 128 * g, dq + g * (TB >> 4) + off, dk + (uint64_t)(stage * (TB >> 4)) + off, idesc_s, k > 0);
+      }
+    };
+    auto issue_pv = [&](int g, int stage, bool first) {
+      const uint32_t t_p = tmem_base + 128 * g, t_o = tmem_base + 256 + 128 * g;
 #pragma unroll
-        for (int k = 0; k < kTileT / 16; ++k) {
-          const uint32_t acc = (!first || k > 0) ? 1u : 0u;
-          if (D == 128 && p.pv_wide) {
-            tc_mma_bf16_ts(t_o, t_p + 8 * k, smem_desc_sw128_1k(vb + k * 2048, kHalfBytes), idesc_pv_wide, acc);
-          } else {
-            tc_mma_bf16_ts(t_o, t_p + 8 * k, smem_desc_sw128_1k(vb + k * 2048), idesc_pv, acc);
-            if (D == 128)
-              tc_mma_bf16_ts(t_o + 64, t_p + 8 * k, smem_desc_sw128_1k(vb + kHalfBytes + k * 2048), idesc_pv, acc);
-          }
-        }
-      };
-      bool ok = mbar_wait(&k_full[0], 0, abort_flag);
-      if (ok) {
-        tc_fence_after_sync();
+      for (int k = 0; k < kTileT / 16; ++k)
+        tc_mma_bf16_ts(t_o, t_p + 8 * k, dv + (uint64_t)(stage * (TB >> 4)) + k * (D / 64) * (2048 >> 4), idesc_pv, (!first || k > 0) ? 1u : 0u);
+    };
+    bool ok = mbar_wait_warp(&k_full[0], 0, abort_flag);
+    if (ok) {
+      tc_fence_after_sync();
+      if (elect_one()) {
         issue_s(0, 0);
         tc_commit(&s_full[0]);
         issue_s(1, 0);
         tc_commit(&s_full[1]);
         tc_commit(&k_empty[0]);
       }
-      for (int it = 0; ok && it < n_tiles; ++it) {
-        const int b = it & 1, nb = b ^ 1;
-        const uint32_t ph = (it >> 1) & 1, nph = ((it + 1) >> 1) & 1;
-        const bool more = it + 1 < n_tiles;
-        if (!mbar_wait(&p_ready[0], it & 1, abort_flag) || !mbar_wait(&v_full[b], ph, abort_flag)) break;
+      __syncwarp();
+    }
+    for (int it = 0; ok && it < n_tiles; ++it) {
+      const int b = it & 1, nb = b ^ 1;
+      const uint32_t ph = (it >> 1) & 1, nph = ((it + 1) >> 1) & 1;
+      const bool more = it + 1 < n_tiles;
+      if (!mbar_wait_warp(&p_ready[0], it & 1, abort_flag) || !mbar_wait_warp(&v_full[b], ph, abort_flag)) break;
+      tc_fence_after_sync();
+      if (elect_one()) issue_pv(0, b, it == 0);
+      __syncwarp();
+      if (more) {
+        if (!mbar_wait_warp(&k_full[nb], nph, abort_flag)) break;
         tc_fence_after_sync();
-        issue_pv(0, b, it == 0);
-        if (more) {
-          if (!mbar_wait(&k_full[nb], nph, abort_flag)) break;
-          tc_fence_after_sync();
+        if (elect_one()) {
           issue_s(0, nb);
           tc_commit(&s_full[0]);
         }
-        if (!mbar_wait(&p_ready[1], it & 1, abort_flag)) break;
-        tc_fence_after_sync();
+        __syncwarp();
+      }
+      if (!mbar_wait_warp(&p_ready[1], it & 1, abort_flag)) break;
+      tc_fence_after_sync();
+      if (elect_one()) {
         issue_pv(1, b, it == 0);
         tc_commit(&v_empty[b]);
         if (more) {
@@ -565,8 +558,9 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
           tc_commit(o_done);
         }
       }
+      __syncwarp();
     }
-  } else {
+  } else {                                              // warps 2 - 9
     const int g = (warp - 2) >> 2;                      // query tile of this softmax group
     const int quarter = warp & 3;
     const int r = g * kRowsT + quarter * 32 + lane;     // packed row within the CTA
@@ -662,7 +656,7 @@ void attention_prefill_tmem(const void* q, long long ldq, const void* k_cache, c
     if (maps.size() > 4096) maps.clear();
     MapPair mp;
     mp.k = make_tmap_2d(k_cache, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, head_dim, head_dim * 2, kPageT, 64, true);
-    mp.v = make_tmap_2d(v_cache, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, rows, head_dim, head_dim * 2, kPageT, 64, true);
+    mp.v = make_tmap_parts(v_cache, rows, head_dim, kPageT, head_dim / 64);
     it = maps.emplace(key, mp).first;
   }
   FaTmemParams p{};
@@ -674,7 +668,6 @@ void attention_prefill_tmem(const void* q, long long ldq, const void* k_cache, c
   p.hkv = hkv; p.group = hq / hkv;
   p.window = window; p.min_q = min_q;
   p.scale = scale; p.scale_log2 = scale * kLog2eT; p.softcap = softcap;
-  p.pv_wide = 1;
   p.tile_variant = tile_variant;
   p.bidir = bidir;
   if (head_dim == 64) launch_tmem<64>(it->second, p, max_q_len, num_seqs, s);
