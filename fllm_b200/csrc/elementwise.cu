@@ -473,6 +473,81 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
   }
 }
 
+// The same for prompts: rotate-half over the whole head, bf16 cache, projection in one piece. A block per token computes the cosines and
+// sines of its position once (a warp per head computes them for every head: 48 accurate sincosf of a token instead of one took
+// 44 us of 2048 x 48 heads of 128, whose 50 MB move in 8); then D / 8 lanes take a head, eight values each: four neighbours and
+// their partners half a head further, so that a rotation stays in its lane and every access is 8 bytes.
+template <int D>
+__global__ void __launch_bounds__(256)
+rope_kv_rows_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __restrict__ positions, const int* __restrict__ slots,
+                    const float* __restrict__ inv_freq, const __nv_bfloat16* __restrict__ q_norm_w, const __nv_bfloat16* __restrict__ k_norm_w,
+                    __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int hq, int hkv, int block_size, float eps,
+                    float attn_factor) {
+  constexpr int LANES = D / 8, HPW = 32 / LANES;          // lanes of a head, heads of a warp
+  __shared__ float2 table[D / 2];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const int slot = slots ? slots[t] : -1;
+  if (threadIdx.x < D / 2) {
+    float sn, cs;
+    sincosf((float)positions[t] * inv_freq[threadIdx.x], &sn, &cs);
+    table[threadIdx.x] = make_float2(cs * attn_factor, sn * attn_factor);
+  }
+  __syncthreads();
+  const int sub = (threadIdx.x & 31) % LANES, e = 4 * sub;
+  const int heads = hq + 2 * hkv;
+  const int blk = slot / block_size, off = slot - blk * block_size;
+  const int first = (threadIdx.x >> 5) * HPW + (threadIdx.x & 31) / LANES;
+  for (int h = first; h - (threadIdx.x & 31) / LANES < heads; h += 8 * HPW) {      // a warp's lanes go together: the sums below are exchanged
+    const bool in = h < heads, is_q = h < hq, is_v = h >= hq + hkv;
+    __nv_bfloat16* src = qkv + (size_t)t * ld_qkv + (size_t)h * D;
+    uint2 a = make_uint2(0, 0), b = make_uint2(0, 0);
+    if (in && (is_q || slot >= 0)) {
+      a = *reinterpret_cast<const uint2*>(src + e);
+      b = *reinterpret_cast<const uint2*>(src + D / 2 + e);
+    }
+    float v[8];
+    {
+      const float2 p0 = unpack_bf16x2(a.x), p1 = unpack_bf16x2(a.y), p2 = unpack_bf16x2(b.x), p3 = unpack_bf16x2(b.y);
+      v[0] = p0.x; v[1] = p0.y; v[2] = p1.x; v[3] = p1.y; v[4] = p2.x; v[5] = p2.y; v[6] = p3.x; v[7] = p3.y;
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o, LANES);
+    if (!is_v) {
+      const __nv_bfloat16* nw = is_q ? q_norm_w : k_norm_w;
+      if (nw) {
+        const float inv = rsqrtf(ss / (float)D + eps);
+        const uint2 wa = *reinterpret_cast<const uint2*>(nw + e), wb = *reinterpret_cast<const uint2*>(nw + D / 2 + e);
+        const uint32_t w[4] = {wa.x, wa.y, wb.x, wb.y};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                     // rounded through bf16, as an unfused norm would
+          const float2 g = unpack_bf16x2(w[j]);
+          const float2 r = unpack_bf16x2(pack_bf16x2(v[2 * j] * inv * g.x, v[2 * j + 1] * inv * g.y));
+          v[2 * j] = r.x; v[2 * j + 1] = r.y;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 cs = table[e + j];
+        const float x = v[j], y = v[j + 4];
+        v[j] = x * cs.x - y * cs.y;
+        v[j + 4] = y * cs.x + x * cs.y;
+      }
+      a = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+      b = make_uint2(pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+    }
+    if (!in || (!is_q && slot < 0)) continue;
+    __nv_bfloat16* dst = src;
+    if (!is_q) dst = (is_v ? v_cache : k_cache) + (((size_t)blk * hkv + (is_v ? h - hq - hkv : h - hq)) * block_size + off) * D;
+    *reinterpret_cast<uint2*>(dst + e) = a;
+    *reinterpret_cast<uint2*>(dst + D / 2 + e) = b;
+  }
+}
+
 void rope_qknorm_kvwrite_bf16(void* qkv, long long ld_qkv, const int* positions, const int* slots,
                               const float* inv_freq, const void* q_norm_w, const void* k_norm_w,
                               void* k_cache, void* v_cache, int tokens, int hq, int hkv,
@@ -488,6 +563,19 @@ void rope_qknorm_kvwrite_bf16(void* qkv, long long ld_qkv, const int* positions,
   auto* kn = (const __nv_bfloat16*)k_norm_w;
   auto* kc = (__nv_bfloat16*)k_cache;
   auto* vc = (__nv_bfloat16*)v_cache;
+  // One block per token needs as many tokens as there are SMs; below, a warp per head finishes sooner.
+  const uintptr_t align = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w) |
+                          reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache);
+  if (tokens >= sm_count() && !partials && !q_out && !kv_fp8 && rope_style == 0 && rot_dim == head_dim && (head_dim == 64 || head_dim == 128) &&
+      (ld_qkv & 3) == 0 && (align & 7) == 0) {
+    if (head_dim == 64)
+      launch_pdl(rope_kv_rows_kernel<64>, dim3(tokens), dim3(256), 0, s, x, ld_qkv, positions, slots, inv_freq, qn, kn, kc, vc, hq, hkv, block_size, eps,
+                 attn_factor);
+    else
+      launch_pdl(rope_kv_rows_kernel<128>, dim3(tokens), dim3(256), 0, s, x, ld_qkv, positions, slots, inv_freq, qn, kn, kc, vc, hq, hkv, block_size, eps,
+                 attn_factor);
+    return;
+  }
 #define FLLM_ROPE(DD)                                                                            \
   launch_pdl(rope_kv_kernel<DD>, dim3(blocks), dim3(128), 0, s, x, ld_qkv, positions, slots, inv_freq, qn, kn, kc, \
              vc, tokens, hq, hkv, block_size, rot_dim, rope_style, eps, attn_factor, kv_fp8, partials, splits,    \
