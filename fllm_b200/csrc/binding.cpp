@@ -258,6 +258,13 @@ void act_(Tensor x, int64_t kind) {
   fllm::act_rows_bf16(x.data_ptr(), x.stride(0), (int)x.size(0), (int)x.size(1), (int)kind, cur_stream());
 }
 
+void widen_rows(const Tensor& x, Tensor out) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && (x.stride(1) == 1 || x.size(1) <= 1), "x: bf16 rows");
+  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kFloat && out.is_contiguous() && out.sizes() == x.sizes(), "out: contiguous fp32 of the same shape");
+  c10::cuda::CUDAGuard guard(x.device());
+  fllm::widen_rows(x.data_ptr(), x.stride(0), out.data_ptr<float>(), (int)x.size(0), (int)x.size(1), cur_stream());
+}
+
 void softcap_(Tensor x, double cap) {
   const bool f32 = x.is_cuda() && x.scalar_type() == at::kFloat;
   if (!f32) check_bf16(x, "x");
@@ -399,6 +406,7 @@ TORCH_LIBRARY(fllm_b200, m) {
   m.def("glu(Tensor x, Tensor(a!) out, int act_kind, float alpha, float limit) -> ()", &glu);
   m.def("gather_rows(Tensor x, Tensor rows, Tensor(a!) out) -> ()", &gather_rows);
   m.def("softcap_(Tensor(a!) x, float cap) -> ()", &softcap_);
+  m.def("widen_rows(Tensor x, Tensor(a!) out) -> ()", &widen_rows);
   m.def("add_layernorm(Tensor(a!) x, Tensor? delta, Tensor w, Tensor? b, Tensor(b!) y, float eps, float w_offset) -> ()", &add_layernorm);
   m.def("act_(Tensor(a!) x, int kind) -> ()", &act_);
   m.def("argmax(Tensor logits, Tensor(a!) out_ids, Tensor? out_vals, int id_offset) -> ()", &argmax);

@@ -4,6 +4,8 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
 
+#include <tuple>
+
 #include "fllm_ops.h"
 
 namespace {
@@ -75,7 +77,7 @@ int64_t linear_w4a16(const Tensor& x, const Tensor& codes, const Tensor& scales,
     ws_bytes = workspace->numel() * workspace->element_size() - (64 << 10);
   }
   return fllm::linear_w4a16(x.data_ptr(), x.stride(0), codes.data_ptr(), scales.data_ptr(), (int)fmt, (float)alpha, b,
-                            y.data_ptr(), y.stride(0), (int)T, (int)N, (int)K, ws, ws_bytes, st, cur_stream());
+                            y.data_ptr(), y.stride(0), (int)T, (int)N, (int)K, ws, ws_bytes, st, cur_stream(), f16);
 }
 
 // x bf16 [T, K] -> xq uint8 [T, K] (e4m3) + sf uint8 [mx_act_scale_bytes(T, K, 0)] (e8m0 atoms per token tile)

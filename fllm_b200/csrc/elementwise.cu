@@ -590,6 +590,32 @@ void rope_qknorm_kvwrite_bf16(void* qkv, long long ld_qkv, const int* positions,
   cuda_check(cudaGetLastError(), "rope_kv_kernel");
 }
 
+// ---------------------------------------------------------------------------- bf16 rows -> fp32
+// Eight values per thread: 16 bytes in, 32 out (the generic copy moved 2.3 TB/s of 200 x 151936 logits, behind a gather of its own).
+__global__ void __launch_bounds__(256) widen_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, float* __restrict__ out, int cols, int vec) {
+  const __nv_bfloat16* src = x + (size_t)blockIdx.y * ldx;
+  float* dst = out + (size_t)blockIdx.y * cols;
+  const int i = (blockIdx.x * 256 + threadIdx.x) * 8;
+  if (i >= cols) return;
+  if (vec && i + 8 <= cols) {
+    const uint4 v = *reinterpret_cast<const uint4*>(src + i);
+    const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
+    reinterpret_cast<float4*>(dst + i)[0] = make_float4(a.x, a.y, b.x, b.y);
+    reinterpret_cast<float4*>(dst + i)[1] = make_float4(c.x, c.y, d.x, d.y);
+  } else {
+    for (int j = i; j < min(i + 8, cols); ++j) dst[j] = __bfloat162float(src[j]);
+  }
+}
+
+void widen_rows(const void* x, long long ldx, float* out, int rows, int cols, cudaStream_t s) {
+  if (rows <= 0 || cols <= 0) return;
+  const int vec = (ldx & 7) == 0 && (cols & 3) == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  for (int r = 0; r < rows; r += 65535)
+    widen_rows_kernel<<<dim3((cols + 2047) / 2048, min(rows - r, 65535)), 256, 0, s>>>((const __nv_bfloat16*)x + (size_t)r * ldx, ldx,
+                                                                                       out + (size_t)r * cols, cols, vec);
+  cuda_check(cudaGetLastError(), "widen_rows_kernel");
+}
+
 // ---------------------------------------------------------------------------- GLU activations
 // act_kind 0: silu(gate) * up with gate = x[:, :I], up = x[:, I:2I]
 // act_kind 1: gelu_tanh(gate) * up (GeGLU)

@@ -187,6 +187,13 @@ class NativeOps(RecurrentNative, LatentNative, TiedNative, MapsNative, PreNormNa
         self.launches += 1
         return x
 
+    def widen_rows(self, x):
+        """fp32 copy of bf16 rows (row pitch free), e.g. logits that leave a captured step's buffer."""
+        out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+        self.k.widen_rows(x, out)
+        self.launches += 1
+        return out
+
     def attention_tree(self, q, k_cache, v_cache, block_tables, row_seq, positions, tree_mask, tree_base, hq, hkv,
                        head_dim, scale, window=0, sinks=None, softcap=0.0):
         """Attention for the nodes of draft trees: row t sees the first tree_base[t] tokens of its sequence and the
@@ -298,12 +305,15 @@ class Fp8BlockWeight:
             wd = self.wq.view(torch.float8_e4m3fn).float().view(self.shape[0] // 128, 128, K // 128, 128) * self.sw[:, None, :, None]
             y = x.float() @ wd.view(self.shape[0], K).t()
             return (y + bias.float() if bias is not None else y).to(x.dtype)
+        if out is None:                                             # quantiser and product behind one call
+            y, n = ops.k.fp8_block_apply(x, self.wq, self.sw, bias, ops.status, ops.workspace)
+            ops.launches += n
+            return y
         xq = torch.empty(T, K, dtype=torch.uint8, device=x.device)
         sx = torch.empty(T, K // 128, dtype=torch.float32, device=x.device)
         ops.k.quant_fp8_1x128(x.contiguous(), xq, sx)
-        y = out if out is not None else torch.empty(T, self.shape[0], dtype=torch.bfloat16, device=x.device)
-        ops.launches += 1 + ops.k.linear_fp8_block(xq, sx, self.wq, self.sw, bias, y, ops.status, ops.workspace)
-        return y
+        ops.launches += 1 + ops.k.linear_fp8_block(xq, sx, self.wq, self.sw, bias, out, ops.status, ops.workspace)
+        return out
 
 
 class Fp8BlockLinear:

@@ -190,6 +190,9 @@ class LLMEngine:
         if self.par.pp == 1:
             halt = torch.empty(cap, dtype=torch.int32, pin_memory=self.is_cuda)
             self._stage_bufs.append((halt, halt.numpy(), self._dev))
+        # a pinned buffer is written again only after the copy out of it is done (no caller has to wait for that)
+        self._stage_done: List[Optional[torch.cuda.Event]] = [None] * len(self._stage_bufs)
+        self._forced_slot = 0
         self._out_alt = torch.empty(512, dtype=torch.int32, pin_memory=self.is_cuda)
         self._flip = 0
         self._out_host = torch.empty(self.cfg.max_num_batched_tokens + 64, dtype=torch.int32,
@@ -336,17 +339,15 @@ class LLMEngine:
         Bp = max(B, pad_to) if pad_to else B
         bs = self.block_size
         host_t, h, dev = self._stage_bufs[slot]
+        if self._stage_done[slot] is not None:
+            self._stage_done[slot].synchronize()
         ids = h[0:Tp]
         pos = h[Tp:2 * Tp]
         slots = h[2 * Tp:3 * Tp]
         rseq = h[3 * Tp:4 * Tp]
         rows: List[int] = []
         max_kv = 0
-        max_blocks = 1
-        for s in seqs:
-            max_blocks = max(max_blocks, len(self.blocks.table(s.req.seq_id)))
-        if pad_to:
-            max_blocks = self.max_blocks_per_seq
+        max_blocks = self.max_blocks_per_seq if pad_to else max([1] + [len(self.blocks.table(s.req.seq_id)) for s in seqs])
         R_cap = Tp
         lrow = h[4 * Tp:4 * Tp + R_cap]
         o_qs, o_kl, o_tab = 5 * Tp, 5 * Tp + Bp + 1, 5 * Tp + 2 * Bp + 1
@@ -357,6 +358,26 @@ class LLMEngine:
         sst = h[o_ss:o_ss + Bp] if self.rstate is not None else None
         max_q, min_q = 1, 1 << 30
         t = 0
+        if step.all_decode and not any(s.verify for s in seqs):
+            # one token per sequence: collected as lists, stored once
+            c_ids, c_pos, c_slot = [], [], []
+            for i, s in enumerate(seqs):
+                r, p0 = s.req, s.start
+                sb = self.blocks.seqs[r.seq_id]
+                c_ids.append(r.output[-1] if p0 == r.num_tokens - 1 else r.all_tokens[p0])
+                c_pos.append(p0)
+                tb = sb.np_table()
+                c_slot.append(int(tb[p0 // bs]) * bs + p0 % bs)
+                tab[i, :tb.shape[0]] = tb
+                if sst is not None:
+                    sst[i] = sb.state_slot
+                if s.wants_logits:
+                    rows.extend([i + j for j in s.rows] if s.rows is not None else [i])
+            ids[:B], pos[:B], slots[:B] = c_ids, c_pos, c_slot
+            rseq[:B] = qst[:B] = np.arange(B, dtype=np.int32)
+            kvl[:B] = pos[:B] + 1
+            max_kv = max([max_kv] + c_pos) + 1
+            min_q, t, seqs = 1, T, []
         for i, s in enumerate(seqs):
             r = s.req
             n = s.count
@@ -406,13 +427,16 @@ class LLMEngine:
         used = o_ss + (Bp if sst is not None else 0)
         if self.is_cuda:
             dev[:used].copy_(host_t[:used], non_blocking=True)
+            if self._stage_done[slot] is None:
+                self._stage_done[slot] = torch.cuda.Event()
+            self._stage_done[slot].record()
         else:
             dev[:used] = host_t[:used]
         self.stats.h2d_bytes += used * 4
         host_seqs = None
         if sst is not None and max_q >= 512 and not pad_to:
             # long prompt chunks of recurrent layers may take a matrix form that is set up from the host
-            host_seqs = [(int(qst[i]), s.count, int(sst[i]), s.start == 0) for i, s in enumerate(seqs)]
+            host_seqs = [(int(qst[i]), s.count, int(sst[i]), s.start == 0) for i, s in enumerate(step.seqs)]
         return StepBatch(
             host_seqs=host_seqs,
             token_ids=dev[0:Tp], positions=dev[Tp:2 * Tp], slots=dev[2 * Tp:3 * Tp],
@@ -430,7 +454,7 @@ class LLMEngine:
                 return b
         return 0
 
-    def _decode_with_graph(self, step: ScheduledStep) -> torch.Tensor:
+    def _decode_with_graph(self, step: ScheduledStep, slot: int = 0) -> torch.Tensor:
         """Pure-decode step through a captured graph; returns greedy ids for the bucket rows."""
         n = len(step.seqs)
         bucket = self._bucket_for(n)
@@ -438,7 +462,7 @@ class LLMEngine:
         if g is None:
             g = _DecodeGraph(self, bucket)
             self._graphs[bucket] = g
-        batch = self._build_batch(step, pad_to=bucket)     # fills the static staging buffer
+        batch = self._build_batch(step, pad_to=bucket, slot=slot)     # fills the static staging buffer
         g.replay()
         self.stats.graph_steps += 1
         return g.tokens, g.logits, batch
@@ -896,12 +920,25 @@ class LLMEngine:
         """Forward of a step whose tokens are all given: fp32 logits of the rows it wants, in batch order. Pure decode steps
         replay the captured graph of their bucket. Nothing is sampled or committed. Single pipeline stage only."""
         self.drain()
-        if self._graph_eligible(step):
-            _, logits, _ = self._decode_with_graph(step)
-            logits = logits[[i for i, s in enumerate(step.seqs) if s.wants_logits]]
+        slot = 0
+        if self.par.pp == 1:             # two pinned buffers over one device buffer: the next step is built while this one runs
+            self._forced_slot ^= 1
+            slot = 0 if self._forced_slot == 0 else len(self._stage_bufs) - 1
+        static = self._graph_eligible(step)
+        if static:
+            _, logits, _ = self._decode_with_graph(step, slot)
+            want = [i for i, s in enumerate(step.seqs) if s.wants_logits]
+            if want == list(range(len(want))):
+                logits = logits[:len(want)]
+            else:
+                logits, static = logits[want], False
         else:
-            logits = self.decoder.forward(self._build_batch(step))
-        return self.decoder.full_logits(logits).float()
+            logits = self.decoder.forward(self._build_batch(step, slot=slot))
+        logits = self.decoder.full_logits(logits)
+        if logits.dtype == torch.bfloat16 and logits.is_cuda and hasattr(self.ops, "k"):
+            return self.ops.widen_rows(logits)
+        out = logits.float()
+        return out.clone() if static and out.data_ptr() == logits.data_ptr() else out      # (not the graph's own buffer)
 
     # ------------------------------------------------------------------ scoring
     @torch.inference_mode()

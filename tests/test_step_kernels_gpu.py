@@ -1,0 +1,127 @@
+"""Kernels of a step at the edges of their tiles and rules: CTA-pair products over splits of K, block-FP8 products of both tile widths,
+rotation of prompt rows, widened logits, and given steps queued without waiting for one another."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from fllm_b200.ops import get_ops
+    return get_ops(torch.device("cuda:0"))
+
+
+def _rand(shape, seed, std=1.0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * std).to(torch.bfloat16).cuda()
+
+
+def _rel(y, ref):
+    return ((y.double() - ref).norm() / ref.norm()).item()
+
+
+@pytest.mark.parametrize("T", [129, 200, 255, 256, 257, 511])
+@pytest.mark.parametrize("N,K", [(256, 4096), (264, 64), (1000, 320), (6144, 4096), (4096, 12288)])
+def test_pairs_over_splits(ops, T, N, K):
+    """One rounding to bf16 is all that a correct product is off (0.17 % in the mean square)."""
+    x, w, b = _rand((T, K), 1), _rand((N, K), 2, 0.05), _rand((N,), 3)
+    ref = x.double() @ w.double().t()
+    assert _rel(ops.linear(x, w), ref) < 2.5e-3
+    assert _rel(ops.linear(x, w, b), ref + b.double()) < 2.5e-3
+    assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("T", [129, 200, 300])
+def test_pairs_leave_their_sums_to_the_norm_and_the_activation(ops, T):
+    x, w, b, nw = _rand((T, 4096), 1), _rand((4096, 4096), 2, 0.02), _rand((4096,), 3), _rand((4096,), 4)
+    res = _rand((T, 4096), 5)
+    y = ops.linear(x, w, b, defer=True)
+    assert type(y).__name__ == "Deferred"
+    a, r1 = res.clone(), res.clone()
+    got = ops.rmsnorm(a, y, nw, 1e-6)
+    want = ops.rmsnorm(r1, ops.linear(x, w, b), nw, 1e-6)
+    assert torch.equal(a, r1) and _rel(got, want.double()) < 1e-3      # (the two norms add a row's squares in other orders)
+    g = _rand((2048, 512), 6, 0.1)                     # gate | up in blocks of 16
+    h = _rand((T, 512), 7)
+    u = (h.double() @ g.double().t()).view(T, 64, 2, 16)
+    ref = (torch.nn.functional.silu(u[:, :, 0]) * u[:, :, 1]).reshape(T, 1024)
+    assert _rel(ops.linear_glu(h, g, None, 0, layout=16), ref) < 8e-3     # partial sums are rounded to bf16 in front of the activation
+
+
+@pytest.mark.parametrize("T,N,K", [(1, 128, 128), (17, 256, 1024), (64, 384, 8192), (65, 128, 256), (128, 7168, 8192), (129, 1280, 8192), (128, 256, 12288),
+                                   (300, 8192, 1024), (1965, 8192, 3584)])
+def test_fp8_block(ops, T, N, K):
+    from fllm_b200.ops.native import Fp8BlockLinear, quantize_weight_fp8_block
+    x, bias = _rand((T, K), 1), _rand((N,), 3)
+    wq, sw = quantize_weight_fp8_block(_rand((N, K), 2, 0.05))
+    xq, sx = torch.empty(T, K, dtype=torch.uint8, device="cuda"), torch.empty(T, K // 128, device="cuda")
+    ops.k.quant_fp8_1x128(x, xq, sx)
+    amax = x.float().view(T, K // 128, 128).abs().amax(-1)
+    assert torch.allclose(sx, amax / 448.0, rtol=1e-6)
+    xd = xq.view(torch.float8_e4m3fn).double().view(T, K // 128, 128) * sx.double()[:, :, None]
+    assert ((xd.view(T, K) - x.double()).abs() <= x.double().abs() / 15.9 + sx.double().repeat_interleave(128, 1) * 2.0 ** -10).all()
+    wd = wq.view(torch.float8_e4m3fn).double().view(N // 128, 128, K // 128, 128) * sw.double()[:, None, :, None]
+    ref = xd.view(T, K) @ wd.view(N, K).t() + bias.double()
+    assert _rel(Fp8BlockLinear(ops, wq, sw, bias)(x), ref) < 2.5e-3
+    out = torch.empty(T, N, dtype=torch.bfloat16, device="cuda")
+    from fllm_b200.ops.native import Fp8BlockWeight
+    assert ops.linear(x, Fp8BlockWeight(wq, sw), bias, out=out) is out and _rel(out, ref) < 2.5e-3
+    assert ops.check_status() == 0
+
+
+@pytest.mark.parametrize("T", [147, 148, 301])
+@pytest.mark.parametrize("D,hq,hkv", [(64, 5, 1), (64, 64, 8), (128, 3, 3), (128, 32, 8)])
+@pytest.mark.parametrize("norm", [False, True])
+def test_rope_of_prompt_rows(ops, T, D, hq, hkv, norm):
+    """On both sides of the number of tokens that the kernel for rows takes over at, against the PyTorch operator."""
+    from fllm_b200.ops.reference import RefOps
+    qkv = _rand((T, (hq + 2 * hkv) * D), 1)
+    blocks = T // 16 + 2
+    pos = (torch.arange(T) * 37 % 9000).int().cuda()
+    slots = torch.randperm(blocks * 16, generator=torch.Generator().manual_seed(2))[:T].int().cuda()
+    slots[3], slots[T - 1] = -1, -1
+    inv = (1e6 ** (-torch.arange(0, D, 2).double() / D)).float().cuda()
+    qn, kn = (_rand((D,), 3) + 1, _rand((D,), 4) + 1) if norm else (None, None)
+    caches = [[torch.zeros(blocks, hkv, 16, D, dtype=torch.bfloat16, device="cuda") for _ in range(2)] for _ in range(2)]
+    got = ops.rope_kv_write(qkv.clone(), pos, slots, inv, qn, kn, *caches[0], hq, hkv, D, D, 0, 1e-6, 1.25)
+    want = RefOps().rope_kv_write(qkv.clone(), pos, slots, inv, qn, kn, *caches[1], hq, hkv, D, D, 0, 1e-6, 1.25)
+    # one rounding to bf16 more or less, and one of a normed value
+    assert _rel(got, want.double()) < 4e-3 and _rel(caches[0][0], caches[1][0].double()) < 4e-3
+    assert torch.equal(caches[0][1], caches[1][1])
+
+
+@pytest.mark.parametrize("rows,cols,pitch", [(1, 1, 8), (3, 7, 8), (5, 4096, 4096), (2, 151936, 151936), (4, 2052, 2056), (3, 2051, 2056)])
+def test_widen_rows(ops, rows, cols, pitch):
+    x = _rand((rows, pitch), 1)[:, :cols]
+    assert torch.equal(ops.widen_rows(x), x.float())
+
+
+def test_given_steps_queue_without_waiting():
+    """Steps of other sizes and other tokens, one after the other without a synchronisation: each gives what it gives alone."""
+    from fllm_b200.config import EngineConfig, preset
+    from fllm_b200.runtime import LLMEngine
+    from fllm_b200.runtime.request import Request, SamplingParams
+    from fllm_b200.runtime.scheduler import ScheduledSeq, ScheduledStep
+    cfg = preset("qwen3-tiny")
+    eng = LLMEngine(cfg, EngineConfig(max_num_seqs=16, max_num_batched_tokens=128, max_model_len=256, num_kv_blocks=256, enable_prefix_caching=False),
+                    device="cuda:0")
+    g = torch.Generator().manual_seed(0)
+    reqs = []
+    for i in range(11):
+        toks = torch.randint(0, cfg.vocab_size, (9 + 5 * i,), generator=g).tolist()
+        r = Request(f"r{i}", 1000 + i, toks, SamplingParams(max_tokens=4))
+        r.output = [7 + i]
+        eng.blocks.allocate(r.seq_id, [])
+        assert eng.blocks.ensure_capacity(r.seq_id, r.num_tokens)
+        reqs.append(r)
+    prompts = [ScheduledStep(seqs=[ScheduledSeq(r, 0, len(r.prompt), True)]) for r in reqs]
+    decodes = [ScheduledStep(seqs=[ScheduledSeq(r, len(r.prompt), 1, j % 3 != 1) for j, r in enumerate(reqs[a:b])]) for a, b in ((0, 11), (2, 5), (4, 11), (0, 1), (3, 11))]
+    alone = []
+    for s in prompts + decodes:
+        alone.append(eng.run_forced(s).cpu())
+        torch.cuda.synchronize()
+    queued = [eng.run_forced(s) for s in prompts + decodes + decodes[::-1]]
+    torch.cuda.synchronize()
+    for a, b in zip(alone + alone[len(prompts):][::-1], queued):
+        assert torch.equal(a, b.cpu())
+    eng.close()
