@@ -30,7 +30,6 @@ namespace fllm {
 constexpr int F8_BM = 128;
 constexpr int F8_BK = 128;      // e4m3 elements = bytes per swizzle row = scale block depth
 constexpr int F8_UMMA_K = 32;
-constexpr int kF8Threads = 64 + 256;      // TMA warp, MMA warp, eight promoting warps
 
 struct Fp8GemmArgs {
   int M, N, K;              // MMA orientation: D[M][N] = A[M][K] B[N][K]^T
@@ -56,19 +55,21 @@ struct Fp8Smem {
   // A K block's product stays in its buffer until the promoting warps have added it up: the tensor core runs ahead by the other buffers.
   static constexpr int kBuffers = BN == 256 ? 2 : 4;
   static constexpr int kTmemCols = kBuffers * BN < 128 ? (kBuffers * BN < 64 ? 64 : kBuffers * BN) : kBuffers * BN;
-  static constexpr int kHalves = BN >= 64 ? 2 : 1;                  // warps that share a lane quarter split the columns
-  static constexpr int kCols = BN / kHalves;                        // columns of a promoting thread
-  static constexpr int kPromote = 128 * kHalves;                    // promoting threads with columns
+  static constexpr int kCols = BN > 64 ? 64 : BN > 32 ? 32 : BN;     // columns of a promoting thread
+  static constexpr int kShares = BN / kCols;                        // warps that share a lane quarter split the columns
+  static constexpr int kPromote = 128 * kShares;                    // promoting threads: four warps per share
+  static constexpr int kThreads = 64 + kPromote;                    // TMA warp, MMA warp, promoting warps
   static constexpr int kTotal = kStages * kStageBytes + kScaleFloats * 4 + 256 + 1024;
   static_assert((2 * kStages + 2 * kBuffers) * 8 + 8 <= 256, "barrier block");
 };
 
 // What bounds it: a 128 x 256 x 128 block is 512 clocks of the tensor core; promoting it is 32768 multiply-adds, 256 issue slots of each
-// scheduler over eight warps, so the products bound it as long as a thread's share costs one multiply-add per value: one factor per row
-// and K block (activation scale x weight scale, read ahead), one accumulator register per column. 128 x 128 tiles read and write shared memory
+// scheduler, so the products bound it as long as a thread's share costs one multiply-add per value (one factor per row and K
+// block, activation scale x weight scale, read ahead; one accumulator register per column) and the latency of the tensor memory is
+// covered: four warps per scheduler with 64 columns each (two with 128 needed 1290 clocks a block). 128 x 128 tiles read and write shared memory
 // twice as often per product; they remain for few tiles.
 template <int BN>
-__global__ void __launch_bounds__(kF8Threads, 1)
+__global__ void __launch_bounds__(Fp8Smem<BN>::kThreads, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const Fp8GemmArgs p) {
   using S = Fp8Smem<BN>;
@@ -90,7 +91,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < NBUF; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 4 * S::kHalves); }
+    for (int a = 0; a < NBUF; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 4 * S::kShares); }
     *abort_flag = 0;
     fence_barrier_init();
   }
@@ -165,7 +166,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         if (++buf == NBUF) { buf = 0; buf_phase ^= 1; }
       }
     }
-  } else if (threadIdx.x - 64 < S::kPromote) {
+  } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
     const int etid = threadIdx.x - 64;
     pdl_wait();                            // scales of the activations; outputs may still be in use by the predecessor
@@ -202,7 +203,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
         if (!mbar_wait(&tfull_bar[buf], buf_phase, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t t_row = tmem_base + buf * BN + half * COLS + ((uint32_t)(q * 32) << 16);
-        constexpr int CH = COLS < 32 ? 16 : 32;
+        constexpr int CH = COLS < 32 || BN == 256 ? 16 : 32;      // (registers: eighteen warps leave 102 a thread)
 #pragma unroll
         for (int c0 = 0; c0 < COLS; c0 += CH) {
           uint32_t r[CH];
@@ -340,7 +341,7 @@ static void launch_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const Fp8Ge
     cuda_check(cudaFuncSetAttribute(gemm_fp8_block_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
                "cudaFuncSetAttribute(gemm_fp8_block_kernel)");
   }
-  launch_pdl(gemm_fp8_block_kernel<BN>, dim3(grid), dim3(kF8Threads), S::kTotal, s, ta, tb, a);
+  launch_pdl(gemm_fp8_block_kernel<BN>, dim3(grid), dim3(S::kThreads), S::kTotal, s, ta, tb, a);
 }
 
 // y[T][N] = dequant(xq, sx) * dequant(wq, sw)^T (+ bias)
