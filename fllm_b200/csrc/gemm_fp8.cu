@@ -42,15 +42,28 @@ struct Fp8GemmArgs {
   const __nv_bfloat16* bias;
   int* status;
   int k_splits, kb_per_split;   // work items are (tile, split): few tiles cannot pull the whole HBM bandwidth otherwise
-  float* ws;                    // [k_splits][tokens][features] fp32 partial sums when k_splits > 1
+  int whole;                    // the first tiles are one item each, over all of K; only those after them are split
+  float* ws;                    // fp32 partial sums when k_splits > 1: [k_splits][tokens][features], or a tile each if whole > 0
 };
 
-template <int BN>
+// Item w of a launch: its tile, its split (-1: a whole tile) and its K blocks.
+struct Fp8Item {
+  int t, split, kb0, kb1;
+  __device__ __forceinline__ Fp8Item(const Fp8GemmArgs& p, int w) : t(w), split(-1), kb0(0), kb1(p.k_blocks) {
+    if (w >= p.whole) {                                     // the split is the fastest index
+      const int v = w - p.whole;
+      split = v % p.k_splits; t = p.whole + v / p.k_splits;
+      kb0 = split * p.kb_per_split; kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+    }
+  }
+};
+
+template <int BN, bool SWAP>
 struct Fp8Smem {
   static constexpr int kABytes = F8_BM * F8_BK;
   static constexpr int kBBytes = BN * F8_BK;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kScaleFloats = BN <= 64 ? 64 * BN : 0;       // token scales of a swap-AB tile, up to 64 K blocks
+  static constexpr int kScaleFloats = SWAP ? 64 * BN : 0;       // token scales of a swap-AB tile, up to 64 K blocks
   static constexpr int kStages = (196 * 1024 - kScaleFloats * 4) / kStageBytes > 10 ? 10 : (196 * 1024 - kScaleFloats * 4) / kStageBytes;
   // A K block's product stays in its buffer until the promoting warps have added it up: the tensor core runs ahead by the other buffers.
   static constexpr int kBuffers = BN == 256 ? 2 : 4;
@@ -68,13 +81,12 @@ struct Fp8Smem {
 // block, activation scale x weight scale, read ahead; one accumulator register per column) and the latency of the tensor memory is
 // covered: four warps per scheduler with 64 columns each (two with 128 needed 1290 clocks a block). 128 x 128 tiles read and write shared memory
 // twice as often per product; they remain for few tiles.
-template <int BN>
-__global__ void __launch_bounds__(Fp8Smem<BN>::kThreads, 1)
+template <int BN, bool SWAP>                // SWAP: tokens in the N dimension
+__global__ void __launch_bounds__(Fp8Smem<BN, SWAP>::kThreads, 1)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const Fp8GemmArgs p) {
-  using S = Fp8Smem<BN>;
+  using S = Fp8Smem<BN, SWAP>;
   constexpr int STAGES = S::kStages, NBUF = S::kBuffers, COLS = S::kCols;
-  constexpr bool SWAP = BN <= 64;          // tokens in the N dimension
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
@@ -102,17 +114,17 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
-  const int tiles = p.m_tiles * p.n_tiles * p.k_splits;      // work items: the split is the fastest index
+  const int items = p.whole + (p.m_tiles * p.n_tiles - p.whole) * p.k_splits;
 
   if (warp == 0) {
     int stage = 0, pre = 0;
     uint32_t phase = 0;
     bool ok = true;
     {                                    // weights are static: the first stages' are requested before waiting for the quantiser
-      const int split = blockIdx.x % p.k_splits, t = blockIdx.x / p.k_splits;
-      const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
-      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-      pre = min(kb1 - kb0, STAGES);
+      const Fp8Item it(p, blockIdx.x);
+      const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
+      const int kb0 = it.kb0;
+      pre = min(it.kb1 - kb0, STAGES);
       if (elect_one()) {
         for (int i = 0; i < pre; ++i) {
           mbar_expect_tx(&full_bar[i], S::kStageBytes);
@@ -123,10 +135,10 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       __syncwarp();
     }
     pdl_wait();
-    for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
-      const int split = w % p.k_splits, t = w / p.k_splits;
-      const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
-      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const Fp8Item it(p, w);
+      const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
+      const int kb0 = it.kb0, kb1 = it.kb1;
       for (int kb = kb0; kb < kb1; ++kb) {
         const bool requested = pre > 0;
         if (requested) --pre;
@@ -146,10 +158,9 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     int stage = 0, buf = 0;
     uint32_t phase = 0, buf_phase = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
-      const int split = w % p.k_splits;
-      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
-      for (int kb = kb0; kb < kb1; ++kb) {
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const Fp8Item it(p, w);
+      for (int kb = it.kb0; kb < it.kb1; ++kb) {
         // each K block gets its own accumulator: wait until the promoting warps drained this buffer
         if (!mbar_wait_warp(&tempty_bar[buf], buf_phase ^ 1, abort_flag) || !mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
@@ -173,10 +184,10 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     int buf = 0;
     uint32_t buf_phase = 0;
     bool ok = true;
-    for (int w = blockIdx.x; w < tiles && ok; w += gridDim.x) {
-      const int split = w % p.k_splits, t = w / p.k_splits;
-      const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
-      const int kb0 = split * p.kb_per_split, kb1 = min(p.k_blocks, kb0 + p.kb_per_split);
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const Fp8Item it(p, w);
+      const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
+      const int kb0 = it.kb0, kb1 = it.kb1;
       const int m = m_idx * F8_BM + q * 32 + lane;
       const int n_base = n_idx * BN + half * COLS;
       if (SWAP) {
@@ -223,12 +234,16 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       }
       if (!ok) break;
       // store
-      if (p.k_splits > 1) {                                   // fp32 partial sums [split][token][feature]; bias in the reduction
-        float* wsp = p.ws + (size_t)split * (size_t)p.N * p.M;
+      if (it.split >= 0) {                                    // fp32 partial sums; bias in the reduction
+        float* wsp = p.ws + (size_t)it.split * (size_t)p.N * p.M;
         if (SWAP) {                                           // lanes run along features: coalesced
 #pragma unroll
           for (int c = 0; c < COLS; ++c)
             if (n_base + c < p.N && m < p.M) wsp[(size_t)(n_base + c) * p.M + m] = acc[c];
+        } else if (p.whole > 0) {
+          wsp = p.ws + (((size_t)it.split * (p.m_tiles * p.n_tiles - p.whole) + (it.t - p.whole)) * F8_BM + q * 32 + lane) * BN + half * COLS;
+#pragma unroll
+          for (int c = 0; c < COLS; c += 4) *reinterpret_cast<float4*>(wsp + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
         } else if (m < p.M) {
 #pragma unroll
           for (int c = 0; c < COLS; c += 4)
@@ -294,6 +309,30 @@ __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ ws, int split
   *reinterpret_cast<uint2*>(out + (size_t)r * ldc + c) = o;
 }
 
+// The same over the tiles after the whole ones, whose partial sums lie tile by tile: ws[s][tile][128][bn].
+__global__ void fp8_tail_reduce_kernel(const Fp8GemmArgs p, int bn) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t tile = (size_t)F8_BM * bn, n = (size_t)(p.m_tiles * p.n_tiles - p.whole) * tile;
+  const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (i4 >= n) return;
+  const int t = p.whole + (int)(i4 / tile), within = (int)(i4 % tile);
+  const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
+  const int r = m_idx * F8_BM + within / bn, c = n_idx * bn + within % bn;
+  if (r >= p.M || c >= p.N) return;
+  float4 acc = *reinterpret_cast<const float4*>(p.ws + i4);
+  for (int s = 1; s < p.k_splits; ++s) {
+    const float4 v = *reinterpret_cast<const float4*>(p.ws + (size_t)s * n + i4);
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  float b[4] = {0.f, 0.f, 0.f, 0.f};
+  if (p.bias) for (int i = 0; i < 4; ++i) b[i] = __bfloat162float(p.bias[c + i]);
+  uint2 o;
+  o.x = pack_bf16x2(acc.x + b[0], acc.y + b[1]);
+  o.y = pack_bf16x2(acc.z + b[2], acc.w + b[3]);
+  *reinterpret_cast<uint2*>(p.out + (size_t)r * p.ldc + c) = o;
+}
+
 // x bf16 [T][K] -> e4m3 [T][K] and scales [T][K/128] (amax / 448 per 128 values). Half a warp per group, 16 bytes per lane (one warp per
 // group with 8 bytes per lane moved 2.3 TB/s at 1965 x 8192).
 __global__ void __launch_bounds__(256) quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ xq,
@@ -333,15 +372,15 @@ void quant_fp8_1x128(const void* x, long long ldx, void* xq, float* sx, int toke
   launch_pdl(quant_fp8_1x128_kernel, dim3((unsigned)((groups + 15) / 16)), dim3(256), 0, s, (const __nv_bfloat16*)x, ldx, (uint8_t*)xq, sx, tokens, K);
 }
 
-template <int BN>
+template <int BN, bool SWAP>
 static void launch_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const Fp8GemmArgs& a, int grid, cudaStream_t s) {
-  using S = Fp8Smem<BN>;
+  using S = Fp8Smem<BN, SWAP>;
   static bool configured[kMaxDevices] = {};
   if (first_call_on_device(configured)) {
-    cuda_check(cudaFuncSetAttribute(gemm_fp8_block_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
+    cuda_check(cudaFuncSetAttribute(gemm_fp8_block_kernel<BN, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
                "cudaFuncSetAttribute(gemm_fp8_block_kernel)");
   }
-  launch_pdl(gemm_fp8_block_kernel<BN>, dim3(grid), dim3(S::kThreads), S::kTotal, s, ta, tb, a);
+  launch_pdl(gemm_fp8_block_kernel<BN, SWAP>, dim3(grid), dim3(S::kThreads), S::kTotal, s, ta, tb, a);
 }
 
 // y[T][N] = dequant(xq, sx) * dequant(wq, sw)^T (+ bias)
@@ -359,23 +398,34 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   const int sms = sm_count();
   a.M = swap ? N : T; a.N = swap ? T : N; a.transposed = swap;
   a.m_tiles = (a.M + F8_BM - 1) / F8_BM;
-  // Tile width and K splits by the rounds of items over the SMs, in units of 1/100 us. A K block takes what its products take, or the
-  // time in which an SM's share of the HBM bandwidth brings its weights (37 per 128 features) when no other tile of the step reads
-  // them, too. 128-wide blocks take 18 and not 14, half of a 256-wide one: they move twice the shared memory per product. Partial sums
-  // are written and read once, and cost a launch.
-  int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1;
+  // Tile and K splits by the rounds of items over the SMs, in units of 1/100 us. A K block takes the time in which an SM's share of the HBM
+  // bandwidth brings its weights (37 per 128 features) when no other tile of the step reads them, too (64-wide tiles spare few tokens the
+  // partial sums or some of them, 28: 128 x 1280 x 8192 13.6 -> 12.0 us, 128 x 8192 x 3584 16.9 -> 15.8; 7168 x 8192 needs them and took 27.7
+  // against 24.9); else what L2 takes for its operands with every SM reading (256-wide tiles 60, 128-wide 36). Partial sums are
+  // written and read once, and cost a launch. With more tiles than SMs either all are split, or those of the last, partly filled
+  // round alone (whole > 0): 1965 x 7168 x 8192 has 448 tiles of 256 for 3 x 148, and the last four took as long
+  // as a full round (172 -> 149 us).
+  int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1, whole = 0;
   const int least = (a.k_blocks + 63) / 64;           // the token scales of a split fit their shared-memory block
   const bool can_split = workspace && (N & 3) == 0;
   long long best = -1;
-  for (int w : {swap ? bn : 256, swap ? 0 : 128}) {
+  for (int w : {swap ? bn : 256, swap ? 0 : 128, swap ? 0 : 64}) {
     if (w == 0 || (w == 256 && N % 256)) continue;
     const int n_tiles = (a.N + w - 1) / w;
-    const long long block = std::max(swap ? 14 : (w == 256 ? 28 : 18), a.m_tiles == 1 || swap ? (w == 256 ? 74 : 37) : 0);
+    const long long block = swap ? 37 : a.m_tiles == 1 ? (w == 256 ? 74 : w == 128 ? 37 : 28) : (w == 256 ? 60 : w == 128 ? 36 : 28);
     for (int s = least; s <= 16 * least && s <= a.k_blocks; ++s) {
       if (s > 1 && (!can_split || (size_t)s * T * N * 4 > workspace_bytes)) break;
       const long long rounds = ((long long)a.m_tiles * n_tiles * s + sms - 1) / sms;
       const long long cost = rounds * ((a.k_blocks + s - 1) / s * block + 100) + (s > 1 ? 250 + (long long)((double)s * T * N * 8 / 60000.0) : 0);
-      if (best < 0 || cost < best) { best = cost; bn = w; splits = s; }
+      if (best < 0 || cost < best) { best = cost; bn = w; splits = s; whole = 0; }
+    }
+    const long long tiles = (long long)a.m_tiles * n_tiles, first = tiles / sms * sms, tail = tiles - first;
+    if (swap || least > 1 || !can_split || first == 0) continue;
+    for (int s = 2; s <= 16 && s <= a.k_blocks && tail; ++s) {
+      const long long bytes = s * tail * F8_BM * w * 4;
+      if ((size_t)bytes > workspace_bytes) break;
+      const long long cost = first / sms * (a.k_blocks * block + 100) + (tail * s + sms - 1) / sms * ((a.k_blocks + s - 1) / s * block + 100) + 250 + bytes / 30000;
+      if (best < 0 || cost < best) { best = cost; bn = w; splits = s; whole = (int)first; }
     }
   }
   if (best < 0) throw std::runtime_error("linear_fp8_block: K above 8192 needs a split-K workspace");
@@ -385,14 +435,23 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   const CUtensorMap &ta = swap ? tw : tx, &tb = swap ? tx : tw;
   a.kb_per_split = (a.k_blocks + splits - 1) / splits;
   a.k_splits = (a.k_blocks + a.kb_per_split - 1) / a.kb_per_split;
+  a.whole = a.k_splits > 1 ? whole : a.m_tiles * a.n_tiles;
   a.ws = reinterpret_cast<float*>(workspace);
-  const int grid = std::min(a.m_tiles * a.n_tiles * a.k_splits, sms);
+  const int grid = std::min(a.whole + (a.m_tiles * a.n_tiles - a.whole) * a.k_splits, sms);
   switch (bn) {
-    case 16: launch_fp8<16>(ta, tb, a, grid, stream); break;
-    case 32: launch_fp8<32>(ta, tb, a, grid, stream); break;
-    case 64: launch_fp8<64>(ta, tb, a, grid, stream); break;
-    case 128: launch_fp8<128>(ta, tb, a, grid, stream); break;
-    default: launch_fp8<256>(ta, tb, a, grid, stream); break;
+    case 16: launch_fp8<16, true>(ta, tb, a, grid, stream); break;
+    case 32: launch_fp8<32, true>(ta, tb, a, grid, stream); break;
+    case 64:
+      if (swap) launch_fp8<64, true>(ta, tb, a, grid, stream);
+      else launch_fp8<64, false>(ta, tb, a, grid, stream);
+      break;
+    case 128: launch_fp8<128, false>(ta, tb, a, grid, stream); break;
+    default: launch_fp8<256, false>(ta, tb, a, grid, stream); break;
+  }
+  if (a.k_splits > 1 && a.whole > 0) {
+    const size_t n = (size_t)(a.m_tiles * a.n_tiles - a.whole) * F8_BM * bn;
+    launch_pdl(fp8_tail_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, a, bn);
+    return 2;
   }
   if (a.k_splits > 1) {
     const size_t n = (size_t)T * N;

@@ -49,7 +49,7 @@ def test_pairs_leave_their_sums_to_the_norm_and_the_activation(ops, T):
 
 
 @pytest.mark.parametrize("T,N,K", [(1, 128, 128), (17, 256, 1024), (64, 384, 8192), (65, 128, 256), (128, 7168, 8192), (129, 1280, 8192), (128, 256, 12288),
-                                   (300, 8192, 1024), (1965, 8192, 3584)])
+                                   (300, 8192, 1024), (513, 1280, 8192), (100, 8192, 384), (257, 512, 128), (1965, 1280, 8192), (2430, 2048, 1024), (1965, 8192, 3584)])
 def test_fp8_block(ops, T, N, K):
     from fllm_b200.ops.native import Fp8BlockLinear, quantize_weight_fp8_block
     x, bias = _rand((T, K), 1), _rand((N,), 3)
