@@ -70,8 +70,8 @@ struct W4Smem {
   static constexpr int kRawBytes = W4_BM * 128;
   static constexpr int kBStep = BN * W4_BK * 2;                // activations of one 64-value step
   static constexpr int kBBytes = 4 * kBStep;
-  static constexpr int kRStages = BN == 128 ? 4 : BN == 64 ? 6 : 8;
-  static constexpr int kBStages = BN == 128 ? 2 : BN == 64 ? 3 : BN == 32 ? 4 : 6;
+  static constexpr int kRStages = BN == 128 ? 4 : BN == 96 ? 5 : BN == 64 ? 6 : 8;
+  static constexpr int kBStages = BN >= 96 ? 2 : BN == 64 ? 3 : BN == 32 ? 4 : 6;
   // tensor memory: two accumulators, then kAStages slots of expanded weights
   static constexpr int kDCols = BN < 32 ? 32 : BN;
   static constexpr int kTmemCols = 512;
@@ -339,7 +339,14 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_cons
           if (kb - g + 4 < nkb) sc = load_scales(srow, kb + 4, nkb);
           else if (more) sc = load_scales(srow_next, g, it.nkb);
           uint32_t s2[4];
-          if (p.fmt == 0) {
+          if (p.fmt == 0 && p.f16) {                        // four e4m3 scales: two conversions, no table
+            uint32_t h01, h23;
+            asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, a;\n\tcvt.rn.f16x2.e4m3x2 %1, b;\n\t}" : "=r"(h01), "=r"(h23) : "r"(sraw));
+            s2[0] = __byte_perm(h01, 0, 0x1010);
+            s2[1] = __byte_perm(h01, 0, 0x3232);
+            s2[2] = __byte_perm(h23, 0, 0x1010);
+            s2[3] = __byte_perm(h23, 0, 0x3232);
+          } else if (p.fmt == 0) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) s2[i] = lut[(sraw >> (8 * i)) & 0xFF];
           } else if (p.fmt == 1) {
@@ -621,6 +628,7 @@ static void launch_w4_bn(int bn, const CUtensorMap& tr, const CUtensorMap& tb, c
     case 16: launch_w4<16>(tr, tb, a, items, s); break;
     case 32: launch_w4<32>(tr, tb, a, items, s); break;
     case 64: launch_w4<64>(tr, tb, a, items, s); break;
+    case 96: launch_w4<96>(tr, tb, a, items, s); break;
     default: launch_w4<128>(tr, tb, a, items, s); break;
   }
 }
@@ -638,7 +646,7 @@ int linear_w4a16(const void* x, long long ldx, const void* codes, const void* sc
   a.M = N; a.N = T; a.K = K; a.m_tiles = (N + W4_BM - 1) / W4_BM; a.k_blocks = K / W4_BK; a.fmt = fmt;
   a.ldc = ldy; a.out = reinterpret_cast<uint16_t*>(y); a.scales = reinterpret_cast<const uint8_t*>(scales);
   a.alpha = alpha; a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.status = status;
-  const int bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
+  const int bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 96 ? 96 : 128;
   // [.. partial sums ..][fp16 rows][row factors]
   const size_t rows_bytes = ((size_t)T * K * 2 + (size_t)T * 4 + 255) & ~(size_t)255;
   a.f16 = f16 && fmt != 2 && workspace && workspace_bytes >= rows_bytes + 256;
@@ -691,7 +699,7 @@ int moe_grouped_linear_w4(const void* xp, long long ldx, const void* codes_stack
   if (rows_cap <= 0 || max_tiles <= 0) return 0;
   if (K % 64 || n_out % 8 || (ldx & 7) || (ldy & 7)) throw std::runtime_error("moe_grouped_linear_w4: K % 64, n_out % 8 and 16-byte rows required");
   if (fmt < 0 || fmt > 2) throw std::runtime_error("moe_grouped_linear_w4: fmt must be 0, 1 or 2");
-  if (bn != 16 && bn != 32 && bn != 64 && bn != 128) throw std::runtime_error("moe_grouped_linear_w4: token tile must be 16, 32, 64 or 128");
+  if (bn != 16 && bn != 32 && bn != 64 && bn != 96 && bn != 128) throw std::runtime_error("moe_grouped_linear_w4: token tile must be 16, 32, 64, 96 or 128");
   W4Args a{};
   a.M = n_out; a.N = rows_cap; a.K = K; a.m_tiles = (n_out + W4_BM - 1) / W4_BM; a.k_blocks = K / W4_BK; a.fmt = fmt;
   a.ldc = ldy; a.out = reinterpret_cast<uint16_t*>(y); a.scales = reinterpret_cast<const uint8_t*>(scales_stack);

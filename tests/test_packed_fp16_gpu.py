@@ -60,7 +60,7 @@ def test_rows_keep_every_value(ops, K):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp4"])
-@pytest.mark.parametrize("T,N,K", [(5, 128, 64), (17, 136, 192), (64, 256, 1088), (65, 1000, 320), (128, 40960, 256), (128, 512, 12288)])
+@pytest.mark.parametrize("T,N,K", [(5, 128, 64), (17, 136, 192), (64, 256, 1088), (65, 1000, 320), (96, 264, 3072), (97, 264, 832), (128, 40960, 256), (128, 512, 12288)])
 def test_dense_against_64_bits(ops, fmt, T, N, K):
     """One rounding to bf16 (2^-9 of a value at most, 0.17 % in the mean square) is all that a correct product is off."""
     x, q = _rand((T, K), 1).cuda(), Fp4Weight.from_dense(_rand((N, K), 2, 0.05).cuda(), fmt)
@@ -82,7 +82,7 @@ def test_scales_beyond_fp16_take_the_bf16_form(ops):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("bn", [16, 32, 64, 128])
+@pytest.mark.parametrize("bn", [16, 32, 64, 96, 128])
 @pytest.mark.parametrize("n,k", [(32, 64), (304, 192), (5760, 2880)])
 @pytest.mark.parametrize("glu", [False, True])
 def test_grouped(ops, bn, n, k, glu):
