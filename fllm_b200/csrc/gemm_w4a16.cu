@@ -181,7 +181,9 @@ __device__ __forceinline__ W4Item w4_item(const W4Args& p, int w) {
   return it;
 }
 
-template <int BN>
+// F16: activations and expanded weights are fp16 (formats 0 and 1). A template parameter: tested at every word of codes, the branches
+// were a tenth of the expanding warps' time.
+template <int BN, bool F16>
 __global__ void __launch_bounds__(W4Smem<BN>::kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_constant__ CUtensorMap tma_b, const W4Args p) {
   using S = W4Smem<BN>;
@@ -218,7 +220,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_cons
     const int i = threadIdx.x - 64;
     const float f = scale_to_float((uint8_t)i, p.fmt);
     const __half2 h = __floats2half2_rn(f, f);
-    lut[i] = p.f16 ? *reinterpret_cast<const uint32_t*>(&h) : pack_bf16x2(f, f);
+    lut[i] = F16 ? *reinterpret_cast<const uint32_t*>(&h) : pack_bf16x2(f, f);
   }
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tma_raw); tma_prefetch_desc(&tma_b); }
   if (warp == 1) { tmem_alloc(tmem_slot, S::kTmemCols); tmem_relinquish(); }
@@ -267,7 +269,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    const uint32_t idesc = p.f16 ? make_idesc(W4_BM, BN, 0, 0) : make_idesc(W4_BM, BN, 1, 1);
+    const uint32_t idesc = F16 ? make_idesc(W4_BM, BN, 0, 0) : make_idesc(W4_BM, BN, 1, 1);
     const uint64_t db0 = make_smem_desc_sw128(smem_u32(sB));
     int bs = 0, as = 0, acc = 0;
     uint32_t bphase = 0, aphase = 0, accphase = 0;
@@ -339,7 +341,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_cons
           if (kb - g + 4 < nkb) sc = load_scales(srow, kb + 4, nkb);
           else if (more) sc = load_scales(srow_next, g, it.nkb);
           uint32_t s2[4];
-          if (p.fmt == 0 && p.f16) {                        // four e4m3 scales: two conversions, no table
+          if (p.fmt == 0 && F16) {                        // four e4m3 scales: two conversions, no table
             uint32_t h01, h23;
             asm("{\n\t.reg .b16 a, b;\n\tmov.b32 {a, b}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, a;\n\tcvt.rn.f16x2.e4m3x2 %1, b;\n\t}" : "=r"(h01), "=r"(h23) : "r"(sraw));
             s2[0] = __byte_perm(h01, 0, 0x1010);
@@ -372,7 +374,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_cons
 #pragma unroll
               for (int c = 0; c < 4; ++c) {                 // 8 codes -> 4 cells of two values each
                 uint32_t o4[4];
-                if (p.f16) e2m1x8_to_f16(words[4 * h + c], s2[2 * h + (c >> 1)], o4);
+                if (F16) e2m1x8_to_f16(words[4 * h + c], s2[2 * h + (c >> 1)], o4);
                 else if (p.fmt == 2) int4x8_to_bf16(words[4 * h + c], s2[2 * h], s2[2 * h + 1], o4);
                 else e2m1x8_to_bf16(words[4 * h + c], s2[2 * h + (c >> 1)], o4);
 #pragma unroll
@@ -610,17 +612,23 @@ void w4_dequant_bf16(const void* codes, const void* scales, int fmt, float alpha
   cuda_check(cudaGetLastError(), "w4_dequant_kernel");
 }
 
-template <int BN>
-static void launch_w4(const CUtensorMap& tr, const CUtensorMap& tb, const W4Args& a, int items, cudaStream_t s) {
+template <int BN, bool F16>
+static void launch_w4_form(const CUtensorMap& tr, const CUtensorMap& tb, const W4Args& a, int items, cudaStream_t s) {
   using S = W4Smem<BN>;
   static bool configured[kMaxDevices] = {};
   if (first_call_on_device(configured)) {
-    cuda_check(cudaFuncSetAttribute(gemm_w4a16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
+    cuda_check(cudaFuncSetAttribute(gemm_w4a16_kernel<BN, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
                "cudaFuncSetAttribute(gemm_w4a16_kernel)");
-    cuda_check(cudaFuncSetAttribute(gemm_w4a16_kernel<BN>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    cuda_check(cudaFuncSetAttribute(gemm_w4a16_kernel<BN, F16>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                     cudaSharedmemCarveoutMaxShared), "cudaFuncSetAttribute(carveout)");
   }
-  launch_pdl(gemm_w4a16_kernel<BN>, dim3(std::min(items, sm_count())), dim3(S::kThreads), S::kTotal, s, tr, tb, a);
+  launch_pdl(gemm_w4a16_kernel<BN, F16>, dim3(std::min(items, sm_count())), dim3(S::kThreads), S::kTotal, s, tr, tb, a);
+}
+
+template <int BN>
+static void launch_w4(const CUtensorMap& tr, const CUtensorMap& tb, const W4Args& a, int items, cudaStream_t s) {
+  if (a.f16) launch_w4_form<BN, true>(tr, tb, a, items, s);
+  else launch_w4_form<BN, false>(tr, tb, a, items, s);
 }
 
 static void launch_w4_bn(int bn, const CUtensorMap& tr, const CUtensorMap& tb, const W4Args& a, int items, cudaStream_t s) {
