@@ -189,6 +189,83 @@ __device__ __forceinline__ void softmax_tile(const FaTmemParams& p, uint32_t t_s
   else softmax_tile_impl<D, false, false, false>(p, t_s, t_o, tok0, lim, beg, have_o, m_used, l);
 }
 
+// The same with a row's 128 scores held in registers between the two passes, for warps that have 208 of them. The first 64 probabilities
+// are handed over (`p_half`) before the others are computed.
+template <int D, bool full, bool capped, bool windowed>
+__device__ __forceinline__ void softmax_row_impl(const FaTmemParams& p, uint32_t t_s, uint32_t t_o, int tok0, int lim, int beg, bool have_o,
+                                                 uint64_t* p_half, float& m_used, float& l) {
+  const float cap_in = capped ? p.scale / p.softcap : 0.f;
+  const float scale = capped ? p.softcap * kLog2eT : p.scale_log2;
+  uint32_t s[4][32];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_s + 32 * c, s[c]);
+  tmem_ld_wait();
+  const int hi = lim - tok0, lo = beg - tok0;
+  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int i = 0; i < 128; ++i) {
+    float a = __uint_as_float(s[i >> 5][i & 31]);
+    if (capped) { a = tanhf(a * cap_in); s[i >> 5][i & 31] = __float_as_uint(a); }
+    if (!full && (i >= hi || (windowed && i < lo))) a = -INFINITY;
+    mx[i & 3] = fmaxf(mx[i & 3], a);
+  }
+  // the scale is positive, so it commutes with the maximum
+  const float m = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;
+  const bool grow = m > m_used + kLazyRescale || (m_used == -INFINITY && m > -INFINITY);
+  if (__any_sync(0xffffffffu, grow)) {
+    const float m_new = fmaxf(m_used, m);
+    const float corr = m_new == -INFINITY ? 1.f : ex2(m_used - m_new);     // m_used = -inf gives 0
+    m_used = m_new;
+    l *= corr;
+    if (have_o) {
+#pragma unroll 1
+      for (int c = 0; c < D / 16; ++c) {
+        uint32_t o[16];
+        tmem_ld_32x16(t_o + 16 * c, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * corr);
+        tmem_st_32x16(t_o + 16 * c, o);
+      }
+    }
+  }
+  const float m_ref = m_used == -INFINITY ? 0.f : m_used;
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t w[16];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const int i = 32 * c + j;
+      float a = ex2(fmaf(__uint_as_float(s[c][j]), scale, -m_ref)), b = ex2(fmaf(__uint_as_float(s[c][j + 1]), scale, -m_ref));
+      if (!full) {
+        if (i >= hi || (windowed && i < lo)) a = 0.f;
+        if (i + 1 >= hi || (windowed && i + 1 < lo)) b = 0.f;
+      }
+      sum[j & 2] += a; sum[(j & 2) + 1] += b;
+      w[j >> 1] = pack_bf16x2(a, b);
+    }
+    tmem_st_32x16(t_s + 16 * c, w);
+    if (c == 1) {
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) mbar_arrive(p_half);
+    }
+  }
+  l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+  tmem_st_wait();
+}
+
+template <int D>
+__device__ __forceinline__ void softmax_row(const FaTmemParams& p, uint32_t t_s, uint32_t t_o, int tok0, int lim, int beg, bool full, bool have_o,
+                                            uint64_t* p_half, float& m_used, float& l) {
+  if (p.softcap > 0.f) softmax_row_impl<D, false, true, true>(p, t_s, t_o, tok0, lim, beg, have_o, p_half, m_used, l);
+  else if (full) softmax_row_impl<D, true, false, false>(p, t_s, t_o, tok0, lim, beg, have_o, p_half, m_used, l);
+  else if (p.window > 0) softmax_row_impl<D, false, false, true>(p, t_s, t_o, tok0, lim, beg, have_o, p_half, m_used, l);
+  else softmax_row_impl<D, false, false, false>(p, t_s, t_o, tok0, lim, beg, have_o, p_half, m_used, l);
+}
+
 // Final normalisation (with the head's sink, if any) and store of one row of O. The tensor memory loads are
 // warp-wide, so rows past the tile's last query take part and only skip the store.
 template <int D>
@@ -286,6 +363,7 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                     // decode rows of a mixed batch, the weights of the next product (not before the allocation)
   const uint32_t t_s = tmem_base;            // S, later P in its first 64 columns
   const uint32_t t_o = tmem_base + 128;
 
@@ -390,9 +468,15 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
 
 // The same pipeline with two 128-row query tiles per CTA sharing every K/V tile (half the K/V traffic per
 // FLOP, which is what bounds the one-tile kernel: its 64 KB per 8.4 MFLOP tile saturates L2 first). Twelve warps:
-// three producers, issuer, and one softmax group of four warps per query tile. The issuer interleaves the two tiles
+// one softmax group of four warps per query tile, three producers, issuer. The issuer interleaves the two tiles
 // (PV0, next S0, PV1, next S1) so that one group's softmax runs under the other tile's MMAs; K and V are
 // double buffered. Tensor memory: S0 S1 O0 O1 = 512 columns, one CTA per SM.
+//
+// What bounds it: the chain of a group. A tile's softmax took 2620 clocks and its PV and next S 1024, of which the other group's chain
+// hides about half; tensor pipe and exponentials are each busy 47 % of the time. So a row's scores stay in registers (one pass over
+// tensor memory instead of two; the warps that need no registers leave theirs), and PV of the first 64 tokens runs while the others'
+// exponentials are computed: 2017 tokens at 8161, 32 query and 8 key heads of 128: 313 -> 293 us. (Two S buffers of 64 tokens per tile
+// took 355: products of 64 columns read Q twice as often.)
 constexpr int kThreadsT2 = 384;
 template <int D> constexpr int smem_two() { return 6 * tile_bytes<D>() + 256 + 1024; }
 
@@ -414,7 +498,8 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   uint64_t* s_full = bars + 8;                 // [2] by query tile
   uint64_t* p_ready = bars + 10;
   uint64_t* o_done = bars + 12;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* p_half = bars + 13;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
@@ -440,14 +525,14 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&k_full[i], D / 64); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
-      mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4);
+      mbar_init(&s_full[i], 1); mbar_init(&p_half[i], 4); mbar_init(&p_ready[i], 4);
     }
     mbar_init(o_done, 1);
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 0 && lane == 0) { tma_prefetch_desc(&tma_k); tma_prefetch_desc(&tma_v); }
-  if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+  if (warp == 8 && lane == 0) { tma_prefetch_desc(&tma_k); tma_prefetch_desc(&tma_v); }
+  if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   for (int i = threadIdx.x; i < 2 * kRowsT * (D / 8); i += kThreadsT2) {
     const int r = i / (D / 8), c = i % (D / 8);
     uint4 v = make_uint4(0, 0, 0, 0);
@@ -463,105 +548,119 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                     // decode rows of a mixed batch, the weights of the next product (not before the allocation)
 
-  if (warp == 0 || warp >= 10) {
-    // Three warps ask for the pages, one box of theirs after the other: warp 0 for the first 64 columns of K, warp 10 for the
-    // others, warp 11 for V. (One warp for all 32 boxes of a tile needed longer than the products of the tile.)
-    const bool is_v = warp == 11;
-    const int half = warp == 10 ? 1 : 0;
-    uint64_t *full = is_v ? v_full : k_full, *empty = is_v ? v_empty : k_empty;
-    const int* table = p.block_tables + (size_t)seq * p.max_blocks;
-    const int last_page = (kv_len + kPageT - 1) / kPageT - 1;
-    int rows[kTileT / kPageT], nxt[kTileT / kPageT];
-#pragma unroll
-    for (int pg = 0; pg < kTileT / kPageT; ++pg)
-      nxt[pg] = table[min(tile_lo * (kTileT / kPageT) + pg, last_page)];
-    for (int it = 0; it < n_tiles && (half == 0 || D == 128); ++it) {
-      const int b = it & 1;
-      const int page1 = (tile_lo + it + 1) * (kTileT / kPageT);
-#pragma unroll
-      for (int pg = 0; pg < kTileT / kPageT; ++pg) {
-        rows[pg] = (nxt[pg] * p.hkv + kvh) * kPageT;
-        nxt[pg] = table[min(page1 + pg, last_page)];
-      }
-      if (it >= 2 && !mbar_wait_warp(&empty[b], ((it >> 1) - 1) & 1, abort_flag)) break;      // phase of the stage's previous use
-      if (elect_one()) {
-        if (is_v) {
-          mbar_expect_tx(&full[b], TB);
-#pragma unroll
-          for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_3d(sv + b * TB + pg * (D / 64) * 2048, &tma_v, &full[b], 0, rows[pg], 0);
-        } else {
-          mbar_expect_tx(&full[b], kHalfBytes);
-#pragma unroll
-          for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_2d(sk + b * TB + half * kHalfBytes + pg * 2048, &tma_k, &full[b], 64 * half, rows[pg]);
+  // The block was launched with 168 registers a thread: 256 x 208 + 128 x 88 = 384 x 168.
+  if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
+    if (warp != 9) {
+      // Three warps ask for the pages, one box of theirs after the other: warp 8 for the first 64 columns of K, warp 10 for the
+      // others, warp 11 for V. (One warp for all 32 boxes of a tile needed longer than the products of the tile.)
+      const bool is_v = warp == 11;
+      const int half = warp == 10 ? 1 : 0;
+      uint64_t *full = is_v ? v_full : k_full, *empty = is_v ? v_empty : k_empty;
+      const int* table = p.block_tables + (size_t)seq * p.max_blocks;
+      const int last_page = (kv_len + kPageT - 1) / kPageT - 1;
+      int rows[kTileT / kPageT], nxt[kTileT / kPageT];
+  #pragma unroll
+      for (int pg = 0; pg < kTileT / kPageT; ++pg)
+        nxt[pg] = table[min(tile_lo * (kTileT / kPageT) + pg, last_page)];
+      for (int it = 0; it < n_tiles && (half == 0 || D == 128); ++it) {
+        const int b = it & 1;
+        const int page1 = (tile_lo + it + 1) * (kTileT / kPageT);
+  #pragma unroll
+        for (int pg = 0; pg < kTileT / kPageT; ++pg) {
+          rows[pg] = (nxt[pg] * p.hkv + kvh) * kPageT;
+          nxt[pg] = table[min(page1 + pg, last_page)];
         }
-      }
-      __syncwarp();
-    }
-  } else if (warp == 1) {
-    constexpr uint32_t idesc_s = make_idesc(128, 128, 1, 1);
-    constexpr uint32_t idesc_pv = make_idesc(128, D, 1, 1) | (1u << 16);     // B is MN-major
-    const uint64_t dq = make_smem_desc_sw128(smem_u32(sq)), dk = make_smem_desc_sw128(smem_u32(sk));
-    const uint64_t dv = smem_desc_sw128_1k(smem_u32(sv), D == 128 ? 2048 : 1024);     // V lands by pages: [page][D / 64][16][64]
-    auto issue_s = [&](int g, int stage) {
-#pragma unroll
-      for (int k = 0; k < D / 16; ++k) {
-        const uint32_t off = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
-        tc_mma_bf16(tmem_base + 128 * g, dq + g * (TB >> 4) + off, dk + (uint64_t)(stage * (TB >> 4)) + off, idesc_s, k > 0);
-      }
-    };
-    auto issue_pv = [&](int g, int stage, bool first) {
-      const uint32_t t_p = tmem_base + 128 * g, t_o = tmem_base + 256 + 128 * g;
-#pragma unroll
-      for (int k = 0; k < kTileT / 16; ++k)
-        tc_mma_bf16_ts(t_o, t_p + 8 * k, dv + (uint64_t)(stage * (TB >> 4)) + k * (D / 64) * (2048 >> 4), idesc_pv, (!first || k > 0) ? 1u : 0u);
-    };
-    bool ok = mbar_wait_warp(&k_full[0], 0, abort_flag);
-    if (ok) {
-      tc_fence_after_sync();
-      if (elect_one()) {
-        issue_s(0, 0);
-        tc_commit(&s_full[0]);
-        issue_s(1, 0);
-        tc_commit(&s_full[1]);
-        tc_commit(&k_empty[0]);
-      }
-      __syncwarp();
-    }
-    for (int it = 0; ok && it < n_tiles; ++it) {
-      const int b = it & 1, nb = b ^ 1;
-      const uint32_t ph = (it >> 1) & 1, nph = ((it + 1) >> 1) & 1;
-      const bool more = it + 1 < n_tiles;
-      if (!mbar_wait_warp(&p_ready[0], it & 1, abort_flag) || !mbar_wait_warp(&v_full[b], ph, abort_flag)) break;
-      tc_fence_after_sync();
-      if (elect_one()) issue_pv(0, b, it == 0);
-      __syncwarp();
-      if (more) {
-        if (!mbar_wait_warp(&k_full[nb], nph, abort_flag)) break;
-        tc_fence_after_sync();
+        if (it >= 2 && !mbar_wait_warp(&empty[b], ((it >> 1) - 1) & 1, abort_flag)) break;      // phase of the stage's previous use
         if (elect_one()) {
-          issue_s(0, nb);
-          tc_commit(&s_full[0]);
+          if (is_v) {
+            mbar_expect_tx(&full[b], TB);
+  #pragma unroll
+            for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_3d(sv + b * TB + pg * (D / 64) * 2048, &tma_v, &full[b], 0, rows[pg], 0);
+          } else {
+            mbar_expect_tx(&full[b], kHalfBytes);
+  #pragma unroll
+            for (int pg = 0; pg < kTileT / kPageT; ++pg) tma_load_2d(sk + b * TB + half * kHalfBytes + pg * 2048, &tma_k, &full[b], 64 * half, rows[pg]);
+          }
         }
         __syncwarp();
       }
-      if (!mbar_wait_warp(&p_ready[1], it & 1, abort_flag)) break;
-      tc_fence_after_sync();
-      if (elect_one()) {
-        issue_pv(1, b, it == 0);
-        tc_commit(&v_empty[b]);
-        if (more) {
-          issue_s(1, nb);
-          tc_commit(&s_full[1]);
-          tc_commit(&k_empty[nb]);
-        } else {
-          tc_commit(o_done);
+    } else {
+      constexpr uint32_t idesc_s = make_idesc(128, 128, 1, 1);
+      constexpr uint32_t idesc_pv = make_idesc(128, D, 1, 1) | (1u << 16);     // B is MN-major
+      const uint64_t dq = make_smem_desc_sw128(smem_u32(sq)), dk = make_smem_desc_sw128(smem_u32(sk));
+      const uint64_t dv = smem_desc_sw128_1k(smem_u32(sv), D == 128 ? 2048 : 1024);     // V lands by pages: [page][D / 64][16][64]
+      auto issue_s = [&](int g, int stage) {
+  #pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint32_t off = ((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
+          tc_mma_bf16(tmem_base + 128 * g, dq + g * (TB >> 4) + off, dk + (uint64_t)(stage * (TB >> 4)) + off, idesc_s, k > 0);
         }
+      };
+      auto issue_pv = [&](int g, int stage, bool first, int part) {            // over tokens [64 part, 64 part + 64)
+        const uint32_t t_p = tmem_base + 128 * g, t_o = tmem_base + 256 + 128 * g;
+  #pragma unroll
+        for (int k = 4 * part; k < 4 * part + 4; ++k)
+          tc_mma_bf16_ts(t_o, t_p + 8 * k, dv + (uint64_t)(stage * (TB >> 4)) + k * (D / 64) * (2048 >> 4), idesc_pv, (!first || k > 0) ? 1u : 0u);
+      };
+      bool ok = mbar_wait_warp(&k_full[0], 0, abort_flag);
+      if (ok) {
+        tc_fence_after_sync();
+        if (elect_one()) {
+          issue_s(0, 0);
+          tc_commit(&s_full[0]);
+          issue_s(1, 0);
+          tc_commit(&s_full[1]);
+          tc_commit(&k_empty[0]);
+        }
+        __syncwarp();
       }
-      __syncwarp();
+      for (int it = 0; ok && it < n_tiles; ++it) {
+        const int b = it & 1, nb = b ^ 1;
+        const uint32_t ph = (it >> 1) & 1, nph = ((it + 1) >> 1) & 1;
+        const bool more = it + 1 < n_tiles;
+        if (!mbar_wait_warp(&p_half[0], it & 1, abort_flag) || !mbar_wait_warp(&v_full[b], ph, abort_flag)) break;
+        tc_fence_after_sync();
+        if (elect_one()) issue_pv(0, b, it == 0, 0);
+        __syncwarp();
+        if (!mbar_wait_warp(&p_ready[0], it & 1, abort_flag)) break;
+        tc_fence_after_sync();
+        if (elect_one()) issue_pv(0, b, it == 0, 1);
+        __syncwarp();
+        if (more) {
+          if (!mbar_wait_warp(&k_full[nb], nph, abort_flag)) break;
+          tc_fence_after_sync();
+          if (elect_one()) {
+            issue_s(0, nb);
+            tc_commit(&s_full[0]);
+          }
+          __syncwarp();
+        }
+        if (!mbar_wait_warp(&p_half[1], it & 1, abort_flag)) break;
+        tc_fence_after_sync();
+        if (elect_one()) issue_pv(1, b, it == 0, 0);
+        __syncwarp();
+        if (!mbar_wait_warp(&p_ready[1], it & 1, abort_flag)) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          issue_pv(1, b, it == 0, 1);
+          tc_commit(&v_empty[b]);
+          if (more) {
+            issue_s(1, nb);
+            tc_commit(&s_full[1]);
+            tc_commit(&k_empty[nb]);
+          } else {
+            tc_commit(o_done);
+          }
+        }
+        __syncwarp();
+      }
     }
-  } else {                                              // warps 2 - 9
-    const int g = (warp - 2) >> 2;                      // query tile of this softmax group
+  } else {                                              // warps 0 - 7
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
+    const int g = warp >> 2;                            // query tile of this softmax group
     const int quarter = warp & 3;
     const int r = g * kRowsT + quarter * 32 + lane;     // packed row within the CTA
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
@@ -580,7 +679,7 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
       if (!mbar_wait(&s_full[g], it & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       const bool full = p.window == 0 && tok0 + kTileT <= (p.bidir ? kv_len : group_first + 1) && group_whole;
-      softmax_tile<D>(p, t_s, t_o, tok0, lim, beg, full, it > 0, m_used, l);
+      softmax_row<D>(p, t_s, t_o, tok0, lim, beg, full, it > 0, &p_half[g], m_used, l);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_ready[g]);
@@ -593,7 +692,7 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   }
   tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
+  if (warp == 9) { tc_fence_after_sync(); tmem_dealloc(tmem_base, 512); }
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicCAS(p.status, FLLM_OK, FLLM_ERR_MBAR_TIMEOUT);
 }
 

@@ -125,3 +125,40 @@ def test_given_steps_queue_without_waiting():
     for a, b in zip(alone + alone[len(prompts):][::-1], queued):
         assert torch.equal(a, b.cpu())
     eng.close()
+
+
+@pytest.mark.parametrize("D,hq,hkv,window", [(128, 32, 8, 0), (64, 32, 8, 0), (128, 32, 8, 70)])
+@pytest.mark.parametrize("kv", [(320, 257, 65, 64), (333, 300, 129, 1), (449, 448, 447, 385)])
+def test_prompt_attention_rescales_between_halves(ops, D, hq, hkv, window, kv):
+    """Scores that grow along the sequence move the row maximum by more than 2^8 in every half tile of 64 tokens, the last of which may
+    be the first half of a tile. Probabilities and results are rounded to bf16 once each: 2^-9 + 2^-9."""
+    from types import SimpleNamespace
+    G, n = hq // hkv, len(kv)
+    starts = [0]
+    for x in kv:
+        starts.append(starts[-1] + x)
+    per = [(x + 15) // 16 for x in kv]
+    tables = torch.zeros(n, max(per), dtype=torch.int32, device="cuda")
+    order = torch.randperm(sum(per), generator=torch.Generator().manual_seed(1)).int().cuda()
+    kc, vc = torch.zeros(sum(per), hkv, 16, D, dtype=torch.bfloat16, device="cuda"), _rand((sum(per), hkv, 16, D), 2)
+    q = (_rand((starts[-1], hq * D), 3, 0.2).float() + 1).to(torch.bfloat16)
+    ref, o = [], 0
+    for i, x in enumerate(kv):
+        blocks = order[o:o + per[i]]
+        o += per[i]
+        tables[i, :per[i]] = blocks
+        k = _rand((per[i] * 16, hkv, D), 4 + i, 0.2).float() + (torch.arange(per[i] * 16, device="cuda") / 8 * D ** -0.5)[:, None, None]
+        kc[blocks.long()] = k.to(torch.bfloat16).view(per[i], 16, hkv, D).transpose(1, 2)
+        k, v = (c[blocks.long()].double().transpose(1, 2).reshape(-1, hkv, D)[:x].repeat_interleave(G, 1) for c in (kc, vc))
+        s = torch.einsum("qhd,khd->hqk", q[starts[i]:starts[i + 1]].double().view(x, hq, D), k) * D ** -0.5
+        d = torch.arange(x, device="cuda")[:, None] - torch.arange(x, device="cuda")[None, :]
+        s = s.masked_fill((d < 0) | ((d >= window) if window else (d < 0)), float("-inf"))
+        ref.append(torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v).reshape(x, hq * D))
+    i32 = dict(dtype=torch.int32, device="cuda")
+    rows = torch.tensor([i for i, x in enumerate(kv) for _ in range(x)], **i32)
+    pos = torch.tensor([j for x in kv for j in range(x)], **i32)
+    meta = SimpleNamespace(q_starts=torch.tensor(starts, **i32), seq_lens=torch.tensor(kv, **i32), num_seqs=n, max_q_len=max(kv),
+                           min_q_len=min(kv), max_kv_len=max(kv))
+    y = ops.attention(q, kc, vc, tables, rows, pos, hq, hkv, D, D ** -0.5, window, None, 0.0, meta=meta)
+    assert _rel(y, torch.cat(ref)) < 2 ** -8
+    assert ops.check_status() == 0
