@@ -82,19 +82,21 @@ def dequantize_fp4(codes: torch.Tensor, scales: torch.Tensor, fmt: int, alpha: f
 
 def fp16_form(codes: torch.Tensor, scales: torch.Tensor, fmt: int) -> bool:
     """Whether every value of a packed matrix is exact in fp16: NVFP4 always; MXFP4 when the scale byte of every block that holds
-    something else than zeros lies in [104, 140] (0.5 x 2^-23 .. 6 x 2^13; scale 0 counts as a factor of 0). Looked at once, when the
-    weight is laid out: the packed GEMM then multiplies fp16 values, otherwise bf16 ones."""
+    something else than zeros lies in [104, 140] (0.5 x 2^-23 .. 6 x 2^13; scale 0 counts as a factor of 0), and that of a block of
+    zeros below 143: 2^16 and above are infinite in fp16, and zero times that is not a number. Looked at once, when the weight is
+    laid out: the packed GEMM then multiplies fp16 values, otherwise bf16 ones."""
     if fmt == NVFP4 or scales.numel() == 0:
         return True
     out = (scales > 140) | ((scales < 104) & (scales != 0))
     if not bool(out.any()):
         return True
-    rows = (codes.reshape(-1, 16)[out.reshape(-1)] & 0x77) != 0
-    return not bool(rows.any())
+    blocks = (codes.reshape(-1, 16)[out.reshape(-1)] & 0x77) != 0
+    return not bool(blocks.any()) and not bool((scales > 142).any())
 
 
 class Fp4Weight:
-    """A [N, K] matrix held as packed FP4 codes + block scales (+ tensor scale)."""
+    """A [N, K] matrix held as packed FP4 codes + block scales (+ tensor scale). Which form multiplies it is decided from the scales
+    here: to change them, make another weight (scales rewritten in place beyond `fp16_form` would overflow)."""
 
     def __init__(self, codes: torch.Tensor, scales: torch.Tensor, fmt: int, alpha: float = 1.0):
         self.codes, self.scales, self.fmt, self.alpha = codes, scales, int(fmt), float(alpha)
@@ -139,7 +141,7 @@ class Fp4Weight:
 class Fp4ExpertStack:
     """The matrices of several experts held packed: codes [E, N, K/2], scales [E, N, K/block] (bytes).
     ``moe_ffn`` hands it to the grouped packed GEMM; gpt-oss checkpoints store their experts this way
-    (MXFP4), so the bytes go from the file to the tensor core unexpanded."""
+    (MXFP4), so the bytes go from the file to the tensor core unexpanded. As with ``Fp4Weight``, other scales are another stack."""
 
     def __init__(self, codes: torch.Tensor, scales: torch.Tensor, fmt: int, alpha: float = 1.0):
         self.codes, self.scales, self.fmt, self.alpha = codes.contiguous(), scales.contiguous(), int(fmt), float(alpha)

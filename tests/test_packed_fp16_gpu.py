@@ -32,6 +32,28 @@ def test_which_weights_are_exact_in_fp16():
         assert fp16_form(codes, scales, 1) == ok
 
 
+def test_zeros_under_a_scale_that_fp16_does_not_hold():
+    """Scales from 2^16 on (byte 143) are infinite in fp16, and zero times that is not a number."""
+    codes = torch.full((2, 32), 0x77, dtype=torch.uint8)
+    codes[1, 16:] = 0x80
+    scales = torch.full((2, 2), 120, dtype=torch.uint8)
+    for s, ok in ((141, True), (142, True), (143, False), (200, False), (255, False)):
+        scales[1, 1] = s
+        assert fp16_form(codes, scales, 1) == ok
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [142, 143, 200])
+def test_blocks_of_zeros_under_large_scales(ops, scale):
+    q = Fp4Weight.from_dense(_rand((256, 512), 2, 0.05).cuda(), "mxfp4")
+    q.codes[7, 32:48], q.scales[7, 2] = 0, scale
+    q = Fp4Weight(q.codes, q.scales, 1)
+    x = _rand((24, 512), 1).cuda()
+    assert _rel(ops.linear(x, q), x.double() @ dequantize_fp4(q.codes, q.scales, 1).double().t()) < 2.5e-3
+    stack = Fp4ExpertStack(q.codes[None], q.scales[None], 1)
+    assert stack.f16 == q.f16 == (scale < 143)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", [64, 320, 2880, 28672])
 def test_rows_keep_every_value(ops, K):
