@@ -133,7 +133,7 @@ int linear_mx(const void* xq, const void* sfb, const void* wq, const void* sfa, 
 void quant_fp8_1x128(const void* x, long long ldx, void* xq, float* sx, int tokens, int K, cudaStream_t s);
 int linear_fp8_block(const void* xq, const float* sx, const void* wq, const float* sw, const void* bias, void* y,
                      long long ldy, int T, int N, int K, int* status, cudaStream_t stream, void* workspace = nullptr,
-                     size_t workspace_bytes = 0);   // workspace: fp32 split-K partials (few tiles, or K above 8192)
+                     size_t workspace_bytes = 0);   // workspace: fp32 split-K partials (few tiles; up to 64 tokens need it for K above 8192)
 
 void widen_rows(const void* x, long long ldx, float* out, int rows, int cols, cudaStream_t s);   // bf16 rows -> fp32
 

@@ -406,14 +406,14 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   // round alone (whole > 0): 1965 x 7168 x 8192 has 448 tiles of 256 for 3 x 148, and the last four took as long
   // as a full round (172 -> 149 us).
   int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1, whole = 0;
-  const int least = (a.k_blocks + 63) / 64;           // the token scales of a split fit their shared-memory block
+  const int deep = (a.k_blocks + 63) / 64, least = swap ? deep : 1;   // swap-AB: the token scales of a split fit their shared-memory block
   const bool can_split = workspace && (N & 3) == 0;
   long long best = -1;
   for (int w : {swap ? bn : 256, swap ? 0 : 128, swap ? 0 : 64}) {
     if (w == 0 || (w == 256 && N % 256)) continue;
     const int n_tiles = (a.N + w - 1) / w;
     const long long block = swap ? 37 : a.m_tiles == 1 ? (w == 256 ? 74 : w == 128 ? 37 : 28) : (w == 256 ? 60 : w == 128 ? 36 : 28);
-    for (int s = least; s <= 16 * least && s <= a.k_blocks; ++s) {
+    for (int s = least; s <= 16 * deep && s <= a.k_blocks; ++s) {
       if (s > 1 && (!can_split || (size_t)s * T * N * 4 > workspace_bytes)) break;
       const long long rounds = ((long long)a.m_tiles * n_tiles * s + sms - 1) / sms;
       const long long cost = rounds * ((a.k_blocks + s - 1) / s * block + 100) + (s > 1 ? 250 + (long long)((double)s * T * N * 8 / 60000.0) : 0);

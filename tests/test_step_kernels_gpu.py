@@ -69,6 +69,24 @@ def test_fp8_block(ops, T, N, K):
     assert ops.check_status() == 0
 
 
+@pytest.mark.parametrize("T,N,K,room", [(2048, 8192, 14336, None), (800, 8192, 28672, None), (65, 256, 8320, 0), (300, 384, 12288, 0), (257, 256, 32768, 0)])
+def test_fp8_block_of_many_tokens_needs_no_room_for_deep_sums(ops, T, N, K, room):
+    """More than 64 tokens read their scales from global memory: K is not limited by what a workspace holds."""
+    from fllm_b200.ops.native import quantize_weight_fp8_block
+    x = _rand((T, K), 1)
+    wq, sw = quantize_weight_fp8_block(_rand((N, K), 2, 0.05))
+    xq, sx = torch.empty(T, K, dtype=torch.uint8, device="cuda"), torch.empty(T, K // 128, device="cuda")
+    ops.k.quant_fp8_1x128(x, xq, sx)
+    y = torch.empty(T, N, dtype=torch.bfloat16, device="cuda")
+    ops.k.linear_fp8_block(xq, sx, wq, sw, None, y, ops.status, ops.workspace if room is None else None)
+    xd = (xq.view(torch.float8_e4m3fn).double().view(T, K // 128, 128) * sx.double()[:, :, None]).view(T, K)
+    for n in range(0, N, 1024):                          # (fp64 copies of a slice of the weights at a time)
+        w, s = wq[n:n + 1024], sw[n // 128:(n + 1024) // 128]
+        wd = w.view(torch.float8_e4m3fn).double().view(-1, 128, K // 128, 128) * s.double()[:, None, :, None]
+        assert _rel(y[:, n:n + 1024], xd @ wd.view(-1, K).t()) < 2.5e-3
+    assert ops.check_status() == 0
+
+
 @pytest.mark.parametrize("T", [147, 148, 301])
 @pytest.mark.parametrize("D,hq,hkv", [(64, 5, 1), (64, 64, 8), (128, 3, 3), (128, 32, 8)])
 @pytest.mark.parametrize("norm", [False, True])
