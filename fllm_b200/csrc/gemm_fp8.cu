@@ -407,7 +407,11 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   // as a full round (172 -> 149 us).
   int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1, whole = 0;
   const int deep = (a.k_blocks + 63) / 64, least = swap ? deep : 1;   // swap-AB: the token scales of a split fit their shared-memory block
-  const bool can_split = workspace && (N & 3) == 0;
+  // Tiles of up to 64 tokens store pairs of features, wider ones eight at a time; the kernels that add partial sums store four.
+  const int unit = swap ? 2 : 8;
+  if (ldy % unit || reinterpret_cast<uintptr_t>(y) % (2 * unit))
+    throw std::runtime_error("linear_fp8_block: output rows must be aligned to 4 bytes for up to 64 tokens, to 16 for more");
+  const bool can_split = workspace && (ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0;
   long long best = -1;
   for (int w : {swap ? bn : 256, swap ? 0 : 128, swap ? 0 : 64}) {
     if (w == 0 || (w == 256 && N % 256)) continue;
@@ -428,7 +432,7 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
       if (best < 0 || cost < best) { best = cost; bn = w; splits = s; whole = (int)first; }
     }
   }
-  if (best < 0) throw std::runtime_error("linear_fp8_block: K above 8192 needs a split-K workspace");
+  if (best < 0) throw std::runtime_error("linear_fp8_block: K above 8192 needs a split-K workspace and output rows aligned to 8 bytes");
   a.n_tiles = (a.N + bn - 1) / bn;
   const CUtensorMap tw = make_tmap_2d(wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, swap ? F8_BM : bn, F8_BK, true);
   const CUtensorMap tx = make_tmap_2d(xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, T, K, K, swap ? bn : F8_BM, F8_BK, true);

@@ -87,6 +87,23 @@ def test_fp8_block_of_many_tokens_needs_no_room_for_deep_sums(ops, T, N, K, room
     assert ops.check_status() == 0
 
 
+@pytest.mark.parametrize("T,N,K", [(8, 19072, 4096), (20, 19072, 4096), (64, 19072, 5120), (3, 256, 1024)])
+def test_fp8_block_into_rows_of_four_bytes(ops, T, N, K):
+    """Rows that the kernels adding partial sums could not store are not split; what no kernel could store is refused."""
+    from fllm_b200.ops.native import Fp8BlockWeight, quantize_weight_fp8_block
+    x, w = _rand((T, K), 1), Fp8BlockWeight(*quantize_weight_fp8_block(_rand((N, K), 2, 0.05)))
+    want = ops.linear(x, w)
+    out = torch.zeros(T, N + 6, dtype=torch.bfloat16, device="cuda")
+    ops.linear(x, w, out=out[:, 2:2 + N])
+    # (two results, each off by one rounding to bf16: 0.17 % in the mean square)
+    assert _rel(out[:, 2:2 + N], want.double()) < 3.4e-3 and not out[:, :2].any() and not out[:, 2 + N:].any()
+    with pytest.raises(RuntimeError, match="aligned"):
+        ops.linear(x, w, out=out[:, 1:1 + N])
+    wide = _rand((65, K), 1)
+    with pytest.raises(RuntimeError, match="aligned"):
+        ops.linear(wide, w, out=torch.zeros(65, N + 6, dtype=torch.bfloat16, device="cuda")[:, 2:2 + N])
+
+
 @pytest.mark.parametrize("T", [147, 148, 301])
 @pytest.mark.parametrize("D,hq,hkv", [(64, 5, 1), (64, 64, 8), (128, 3, 3), (128, 32, 8)])
 @pytest.mark.parametrize("norm", [False, True])
