@@ -624,7 +624,7 @@ void widen_rows(const void* x, long long ldx, float* out, int rows, int cols, cu
 // layout: 0 = the kind's natural one (halves; pairs for kind 2), 16 = blocks of 16 gate columns followed
 // by the 16 up columns of the same features (the order the GEMM's gated epilogue wants its weight rows in).
 // ws != null: x is not read; the columns are the sums of fp32 split-K partials [splits][rows][2 * inter]
-// (+ bias), rounded to bf16 like the reduction kernel would have stored them.
+// (+ bias), kept in fp32 in front of the activation as the epilogue of an unsplit product keeps them.
 __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                            __nv_bfloat16* __restrict__ out, long long ldo, int inter, int act_kind,
                            float alpha, float limit, int layout, const float* __restrict__ ws, int splits,
@@ -685,8 +685,6 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         if (bias) { g[j] += __bfloat162float(bias[col(j, false)]); u[j] += __bfloat162float(bias[col(j, true)]); }
-        g[j] = __bfloat162float(__float2bfloat16(g[j]));
-        u[j] = __bfloat162float(__float2bfloat16(u[j]));
       }
     }
   } else if (act_kind == 2) {

@@ -45,7 +45,29 @@ def test_pairs_leave_their_sums_to_the_norm_and_the_activation(ops, T):
     h = _rand((T, 512), 7)
     u = (h.double() @ g.double().t()).view(T, 64, 2, 16)
     ref = (torch.nn.functional.silu(u[:, :, 0]) * u[:, :, 1]).reshape(T, 1024)
-    assert _rel(ops.linear_glu(h, g, None, 0, layout=16), ref) < 8e-3     # partial sums are rounded to bf16 in front of the activation
+    assert _rel(ops.linear_glu(h, g, None, 0, layout=16), ref) < 2.5e-3
+
+
+@pytest.mark.parametrize("T,N,K", [(200, 4768, 4096), (5, 2048, 4096), (129, 2048, 512), (512, 2336, 4096)])
+@pytest.mark.parametrize("kind,layout", [(0, 16), (1, 16), (2, 0)])
+def test_gate_and_up_sums_stay_in_fp32(ops, T, N, K, kind, layout):
+    """A product over splits of K feeds the activation its fp32 sums: one rounding to bf16, behind the activation."""
+    w, h, b = _rand((N, K), 6, 0.02), _rand((T, K), 7), _rand((N,), 8, 0.3)
+    y = torch.empty(T, N // 2, dtype=torch.bfloat16, device="cuda")
+    ref = h.double() @ w.double().t() + b.double()
+    u = ref.view(T, N // 32, 2, 16) if layout else ref.view(T, N // 2, 2)
+    gate, up = (u[:, :, 0], u[:, :, 1]) if layout else (u[..., 0], u[..., 1])
+    if kind == 2:
+        gate, up = gate.clamp(max=7.0), up.clamp(-7.0, 7.0)
+        want = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+    else:
+        want = (torch.nn.functional.silu(gate) if kind == 0 else torch.nn.functional.gelu(gate, approximate="tanh")) * up
+    _, splits = ops.k.linear_ex(h, w, b, y, ops.workspace, ops.status, 2, kind + 1, 16 if layout else 1, 1.702, 7.0, True)
+    assert splits == 2
+    ops.k.glu_ex(None, y, kind, 1.702, 7.0, layout, ops.workspace, splits, b)
+    assert _rel(y, want.reshape(T, N // 2)) < 2.5e-3
+    assert _rel(ops.linear_glu(h, w, b, kind, 1.702, 7.0, layout), want.reshape(T, N // 2)) < 2.5e-3
+    assert ops.check_status() == 0
 
 
 @pytest.mark.parametrize("T,N,K", [(1, 128, 128), (17, 256, 1024), (64, 384, 8192), (65, 128, 256), (128, 7168, 8192), (129, 1280, 8192), (128, 256, 12288),
