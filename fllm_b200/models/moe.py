@@ -163,17 +163,20 @@ def _fp16_experts(lw) -> bool:
 
 
 def _oai_scale(alpha: float, limit: float) -> float:
-    """Power of two that brings the largest value of the clamped SwiGLU-OAI, limit (limit + 1), below the largest fp16 value; 0 where the
-    activation has no such bound. (The gate is not clamped from below: x sigmoid(alpha x) >= -0.279 / alpha.)"""
+    """Power of two that brings the largest value of the clamped SwiGLU-OAI, limit (limit + 1), below the largest fp16 value. (The gate
+    is not clamped from below: x sigmoid(alpha x) >= -0.279 / alpha.) fp16 keeps the eight bits of bf16 down to 2^-16, so a factor of
+    2^10 (limits up to 7) keeps those of activations down to 2^-26, and a smaller one is off by 2^-35 at most. Larger limits leave
+    less below: 0 for them, and for an activation without such a bound."""
     if not (alpha > 0 and limit > 0):
         return 0.0
     top = max(limit, 0.279 / alpha) * (limit + 1)
-    return 2.0 ** min(12, math.floor(math.log2(60000 / top))) if top < 60000 else 0.0
+    power = math.floor(math.log2(60000 / top))
+    return 2.0 ** min(12, power) if power >= 10 else 0.0
 
 
 def _packed_ffn(cfg, ops, spec: MoeSpec, lw, x: torch.Tensor, token_of, row_w, tile_e, tile_r, ntiles, bn: int, rows: int) -> torch.Tensor:
     """Expert networks on packed stacks in fp16: rows gathered and converted in one kernel, the activation in the epilogue of the first
-    product where it is bounded (its fp16 values times a constant need no factor per row), else on rows converted again."""
+    product where its bound leaves fp16 enough range for one factor for all rows (`_oai_scale`), else on rows converted again."""
     H, k_ops = x.shape[1], ops.k
     gu, dn = lw.exp_gate_up, lw.exp_down
     where = (tile_e, tile_r, ntiles, bn, ops.status)

@@ -54,6 +54,59 @@ def test_blocks_of_zeros_under_large_scales(ops, scale):
     assert stack.f16 == q.f16 == (scale < 143)
 
 
+def test_one_factor_for_an_activation_needs_room_below():
+    from fllm_b200.models.moe import _oai_scale
+    assert _oai_scale(1.702, 7.0) == 1024.0 and _oai_scale(1.702, 0.5) == 4096.0
+    for limit in (8.0, 100.0, 240.0, 1e6, 0.0):
+        assert _oai_scale(1.702, limit) == 0.0
+    assert _oai_scale(1e-3, 7.0) == 0.0
+
+
+def _experts(ops, counts, k, act, limit=7.0, size=1.0, weigh=False, alpha=1.702):
+    """moe_ffn over MXFP4 experts, expert e chosen by counts[e] (token, place) pairs, and the same in 64 bits. The first values of a row are
+    its router logits (times ``size``)."""
+    from types import SimpleNamespace
+    from fllm_b200.config import ModelConfig, MoeSpec
+    from fllm_b200.models.moe import moe_ffn
+    from fllm_b200.models.weights import LayerWeights
+    E, H, I, T = len(counts), 256, 192, sum(counts) // k
+    cfg = ModelConfig(hidden_size=H, num_experts=E, experts_per_token=k, moe_intermediate_size=I, act=act, swiglu_limit=limit, swiglu_alpha=alpha)
+    lw = LayerWeights(attn_norm=None, wqkv=None, wo=None, ffn_norm=None)
+    lw.moe = MoeSpec(E, k, act=act, weigh_input=weigh)
+    lw.router_w = torch.eye(max(E, 8), H, dtype=torch.bfloat16, device="cuda")[:E]
+    lw.exp_gate_up, lw.exp_down = Fp4ExpertStack.from_dense(_rand((E, 2 * I, H), 3, 0.01).cuda()), Fp4ExpertStack.from_dense(_rand((E, H, I), 5, 0.05).cuda())
+    ids = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)]).view(k, T).t()
+    h = _rand((T, H), 7)
+    h[:, :E] = 0
+    h.scatter_(1, ids, torch.tensor([[4.0, 3.0, 2.5, 2.0][:k]]).expand(T, k).to(torch.bfloat16))
+    h = (h * size).cuda()
+    w = torch.softmax(torch.tensor([[4.0, 3.0, 2.5, 2.0][:k]]).double() * size, -1)
+    got = moe_ffn(SimpleNamespace(cfg=cfg, ops=ops, spec=SimpleNamespace(expert_parallel=False, expert_start=0)), lw, h)
+    gu, dn, ref = lw.exp_gate_up.dense().double(), lw.exp_down.dense().double(), torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for j in range(k):
+        for e in range(E):
+            t = (ids[:, j] == e).nonzero().flatten().cuda()
+            x = h[t].double() * (w[0, j].item() if weigh else 1.0)
+            u = x @ gu[e].t()
+            if act == "swiglu_oai":
+                g, u = u[:, 0::2].clamp(max=limit), u[:, 1::2].clamp(-limit, limit)
+                u = g * torch.sigmoid(alpha * g) * (u + 1)
+            else:
+                u = torch.nn.functional.silu(u[:, :I]) * u[:, I:]
+            ref[t] += u @ dn[e].t() * (1.0 if weigh else w[0, j].item())
+    assert ops.check_status() == 0
+    return _rel(got, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit", [7.0, 100.0, 240.0])
+@pytest.mark.parametrize("size", [1.0, 2.0 ** -10, 2.0 ** -18])
+def test_small_activations_of_experts(ops, limit, size):
+    """Activations of 2^-5, 2^-15 and 2^-23 under limits that leave them room above. Rounded to bf16 are gate and up, the activation, an
+    expert's result and their sum: four roundings of 0.17 % in the mean square."""
+    assert _experts(ops, [5, 4, 0, 9], 2, "swiglu_oai", limit, size) < 4 * 1.7e-3
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", [64, 320, 2880, 28672])
 def test_rows_keep_every_value(ops, K):
