@@ -853,7 +853,7 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
   constexpr size_t kCounterBytes = 64 * 1024;
   // Local products of more tokens than one swap-AB tile holds go to the CTA-pair kernel (cta_group::2, 256 x 256 tiles), over splits of K
   // while its tiles do not fill the machine (200 tokens, 6144 x 4096: 25.4 us on one-CTA tiles, which read every weight twice).
-  if (!tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && T > 128 && N >= 256 && K >= BK) {
+  if (!tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && linear_bf16_pair_supported(T, N, K)) {
     int splits = 1;
     if ((long long)((T + 255) / 256) * ((N + 255) / 256) < sms / 2)
       splits = linear_bf16_pair_splits(T, N, K, workspace && workspace_bytes > kCounterBytes && (!glu || defer) ? workspace_bytes - kCounterBytes : 0);

@@ -274,7 +274,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
   if (threadIdx.x == 0 && *abort_flag && p.status) atomicCAS(p.status, FLLM_OK, FLLM_ERR_MBAR_TIMEOUT);
 }
 
-bool linear_bf16_pair_supported(int T, int N, int K) { return T >= 256 && N % 8 == 0 && N >= 256 && K % 8 == 0 && K >= P2_BK; }
+bool linear_bf16_pair_supported(int T, int N, int K) { return T > 128 && N % 8 == 0 && N >= 256 && K % 8 == 0 && K >= P2_BK; }
 
 // K splits with which pairs finish a product of more than 128 tokens that has fewer tiles than pairs, or 0 when `workspace_bytes` holds
 // no split. In units of 10 ns: a K block of a tile takes 37, its share of the HBM bandwidth (27 for its products), an item 300 to start and
@@ -297,8 +297,8 @@ int linear_bf16_pair_splits(int T, int N, int K, size_t workspace_bytes) {
 // (without bias or activation); returns the number of them.
 int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* y, long long ldy,
                      int T, int N, int K, int* status, cudaStream_t stream, const LinearExtras* ex, int splits, float* partials) {
-  if (T <= 128 || N < 256 || N % 8 || K % 8 || K < P2_BK) throw std::runtime_error("linear_bf16_pair: needs more than 128 tokens, N >= 256, N % 8 == 0, K % 8 == 0");
-  if ((ldy & 7)) throw std::runtime_error("linear_bf16_pair: output rows must be 16-byte aligned");
+  if (!linear_bf16_pair_supported(T, N, K)) throw std::runtime_error("linear_bf16_pair: needs more than 128 tokens, N >= 256, N % 8 == 0, K >= 64, K % 8 == 0");
+  if ((ldy & 7) || (reinterpret_cast<uintptr_t>(y) & 15)) throw std::runtime_error("linear_bf16_pair: output rows must be 16-byte aligned");
   const int glu = ex ? ex->glu : 0;
   if (glu && ((N & 31) || (ex->glu_pd != 16 && ex->glu_pd != 1))) throw std::runtime_error("linear_bf16_pair: GLU needs N % 32 == 0 and a pair distance of 16 or 1");
   Gemm2Args a{};

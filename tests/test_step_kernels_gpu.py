@@ -31,6 +31,25 @@ def test_pairs_over_splits(ops, T, N, K):
     assert ops.check_status() == 0
 
 
+@pytest.mark.parametrize("T", [129, 200, 255, 257, 511])
+@pytest.mark.parametrize("N,K", [(256, 4096), (264, 64), (1000, 320), (4096, 1088)])
+def test_pair_kernel_over_each_number_of_splits(ops, T, N, K):
+    """The kernel itself, whatever the planner picks: an unsplit product is off by one rounding, fp32 sums over parts of K by none."""
+    x, w, b = _rand((T, K), 1), _rand((N, K), 2, 0.05), _rand((N,), 3)
+    ref = x.double() @ w.double().t()
+    y = torch.empty(T, N, dtype=torch.bfloat16, device="cuda")
+    assert ops.k.linear_pair(x, w, b, y, ops.status) == 1
+    assert _rel(y, ref + b.double()) < 2.5e-3
+    for splits in (2, 3, 8):
+        part = torch.full((splits + 1, T, N), 7.0, device="cuda")
+        n = ops.k.linear_pair(x, w, None, y, ops.status, splits, part[:splits])
+        assert 1 <= n <= splits and (part[n if n > 1 else 0:] == 7.0).all()
+        assert n == 1 or _rel(part[:n].double().sum(0), ref) < 1e-5
+    with pytest.raises(RuntimeError, match="partials"):
+        ops.k.linear_pair(x, w, None, y, ops.status, 2, None)
+    assert ops.check_status() == 0
+
+
 @pytest.mark.parametrize("T", [129, 200, 300])
 def test_pairs_leave_their_sums_to_the_norm_and_the_activation(ops, T):
     x, w, b, nw = _rand((T, 4096), 1), _rand((4096, 4096), 2, 0.02), _rand((4096,), 3), _rand((4096,), 4)
