@@ -77,6 +77,12 @@ int64_t linear_pair(const Tensor& x, const Tensor& w, const optional<Tensor>& bi
                                 y.stride(0), (int)x.size(0), (int)w.size(0), (int)x.size(1), st, cur_stream(), nullptr, (int)splits, sums);
 }
 
+// The form that `linear` takes for a product on a device of `sms` SMs: splits over K on CTA pairs, or 0 for one-CTA tiles.
+int64_t linear_plan_pair(int64_t tokens, int64_t features, int64_t k, int64_t sms, int64_t workspace_bytes, bool gated, bool deferred) {
+  TORCH_CHECK(tokens > 0 && features > 0 && k > 0 && sms > 0 && workspace_bytes >= 0, "linear_plan_pair: sizes");
+  return fllm::linear_bf16_plan_pair((int)tokens, (int)features, (int)k, (int)sms, (size_t)workspace_bytes, gated, deferred);
+}
+
 // linear with the optional behaviours of fllm::LinearExtras. glu > 0: y is [T, N / 2] (the activation runs in the
 // epilogue, or in the caller's consumer when the call deferred split-K). Returns [kernels launched, deferred splits].
 std::vector<int64_t> linear_ex(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, Tensor y,
@@ -405,6 +411,7 @@ int64_t sample_row_bytes() { return (int64_t)sizeof(fllm::SampleRow); }
 
 TORCH_LIBRARY(fllm_b200, m) {
   m.def("linear(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status, int force_splits) -> int", &linear);
+  m.def("linear_plan_pair(int tokens, int features, int k, int sms, int workspace_bytes, bool gated, bool deferred) -> int", &linear_plan_pair);
   m.def("linear_pair(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? status, int splits=1, Tensor(b!)? partials=None) -> int", &linear_pair);
   m.def("linear_ex(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status, int force_splits, int glu, int glu_pd, float glu_alpha, float glu_limit, bool defer_reduce) -> int[]", &linear_ex);
   m.def("rmsnorm_splitk(Tensor(a!) residual, Tensor workspace, int splits, Tensor? bias, Tensor w, Tensor(b!) y, float eps, float w_offset) -> ()", &rmsnorm_splitk);

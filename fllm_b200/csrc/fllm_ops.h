@@ -103,7 +103,9 @@ bool linear_bf16_pair_supported(int T, int N, int K);
 int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* y, long long ldy,
                      int T, int N, int K, int* status, cudaStream_t stream, const struct LinearExtras* ex = nullptr, int splits = 1,
                      float* partials = nullptr);                    // splits > 1: partial sums only; returns their number
-int linear_bf16_pair_splits(int T, int N, int K, size_t workspace_bytes);
+// Whether a local product of linear_bf16 takes the CTA pairs, and over how many splits of K (0: one-CTA tiles). `workspace_bytes`: of the
+// whole workspace; gated: the activation follows the product; deferred: the consumer adds partial sums.
+int linear_bf16_plan_pair(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred);
 
 // Packed 4-bit weights x at most 4 tokens on dp4a (int8 activations quantised inside the kernel); formats as linear_w4a16.
 bool gemv_w4_supported(int T, int K);

@@ -815,6 +815,50 @@ static void plan_linear(int T, int N, int sms, bool* swap, int* bn) {
   }
 }
 
+constexpr size_t kCounterBytes = 64 * 1024;      // workspace = [tile counters, zero between launches] [fp32 partial sums]
+
+// Splits over K of a product on one-CTA tiles when the tile list cannot fill the machine and K is deep enough: with fewer tiles than 3/4 of
+// the resident CTA slots K is cut so that every SM streams weights. `whole`: the product needs complete sums.
+static int plan_splits(int tiles, int bn, int k_blocks, int sms, size_t workspace_bytes, bool whole) {
+  const int slots = sms * (bn <= 64 ? 2 : 1);
+  if (whole || tiles * 4 > slots * 3 || k_blocks < 8) return 1;
+  int splits = min(min(slots / tiles, k_blocks / 4), 16);
+  if (workspace_bytes <= kCounterBytes || (size_t)tiles * 4 > kCounterBytes || bn > 128) return 1;
+  while (splits > 1 && kCounterBytes + (size_t)splits * tiles * BM * bn * sizeof(float) > workspace_bytes) --splits;
+  return splits;
+}
+
+// Times of the two forms by the rounds of their items over the machine, in units of 10 ns, fitted to 231 products of 256 .. 24576
+// features, K of 320 .. 12288 and 129 .. 2048 tokens (11 % off in the mean; what they choose is 0.1 % behind the other form in the
+// mean, 9 % at most): a K block of a 128-wide one-CTA tile takes 31, of a 256-wide one 38, of a pair's 256 x 256 tile 29; a round 110, 480 and
+// 225 more; a launch 330, and 610 for pairs, whose launch overlaps with no other; a kernel that adds partial sums 165 or, behind
+// pairs, 305; the sums themselves 5.7 TB/s. The gated epilogue of a one-CTA tile takes 900 (256-wide 1500) more a round. So few
+// tiles of short sums go to one-CTA tiles (512 x 3072 x 2048: 14.5 us against 22.1 on pairs; 200 x 2048 x 2048: 10.0 against 15.4), most
+// others to pairs (1024 x 2048 x 8192: 36.8 us against 42.0; 200 x 24576 x 4096: 54.9 against 66.1).
+int linear_bf16_plan_pair(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred) {
+  if (!linear_bf16_pair_supported(T, N, K)) return 0;
+  const int kbs = (K + BK - 1) / BK;
+  const bool whole = gated && !deferred;
+  auto sums = [&](int s, int launch) {
+    return s > 1 ? (deferred && !gated ? 0 : launch) + (long long)((double)s * T * N * 8 / 57000.0) : 0;
+  };
+  bool swap;
+  int bn;
+  plan_linear(T, N, sms, &swap, &bn);
+  const int tiles = ((T + BM - 1) / BM) * ((N + bn - 1) / bn), s1 = plan_splits(tiles, bn, kbs, sms, workspace_bytes, whole);
+  const long long round = (kbs + s1 - 1) / s1 * (bn == 256 ? 38 : 31) + (bn == 256 ? 480 : 110) + (gated && s1 == 1 ? (bn == 256 ? 1500 : 900) : 0);
+  const long long one = 330 + (tiles * s1 + sms - 1) / sms * round + sums(s1, 165);
+  const long long pair_tiles = (long long)((T + 255) / 256) * ((N + 255) / 256), pairs = sms / 2;
+  long long best = one;
+  int splits = 0;
+  for (int s = 1; s == 1 || (s <= 8 && s * 4 <= kbs); ++s) {
+    if (s > 1 && (whole || kCounterBytes + (size_t)s * T * N * sizeof(float) > workspace_bytes)) break;
+    const long long cost = 610 + (pair_tiles * s + pairs - 1) / pairs * ((kbs + s - 1) / s * 29 + 225) + sums(s, 305);
+    if (cost < best) { best = cost; splits = s; }
+  }
+  return splits;
+}
+
 // Flag bumps rank `dest` receives from EACH source rank for one reduce-scatter linear of this
 // shape: 4 epilogue warps x feature tiles x token tiles that overlap the rows `dest` owns.
 int linear_rs_expected_signals(int T, int N, int rows_per, int dest) {
@@ -850,15 +894,14 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
   if ((K & 7) || (N & 7) || (ldx & 7) || (ldw & 7) || (ldy & 1))
     throw std::runtime_error("linear_bf16: K, N and the row pitches must be multiples of 8");
   const int sms = sm_count();
-  constexpr size_t kCounterBytes = 64 * 1024;
-  // Local products of more tokens than one swap-AB tile holds go to the CTA-pair kernel (cta_group::2, 256 x 256 tiles), over splits of K
-  // while its tiles do not fill the machine (200 tokens, 6144 x 4096: 25.4 us on one-CTA tiles, which read every weight twice).
-  if (!tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0 && linear_bf16_pair_supported(T, N, K)) {
-    int splits = 1;
-    if ((long long)((T + 255) / 256) * ((N + 255) / 256) < sms / 2)
-      splits = linear_bf16_pair_splits(T, N, K, workspace && workspace_bytes > kCounterBytes && (!glu || defer) ? workspace_bytes - kCounterBytes : 0);
+  if (!workspace) workspace_bytes = 0;
+  // Local products of more tokens than one swap-AB tile holds: CTA pairs (cta_group::2, 256 x 256 tiles), over splits of K while their tiles
+  // do not fill the machine, or the one-CTA tiles below.
+  int splits = !tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0
+                   ? linear_bf16_plan_pair(T, N, K, sms, workspace_bytes, glu != 0, defer) : 0;
+  if (splits > 0) {
     float* partials = splits > 1 ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + kCounterBytes) : nullptr;
-    splits = linear_bf16_pair(x, ldx, w, ldw, bias, y, ldy, T, N, K, status, stream, glu && splits <= 1 ? ex : nullptr, max(splits, 1), partials);
+    splits = linear_bf16_pair(x, ldx, w, ldw, bias, y, ldy, T, N, K, status, stream, glu && splits == 1 ? ex : nullptr, splits, partials);
     if (splits == 1) return 1;
     if (defer) {
       ex->deferred_splits = splits;
@@ -911,22 +954,14 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
   a.n_tiles = (a.N + bn - 1) / bn;
   const int tiles = a.m_tiles * a.n_tiles;
 
-  // split-K when the tile list cannot fill the machine and K is deep enough
-  int splits = 1;
-  if (force_splits > 0) {
-    splits = force_splits;
-  } else if (tiles * 4 <= sms * (bn <= 64 ? 2 : 1) * 3 && a.k_blocks >= 8) {
-    // fewer tiles than 3/4 of the resident CTA slots: cut K so that every SM streams weights
-    const int slots = sms * (bn <= 64 ? 2 : 1);
-    splits = min(min(slots / tiles, a.k_blocks / 4), 16);
-  }
-  // workspace = [tile counters (kCounterBytes, zero between launches)] [fp32 partial tiles]
-  if (splits > 1 && (!workspace || workspace_bytes <= kCounterBytes || (size_t)tiles * 4 > kCounterBytes || bn > 128))
-    splits = 1;
-  while (splits > 1 && kCounterBytes + (size_t)splits * tiles * BM * bn * sizeof(float) > workspace_bytes) --splits;
   // A gated epilogue needs complete sums: no split-K, unless the caller takes the fp32 partials and
   // applies the activation while it adds them.
-  if (glu && splits > 1 && !defer) splits = 1;
+  splits = plan_splits(tiles, bn, a.k_blocks, sms, workspace_bytes, glu && !defer);
+  if (force_splits > 0) {
+    splits = force_splits;
+    if (splits > 1 && (workspace_bytes <= kCounterBytes || (size_t)tiles * 4 > kCounterBytes || bn > 128 || (glu && !defer))) splits = 1;
+    while (splits > 1 && kCounterBytes + (size_t)splits * tiles * BM * bn * sizeof(float) > workspace_bytes) --splits;
+  }
   // Broadcast destination + split-K: the GEMM keeps its fast local split path and the reduction
   // kernel does the pushing. Scatter destination + split-K: the last-arriving CTA finishes the tile.
   const bool push_reduce = rs && tpa->rs_bcast && splits > 1;

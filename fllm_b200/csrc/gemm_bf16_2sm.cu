@@ -276,22 +276,6 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
 
 bool linear_bf16_pair_supported(int T, int N, int K) { return T > 128 && N % 8 == 0 && N >= 256 && K % 8 == 0 && K >= P2_BK; }
 
-// K splits with which pairs finish a product of more than 128 tokens that has fewer tiles than pairs, or 0 when `workspace_bytes` holds
-// no split. In units of 10 ns: a K block of a tile takes 37, its share of the HBM bandwidth (27 for its products), an item 300 to start and
-// drain, a partial sum is written and read at 5 TB/s; a round of items is as long as one.
-int linear_bf16_pair_splits(int T, int N, int K, size_t workspace_bytes) {
-  const int pairs = sm_count() / 2, kbs = (K + P2_BK - 1) / P2_BK;
-  const long long tiles = (long long)((T + P2_TILE - 1) / P2_TILE) * ((N + P2_TILE - 1) / P2_TILE);
-  long long best = -1;
-  int splits = 0;
-  for (int s = 1; s <= 8 && s * 4 <= kbs; ++s) {
-    if (s > 1 && (size_t)s * T * N * sizeof(float) > workspace_bytes) break;
-    const long long cost = (tiles * s + pairs - 1) / pairs * ((kbs + s - 1) / s * 37 + 300) + (s > 1 ? (long long)(s * (double)T * N * 8 / 50000.0) : 0);
-    if (best < 0 || cost < best) { best = cost; splits = s; }
-  }
-  return splits;
-}
-
 // y[T, N] = x[T, K] * w[N, K]^T (+ bias[N]); row pitches in elements. With ex->glu the gated activation runs in the
 // epilogue and y is [T, N / 2] (N a multiple of 32). splits > 1: fp32 partial sums [splits][T][N] go to `partials` instead
 // (without bias or activation); returns the number of them.
