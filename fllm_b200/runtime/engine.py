@@ -193,6 +193,7 @@ class LLMEngine:
         # a pinned buffer is written again only after the copy out of it is done (no caller has to wait for that)
         self._stage_done: List[Optional[torch.cuda.Event]] = [None] * len(self._stage_bufs)
         self._forced_slot = 0
+        self._step_stream = None         # where the last step was queued
         self._out_alt = torch.empty(512, dtype=torch.int32, pin_memory=self.is_cuda)
         self._flip = 0
         self._out_host = torch.empty(self.cfg.max_num_batched_tokens + 64, dtype=torch.int32,
@@ -331,6 +332,14 @@ class LLMEngine:
         return self.export_request(rid), [e for e in events if e.request_id != rid] if mine is not None else events
 
     # ------------------------------------------------------------------ batch building
+    def _follow_last_step(self) -> None:
+        """Order the current stream behind the last step, wherever that was queued: device buffers, graphs and the cache are its own."""
+        if self.is_cuda:
+            stream = torch.cuda.current_stream(self.device)
+            if self._step_stream is not None and self._step_stream != stream:
+                stream.wait_stream(self._step_stream)
+            self._step_stream = stream
+
     def _build_batch(self, step: ScheduledStep, pad_to: int = 0, slot: int = 0) -> StepBatch:
         seqs = step.seqs
         T = step.num_tokens
@@ -341,6 +350,7 @@ class LLMEngine:
         host_t, h, dev = self._stage_bufs[slot]
         if self._stage_done[slot] is not None:
             self._stage_done[slot].synchronize()
+        self._follow_last_step()
         ids = h[0:Tp]
         pos = h[Tp:2 * Tp]
         slots = h[2 * Tp:3 * Tp]
@@ -1185,6 +1195,7 @@ class _DecodeGraph:
             num_seqs=n, num_tokens=n, max_kv_len=eng.cfg.max_model_len, all_decode=True,
             max_q_len=1, min_q_len=1)
         # harmless contents for warm-up / capture: all rows padded
+        eng._follow_last_step()
         dev[0:2 * n].zero_()
         dev[2 * n:3 * n].fill_(-1)
         dev[3 * n:4 * n].zero_()

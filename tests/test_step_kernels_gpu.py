@@ -200,6 +200,14 @@ def test_given_steps_queue_without_waiting():
     torch.cuda.synchronize()
     for a, b in zip(alone + alone[len(prompts):][::-1], queued):
         assert torch.equal(a, b.cpu())
+    # from streams that know nothing of one another: each step waits for the one before, wherever that was queued
+    streams, spread = [torch.cuda.Stream() for _ in range(2)], []
+    for i, s in enumerate(prompts + decodes):
+        with torch.cuda.stream(streams[i % 2]):
+            spread.append(eng.run_forced(s))
+    torch.cuda.synchronize()
+    for a, b in zip(alone, spread):
+        assert torch.equal(a, b.cpu())
     eng.close()
 
 
