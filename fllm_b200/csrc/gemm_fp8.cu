@@ -58,13 +58,14 @@ struct Fp8Item {
   }
 };
 
-template <int BN, bool SWAP>
+template <int BN, bool SWAP, int PER>
 struct Fp8Smem {
   static constexpr int kABytes = F8_BM * F8_BK;
   static constexpr int kBBytes = BN * F8_BK;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kScaleFloats = SWAP ? 64 * BN : 0;       // token scales of a swap-AB tile, up to 64 K blocks
-  static constexpr int kStages = (196 * 1024 - kScaleFloats * 4) / kStageBytes > 10 ? 10 : (196 * 1024 - kScaleFloats * 4) / kStageBytes;
+  static constexpr int kRing = (PER == 2 ? 96 : 196) * 1024 - kScaleFloats * 4;
+  static constexpr int kStages = kRing / kStageBytes > 10 ? 10 : kRing / kStageBytes;
   // A K block's product stays in its buffer until the promoting warps have added it up: the tensor core runs ahead by the other buffers.
   static constexpr int kBuffers = BN == 256 ? 2 : 4;
   static constexpr int kTmemCols = kBuffers * BN < 128 ? (kBuffers * BN < 64 ? 64 : kBuffers * BN) : kBuffers * BN;
@@ -81,11 +82,11 @@ struct Fp8Smem {
 // block, activation scale x weight scale, read ahead; one accumulator register per column) and the latency of the tensor memory is
 // covered: four warps per scheduler with 64 columns each (two with 128 needed 1290 clocks a block). 128 x 128 tiles read and write shared memory
 // twice as often per product; they remain for few tiles.
-template <int BN, bool SWAP>                // SWAP: tokens in the N dimension
-__global__ void __launch_bounds__(Fp8Smem<BN, SWAP>::kThreads, 1)
+template <int BN, bool SWAP, int PER>       // SWAP: tokens in the N dimension; PER: CTAs per SM
+__global__ void __launch_bounds__(Fp8Smem<BN, SWAP, PER>::kThreads, PER)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                       const Fp8GemmArgs p) {
-  using S = Fp8Smem<BN, SWAP>;
+  using S = Fp8Smem<BN, SWAP, PER>;
   constexpr int STAGES = S::kStages, NBUF = S::kBuffers, COLS = S::kCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -372,15 +373,15 @@ void quant_fp8_1x128(const void* x, long long ldx, void* xq, float* sx, int toke
   launch_pdl(quant_fp8_1x128_kernel, dim3((unsigned)((groups + 15) / 16)), dim3(256), 0, s, (const __nv_bfloat16*)x, ldx, (uint8_t*)xq, sx, tokens, K);
 }
 
-template <int BN, bool SWAP>
+template <int BN, bool SWAP, int PER = 1>
 static void launch_fp8(const CUtensorMap& ta, const CUtensorMap& tb, const Fp8GemmArgs& a, int grid, cudaStream_t s) {
-  using S = Fp8Smem<BN, SWAP>;
+  using S = Fp8Smem<BN, SWAP, PER>;
   static bool configured[kMaxDevices] = {};
   if (first_call_on_device(configured)) {
-    cuda_check(cudaFuncSetAttribute(gemm_fp8_block_kernel<BN, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
+    cuda_check(cudaFuncSetAttribute(gemm_fp8_block_kernel<BN, SWAP, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal),
                "cudaFuncSetAttribute(gemm_fp8_block_kernel)");
   }
-  launch_pdl(gemm_fp8_block_kernel<BN, SWAP>, dim3(grid), dim3(S::kThreads), S::kTotal, s, ta, tb, a);
+  launch_pdl(gemm_fp8_block_kernel<BN, SWAP, PER>, dim3(grid), dim3(S::kThreads), S::kTotal, s, ta, tb, a);
 }
 
 // y[T][N] = dequant(xq, sx) * dequant(wq, sw)^T (+ bias)
@@ -404,8 +405,10 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   // against 24.9); else what L2 takes for its operands with every SM reading (256-wide tiles 60, 128-wide 36). Partial sums are
   // written and read once, and cost a launch. With more tiles than SMs either all are split, or those of the last, partly filled
   // round alone (whole > 0): 1965 x 7168 x 8192 has 448 tiles of 256 for 3 x 148, and the last four took as long
-  // as a full round (172 -> 149 us).
-  int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1, whole = 0;
+  // as a full round (172 -> 149 us). 16-wide tiles may run as two CTAs per SM with half of the ring each, which share its bandwidth: one's
+  // scales, last blocks and stores lie under the other's stream, and the rounds are half as many (16 x 57344 x 8192 with its quantiser
+  // 89.8 -> 82.0 us, 16 x 28672 x 4096 27.6 -> 23.5); with few tiles one CTA and its whole ring are faster (1 x 16384 x 2048 9.7 against 10.3).
+  int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1, whole = 0, per = 1;
   const int deep = (a.k_blocks + 63) / 64, least = swap ? deep : 1;   // swap-AB: the token scales of a split fit their shared-memory block
   // Tiles of up to 64 tokens store pairs of features, wider ones eight at a time; the kernels that add partial sums store four.
   const int unit = swap ? 2 : 8;
@@ -419,9 +422,13 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
     const long long block = swap ? 37 : a.m_tiles == 1 ? (w == 256 ? 74 : w == 128 ? 37 : 28) : (w == 256 ? 60 : w == 128 ? 36 : 28);
     for (int s = least; s <= 16 * deep && s <= a.k_blocks; ++s) {
       if (s > 1 && (!can_split || (size_t)s * T * N * 4 > workspace_bytes)) break;
-      const long long rounds = ((long long)a.m_tiles * n_tiles * s + sms - 1) / sms;
-      const long long cost = rounds * ((a.k_blocks + s - 1) / s * block + 100) + (s > 1 ? 250 + (long long)((double)s * T * N * 8 / 60000.0) : 0);
-      if (best < 0 || cost < best) { best = cost; bn = w; splits = s; whole = 0; }
+      const long long items = (long long)a.m_tiles * n_tiles * s;
+      for (int two = 1; two <= (w == 16 ? 2 : 1); ++two) {
+        const long long rounds = (items + sms * two - 1) / (sms * two);
+        const long long cost = rounds * ((a.k_blocks + s - 1) / s * (two == 2 && items > sms ? 2 * block : block) + 100) +
+                               (s > 1 ? 250 + (long long)((double)s * T * N * 8 / 60000.0) : 0);
+        if (best < 0 || cost < best) { best = cost; bn = w; splits = s; whole = 0; per = two; }
+      }
     }
     const long long tiles = (long long)a.m_tiles * n_tiles, first = tiles / sms * sms, tail = tiles - first;
     if (swap || least > 1 || !can_split || first == 0) continue;
@@ -441,9 +448,12 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   a.k_splits = (a.k_blocks + a.kb_per_split - 1) / a.kb_per_split;
   a.whole = a.k_splits > 1 ? whole : a.m_tiles * a.n_tiles;
   a.ws = reinterpret_cast<float*>(workspace);
-  const int grid = std::min(a.whole + (a.m_tiles * a.n_tiles - a.whole) * a.k_splits, sms);
+  const int grid = std::min(a.whole + (a.m_tiles * a.n_tiles - a.whole) * a.k_splits, sms * per);
   switch (bn) {
-    case 16: launch_fp8<16, true>(ta, tb, a, grid, stream); break;
+    case 16:
+      if (per == 2) launch_fp8<16, true, 2>(ta, tb, a, grid, stream);
+      else launch_fp8<16, true>(ta, tb, a, grid, stream);
+      break;
     case 32: launch_fp8<32, true>(ta, tb, a, grid, stream); break;
     case 64:
       if (swap) launch_fp8<64, true>(ta, tb, a, grid, stream);

@@ -110,6 +110,22 @@ def test_fp8_block(ops, T, N, K):
     assert ops.check_status() == 0
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 19072, 256), (16, 18944, 512), (16, 19072, 512), (13, 38016, 1152), (9, 7168, 8192), (16, 8192, 28672), (17, 19072, 512)])
+def test_fp8_block_of_few_tokens_over_more_tiles_than_sms(ops, T, N, K):
+    """Up to 16 tokens: on both sides of the number of tiles from which two CTAs share an SM, with and without splits."""
+    from fllm_b200.ops.native import Fp8BlockLinear, quantize_weight_fp8_block
+    x, bias = _rand((T, K), 1), _rand((N,), 3)
+    wq, sw = quantize_weight_fp8_block(_rand((N, K), 2, 0.05))
+    xq, sx = torch.empty(T, K, dtype=torch.uint8, device="cuda"), torch.empty(T, K // 128, device="cuda")
+    ops.k.quant_fp8_1x128(x, xq, sx)
+    xd = (xq.view(torch.float8_e4m3fn).double().view(T, K // 128, 128) * sx.double()[:, :, None]).view(T, K)
+    wd = (wq.view(torch.float8_e4m3fn).float().view(N // 128, 128, K // 128, 128) * sw[:, None, :, None]).view(N, K)
+    ref = xd @ wd.double().t() + bias.double()
+    y = Fp8BlockLinear(ops, wq, sw, bias)(x)
+    assert _rel(y, ref) < 2.5e-3 and max(_rel(y[t], ref[t]) for t in range(T)) < 2.8e-3
+    assert ops.check_status() == 0
+
+
 @pytest.mark.parametrize("T,N,K,room", [(2048, 8192, 14336, None), (800, 8192, 28672, None), (65, 256, 8320, 0), (300, 384, 12288, 0), (257, 256, 32768, 0)])
 def test_fp8_block_of_many_tokens_needs_no_room_for_deep_sums(ops, T, N, K, room):
     """More than 64 tokens read their scales from global memory: K is not limited by what a workspace holds."""
