@@ -8,8 +8,8 @@
 // scales per 32 values), so every 128-deep K block is multiplied unscaled into a fresh TMEM
 // accumulator (tcgen05.mma kind::f8f6f4, four K=32 instructions) and the epilogue warps
 // promote it: they read the partial sums out of TMEM, multiply by sx * sw of that K block and
-// add them into fp32 registers. Two TMEM buffers alternate, so the tensor core works on K block
-// i+1 while block i is being promoted. Warp roles, TMA staging (128-byte swizzle, one K block
+// add them into fp32 registers. TMEM buffers alternate (two of 256 columns, four of fewer), so the
+// tensor core works on the next K blocks while one is being promoted. Warp roles, TMA staging (128-byte swizzle, one K block
 // = one 128-byte row) and the swap-AB orientation for small token counts are those of
 // gemm_bf16.cu.
 //

@@ -216,7 +216,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tma_raw, const __grid_cons
     *abort_flag = 0;
     fence_barrier_init();
   }
-  if (threadIdx.x >= 64 && threadIdx.x < 64 + 256) {    // scale byte -> {s, s}
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + 256 && !(F16 && p.fmt == 0)) {    // scale byte -> {s, s} (fp16 NVFP4 converts its scales)
     const int i = threadIdx.x - 64;
     const float f = scale_to_float((uint8_t)i, p.fmt);
     const __half2 h = __floats2half2_rn(f, f);
