@@ -80,6 +80,13 @@ int64_t linear_w4a16(const Tensor& x, const Tensor& codes, const Tensor& scales,
                             y.data_ptr(), y.stride(0), (int)T, (int)N, (int)K, ws, ws_bytes, st, cur_stream(), f16);
 }
 
+// [splits over K, fp16 form] that linear_w4a16 takes on a device of `sms` SMs with so many bytes for partial sums and rows
+std::vector<int64_t> linear_w4_plan(int64_t tokens, int64_t features, int64_t k, int64_t sms, int64_t workspace_bytes, bool f16) {
+  TORCH_CHECK(tokens > 0 && tokens <= 128 && features > 0 && k > 0 && sms > 0 && workspace_bytes >= 0, "linear_w4_plan: sizes");
+  const fllm::W4Plan p = fllm::w4_plan((int)tokens, (int)features, (int)k, (int)sms, f16, (size_t)workspace_bytes);
+  return {p.splits, p.f16 ? 1 : 0};
+}
+
 // x bf16 [T, K] -> xq uint8 [T, K] (e4m3) + sf uint8 [mx_act_scale_bytes(T, K, 0)] (e8m0 atoms per token tile)
 void quant_mx(const Tensor& x, Tensor xq, Tensor sf) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1 && x.stride(0) % 4 == 0, "x: bf16 rows");
@@ -227,6 +234,7 @@ TORCH_LIBRARY_FRAGMENT(fllm_b200, m) {
   m.def("quant_fp8_1x128(Tensor x, Tensor(a!) xq, Tensor(b!) sx) -> ()", &quant_fp8_1x128);
   m.def("linear_fp8_block(Tensor xq, Tensor sx, Tensor wq, Tensor sw, Tensor? bias, Tensor(a!) y, Tensor? status, Tensor? workspace=None) -> int", &linear_fp8_block);
   m.def("fp8_block_apply(Tensor x, Tensor wq, Tensor sw, Tensor? bias, Tensor? status, Tensor? workspace) -> (Tensor, int)", &fp8_block_apply);
+  m.def("linear_w4_plan(int tokens, int features, int k, int sms, int workspace_bytes, bool f16) -> int[]", &linear_w4_plan);
   m.def("linear_w4a16(Tensor x, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status, bool f16=False) -> int", &linear_w4a16);
   m.def("quant_mx(Tensor x, Tensor(a!) xq, Tensor(b!) sf) -> ()", &quant_mx);
   m.def("quant_rows_8bit(Tensor x, Tensor(a!) xq, Tensor(b!) tok_scale, bool is_int8) -> ()", &quant_rows_8bit);

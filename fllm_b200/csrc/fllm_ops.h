@@ -143,6 +143,12 @@ void widen_rows(const void* x, long long ldx, float* out, int rows, int cols, cu
 int linear_w4a16(const void* x, long long ldx, const void* codes, const void* scales, int fmt, float alpha,
                  const void* bias, void* y, long long ldy, int T, int N, int K, void* workspace, size_t workspace_bytes,
                  int* status, cudaStream_t stream, bool f16 = false);
+// Form (fp16 or bf16 values) and splits over K that linear_w4a16 takes; f16: the weight allows the fp16 form.
+struct W4Plan {
+  int splits;
+  bool f16;
+};
+W4Plan w4_plan(int T, int N, int K, int sms, bool f16, size_t workspace_bytes);
 // bf16 rows -> fp16 rows times 2^-e and factor[row] = 2^e; row r reads x[token_of[r]] (null: x[r]; -1: zeros)
 void rows_f16(const void* x, long long ldx, const int* token_of, const float* row_weight, void* out, float* factor, int rows, int K, cudaStream_t s);
 struct W4Rows {               // fp16 activation rows of a grouped product

@@ -641,8 +641,40 @@ static void launch_w4_bn(int bn, const CUtensorMap& tr, const CUtensorMap& tb, c
   }
 }
 
+static int w4_token_tile(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 96 ? 96 : 128; }
+
+// fp16 rows and their factors at the end of the workspace: [.. partial sums ..][fp16 rows][row factors]
+static size_t w4_rows_bytes(int T, int K) { return ((size_t)T * K * 2 + (size_t)T * 4 + 255) & ~(size_t)255; }
+
+// Form and splits over K of a dense product. One CTA per SM streams whole items, so the time goes by the rounds of items over the SMs. In
+// units of 10 ns, fitted to 72 products of 1024 .. 57344 features, K of 1024 .. 28672 and 8 .. 128 tokens (what is chosen is 0.6 % behind the best
+// in the mean, 6 % at most): a slot of 256 values of K takes 68 to 88 by the token tile in the fp16 form, 99 to 107 in the bf16 form; an
+// item 21 to 301 more until its sums have left; partial sums a kernel of 134, 48 a split, and their bytes at 12.7 TB/s; the conversion of the
+// rows 141 and 2 per 10000 values. (By rounds alone 64 x 24576 x 4096 was cut in eight: 52 us for 31. The conversion of 128 rows of
+// 1024 took 3 of 12 us.)
+W4Plan w4_plan(int T, int N, int K, int sms, bool f16, size_t workspace_bytes) {
+  const int bn = w4_token_tile(T);
+  const size_t rows_bytes = w4_rows_bytes(T, K) + 256;
+  if (workspace_bytes < rows_bytes) f16 = false;
+  const int m_tiles = (N + W4_BM - 1) / W4_BM, slots = (K / W4_BK + 3) / 4, tile = bn == 16 ? 0 : bn == 32 ? 1 : bn == 64 ? 2 : bn == 96 ? 3 : 4;
+  W4Plan best{1, false};
+  long long least = -1;
+  for (int form = 0; form <= (f16 ? 1 : 0); ++form) {
+    for (int s = 1; s <= std::min(8, slots); ++s) {
+      if (s > 1 && (size_t)s * T * N * 4 > workspace_bytes - (form ? rows_bytes : 0)) break;
+      const int per = (slots + s - 1) / s, parts = (slots + per - 1) / per;
+      const long long rounds = ((long long)m_tiles * parts + sms - 1) / sms;
+      const long long cost = rounds * (per * (form ? 68 + 5 * tile : 99 + 2 * tile) + 21 + 70 * tile) + (form ? 141 + (long long)T * K / 5000 : 0) +
+                             (parts > 1 ? 134 + 48 * parts + (long long)((double)parts * T * N * 8 / 127000.0) : 0);
+      if (least < 0 || cost < least) { least = cost; best = W4Plan{s, form == 1}; }
+    }
+  }
+  return best;
+}
+
 // y[T][N] = x[T][K] * dequant(codes, scales)^T * alpha (+ bias); T <= 128. f16: the block scales of the format allow the fp16 form
-// (NVFP4 always; MXFP4 with scales of 104 .. 140, or 0); the rows are converted into the end of the workspace first.
+// (NVFP4 always; MXFP4 with scales of 104 .. 140, or 0), which the plan takes where it is faster: the rows are then converted into the end of
+// the workspace first.
 int linear_w4a16(const void* x, long long ldx, const void* codes, const void* scales, int fmt, float alpha,
                  const void* bias, void* y, long long ldy, int T, int N, int K, void* workspace, size_t workspace_bytes,
                  int* status, cudaStream_t stream, bool f16) {
@@ -654,10 +686,11 @@ int linear_w4a16(const void* x, long long ldx, const void* codes, const void* sc
   a.M = N; a.N = T; a.K = K; a.m_tiles = (N + W4_BM - 1) / W4_BM; a.k_blocks = K / W4_BK; a.fmt = fmt;
   a.ldc = ldy; a.out = reinterpret_cast<uint16_t*>(y); a.scales = reinterpret_cast<const uint8_t*>(scales);
   a.alpha = alpha; a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.status = status;
-  const int bn = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 96 ? 96 : 128;
-  // [.. partial sums ..][fp16 rows][row factors]
-  const size_t rows_bytes = ((size_t)T * K * 2 + (size_t)T * 4 + 255) & ~(size_t)255;
-  a.f16 = f16 && fmt != 2 && workspace && workspace_bytes >= rows_bytes + 256;
+  const int bn = w4_token_tile(T);
+  const size_t rows_bytes = w4_rows_bytes(T, K);
+  const W4Plan plan = w4_plan(T, N, K, sm_count(), f16 && fmt != 2, workspace ? workspace_bytes : 0);
+  const int splits = plan.splits;
+  a.f16 = plan.f16;
   int launches = 1;
   if (a.f16) {
     uint8_t* end = reinterpret_cast<uint8_t*>(reinterpret_cast<uintptr_t>(workspace) + workspace_bytes & ~(uintptr_t)255);
@@ -668,18 +701,6 @@ int linear_w4a16(const void* x, long long ldx, const void* codes, const void* sc
     workspace_bytes -= rows_bytes + 256;
     ++launches;
   }
-  // One CTA per SM streams whole items: split K where the rounds over the SMs, times the length of an item, become fewer. A split costs
-  // its partial sums and one kernel more, so it has to save a tenth.
-  int splits = 1;
-  {
-    const int slots = (a.k_blocks + 3) / 4, sms = sm_count();
-    long long best = (long long)((a.m_tiles + sms - 1) / sms) * slots * 9;
-    for (int s = 2; s <= std::min(8, slots / 2); ++s) {
-      const long long cost = (long long)((a.m_tiles * s + sms - 1) / sms) * ((slots + s - 1) / s) * 10;
-      if (cost < best) { best = cost; splits = s; }
-    }
-  }
-  while (splits > 1 && (!workspace || (size_t)splits * T * N * 4 > workspace_bytes)) --splits;
   a.kb_per_split = ((a.k_blocks + splits - 1) / splits + 3) & ~3;      // code slots cover four K steps
   a.k_splits = (a.k_blocks + a.kb_per_split - 1) / a.kb_per_split;
   a.ws = reinterpret_cast<float*>(workspace);

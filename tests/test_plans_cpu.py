@@ -24,9 +24,9 @@ def plan():
     if not LIB_CUDA.exists():
         pytest.skip("the CUDA library is not built")
 
-    def ask(calls):
+    def ask(calls, rule="linear_plan_pair"):
         code = ("import json, sys\nfrom fllm_b200.ops._lib import load_cuda\nk = load_cuda(build_if_missing=False)\n"
-                "print(json.dumps([k.linear_plan_pair(*c) for c in json.load(sys.stdin)]))")
+                f"print(json.dumps([k.{rule}(*c) for c in json.load(sys.stdin)]))")
         out = subprocess.run([sys.executable, "-c", code], input=json.dumps(calls), capture_output=True, text=True, check=True, cwd=ROOT.parent, timeout=300)
         return json.loads(out.stdout.splitlines()[-1])
     return ask
@@ -48,3 +48,31 @@ def test_plan_of_pairs_keeps_to_its_limits(plan):
             assert t > 128 and n >= 256 and n % 8 == 0 and k >= 64
         if p > 1:
             assert not (gated and not deferred) and 65536 + p * t * n * 4 <= ws and p * 4 <= -(-k // 64)
+
+
+# us of packed 4-bit products by [fp16 form][splits over K]
+PACKED = {(64, 24576, 4096): {1: {1: 30.9, 2: 30.2, 3: 30.6, 4: 36.8, 6: 42.5, 8: 52.4}, 0: {1: 38.2, 2: 38.8, 3: 37.6, 8: 53.2}},
+          (128, 24576, 4096): {1: {1: 38.0, 2: 41.4, 3: 45.7, 8: 73.9}, 0: {1: 40.9, 2: 43.2, 8: 69.5}},
+          (128, 1024, 1024): {1: {1: 9.4, 2: 11.8, 4: 11.5}, 0: {1: 6.9, 2: 8.9, 4: 8.6}},
+          (8, 57344, 8192): {1: {1: 91.9, 2: 85.4, 4: 83.5}, 0: {1: 138.9, 2: 125.6, 4: 121.5}},
+          (128, 16384, 2048): {1: {1: 15.6, 2: 24.6, 4: 35.1}, 0: {1: 14.0, 2: 23.3, 8: 46.5}},
+          (64, 8192, 28672): {1: {1: 90.2, 2: 59.0, 4: 60.8}, 0: {1: 124.8, 2: 70.8, 4: 71.8}},
+          (16, 4096, 12288): {1: {1: 37.6, 2: 22.9, 3: 18.6, 4: 17.4, 8: 17.9}, 0: {1: 53.4, 4: 17.5, 8: 18.0}},
+          (96, 28672, 4096): {1: {1: 34.0, 2: 41.5, 4: 53.1}, 0: {1: 40.0, 2: 50.4, 8: 82.4}}}
+
+
+def test_packed_products_take_a_fast_form(plan):
+    """Within a tenth of the fastest measured form and number of splits."""
+    got = plan([[t, n, k, 148, WORKSPACE - 65536, True] for t, n, k in PACKED], "linear_w4_plan")
+    for (size, times), (splits, f16) in zip(PACKED.items(), got):
+        assert times[f16][splits] <= 1.1 * min(min(v.values()) for v in times.values()), (size, splits, f16)
+
+
+def test_plan_of_packed_products_keeps_to_its_limits(plan):
+    """Partial sums and fp16 rows that have to fit the workspace together, weights that are not exact in fp16, no workspace at all."""
+    calls = [[t, n, k, 148, ws, f16] for t in (1, 16, 17, 97, 128) for n in (8, 136, 1024, 57344) for k in (64, 320, 4096, 28672)
+             for ws in (0, 4096, 1 << 20, 8 << 20, WORKSPACE) for f16 in (False, True)]
+    for (t, n, k, sms, ws, f16), (splits, form) in zip(calls, plan(calls, "linear_w4_plan")):
+        rows = (t * k * 2 + t * 4 + 255) // 256 * 256 + 256
+        assert 1 <= splits <= 8 and splits <= -(-k // 256) and form <= f16
+        assert (splits * t * n * 4 if splits > 1 else 0) + (rows if form else 0) <= ws
