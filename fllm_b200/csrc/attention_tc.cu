@@ -244,12 +244,13 @@ __global__ void __launch_bounds__(128) fa_decode_kernel(const FaParams p) {
   const int G = p.group;
   pdl_launch_dependents();
   // Under a prefill kernel the inputs are there already (that kernel started after all before it had ended); what waits for this kernel has
-  // to wait for that one, too, so this one ends after it.
+  // to wait for that one, too, so this one's last CTA ends after it (all of them would hold the SMs from the CTAs still to come).
+  const bool last_cta = blockIdx.x + 1 == gridDim.x && blockIdx.y + 1 == gridDim.y && blockIdx.z + 1 == gridDim.z;
   if (!p.under_prefill) pdl_wait();
   const int q0 = p.q_starts[seq];
   const int qn = p.q_starts[seq + 1] - q0;
   if (qn <= 0 || qn > p.decode_max_q) {
-    if (p.under_prefill) pdl_wait();
+    if (p.under_prefill && last_cta) pdl_wait();
     return;
   }
   const int kv_len = p.kv_lens[seq];
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(128) fa_decode_kernel(const FaParams p) {
       }
     }
   }
-  if (p.under_prefill) pdl_wait();
+  if (p.under_prefill && last_cta) pdl_wait();
 }
 
 // One warp per (token row, head): combine split partials, add the sink, normalise. Every lane fetches one split's maximum and sum (at most

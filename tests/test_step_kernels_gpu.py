@@ -262,3 +262,51 @@ def test_prompt_attention_rescales_between_halves(ops, D, hq, hkv, window, kv):
     y = ops.attention(q, kc, vc, tables, rows, pos, hq, hkv, D, D ** -0.5, window, None, 0.0, meta=meta)
     assert _rel(y, torch.cat(ref)) < 2 ** -8
     assert ops.check_status() == 0
+
+
+def _attention(ops, q_lens, kv_lens, D, hq, hkv, window, softcap=0.0, sinks=False, seed=1):
+    """Paged attention of sequences whose last q_lens tokens are queries -> (kernel's result, the same in 64 bits)."""
+    from types import SimpleNamespace
+    G, n = hq // hkv, len(kv_lens)
+    per = [(x + 15) // 16 for x in kv_lens]
+    tables = torch.zeros(n, max(per), dtype=torch.int32, device="cuda")
+    order = torch.randperm(sum(per), generator=torch.Generator().manual_seed(seed)).int().cuda()
+    kc, vc, q = _rand((sum(per), hkv, 16, D), seed + 1), _rand((sum(per), hkv, 16, D), seed + 2), _rand((sum(q_lens), hq * D), seed + 3)
+    sk = _rand((hq,), seed + 4).float() if sinks else None
+    starts, ref, o = [0], [], 0
+    for m, x, b in zip(q_lens, kv_lens, per):
+        blocks = order[o:o + b]
+        tables[len(starts) - 1, :b] = blocks
+        o += b
+        k, v = (c[blocks.long()].double().transpose(1, 2).reshape(-1, hkv, D)[:x].repeat_interleave(G, 1) for c in (kc, vc))
+        s = torch.einsum("qhd,khd->hqk", q[starts[-1]:starts[-1] + m].double().view(m, hq, D), k) * D ** -0.5
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        d = torch.arange(x - m, x, device="cuda")[:, None] - torch.arange(x, device="cuda")[None, :]
+        s = s.masked_fill((d < 0) | ((d >= window) if window else (d < 0)), float("-inf"))
+        if sinks:
+            s = torch.cat([s, sk.double()[:, None, None].expand(hq, m, 1)], -1)
+        p = torch.softmax(s, -1)[..., :x]
+        ref.append(torch.einsum("hqk,khd->qhd", p, v).reshape(m, hq * D))
+        starts.append(starts[-1] + m)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    meta = SimpleNamespace(q_starts=torch.tensor(starts, **i32), seq_lens=torch.tensor(kv_lens, **i32), num_seqs=n, max_q_len=max(q_lens),
+                           min_q_len=min(q_lens), max_kv_len=max(kv_lens))
+    rows = torch.tensor([i for i, m in enumerate(q_lens) for _ in range(m)], **i32)
+    pos = torch.tensor([x - m + j for m, x in zip(q_lens, kv_lens) for j in range(m)], **i32)
+    y = ops.attention(q, kc, vc, tables, rows, pos, hq, hkv, D, D ** -0.5, window, sk, softcap, meta=meta)
+    assert ops.check_status() == 0
+    return y, torch.cat(ref)
+
+
+@pytest.mark.parametrize("D,hq,hkv,window", [(128, 32, 8, 0), (64, 64, 8, 128), (64, 32, 8, 0), (128, 16, 16, 100)])
+@pytest.mark.parametrize("q_lens", [[1] * 40 + [300], [300] + [1] * 40, [1, 2, 700, 1, 64, 1, 1, 129, 1], [1] * 500 + [40], [1] * 3 + [1000, 1000] + [2] * 200])
+def test_decode_rows_beside_prompts(ops, D, hq, hkv, window, q_lens):
+    """Many decode rows and a few prompts in one call, in any order: every row is written, none by another's tile."""
+    kv = [m + (i * 37) % 300 for i, m in enumerate(q_lens)]
+    y, ref = _attention(ops, q_lens, kv, D, hq, hkv, window)
+    o = 0
+    for m in q_lens:
+        assert _rel(y[o:o + m], ref[o:o + m]) < 2 ** -7     # (a single row: twice the mean square of all)
+        o += m
+    assert _rel(y, ref) < 2 ** -8
