@@ -299,6 +299,16 @@ def _attention(ops, q_lens, kv_lens, D, hq, hkv, window, softcap=0.0, sinks=Fals
     return y, torch.cat(ref)
 
 
+@pytest.mark.parametrize("D,hq,hkv", [(128, 32, 8), (64, 64, 8)])
+@pytest.mark.parametrize("window", [1, 127, 128, 129, 159, 160, 161, 191, 192, 193, 256, 300, 511, 2000])
+@pytest.mark.parametrize("sinks", [False, True])
+def test_prompt_attention_under_windows(ops, D, hq, hkv, window, sinks):
+    """Windows around the tiles of 128 keys and the 32 and 64 queries of a tile: tiles that every row sees whole, and those at both edges.
+    Probabilities and results are rounded to bf16 once each: 2^-9 + 2^-9."""
+    y, ref = _attention(ops, (700, 513, 1, 300), (700, 1100, 400, 333), D, hq, hkv, window, sinks=sinks)
+    assert _rel(y, ref) < 2 ** -8
+
+
 @pytest.mark.parametrize("D,hq,hkv,window", [(128, 32, 8, 0), (64, 64, 8, 128), (64, 32, 8, 0), (128, 16, 16, 100)])
 @pytest.mark.parametrize("q_lens", [[1] * 40 + [300], [300] + [1] * 40, [1, 2, 700, 1, 64, 1, 1, 129, 1], [1] * 500 + [40], [1] * 3 + [1000, 1000] + [2] * 200])
 def test_decode_rows_beside_prompts(ops, D, hq, hkv, window, q_lens):
