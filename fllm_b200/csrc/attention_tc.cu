@@ -668,7 +668,7 @@ static int launch_tc(FaParams p, int tokens, int num_seqs, int max_q_len, int mi
   if (tmem) {
     attention_prefill_tmem(p.q, p.ldq, p.k_cache, p.v_cache, p.num_kv_blocks, p.block_tables, p.max_blocks, p.q_starts,
                            p.kv_lens, p.out, p.ldo, num_seqs, max_q_len, decode_max_q + 1, p.hq, p.hkv, D, p.scale,
-                           p.window, p.sinks, p.softcap, p.status, s, 0, p.bidir);
+                           p.window, p.sinks, p.softcap, p.status, s, 0, p.bidir, min_q_len <= decode_max_q ? tokens : 0);
     ++launches;
   }
   if (decode_max_q >= 1 && min_q_len <= decode_max_q) {

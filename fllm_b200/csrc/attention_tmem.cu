@@ -56,6 +56,7 @@ struct FaTmemParams {
   float scale_log2, softcap, scale;
   int tile_variant;      // 0: pick by shape; 1 / 2: force one / two query tiles per CTA
   int bidir;             // 1: no causal mask, every query row sees all kv_len tokens (encoders)
+  int list_seqs;         // > 0: blockIdx.x counts the tiles of these sequences' prompts (tile_of_list), blockIdx.z is 0
 };
 
 __device__ __forceinline__ float ex2(float x) {
@@ -306,6 +307,41 @@ __device__ __forceinline__ void store_row(const FaTmemParams& p, uint32_t t_o, b
   }
 }
 
+// The CTA's sequence and query tile when it is the blockIdx.x-th tile of all prompts; false past the last. (A CTA per tile and sequence
+// leaves the decode rows of a mixed step CTAs that find nothing to do, each of which still takes an SM for its launch: 200 rows beside a prompt
+// of 1500, 64 query and 8 key heads of 64, window of 128: 442 -> 77 us with the decode rows.) Called by all THREADS; sums over as many sequences
+// at a time.
+template <int THREADS>
+__device__ bool tile_of_list(const FaTmemParams& p, int rq, int& seq, int& tile) {
+  __shared__ int warp_sum[THREADS / 32], found[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, want = blockIdx.x;
+  if (threadIdx.x == 0) found[0] = -1;
+  int before = 0;
+  for (int s0 = 0; s0 < p.list_seqs; s0 += THREADS) {
+    const int s = s0 + threadIdx.x;
+    const int qn = s < p.list_seqs ? p.q_starts[s + 1] - p.q_starts[s] : 0;
+    const int mine = qn >= p.min_q ? (qn + rq - 1) / rq : 0;
+    int sum = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += v;
+    }
+    if (lane == 31) warp_sum[warp] = sum;
+    __syncthreads();
+    int first = before + sum - mine;
+    for (int w = 0; w < THREADS / 32; ++w) {
+      if (w < warp) first += warp_sum[w];
+      before += warp_sum[w];
+    }
+    if (want >= first && want < first + mine) { found[0] = s; found[1] = mine - 1 - (want - first); }      // the longest KV range first
+    __syncthreads();
+    if (found[0] >= 0 || want < before) break;
+  }
+  seq = found[0]; tile = found[1];
+  return seq >= 0;
+}
+
 template <int D>
 __global__ void __launch_bounds__(kThreadsT, 2)
 fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_constant__ CUtensorMap tma_v,
@@ -328,10 +364,11 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;      // the tiles with the longest KV range start first
-  const int kvh = blockIdx.y, seq = blockIdx.z;
+  int qt = gridDim.x - 1 - blockIdx.x, seq = blockIdx.z;      // the tiles with the longest KV range start first
+  const int kvh = blockIdx.y;
   const int G = p.group;
   const int RQ = kRowsT / G;
+  if (p.list_seqs > 0 && !tile_of_list<kThreadsT>(p, RQ, seq, qt)) return;
   const int q0 = p.q_starts[seq];
   const int qn = p.q_starts[seq + 1] - q0;
   if (qn < p.min_q) return;
@@ -511,10 +548,11 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  const int qt = gridDim.x - 1 - blockIdx.x;
-  const int kvh = blockIdx.y, seq = blockIdx.z;
+  int qt = gridDim.x - 1 - blockIdx.x, seq = blockIdx.z;
+  const int kvh = blockIdx.y;
   const int G = p.group;
   const int RQ = 2 * kRowsT / G;
+  if (p.list_seqs > 0 && !tile_of_list<kThreadsT2>(p, RQ, seq, qt)) return;
   const int q0 = p.q_starts[seq];
   const int qn = p.q_starts[seq + 1] - q0;
   if (qn < p.min_q) return;
@@ -721,7 +759,7 @@ struct MapKeyHash {
 struct MapPair { CUtensorMap k, v; };
 
 template <int D>
-void launch_tmem(const MapPair& maps, const FaTmemParams& p, int max_q_len, int num_seqs, cudaStream_t s) {
+void launch_tmem(const MapPair& maps, FaTmemParams p, int max_q_len, int num_seqs, int mixed_rows, cudaStream_t s) {
   static bool configured[kMaxDevices] = {};
   if (first_call_on_device(configured)) {
     cuda_check(cudaFuncSetAttribute(fa_prefill_tmem_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_one<D>()),
@@ -734,14 +772,14 @@ void launch_tmem(const MapPair& maps, const FaTmemParams& p, int max_q_len, int 
   const int rq2 = 2 * kRowsT / p.group;
   const long long ctas2 = (long long)((max_q_len + rq2 - 1) / rq2) * p.hkv * num_seqs;
   const bool two = forced ? forced == 2 : (max_q_len * p.group >= 2 * kRowsT && ctas2 >= sm_count());
-  if (two) {
-    dim3 grid((max_q_len + rq2 - 1) / rq2, p.hkv, num_seqs);
-    fa_prefill_tmem2_kernel<D><<<grid, kThreadsT2, smem_two<D>(), s>>>(maps.k, maps.v, p);
-  } else {
-    const int rq = kRowsT / p.group;
-    dim3 grid((max_q_len + rq - 1) / rq, p.hkv, num_seqs);
-    fa_prefill_tmem_kernel<D><<<grid, kThreadsT, smem_one<D>(), s>>>(maps.k, maps.v, p);
+  const int rq = two ? rq2 : kRowsT / p.group, tiles = (max_q_len + rq - 1) / rq;
+  dim3 grid(tiles, p.hkv, num_seqs);
+  if (mixed_rows > 0) {                // P prompts of q rows each have at most sum(q) / rq + P tiles
+    const long long bound = mixed_rows / rq + min(num_seqs, mixed_rows / max(p.min_q, 1));
+    if (bound < (long long)tiles * num_seqs) { grid = dim3((unsigned)bound, p.hkv, 1); p.list_seqs = num_seqs; }
   }
+  if (two) fa_prefill_tmem2_kernel<D><<<grid, kThreadsT2, smem_two<D>(), s>>>(maps.k, maps.v, p);
+  else fa_prefill_tmem_kernel<D><<<grid, kThreadsT, smem_one<D>(), s>>>(maps.k, maps.v, p);
   cuda_check(cudaGetLastError(), "fa_prefill_tmem launch");
 }
 
@@ -756,7 +794,7 @@ void attention_prefill_tmem(const void* q, long long ldq, const void* k_cache, c
                             const int* block_tables, int max_blocks, const int* q_starts, const int* kv_lens,
                             void* out, long long ldo, int num_seqs, int max_q_len, int min_q, int hq, int hkv,
                             int head_dim, float scale, int window, const float* sinks, float softcap, int* status,
-                            cudaStream_t s, int tile_variant, int bidir) {
+                            cudaStream_t s, int tile_variant, int bidir, int mixed_rows) {
   static std::unordered_map<MapKey, MapPair, MapKeyHash> maps;
   const uint64_t rows = (uint64_t)num_blocks * hkv * kPageT;
   const MapKey key{k_cache, v_cache, rows, head_dim};
@@ -779,8 +817,8 @@ void attention_prefill_tmem(const void* q, long long ldq, const void* k_cache, c
   p.scale = scale; p.scale_log2 = scale * kLog2eT; p.softcap = softcap;
   p.tile_variant = tile_variant;
   p.bidir = bidir;
-  if (head_dim == 64) launch_tmem<64>(it->second, p, max_q_len, num_seqs, s);
-  else launch_tmem<128>(it->second, p, max_q_len, num_seqs, s);
+  if (head_dim == 64) launch_tmem<64>(it->second, p, max_q_len, num_seqs, mixed_rows, s);
+  else launch_tmem<128>(it->second, p, max_q_len, num_seqs, mixed_rows, s);
 }
 
 }  // namespace fllm

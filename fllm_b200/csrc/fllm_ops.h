@@ -261,7 +261,8 @@ void attention_prefill_tmem(const void* q, long long ldq, const void* k_cache, c
                             const int* block_tables, int max_blocks, const int* q_starts, const int* kv_lens,
                             void* out, long long ldo, int num_seqs, int max_q_len, int min_q, int hq, int hkv,
                             int head_dim, float scale, int window, const float* sinks, float softcap, int* status,
-                            cudaStream_t s, int tile_variant = 0, int bidir = 0);
+                            cudaStream_t s, int tile_variant = 0, int bidir = 0,
+                            int mixed_rows = 0);   // > 0: shorter sequences are among them, and so many query rows in all
 size_t attention_tc_workspace_bytes(int tokens, int hq, int head_dim, int max_splits);
 
 // ---- sampling -----------------------------------------------------------------------
