@@ -410,17 +410,17 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   // 89.8 -> 82.0 us, 16 x 28672 x 4096 27.6 -> 23.5); with few tiles one CTA and its whole ring are faster (1 x 16384 x 2048 9.7 against 10.3).
   int bn = T <= 16 ? 16 : (T <= 32 ? 32 : 64), splits = 1, whole = 0, per = 1;
   const int deep = (a.k_blocks + 63) / 64, least = swap ? deep : 1;   // swap-AB: the token scales of a split fit their shared-memory block
-  // Tiles of up to 64 tokens store pairs of features, wider ones eight at a time; the kernels that add partial sums store four.
-  const int unit = swap ? 2 : 8;
-  if (ldy % unit || reinterpret_cast<uintptr_t>(y) % (2 * unit))
-    throw std::runtime_error("linear_fp8_block: output rows must be aligned to 4 bytes for up to 64 tokens, to 16 for more");
-  const bool can_split = workspace && (ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0;
+  // Tiles of up to 64 tokens store pairs of features, wider ones eight at a time; the kernels that add partial sums store four. So rows
+  // aligned to 4 bytes are not split, and more than 64 tokens go into rows aligned to 8 bytes only as partial sums of all tiles.
+  auto rows_of = [&](int n) { return ldy % n == 0 && reinterpret_cast<uintptr_t>(y) % (2 * n) == 0; };
+  const bool can_split = workspace && rows_of(4), can_store = rows_of(swap ? 2 : 8);
   long long best = -1;
   for (int w : {swap ? bn : 256, swap ? 0 : 128, swap ? 0 : 64}) {
     if (w == 0 || (w == 256 && N % 256)) continue;
     const int n_tiles = (a.N + w - 1) / w;
     const long long block = swap ? 37 : a.m_tiles == 1 ? (w == 256 ? 74 : w == 128 ? 37 : 28) : (w == 256 ? 60 : w == 128 ? 36 : 28);
     for (int s = least; s <= 16 * deep && s <= a.k_blocks; ++s) {
+      if (s == 1 && !can_store) continue;
       if (s > 1 && (!can_split || (size_t)s * T * N * 4 > workspace_bytes)) break;
       const long long items = (long long)a.m_tiles * n_tiles * s;
       for (int two = 1; two <= (w == 16 ? 2 : 1); ++two) {
@@ -431,7 +431,7 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
       }
     }
     const long long tiles = (long long)a.m_tiles * n_tiles, first = tiles / sms * sms, tail = tiles - first;
-    if (swap || least > 1 || !can_split || first == 0) continue;
+    if (swap || !can_split || !can_store || first == 0) continue;
     for (int s = 2; s <= 16 && s <= a.k_blocks && tail; ++s) {
       const long long bytes = s * tail * F8_BM * w * 4;
       if ((size_t)bytes > workspace_bytes) break;
@@ -439,6 +439,8 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
       if (best < 0 || cost < best) { best = cost; bn = w; splits = s; whole = (int)first; }
     }
   }
+  if (best < 0 && !can_store)
+    throw std::runtime_error("linear_fp8_block: output rows must be aligned to 4 bytes for up to 64 tokens, to 16 for more (8 where there is room for partial sums)");
   if (best < 0) throw std::runtime_error("linear_fp8_block: K above 8192 needs a split-K workspace and output rows aligned to 8 bytes");
   a.n_tiles = (a.N + bn - 1) / bn;
   const CUtensorMap tw = make_tmap_2d(wq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, K, swap ? F8_BM : bn, F8_BK, true);

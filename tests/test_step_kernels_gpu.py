@@ -161,6 +161,22 @@ def test_fp8_block_into_rows_of_four_bytes(ops, T, N, K):
         ops.linear(wide, w, out=torch.zeros(65, N + 6, dtype=torch.bfloat16, device="cuda")[:, 2:2 + N])
 
 
+@pytest.mark.parametrize("T,N,K", [(65, 7168, 8192), (128, 1280, 8192), (300, 2048, 1024), (1000, 7168, 256)])
+def test_fp8_block_of_many_tokens_into_rows_of_eight_bytes(ops, T, N, K):
+    """Stored by the kernel that adds partial sums, four features at a time; where there is no room for them, refused."""
+    from fllm_b200.ops.native import Fp8BlockWeight, quantize_weight_fp8_block
+    x, w = _rand((T, K), 1), Fp8BlockWeight(*quantize_weight_fp8_block(_rand((N, K), 2, 0.05)))
+    want = ops.linear(x, w)
+    out = torch.zeros(T, N + 12, dtype=torch.bfloat16, device="cuda")
+    ops.linear(x, w, out=out[:, 4:4 + N])
+    assert _rel(out[:, 4:4 + N], want.double()) < 3.4e-3 and not out[:, :4].any() and not out[:, 4 + N:].any()     # (one rounding each)
+    xq, sx = torch.empty(T, K, dtype=torch.uint8, device="cuda"), torch.empty(T, K // 128, device="cuda")
+    ops.k.quant_fp8_1x128(x, xq, sx)
+    with pytest.raises(RuntimeError, match="aligned"):
+        ops.k.linear_fp8_block(xq, sx, w.wq, w.sw, None, out[:, 4:4 + N], ops.status, None)
+    assert ops.check_status() == 0
+
+
 @pytest.mark.parametrize("T", [147, 148, 301])
 @pytest.mark.parametrize("D,hq,hkv", [(64, 5, 1), (64, 64, 8), (128, 3, 3), (128, 32, 8)])
 @pytest.mark.parametrize("norm", [False, True])
