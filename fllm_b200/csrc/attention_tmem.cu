@@ -775,7 +775,7 @@ void launch_tmem(const MapPair& maps, FaTmemParams p, int max_q_len, int num_seq
   const int rq = two ? rq2 : kRowsT / p.group, tiles = (max_q_len + rq - 1) / rq;
   dim3 grid(tiles, p.hkv, num_seqs);
   if (mixed_rows > 0) {                // P prompts of q rows each have at most sum(q) / rq + P tiles
-    const long long bound = mixed_rows / rq + min(num_seqs, mixed_rows / max(p.min_q, 1));
+    const long long bound = max(1, mixed_rows / rq + min(num_seqs, mixed_rows / max(p.min_q, 1)));    // (max_q_len may be an upper bound)
     if (bound < (long long)tiles * num_seqs) { grid = dim3((unsigned)bound, p.hkv, 1); p.list_seqs = num_seqs; }
   }
   if (two) fa_prefill_tmem2_kernel<D><<<grid, kThreadsT2, smem_two<D>(), s>>>(maps.k, maps.v, p);

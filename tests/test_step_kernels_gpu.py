@@ -280,7 +280,7 @@ def test_prompt_attention_rescales_between_halves(ops, D, hq, hkv, window, kv):
     assert ops.check_status() == 0
 
 
-def _attention(ops, q_lens, kv_lens, D, hq, hkv, window, softcap=0.0, sinks=False, seed=1):
+def _attention(ops, q_lens, kv_lens, D, hq, hkv, window, softcap=0.0, sinks=False, seed=1, longest=0):
     """Paged attention of sequences whose last q_lens tokens are queries -> (kernel's result, the same in 64 bits)."""
     from types import SimpleNamespace
     G, n = hq // hkv, len(kv_lens)
@@ -306,7 +306,7 @@ def _attention(ops, q_lens, kv_lens, D, hq, hkv, window, softcap=0.0, sinks=Fals
         ref.append(torch.einsum("hqk,khd->qhd", p, v).reshape(m, hq * D))
         starts.append(starts[-1] + m)
     i32 = dict(dtype=torch.int32, device="cuda")
-    meta = SimpleNamespace(q_starts=torch.tensor(starts, **i32), seq_lens=torch.tensor(kv_lens, **i32), num_seqs=n, max_q_len=max(q_lens),
+    meta = SimpleNamespace(q_starts=torch.tensor(starts, **i32), seq_lens=torch.tensor(kv_lens, **i32), num_seqs=n, max_q_len=max(longest, *q_lens),
                            min_q_len=min(q_lens), max_kv_len=max(kv_lens))
     rows = torch.tensor([i for i, m in enumerate(q_lens) for _ in range(m)], **i32)
     pos = torch.tensor([x - m + j for m, x in zip(q_lens, kv_lens) for j in range(m)], **i32)
@@ -336,3 +336,10 @@ def test_decode_rows_beside_prompts(ops, D, hq, hkv, window, q_lens):
         assert _rel(y[o:o + m], ref[o:o + m]) < 2 ** -7     # (a single row: twice the mean square of all)
         o += m
     assert _rel(y, ref) < 2 ** -8
+
+
+@pytest.mark.parametrize("q_lens", [[1], [1, 2], [1, 2, 7]])
+def test_longest_prompt_given_as_an_upper_bound(ops, q_lens):
+    """Fewer rows in all than the shortest prompt has: the prompt kernel finds nothing or one sequence, the decode kernel does the rest."""
+    y, ref = _attention(ops, q_lens, [m + 50 for m in q_lens], 128, 32, 8, 0, longest=64)
+    assert _rel(y, ref) < 2 ** -7
