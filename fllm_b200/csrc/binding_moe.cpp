@@ -70,19 +70,21 @@ void moe_route_fp32(const optional<Tensor>& logits, const optional<Tensor>& work
 
 void moe_align(const Tensor& ids, int64_t experts, int64_t expert_lo, int64_t expert_hi, int64_t bn, Tensor row_of,
                Tensor token_of, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, const optional<Tensor>& weights,
-               const optional<Tensor>& row_weight) {
+               const optional<Tensor>& row_weight, const optional<Tensor>& tile_rows) {
   TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == at::kInt && ids.dim() == 2 && ids.is_contiguous(), "ids: [tokens, k] int32");
   TORCH_CHECK(num_tiles.numel() >= 2 && expert_lo >= 0 && expert_lo <= expert_hi && expert_hi <= experts, "num_tiles needs two ints; a range of the experts");
   const bool weighed = row_weight.has_value() && row_weight->defined();
   TORCH_CHECK(!weighed || (weights.has_value() && weights->scalar_type() == at::kFloat && weights->is_contiguous() && weights->numel() == ids.numel() &&
                            row_weight->scalar_type() == at::kFloat && row_weight->is_contiguous() && row_weight->numel() >= token_of.numel()),
               "weights fp32 like ids, row_weight fp32 like token_of");
+  const bool counted = tile_rows.has_value() && tile_rows->defined();
+  TORCH_CHECK(!counted || (tile_rows->scalar_type() == at::kInt && tile_rows->is_contiguous() && tile_rows->numel() >= tile_expert.numel()), "tile_rows: int32 like tile_expert");
   c10::cuda::CUDAGuard guard(ids.device());
   fllm::moe_align(ids.data_ptr<int>(), (int)ids.size(0), (int)ids.size(1), (int)expert_lo, (int)expert_hi,
                   (int)bn, row_of.data_ptr<int>(), token_of.data_ptr<int>(), (int)token_of.numel(),
                   tile_expert.data_ptr<int>(), tile_row0.data_ptr<int>(), num_tiles.data_ptr<int>(),
                   (int)tile_expert.numel(), cur_stream(), weighed ? weights->data_ptr<float>() : nullptr,
-                  weighed ? row_weight->data_ptr<float>() : nullptr);
+                  weighed ? row_weight->data_ptr<float>() : nullptr, counted ? tile_rows->data_ptr<int>() : nullptr);
 }
 
 inline bool f32_rows(const Tensor& t) {
@@ -157,7 +159,7 @@ TORCH_LIBRARY_FRAGMENT(fllm_b200, m) {
         &moe_route_fp32);
   m.def("moe_grouped_linear_f32(Tensor xp, Tensor w_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn) -> ()",
         &moe_grouped_linear_f32);
-  m.def("moe_align(Tensor ids, int experts, int expert_lo, int expert_hi, int bn, Tensor(a!) row_of, Tensor(b!) token_of, Tensor(c!) tile_expert, Tensor(d!) tile_row0, Tensor(e!) num_tiles, Tensor? weights=None, Tensor(f!)? row_weight=None) -> ()", &moe_align);
+  m.def("moe_align(Tensor ids, int experts, int expert_lo, int expert_hi, int bn, Tensor(a!) row_of, Tensor(b!) token_of, Tensor(c!) tile_expert, Tensor(d!) tile_row0, Tensor(e!) num_tiles, Tensor? weights=None, Tensor(f!)? row_weight=None, Tensor(g!)? tile_rows=None) -> ()", &moe_align);
   m.def("moe_gather(Tensor x, Tensor token_of, Tensor(a!) xp, Tensor? row_weight=None) -> ()", &moe_gather);
   m.def("moe_grouped_linear(Tensor xp, Tensor w_stack, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status) -> int", &moe_grouped_linear);
   m.def("moe_combine(Tensor y, Tensor row_of, Tensor? weights, Tensor(a!) out, Tensor? add=None, Tensor? add_gate=None) -> ()", &moe_combine);

@@ -79,6 +79,62 @@ int64_t moe_grouped_linear_w4_f16(const Tensor& xp, const optional<Tensor>& fact
                                      st, cur_stream(), &r);
 }
 
+// x bf16 [tokens, k] -> two pieces of e4m3 per row, xq bytes [rows * 2, k] in groups of 16 rows, and their scale atoms (csrc/gemm_mx4_rows.cu: rows_mx)
+void moe_rows_mx(const Tensor& x, const optional<Tensor>& token_of, Tensor xq, Tensor sf, int64_t bn, const optional<Tensor>& row_weight) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1, "x: bf16 rows");
+  TORCH_CHECK(xq.is_cuda() && xq.element_size() == 1 && xq.dim() == 2 && xq.is_contiguous() && xq.size(1) == x.size(1) && xq.size(0) % 2 == 0, "xq: contiguous bytes [rows * 2, k]");
+  const int64_t rows = xq.size(0) / 2;
+  TORCH_CHECK(bn > 0 && bn % 16 == 0 && rows % bn == 0, "whole tiles of a multiple of 16 rows");
+  TORCH_CHECK(sf.is_cuda() && sf.is_contiguous() && sf.nbytes() >= fllm::mx4_scale_bytes((int)rows, (int)x.size(1), (int)bn, 2), "sf: scale atoms of every tile");
+  const int* t = nullptr;
+  if (token_of.has_value() && token_of->defined()) {
+    TORCH_CHECK(token_of->scalar_type() == at::kInt && token_of->is_contiguous() && token_of->numel() >= rows, "token_of: int32 [rows]");
+    t = token_of->data_ptr<int>();
+  } else {
+    TORCH_CHECK(rows <= x.size(0), "xq: as many rows as x");
+  }
+  const float* w = nullptr;
+  if (row_weight.has_value() && row_weight->defined()) {
+    TORCH_CHECK(row_weight->scalar_type() == at::kFloat && row_weight->is_contiguous() && row_weight->numel() >= rows, "row_weight: fp32 [rows]");
+    w = row_weight->data_ptr<float>();
+  }
+  c10::cuda::CUDAGuard guard(x.device());
+  fllm::rows_mx(x.data_ptr(), x.stride(0), t, w, xq.data_ptr(), sf.data_ptr(), (int)rows, (int)x.size(1), (int)bn, cur_stream());
+}
+
+// Grouped product of such rows (`pieces` each) with a stack of MXFP4 matrices: codes [E, n, k/2] bytes, atoms [E, ceil(n / 128), ceil(k / 128), 512] their
+// scales. y: bf16 [rows, n]; or, with y_sf, the clamped SwiGLU-OAI of it as bytes [rows * 3, n / 2] with the scale atoms y_sf.
+int64_t moe_grouped_linear_mx4(const Tensor& xq, const Tensor& sf, int64_t pieces, const Tensor& codes, const Tensor& atoms, double alpha,
+                               const optional<Tensor>& bias_stack, Tensor y, const optional<Tensor>& y_sf, const Tensor& tile_expert, const Tensor& tile_row0,
+                               const Tensor& tile_rows, const Tensor& num_tiles, int64_t bn, const optional<Tensor>& status, double glu_alpha,
+                               double glu_limit) {
+  TORCH_CHECK(codes.is_cuda() && codes.dim() == 3 && codes.is_contiguous() && codes.element_size() == 1, "codes: contiguous [E, n, k/2] bytes");
+  const int64_t E = codes.size(0), n = codes.size(1), k = codes.size(2) * 2;
+  TORCH_CHECK(k % 128 == 0 || codes.storage().nbytes() >= (size_t)(codes.storage_offset() + codes.numel() + 32), "codes: 32 bytes behind the stack where k % 128 != 0");
+  TORCH_CHECK(atoms.is_cuda() && atoms.is_contiguous() && atoms.nbytes() == (size_t)(E * ((n + 127) / 128) * ((k + 127) / 128) * 512), "atoms: scales of every 128 x 128 codes");
+  TORCH_CHECK((pieces == 2 || pieces == 3) && xq.is_cuda() && xq.dim() == 2 && xq.is_contiguous() && xq.element_size() == 1 && xq.size(1) == k && xq.size(0) % pieces == 0,
+              "xq: bytes [rows * pieces, k]");
+  const int64_t rows = xq.size(0) / pieces;
+  TORCH_CHECK(bn > 0 && rows % bn == 0 && sf.is_cuda() && sf.is_contiguous() && sf.nbytes() >= fllm::mx4_scale_bytes((int)rows, (int)k, (int)bn, (int)pieces), "sf: scale atoms of every tile");
+  TORCH_CHECK(tile_rows.numel() >= tile_expert.numel() && tile_row0.numel() >= tile_expert.numel(), "a row and a number of rows per tile");
+  const fllm::Mx4Rows x{xq.data_ptr(), sf.data_ptr(), (int)rows, (int)pieces};
+  const fllm::Mx4Tiles tiles{tile_expert.data_ptr<int>(), tile_row0.data_ptr<int>(), tile_rows.data_ptr<int>(), num_tiles.data_ptr<int>(), (int)tile_expert.numel(), (int)bn};
+  fllm::Mx4Glu g{(float)glu_alpha, (float)glu_limit, nullptr, nullptr};
+  const bool glu = y_sf.has_value() && y_sf->defined();
+  if (glu) {
+    TORCH_CHECK(y.dim() == 2 && y.is_contiguous() && y.element_size() == 1 && y.size(0) == rows * 3 && y.size(1) == n / 2, "y: bytes [rows * 3, n / 2]");
+    TORCH_CHECK(y_sf->is_cuda() && y_sf->is_contiguous() && y_sf->nbytes() >= fllm::mx4_scale_bytes((int)rows, (int)n / 2, (int)bn, 3), "y_sf: scale atoms of every tile");
+    g.q = y.data_ptr();
+    g.sf = y_sf->data_ptr();
+  } else {
+    TORCH_CHECK(y.dim() == 2 && y.stride(1) == 1 && y.size(0) == rows && y.size(1) == n && y.scalar_type() == at::kBFloat16, "y: [rows, n] bf16");
+  }
+  c10::cuda::CUDAGuard guard(xq.device());
+  int* st = status.has_value() && status->defined() ? status->data_ptr<int>() : nullptr;
+  return fllm::moe_grouped_linear_mx4(x, codes.data_ptr(), atoms.data_ptr(), (int)E, (int)n, (int)k, (float)alpha, optp(bias_stack), y.data_ptr(), y.stride(0),
+                                      glu ? &g : nullptr, tiles, st, cur_stream());
+}
+
 // ---- expert-parallel all-to-all: a context of every rank's buffer addresses, then the four steps
 std::vector<fllm::EpArgs> g_ep;
 
@@ -153,6 +209,8 @@ TORCH_LIBRARY_FRAGMENT(fllm_b200, m) {
   m.def("moe_grouped_linear_w4(Tensor xp, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status) -> int", &moe_grouped_linear_w4);
   m.def("moe_rows_f16(Tensor x, Tensor? token_of, Tensor(a!) xp, Tensor(b!) factor, Tensor? row_weight=None) -> ()", &moe_rows_f16);
   m.def("moe_grouped_linear_w4_f16(Tensor xp, Tensor? factor, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status, float glu_alpha=1.0, float glu_limit=0.0, float glu_scale=0.0) -> int", &moe_grouped_linear_w4_f16);
+  m.def("moe_rows_mx(Tensor x, Tensor? token_of, Tensor(a!) xq, Tensor(b!) sf, int bn, Tensor? row_weight=None) -> ()", &moe_rows_mx);
+  m.def("moe_grouped_linear_mx4(Tensor xq, Tensor sf, int pieces, Tensor codes, Tensor atoms, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor(b!)? y_sf, Tensor tile_expert, Tensor tile_row0, Tensor tile_rows, Tensor num_tiles, int bn, Tensor? status, float glu_alpha=1.0, float glu_limit=0.0) -> int", &moe_grouped_linear_mx4);
   m.def("ep_ctx_create(int ranks, int my_rank, int cap, int hidden, int experts_per_rank, int[] recv_x, int[] recv_meta, int[] ctrl, int[] comb_y) -> int", &ep_ctx_create);
   m.def("ep_dispatch(int ctx, Tensor x, Tensor ids, int epoch, Tensor? status, Tensor(a!)? call_ctr=None) -> ()", &ep_dispatch);
   m.def("ep_ingest(int ctx, int epoch, Tensor(a!) ids_out, Tensor(b!) count_out, Tensor? status, Tensor? call_ctr=None) -> ()", &ep_ingest);

@@ -159,6 +159,23 @@ int moe_grouped_linear_w4(const void* xp, long long ldx, const void* codes_stack
                           float alpha, const void* bias_stack, void* y, long long ldy, int rows_cap, int n_out, int K,
                           int experts, const int* tile_expert, const int* tile_row0, const int* num_tiles, int max_tiles,
                           int bn, int* status, cudaStream_t stream, const W4Rows* rows = nullptr);
+// ---- MXFP4 expert stacks on the block-scaled tensor cores (csrc/gemm_mx4_rows.cu): rows as sums of e4m3 pieces, scales in 512-byte atoms
+struct Mx4Rows {
+  const void *q, *sf;         // [rows * pieces][K] e4m3 bytes; [tiles][ceil(K / 128)][ceil(bn * pieces / 128)][512]
+  int rows, pieces;           // rows: a multiple of the token tile
+};
+struct Mx4Tiles {             // of moe_align
+  const int *expert, *row0, *rows, *count;
+  int max_tiles, bn;
+};
+struct Mx4Glu {               // clamped SwiGLU-OAI in the epilogue; its result as rows of three pieces
+  float alpha, limit;
+  void *q, *sf;
+};
+size_t mx4_scale_bytes(int rows, int K, int bn, int pieces);
+void rows_mx(const void* x, long long ldx, const int* token_of, const float* row_weight, void* xq, void* sf, int rows, int K, int bn, cudaStream_t s);
+int moe_grouped_linear_mx4(const Mx4Rows& x, const void* codes, const void* sfa, int experts, int n_out, int K, float alpha, const void* bias, void* y,
+                           long long ldy, const Mx4Glu* glu, const Mx4Tiles& tiles, int* status, cudaStream_t stream);
 void w4_dequant_bf16(const void* codes, const void* scales, int fmt, float alpha, void* out, long long rows, int K,
                      cudaStream_t s);
 
@@ -202,7 +219,8 @@ void moe_route(const void* logits, long long ld, const void* bias, int tokens, i
                int* ids, float* weights, cudaStream_t s);
 void moe_align(const int* ids, int tokens, int k, int expert_lo, int expert_hi, int bn, int* row_of,
                int* token_of, int rows_cap, int* tile_expert, int* tile_row0, int* num_tiles, int max_tiles,
-               cudaStream_t s, const float* weights = nullptr, float* row_weight = nullptr);   // row_weight [rows_cap]: weights [tokens * k] by row
+               cudaStream_t s, const float* weights = nullptr, float* row_weight = nullptr,   // row_weight [rows_cap]: weights [tokens * k] by row
+               int* tile_rows = nullptr);                                                     // rows that each tile of the list has
 void moe_gather(const void* x, long long ldx, const int* token_of, void* xp, int rows_cap, int hidden, cudaStream_t s,
                 const float* row_weight = nullptr, int f32 = 0);
 // weights null: the rows are summed as they are; add (optional): [tokens] rows added to the result

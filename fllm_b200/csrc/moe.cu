@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
                                                          int rows_cap, int* __restrict__ tile_expert,
                                                          int* __restrict__ tile_row0, int* __restrict__ num_tiles,
                                                          int max_tiles, const float* __restrict__ weights,
-                                                         float* __restrict__ row_weight) {
-  __shared__ int off[512], first_tile[512], cnt[512];
+                                                         float* __restrict__ row_weight, int* __restrict__ tile_rows) {
+  __shared__ int off[512], first_tile[512], cnt[512], sums[512];
   extern __shared__ int fill[];               // [warp][local expert]: counts, then next positions
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int local = expert_hi - expert_lo;
@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
       sum += c;
     }
     cnt[e] = (sum + bn - 1) / bn;             // tiles of the expert
+    sums[e] = sum;
   }
   __syncthreads();
   if (warp == 0) {                            // prefix of the tiles
@@ -295,6 +296,7 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
     for (int t = 0; t < cnt[e] && first_tile[e] + t < max_tiles; ++t) {
       tile_expert[first_tile[e] + t] = e;
       tile_row0[first_tile[e] + t] = off[e] + t * bn;
+      if (tile_rows) tile_rows[first_tile[e] + t] = min(bn, sums[e] - t * bn);
     }
   for (int base = lo; base < hi; base += 32) {
     const int i = base + lane, e = i < hi ? ids[i] - expert_lo : -1;
@@ -315,14 +317,14 @@ __global__ void __launch_bounds__(1024) moe_align_kernel(const int* __restrict__
 
 void moe_align(const int* ids, int tokens, int k, int expert_lo, int expert_hi, int bn, int* row_of,
                int* token_of, int rows_cap, int* tile_expert, int* tile_row0, int* num_tiles, int max_tiles,
-               cudaStream_t s, const float* weights, float* row_weight) {
+               cudaStream_t s, const float* weights, float* row_weight, int* tile_rows) {
   if (expert_hi - expert_lo > 512) throw std::runtime_error("moe_align: at most 512 local experts");
   const size_t smem = (size_t)32 * std::max(expert_hi - expert_lo, 1) * sizeof(int);      // 64 KiB at most
   static bool configured[kMaxDevices] = {};
   if (first_call_on_device(configured))
     cuda_check(cudaFuncSetAttribute(moe_align_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024), "moe_align smem");
   moe_align_kernel<<<1, 1024, smem, s>>>(ids, tokens * k, expert_lo, expert_hi, bn, k, row_of, token_of, rows_cap, tile_expert, tile_row0, num_tiles,
-                                         max_tiles, weights, row_weight);
+                                         max_tiles, weights, row_weight, tile_rows);
   cuda_check(cudaGetLastError(), "moe_align_kernel");
 }
 

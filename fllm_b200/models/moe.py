@@ -134,6 +134,17 @@ def _packed_tile(rows_per_expert: float) -> int:
     return 128
 
 
+def _mx_tile(lw, rows_per_expert: float) -> int:
+    """Token tile of MXFP4 experts on the block-scaled tensor cores (csrc/gemm_mx4_rows.cu), 0: expanded to fp16. A tile's products and reads follow the rows
+    that it has, so a wider one costs slots of codes in flight alone. Tiles hold 80 rows, which nearly every expert of 64 in the mean fits into; with 96 in
+    the mean most experts need two, and the fp16 form's tiles of 128 are faster (us per layer of 128 experts of 2880 x 2880 x 3: 624 against 674 at 64 rows
+    per expert, 1065 against 800 at 96)."""
+    if any(getattr(w, "atoms", None) is None for w in (lw.exp_gate_up, lw.exp_down)) or rows_per_expert > 64:
+        return 0
+    most = rows_per_expert + 3 * math.sqrt(rows_per_expert)
+    return 16 if most <= 16 else 32 if most <= 32 else 80
+
+
 def _dense_experts(lw):
     """LayerWeights view with packed expert stacks expanded (oracle / CPU path)."""
     if isinstance(lw.exp_gate_up, torch.Tensor) and isinstance(lw.exp_down, torch.Tensor):
@@ -197,6 +208,36 @@ def _packed_ffn(cfg, ops, spec: MoeSpec, lw, x: torch.Tensor, token_of, row_w, t
         k_ops.moe_rows_f16(u, None, act, factor)
     y = new(H, torch.bfloat16)
     k_ops.moe_grouped_linear_w4_f16(act, factor, dn.codes, dn.scales, dn.fmt, dn.alpha / scale, lw.exp_down_b, y, *where)
+    return y
+
+
+def _mx_ffn(cfg, ops, spec: MoeSpec, lw, x: torch.Tensor, token_of, row_w, tile_e, tile_r, tile_n, ntiles, bn: int, rows: int) -> torch.Tensor:
+    """Expert networks on MXFP4 stacks without expanding them: rows as sums of two e4m3 pieces, the clamped SwiGLU-OAI in the epilogue of the first product,
+    which writes three; other activations between the products."""
+    H, k_ops = x.shape[1], ops.k
+    gu, dn = lw.exp_gate_up, lw.exp_down
+    where = (tile_e, tile_r, tile_n, ntiles, bn, ops.status)
+
+    def room(pieces, n):
+        atoms = rows // bn * -(-n // 128) * -(-bn * pieces // 128)
+        return (torch.empty(rows * pieces, n, dtype=torch.uint8, device=x.device), torch.empty(atoms, 512, dtype=torch.uint8, device=x.device))
+
+    xq, xs = room(2, H)
+    k_ops.moe_rows_mx(x, token_of, xq, xs, bn, row_w)
+    limit = cfg.swiglu_limit if spec.limit is None else spec.limit
+    if spec.act == "swiglu_oai" and cfg.mlp_kind != "plain" and gu.shape[1] % 128 == 0:
+        pieces = 3
+        aq, as_ = room(3, gu.shape[1] // 2)
+        k_ops.moe_grouped_linear_mx4(xq, xs, 2, gu.codes, gu.atoms, gu.alpha, lw.exp_gate_up_b, aq, as_, *where, cfg.swiglu_alpha, limit)
+    else:
+        pieces = 2
+        u = torch.empty(rows, gu.shape[1], dtype=torch.bfloat16, device=x.device)
+        k_ops.moe_grouped_linear_mx4(xq, xs, 2, gu.codes, gu.atoms, gu.alpha, lw.exp_gate_up_b, u, None, *where)
+        u = ops.act_(u, spec.act) if cfg.mlp_kind == "plain" else ops.glu(u, ACT_KIND.get(spec.act, 0), cfg.swiglu_alpha, limit)
+        aq, as_ = room(2, u.shape[1])
+        k_ops.moe_rows_mx(u, None, aq, as_, bn)
+    y = torch.empty(rows, H, dtype=torch.bfloat16, device=x.device)
+    k_ops.moe_grouped_linear_mx4(aq, as_, pieces, dn.codes, dn.atoms, dn.alpha, lw.exp_down_b, y, None, *where)
     return y
 
 
@@ -284,7 +325,8 @@ def moe_ffn(dec, lw, h: torch.Tensor, xe: Optional[torch.Tensor] = None, add: Op
     share = e_local / spec.experts
     fp16 = h.dtype == torch.bfloat16 and _fp16_experts(lw)
     per_expert = T * k * share / max(e_local, 1)
-    bn = 64 if h.dtype == torch.float32 else _packed_tile(per_expert) if fp16 else _token_tile(per_expert)
+    mx = _mx_tile(lw, per_expert) if fp16 else 0
+    bn = 64 if h.dtype == torch.float32 else mx or _packed_tile(per_expert) if fp16 else _token_tile(per_expert)
     rows_cap = -(-(T * k + e_local * (bn - 1)) // bn) * bn
     max_tiles = rows_cap // bn
     i32 = dict(dtype=torch.int32, device=h.device)
@@ -293,8 +335,11 @@ def moe_ffn(dec, lw, h: torch.Tensor, xe: Optional[torch.Tensor] = None, add: Op
     tile_e, tile_r = torch.empty(max_tiles, **i32), torch.empty(max_tiles, **i32)
     ntiles = torch.zeros(2, **i32)
     row_w = torch.empty(rows_cap, dtype=torch.float32, device=h.device) if spec.weigh_input else None
-    k_ops.moe_align(ids, spec.experts, lo, lo + e_local, bn, row_of, token_of, tile_e, tile_r, ntiles, wts if spec.weigh_input else None, row_w)
-    if fp16:
+    tile_n = torch.empty(max_tiles, **i32) if mx else None
+    k_ops.moe_align(ids, spec.experts, lo, lo + e_local, bn, row_of, token_of, tile_e, tile_r, ntiles, wts if spec.weigh_input else None, row_w, tile_n)
+    if mx:
+        y = _mx_ffn(cfg, ops, spec, lw, h if xe is None else xe, token_of, row_w, tile_e, tile_r, tile_n, ntiles, bn, rows_cap)
+    elif fp16:
         y = _packed_ffn(cfg, ops, spec, lw, h if xe is None else xe, token_of, row_w, tile_e, tile_r, ntiles, bn, rows_cap)
     else:
         xp = torch.empty(rows_cap, H, dtype=h.dtype, device=h.device)

@@ -138,6 +138,14 @@ class Fp4Weight:
         return ops.linear(x, dense, bias, out)
 
 
+def scale_atoms(scales: torch.Tensor) -> torch.Tensor:
+    """[E, N, K/32] e8m0 bytes -> [E, ceil(N / 128), ceil(K / 128), 512]: the scales of 128 rows x 128 values, four per row, as
+    tcgen05.cp lays them into tensor memory (byte (r % 32) 16 + (r / 32) 4 + j); 1.0 where the matrix ends."""
+    E, N, G = scales.shape
+    padded = torch.nn.functional.pad(scales, (0, -G % 4, 0, -N % 128), value=127)
+    return padded.view(E, padded.shape[1] // 128, 4, 32, padded.shape[2] // 4, 4).permute(0, 1, 4, 3, 2, 5).reshape(E, padded.shape[1] // 128, -1, 512).contiguous()
+
+
 class Fp4ExpertStack:
     """The matrices of several experts held packed: codes [E, N, K/2], scales [E, N, K/block] (bytes).
     ``moe_ffn`` hands it to the grouped packed GEMM; gpt-oss checkpoints store their experts this way
@@ -148,6 +156,14 @@ class Fp4ExpertStack:
         self.shape = (codes.shape[0], codes.shape[1], codes.shape[2] * 2)
         self.device = codes.device
         self.f16 = fp16_form(self.codes, self.scales, self.fmt)
+        # MXFP4 on the block-scaled tensor cores (csrc/gemm_mx4_rows.cu): scales in the order in which they read them, and, where K ends in the
+        # middle of a block of 128, 32 bytes behind the codes that the last row's last box covers
+        self.atoms = None
+        if self.fmt == MXFP4 and self.codes.is_cuda and self.f16 and self.shape[2] % 64 == 0 and self.shape[1] % 8 == 0 and self.codes.numel():
+            if self.shape[2] % 128 and self.codes.untyped_storage().nbytes() < self.codes.storage_offset() + self.codes.numel() + 32:
+                room = torch.empty(self.codes.numel() + 32, dtype=torch.uint8, device=self.device)
+                self.codes = room[:self.codes.numel()].view(self.codes.shape).copy_(self.codes.view(torch.uint8))
+            self.atoms = scale_atoms(self.scales.view(torch.uint8))
 
     @classmethod
     def from_dense(cls, stack: torch.Tensor, fmt="mxfp4") -> "Fp4ExpertStack":
