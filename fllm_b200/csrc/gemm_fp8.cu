@@ -58,6 +58,15 @@ struct Fp8Item {
   }
 };
 
+// Waits for the loads from tensor memory; `r` is used behind it.
+__device__ __forceinline__ void tmem_ld_wait_of(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]),
+                 "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]), "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]),
+                 "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+               :: "memory");
+}
+
 template <int BN, bool SWAP, int PER>
 struct Fp8Smem {
   static constexpr int kABytes = F8_BM * F8_BK;
@@ -69,19 +78,23 @@ struct Fp8Smem {
   // A K block's product stays in its buffer until the promoting warps have added it up: the tensor core runs ahead by the other buffers.
   static constexpr int kBuffers = BN == 256 ? 2 : 4;
   static constexpr int kTmemCols = kBuffers * BN < 128 ? (kBuffers * BN < 64 ? 64 : kBuffers * BN) : kBuffers * BN;
-  static constexpr int kCols = BN > 64 ? 64 : BN > 32 ? 32 : BN;     // columns of a promoting thread
+  static constexpr int kCols = BN == 256 ? 128 : BN > 64 ? 64 : BN > 32 ? 32 : BN;     // columns of a promoting thread
   static constexpr int kShares = BN / kCols;                        // warps that share a lane quarter split the columns
   static constexpr int kPromote = 128 * kShares;                    // promoting threads: four warps per share
-  static constexpr int kThreads = 64 + kPromote;                    // TMA warp, MMA warp, promoting warps
+  // TMA warp, MMA warp, promoting warps; with 256 columns two more warps fill up the first four, whose registers go to the others
+  static constexpr bool kSplitRegs = BN == 256;
+  static constexpr int kFirst = kSplitRegs ? 4 : 2;                 // the first promoting warp
+  static constexpr int kThreads = 32 * kFirst + kPromote;
   static constexpr int kTotal = kStages * kStageBytes + kScaleFloats * 4 + 256 + 1024;
   static_assert((2 * kStages + 2 * kBuffers) * 8 + 8 <= 256, "barrier block");
 };
 
-// What bounds it: a 128 x 256 x 128 block is 512 clocks of the tensor core; promoting it is 32768 multiply-adds, 256 issue slots of each
-// scheduler, so the products bound it as long as a thread's share costs one multiply-add per value (one factor per row and K
-// block, activation scale x weight scale, read ahead; one accumulator register per column) and the latency of the tensor memory is
-// covered: four warps per scheduler with 64 columns each (two with 128 needed 1290 clocks a block). 128 x 128 tiles read and write shared memory
-// twice as often per product; they remain for few tiles.
+// What bounds it: a 128 x 256 x 128 block is 512 clocks of the tensor core, its operands some 700 of L2 with every SM reading (19.6 TB/s in all), its promotion
+// 32768 multiply-adds, 256 issue slots of each scheduler, and it takes 1000: the promoting warps go through every block one after the other, and what
+// surrounds their multiply-adds (a wait, the first load's latency, the scales, the way back to the top of 2 KB of code) adds up to as much as
+// these. So few warps with many columns each: eight of 128, with 224 registers that the first four warps leave them, the next 32 columns on their way
+// while 32 are added, the scales read under the first load. Sixteen warps of 64 columns: 141 us for 1965 x 7168 x 8192, this 132 (where the product and wait
+// loops were still voted on by whole warps: 147). 128 x 128 tiles read and write shared memory twice as often per product; they remain for few tiles.
 template <int BN, bool SWAP, int PER>       // SWAP: tokens in the N dimension; PER: CTAs per SM
 __global__ void __launch_bounds__(Fp8Smem<BN, SWAP, PER>::kThreads, PER)
 gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
@@ -117,70 +130,74 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   pdl_launch_dependents();
   const int items = p.whole + (p.m_tiles * p.n_tiles - p.whole) * p.k_splits;
 
-  if (warp == 0) {
-    int stage = 0, pre = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    {                                    // weights are static: the first stages' are requested before waiting for the quantiser
-      const Fp8Item it(p, blockIdx.x);
-      const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
-      const int kb0 = it.kb0;
-      pre = min(it.kb1 - kb0, STAGES);
-      if (elect_one()) {
-        for (int i = 0; i < pre; ++i) {
-          mbar_expect_tx(&full_bar[i], S::kStageBytes);
-          if (SWAP) tma_load_2d(sA + i * S::kABytes, &tma_a, &full_bar[i], (kb0 + i) * F8_BK, m_idx * F8_BM);
-          else tma_load_2d(sB + i * S::kBBytes, &tma_b, &full_bar[i], (kb0 + i) * F8_BK, n_idx * BN);
-        }
-      }
-      __syncwarp();
-    }
-    pdl_wait();
-    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-      const Fp8Item it(p, w);
-      const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
-      const int kb0 = it.kb0, kb1 = it.kb1;
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const bool requested = pre > 0;
-        if (requested) --pre;
-        else if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+  if (warp < S::kFirst) {
+    if constexpr (S::kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");      // launched with 168 a thread: 128 x 56 + 256 x 224 = 384 x 168
+    if (warp == 0) {
+      int stage = 0, pre = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      {                                    // weights are static: the first stages' are requested before waiting for the quantiser
+        const Fp8Item it(p, blockIdx.x);
+        const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
+        const int kb0 = it.kb0;
+        pre = min(it.kb1 - kb0, STAGES);
         if (elect_one()) {
+          for (int i = 0; i < pre; ++i) {
+            mbar_expect_tx(&full_bar[i], S::kStageBytes);
+            if (SWAP) tma_load_2d(sA + i * S::kABytes, &tma_a, &full_bar[i], (kb0 + i) * F8_BK, m_idx * F8_BM);
+            else tma_load_2d(sB + i * S::kBBytes, &tma_b, &full_bar[i], (kb0 + i) * F8_BK, n_idx * BN);
+          }
+        }
+        __syncwarp();
+      }
+      pdl_wait();
+      ok = elect_one();
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const Fp8Item it(p, w);
+        const int n_idx = it.t / p.m_tiles, m_idx = it.t - n_idx * p.m_tiles;
+        const int kb0 = it.kb0, kb1 = it.kb1;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const bool requested = pre > 0;
+          if (requested) --pre;
+          else if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
           if (!requested) mbar_expect_tx(&full_bar[stage], S::kStageBytes);
           if (!requested || !SWAP) tma_load_2d(sA + stage * S::kABytes, &tma_a, &full_bar[stage], kb * F8_BK, m_idx * F8_BM);
           if (!requested || SWAP) tma_load_2d(sB + stage * S::kBBytes, &tma_b, &full_bar[stage], kb * F8_BK, n_idx * BN);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        __syncwarp();
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
-    }
-  } else if (warp == 1) {
-    constexpr uint32_t idesc = make_idesc(F8_BM, BN, 0, 0);      // e4m3 x e4m3
-    const uint64_t da0 = make_smem_desc_sw128(smem_u32(sA)), db0 = make_smem_desc_sw128(smem_u32(sB));
-    int stage = 0, buf = 0;
-    uint32_t phase = 0, buf_phase = 0;
-    bool ok = true;
-    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
-      const Fp8Item it(p, w);
-      for (int kb = it.kb0; kb < it.kb1; ++kb) {
-        // each K block gets its own accumulator: wait until the promoting warps drained this buffer
-        if (!mbar_wait_warp(&tempty_bar[buf], buf_phase ^ 1, abort_flag) || !mbar_wait_warp(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-        tc_fence_after_sync();
-        if (elect_one()) {
+      __syncwarp();
+    } else if (warp == 1) {
+      constexpr uint32_t idesc = make_idesc(F8_BM, BN, 0, 0);      // e4m3 x e4m3
+      const uint64_t da0 = make_smem_desc_sw128(smem_u32(sA)), db0 = make_smem_desc_sw128(smem_u32(sB));
+      // One lane runs the role and asks both barriers before it uses either answer: an elected region per K block with two waits of the whole warp in front
+      // took 750 clocks, half again as many as the products of the block.
+      int stage = 0, buf = 0;
+      uint32_t phase = 0, buf_phase = 0;
+      bool ok = elect_one();
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const Fp8Item it(p, w);
+        for (int kb = it.kb0; kb < it.kb1; ++kb) {
+          // each K block gets its own accumulator: wait until the promoting warps drained this buffer
+          const bool drained = mbar_try_wait(&tempty_bar[buf], buf_phase ^ 1), landed = mbar_try_wait(&full_bar[stage], phase);
+          if (!(drained || mbar_wait(&tempty_bar[buf], buf_phase ^ 1, abort_flag)) || !(landed || mbar_wait(&full_bar[stage], phase, abort_flag))) { ok = false; break; }
+          tc_fence_after_sync();
           const uint64_t da = da0 + (uint64_t)(stage * (S::kABytes >> 4)), db = db0 + (uint64_t)(stage * (S::kBBytes >> 4));
 #pragma unroll
           for (int k = 0; k < F8_BK / F8_UMMA_K; ++k)
             tc_mma_f8f6f4(tmem_base + buf * BN, da + 2 * k, db + 2 * k, idesc, k > 0 ? 1u : 0u);
           tc_commit(&empty_bar[stage]);
           tc_commit(&tfull_bar[buf]);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++buf == NBUF) { buf = 0; buf_phase ^= 1; }
         }
-        __syncwarp();
-        if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        if (++buf == NBUF) { buf = 0; buf_phase ^= 1; }
       }
+      __syncwarp();
     }
   } else {
-    const int q = warp & 3, half = (warp - 2) >> 2;
-    const int etid = threadIdx.x - 64;
+    if constexpr (S::kSplitRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+    const int q = warp & 3, half = (warp - S::kFirst) >> 2;
+    const int etid = threadIdx.x - 32 * S::kFirst;
     pdl_wait();                            // scales of the activations; outputs may still be in use by the predecessor
     int buf = 0;
     uint32_t buf_phase = 0;
@@ -204,33 +221,59 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       // scale of the weights: features lie along the rows (one block of 128 per tile), or along the columns (one per thread: COLS divides 128)
       const float* wrow = p.sw + (size_t)(SWAP ? m_idx : min(n_base, p.N - 1) >> 7) * p.k_blocks;
       const float* xrow = p.sx + (size_t)(SWAP ? 0 : min(m, p.M - 1)) * p.k_blocks;
-      auto factor = [&](int kb) { return kb < kb1 ? (SWAP ? wrow[kb] : xrow[kb] * wrow[kb]) : 0.f; };
+      // (read ahead as they are: a product of the two scales formed at once would wait for them, 400 clocks a block)
+      auto wscale = [&](int kb) { return wrow[min(kb, kb1 - 1)]; };
+      auto xscale = [&](int kb) { return SWAP ? 1.f : xrow[min(kb, kb1 - 1)]; };
       float acc[COLS];
 #pragma unroll
       for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
-      float f0 = factor(kb0), f1 = factor(kb0 + 1);
+      float w0 = wscale(kb0), w1 = wscale(kb0 + 1), x0 = xscale(kb0), x1 = xscale(kb0 + 1);
       for (int kb = kb0; kb < kb1; ++kb) {
-        const float f = f0;
-        f0 = f1; f1 = factor(kb + 2);
+        float f = 0.f;
+        auto next_scales = [&]() {
+          f = SWAP ? w0 : x0 * w0;
+          w0 = w1; w1 = wscale(kb + 2);
+          x0 = x1; x1 = xscale(kb + 2);
+        };
         if (!mbar_wait(&tfull_bar[buf], buf_phase, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t t_row = tmem_base + buf * BN + half * COLS + ((uint32_t)(q * 32) << 16);
-        constexpr int CH = COLS < 32 || BN == 256 ? 16 : 32;      // (registers: eighteen warps leave 102 a thread)
+        if constexpr (BN == 256) {                           // the next 32 columns are on their way while these are added
+          uint32_t r[2][32];
+          tmem_ld_32x32(t_row, r[0]);
+          next_scales();
+          tmem_ld_wait_of(r[0]);
 #pragma unroll
-        for (int c0 = 0; c0 < COLS; c0 += CH) {
-          uint32_t r[CH];
-          if constexpr (CH == 32) tmem_ld_32x32(t_row + c0, r);
-          else tmem_ld_32x16(t_row + c0, r);
-          tmem_ld_wait();
+          for (int i = 0; i < 4; ++i) {
+            if (i < 3) tmem_ld_32x32(t_row + 32 * (i + 1), r[(i + 1) & 1]);
+            else {                                           // all of the buffer is in registers
+              tc_fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&tempty_bar[buf]);
+            }
 #pragma unroll
-          for (int c = 0; c < CH; ++c) {
-            if (SWAP) acc[c0 + c] += __uint_as_float(r[c]) * (f * s_scale[(kb - kb0) * BN + half * COLS + c0 + c]);
-            else acc[c0 + c] += __uint_as_float(r[c]) * f;
+            for (int c = 0; c < 32; ++c) acc[32 * i + c] += __uint_as_float(r[i & 1][c]) * f;
+            if (i < 3) tmem_ld_wait_of(r[(i + 1) & 1]);
           }
+        } else {
+          next_scales();
+          constexpr int CH = COLS < 32 ? 16 : 32;
+#pragma unroll
+          for (int c0 = 0; c0 < COLS; c0 += CH) {
+            uint32_t r[CH];
+            if constexpr (CH == 32) tmem_ld_32x32(t_row + c0, r);
+            else tmem_ld_32x16(t_row + c0, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+              if (SWAP) acc[c0 + c] += __uint_as_float(r[c]) * (f * s_scale[(kb - kb0) * BN + half * COLS + c0 + c]);
+              else acc[c0 + c] += __uint_as_float(r[c]) * f;
+            }
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tempty_bar[buf]);
         if (++buf == NBUF) { buf = 0; buf_phase ^= 1; }
       }
       if (!ok) break;
@@ -335,16 +378,17 @@ __global__ void fp8_tail_reduce_kernel(const Fp8GemmArgs p, int bn) {
 }
 
 // x bf16 [T][K] -> e4m3 [T][K] and scales [T][K/128] (amax / 448 per 128 values). Half a warp per group, 16 bytes per lane (one warp per
-// group with 8 bytes per lane moved 2.3 TB/s at 1965 x 8192).
+// group with 8 bytes per lane moved 2.3 TB/s at 1965 x 8192). Groups are counted in 32 bits: with a 64-bit quotient per thread the kernel was bound by
+// its instructions (1965 x 8192: 13.1 -> 12.3 us).
 __global__ void __launch_bounds__(256) quant_fp8_1x128_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ xq,
                                                               float* __restrict__ sx, int tokens, int K) {
   pdl_launch_dependents();
   pdl_wait();
   const int kb_n = K / 128;
-  const long long g = ((long long)blockIdx.x * 256 + threadIdx.x) >> 4;
+  const unsigned g = blockIdx.x * 16u + (threadIdx.x >> 4);
   const int l = threadIdx.x & 15;
-  const bool in = g < (long long)tokens * kb_n;
-  const int t = in ? (int)(g / kb_n) : 0, kb = in ? (int)(g - (long long)t * kb_n) : 0;
+  const bool in = g < (unsigned)tokens * (unsigned)kb_n;
+  const int t = in ? (int)(g / (unsigned)kb_n) : 0, kb = in ? (int)(g - (unsigned)t * (unsigned)kb_n) : 0;
   uint4 raw = make_uint4(0, 0, 0, 0);
   if (in) {
     const __nv_bfloat16* src = x + (size_t)t * ldx + kb * 128 + l * 8;
@@ -370,6 +414,7 @@ void quant_fp8_1x128(const void* x, long long ldx, void* xq, float* sx, int toke
   if (tokens <= 0) return;
   if (K % 128) throw std::runtime_error("quant_fp8_1x128: K must be a multiple of 128");
   const long long groups = (long long)tokens * (K / 128);
+  if (groups >= (1ll << 31)) throw std::runtime_error("quant_fp8_1x128: more than 2^31 groups");
   launch_pdl(quant_fp8_1x128_kernel, dim3((unsigned)((groups + 15) / 16)), dim3(256), 0, s, (const __nv_bfloat16*)x, ldx, (uint8_t*)xq, sx, tokens, K);
 }
 
