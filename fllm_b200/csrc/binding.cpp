@@ -54,10 +54,10 @@ int64_t linear(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, T
                     ws_bytes, st, (int)force_splits, cur_stream());
 }
 
-// y = x @ w^T (+ bias) on CTA pairs (cta_group::2, 256 x 256 tiles): more than 128 tokens. splits > 1: fp32 sums over parts of K go to
+// y = x @ w^T (+ bias) on CTA pairs (cta_group::2, tiles of 256 tokens x `width` features): more than 128 tokens. splits > 1: fp32 sums over parts of K go to
 // `partials` [splits, T, N] instead, without the bias; returns how many were written.
 int64_t linear_pair(const Tensor& x, const Tensor& w, const optional<Tensor>& bias, Tensor y, const optional<Tensor>& status, int64_t splits,
-                    const optional<Tensor>& partials) {
+                    const optional<Tensor>& partials, int64_t width) {
   check_bf16(x, "x"); check_bf16(w, "w"); check_bf16(y, "y");
   check_rows(x, "x"); check_rows(w, "w"); check_rows(y, "y");
   TORCH_CHECK(x.size(1) == w.size(1), "linear_pair: K mismatch");
@@ -74,10 +74,17 @@ int64_t linear_pair(const Tensor& x, const Tensor& w, const optional<Tensor>& bi
   c10::cuda::CUDAGuard guard(x.device());
   int* st = status.has_value() && status->defined() ? status->data_ptr<int>() : nullptr;
   return fllm::linear_bf16_pair(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), opt_ptr<void>(bias), y.data_ptr(),
-                                y.stride(0), (int)x.size(0), (int)w.size(0), (int)x.size(1), st, cur_stream(), nullptr, (int)splits, sums);
+                                y.stride(0), (int)x.size(0), (int)w.size(0), (int)x.size(1), st, cur_stream(), nullptr, (int)splits, sums, (int)width);
 }
 
-// The form that `linear` takes for a product on a device of `sms` SMs: splits over K on CTA pairs, or 0 for one-CTA tiles.
+// What `linear` takes for a product on a device of `sms` SMs: [splits over K on CTA pairs (0: one-CTA tiles), features of their tiles].
+std::vector<int64_t> linear_plan(int64_t tokens, int64_t features, int64_t k, int64_t sms, int64_t workspace_bytes, bool gated, bool deferred) {
+  TORCH_CHECK(tokens > 0 && features > 0 && k > 0 && sms > 0 && workspace_bytes >= 0, "linear_plan: sizes");
+  const fllm::PairPlan p = fllm::linear_bf16_plan_width((int)tokens, (int)features, (int)k, (int)sms, (size_t)workspace_bytes, gated, deferred);
+  return {p.splits, p.width};
+}
+
+// Square tiles against one-CTA tiles alone: splits over K on CTA pairs, or 0 for one-CTA tiles.
 int64_t linear_plan_pair(int64_t tokens, int64_t features, int64_t k, int64_t sms, int64_t workspace_bytes, bool gated, bool deferred) {
   TORCH_CHECK(tokens > 0 && features > 0 && k > 0 && sms > 0 && workspace_bytes >= 0, "linear_plan_pair: sizes");
   return fllm::linear_bf16_plan_pair((int)tokens, (int)features, (int)k, (int)sms, (size_t)workspace_bytes, gated, deferred);
@@ -411,8 +418,9 @@ int64_t sample_row_bytes() { return (int64_t)sizeof(fllm::SampleRow); }
 
 TORCH_LIBRARY(fllm_b200, m) {
   m.def("linear(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status, int force_splits) -> int", &linear);
+  m.def("linear_plan(int tokens, int features, int k, int sms, int workspace_bytes, bool gated, bool deferred) -> int[]", &linear_plan);
   m.def("linear_plan_pair(int tokens, int features, int k, int sms, int workspace_bytes, bool gated, bool deferred) -> int", &linear_plan_pair);
-  m.def("linear_pair(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? status, int splits=1, Tensor(b!)? partials=None) -> int", &linear_pair);
+  m.def("linear_pair(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? status, int splits=1, Tensor(b!)? partials=None, int width=256) -> int", &linear_pair);
   m.def("linear_ex(Tensor x, Tensor w, Tensor? bias, Tensor(a!) y, Tensor? workspace, Tensor? status, int force_splits, int glu, int glu_pd, float glu_alpha, float glu_limit, bool defer_reduce) -> int[]", &linear_ex);
   m.def("rmsnorm_splitk(Tensor(a!) residual, Tensor workspace, int splits, Tensor? bias, Tensor w, Tensor(b!) y, float eps, float w_offset) -> ()", &rmsnorm_splitk);
   m.def("rope_kv_write_splitk(Tensor workspace, int splits, Tensor? bias, Tensor(a!) q_out, Tensor positions, Tensor? slots, Tensor inv_freq, Tensor? q_norm_w, Tensor? k_norm_w, Tensor(b!) k_cache, Tensor(c!) v_cache, int hq, int hkv, int head_dim, int rot_dim, int rope_style, float eps, float attn_factor) -> ()", &rope_kv_write_splitk);

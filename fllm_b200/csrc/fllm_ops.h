@@ -102,9 +102,14 @@ void symm_close(void* p);
 bool linear_bf16_pair_supported(int T, int N, int K);
 int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* y, long long ldy,
                      int T, int N, int K, int* status, cudaStream_t stream, const struct LinearExtras* ex = nullptr, int splits = 1,
-                     float* partials = nullptr);                    // splits > 1: partial sums only; returns their number
-// Whether a local product of linear_bf16 takes the CTA pairs, and over how many splits of K (0: one-CTA tiles). `workspace_bytes`: of the
-// whole workspace; gated: the activation follows the product; deferred: the consumer adds partial sums.
+                     float* partials = nullptr, int width = 256);   // splits > 1: partial sums only; returns their number. width: features of a tile
+// Splits of K over which CTA pairs of 256 x 256 tiles are faster than one-CTA tiles (0: they are not), and what a local product of linear_bf16 takes: splits (0:
+// one-CTA tiles) and width of the pairs' tiles. `workspace_bytes`: of the whole workspace; gated: the activation follows the product; deferred: the
+// consumer adds partial sums.
+struct PairPlan {
+  int splits, width;
+};
+PairPlan linear_bf16_plan_width(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred);
 int linear_bf16_plan_pair(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred);
 
 // Packed 4-bit weights x at most 4 tokens on dp4a (int8 activations quantised inside the kernel); formats as linear_w4a16.

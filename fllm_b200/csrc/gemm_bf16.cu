@@ -828,35 +828,64 @@ static int plan_splits(int tiles, int bn, int k_blocks, int sms, size_t workspac
   return splits;
 }
 
-// Times of the two forms by the rounds of their items over the machine, in units of 10 ns, fitted to 231 products of 256 .. 24576
-// features, K of 320 .. 12288 and 129 .. 2048 tokens (11 % off in the mean; what they choose is 0.1 % behind the other form in the
-// mean, 9 % at most): a K block of a 128-wide one-CTA tile takes 31, of a 256-wide one 38, of a pair's 256 x 256 tile 29; a round 110, 480 and
-// 225 more; a launch 330, and 610 for pairs, whose launch overlaps with no other; a kernel that adds partial sums 165 or, behind
-// pairs, 305; the sums themselves 5.7 TB/s. The gated epilogue of a one-CTA tile takes 900 (256-wide 1500) more a round. So few
-// tiles of short sums go to one-CTA tiles (512 x 3072 x 2048: 14.5 us against 22.1 on pairs; 200 x 2048 x 2048: 10.0 against 15.4), most
-// others to pairs (1024 x 2048 x 8192: 36.8 us against 42.0; 200 x 24576 x 4096: 54.9 against 66.1).
+// Time of a product on one-CTA tiles by the rounds of its items over the machine, in units of 10 ns, fitted with that of pairs of 256 x 256 tiles to 231
+// products of 256 .. 24576 features, K of 320 .. 12288 and 129 .. 2048 tokens (11 % off in the mean): a K block of a 128-wide tile
+// takes 31, of a 256-wide one 38; a round 110 and 480 more; a launch 330; a kernel that adds partial sums 165; the sums themselves 5.7 TB/s. The
+// gated epilogue takes 900 (256-wide 1500) more a round.
+static long long sums_cost(int T, int N, int s, int launch, bool left_to_consumer) {
+  return s > 1 ? (left_to_consumer ? 0 : launch) + (long long)((double)s * T * N * 8 / 57000.0) : 0;
+}
+static long long one_cta_cost(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred) {
+  const int kbs = (K + BK - 1) / BK;
+  bool swap;
+  int bn;
+  plan_linear(T, N, sms, &swap, &bn);
+  const int tiles = ((T + BM - 1) / BM) * ((N + bn - 1) / bn), s1 = plan_splits(tiles, bn, kbs, sms, workspace_bytes, gated && !deferred);
+  const long long round = (kbs + s1 - 1) / s1 * (bn == 256 ? 38 : 31) + (bn == 256 ? 480 : 110) + (gated && s1 == 1 ? (bn == 256 ? 1500 : 900) : 0);
+  return 330 + (tiles * s1 + sms - 1) / sms * round + sums_cost(T, N, s1, 165, deferred && !gated);
+}
+
+// Splits over K on which pairs of 256 x 256 tiles are faster than one-CTA tiles; 0: they are not. A K block of a pair takes 29, a round 225 more, a launch
+// 610, which overlaps with no other, a kernel that adds partial sums 305 behind pairs (what this chooses is 0.1 % behind the other form in the
+// mean, 9 % at most).
 int linear_bf16_plan_pair(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred) {
   if (!linear_bf16_pair_supported(T, N, K)) return 0;
   const int kbs = (K + BK - 1) / BK;
   const bool whole = gated && !deferred;
-  auto sums = [&](int s, int launch) {
-    return s > 1 ? (deferred && !gated ? 0 : launch) + (long long)((double)s * T * N * 8 / 57000.0) : 0;
-  };
-  bool swap;
-  int bn;
-  plan_linear(T, N, sms, &swap, &bn);
-  const int tiles = ((T + BM - 1) / BM) * ((N + bn - 1) / bn), s1 = plan_splits(tiles, bn, kbs, sms, workspace_bytes, whole);
-  const long long round = (kbs + s1 - 1) / s1 * (bn == 256 ? 38 : 31) + (bn == 256 ? 480 : 110) + (gated && s1 == 1 ? (bn == 256 ? 1500 : 900) : 0);
-  const long long one = 330 + (tiles * s1 + sms - 1) / sms * round + sums(s1, 165);
   const long long pair_tiles = (long long)((T + 255) / 256) * ((N + 255) / 256), pairs = sms / 2;
-  long long best = one;
+  long long best = one_cta_cost(T, N, K, sms, workspace_bytes, gated, deferred);
   int splits = 0;
   for (int s = 1; s == 1 || (s <= 8 && s * 4 <= kbs); ++s) {
     if (s > 1 && (whole || kCounterBytes + (size_t)s * T * N * sizeof(float) > workspace_bytes)) break;
-    const long long cost = 610 + (pair_tiles * s + pairs - 1) / pairs * ((kbs + s - 1) / s * 29 + 225) + sums(s, 305);
+    const long long cost = 610 + (pair_tiles * s + pairs - 1) / pairs * ((kbs + s - 1) / s * 29 + 225) + sums_cost(T, N, s, 305, deferred && !gated);
     if (cost < best) { best = cost; splits = s; }
   }
   return splits;
+}
+
+// What a product takes: one-CTA tiles (splits 0) or pairs, whole or over splits as for square tiles, with the number of splits and the width of a tile (96 .. 256
+// features) that are fastest then. Square tiles leave most clusters without work in their last round, which is the second one for 129 to 256
+// tokens of the usual matrices: 200 x 24576 x 4096 has 96 of them for 74 clusters, and 128 of 192 features. In units of 10 ns, fitted to 1100
+// products of 2048 .. 24576 features, K of 2048 .. 12288 and 140 .. 2048 tokens (7 % off in the mean): a K block takes 12.4 and 0.062 a
+// feature, a round 1.9 a feature less 86. Partial sums cost the same whether their consumer adds them or a kernel, so that both give the same bits. us, square
+// tiles over the best number of splits -> this: 200 x 24576 x 4096 57.5 -> 49.4, 200 x 6144 x 4096 22.9 -> 21.3, 200 x 4096 x 4096 17.0 -> 14.9,
+// 512 x 6144 x 4096 29.4 -> 24.4, 768 x 4096 x 4096 27.2 -> 22.6, 1024 x 6144 x 4096 48.2 -> 39.9, 2048 x 24576 x 4096 266.8 -> 264.6.
+PairPlan linear_bf16_plan_width(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred) {
+  PairPlan plan{linear_bf16_plan_pair(T, N, K, sms, workspace_bytes, gated, deferred), 256};
+  if (plan.splits == 0) return plan;
+  const int kbs = (K + BK - 1) / BK, m_tiles = (T + 255) / 256, pairs = sms / 2, first = plan.splits > 1 ? 2 : 1, last = plan.splits > 1 ? 8 : 1;
+  double best = -1;
+  for (int s = first; s <= last && (s == 1 || s * 4 <= kbs); ++s) {
+    if (s > 1 && kCounterBytes + (size_t)s * T * N * sizeof(float) > workspace_bytes) break;
+    const int per = (kbs + s - 1) / s, parts = (kbs + per - 1) / per;
+    if (parts < s) continue;
+    for (int w = 256; w >= 96; w -= 32) {
+      const long long rounds = ((long long)m_tiles * ((N + w - 1) / w) * s + pairs - 1) / pairs;
+      const double cost = rounds * (per * (12.4 + 0.062 * w) + 1.9 * w - 86) + sums_cost(T, N, s, 0, true);
+      if (best < 0 || cost < best) { best = cost; plan = PairPlan{s, w}; }
+    }
+  }
+  return plan;
 }
 
 // Flag bumps rank `dest` receives from EACH source rank for one reduce-scatter linear of this
@@ -895,13 +924,14 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
     throw std::runtime_error("linear_bf16: K, N and the row pitches must be multiples of 8");
   const int sms = sm_count();
   if (!workspace) workspace_bytes = 0;
-  // Local products of more tokens than one swap-AB tile holds: CTA pairs (cta_group::2, 256 x 256 tiles), over splits of K while their tiles
+  // Local products of more tokens than one swap-AB tile holds: CTA pairs (cta_group::2, 256 tokens wide), over splits of K while their tiles
   // do not fill the machine, or the one-CTA tiles below.
-  int splits = !tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0
-                   ? linear_bf16_plan_pair(T, N, K, sms, workspace_bytes, glu != 0, defer) : 0;
+  const PairPlan pairs = !tpa && force_splits <= 0 && (ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0
+                             ? linear_bf16_plan_width(T, N, K, sms, workspace_bytes, glu != 0, defer) : PairPlan{0, 256};
+  int splits = pairs.splits;
   if (splits > 0) {
     float* partials = splits > 1 ? reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(workspace) + kCounterBytes) : nullptr;
-    splits = linear_bf16_pair(x, ldx, w, ldw, bias, y, ldy, T, N, K, status, stream, glu && splits == 1 ? ex : nullptr, splits, partials);
+    splits = linear_bf16_pair(x, ldx, w, ldw, bias, y, ldy, T, N, K, status, stream, glu && splits == 1 ? ex : nullptr, splits, partials, pairs.width);
     if (splits == 1) return 1;
     if (defer) {
       ex->deferred_splits = splits;

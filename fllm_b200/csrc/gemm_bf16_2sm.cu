@@ -37,6 +37,7 @@ constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;                // shared-window a
 struct Gemm2Args {
   int M, N, K;                               // M = tokens, N = features
   int m_tiles, n_tiles, k_blocks;
+  int width;                                 // features of a tile: a multiple of 32, at most 256; each CTA stages half of them
   int k_splits, kb_per_split;                // items are (split, tile); more than one split: fp32 partial sums in ws, [split][token][feature]
   float* ws;
   long long ldc;
@@ -138,6 +139,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
   const int n_clusters = gridDim.x >> 1, cluster_id = blockIdx.x >> 1;
 
   if (warp == 0) {
+    const uint32_t stage_bytes = 2 * (kP2OperandBytes + p.width / 2 * P2_BK * 2);      // of both CTAs
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -148,9 +150,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
         if (elect_one()) {
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * kP2StageBytes);
+          if (leader) mbar_expect_tx(&full_bar[stage], stage_bytes);
           tma_load_2d_pair(sX + stage * kP2OperandBytes, &tma_x, &full_bar[stage], kb * P2_BK, m_idx * P2_TILE + (int)rank * P2_ROWS);
-          tma_load_2d_pair(sW + stage * kP2OperandBytes, &tma_w, &full_bar[stage], kb * P2_BK, n_idx * P2_TILE + (int)rank * P2_ROWS);
+          tma_load_2d_pair(sW + stage * kP2OperandBytes, &tma_w, &full_bar[stage], kb * P2_BK, n_idx * p.width + (int)rank * (p.width / 2));
         }
         __syncwarp();
         if (++stage == P2_STAGES) { stage = 0; phase ^= 1; }
@@ -158,7 +160,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
     }
   } else if (warp == 1) {
     if (leader) {
-      constexpr uint32_t idesc = make_idesc(P2_TILE, P2_TILE, 1, 1);       // bf16 x bf16, M = 256 over the pair, N = 256
+      const uint32_t idesc = make_idesc(P2_TILE, 0, 1, 1) | (uint32_t)(p.width >> 3) << 17;       // bf16 x bf16, M = 256 over the pair
       const uint64_t da0 = make_smem_desc_sw128(smem_u32(sX)), db0 = make_smem_desc_sw128(smem_u32(sW));
       int stage = 0, buf = 0;
       uint32_t phase = 0, buf_phase = 0;
@@ -195,7 +197,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
       if (!mbar_wait(&tfull_bar[buf], buf_phase, abort_flag)) break;
       tc_fence_after_sync();
       const int m = m_idx * P2_TILE + (int)rank * P2_ROWS + q * 32 + lane;
-      const int n_base = n_idx * P2_TILE;
+      const int n_base = n_idx * p.width;
       const uint32_t t_row = tmem_base + buf * P2_TILE + ((uint32_t)(q * 32) << 16);
       __nv_bfloat16* dst = p.out + (size_t)m * p.ldc + n_base;
       auto gated = [&](float g, float u) -> float {
@@ -209,7 +211,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_co
         return __fdividef(gg, 1.f + __expf(-p.glu_alpha * gg)) * (uu + 1.f);
       };
 #pragma unroll 1
-      for (int c0 = 0; c0 < P2_TILE; c0 += 32) {
+      for (int c0 = 0; c0 < p.width; c0 += 32) {
         uint32_t r[32];
         tmem_ld_32x32(t_row + c0, r);
         tmem_ld_wait();
@@ -280,21 +282,22 @@ bool linear_bf16_pair_supported(int T, int N, int K) { return T > 128 && N % 8 =
 // epilogue and y is [T, N / 2] (N a multiple of 32). splits > 1: fp32 partial sums [splits][T][N] go to `partials` instead
 // (without bias or activation); returns the number of them.
 int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* y, long long ldy,
-                     int T, int N, int K, int* status, cudaStream_t stream, const LinearExtras* ex, int splits, float* partials) {
+                     int T, int N, int K, int* status, cudaStream_t stream, const LinearExtras* ex, int splits, float* partials, int width) {
   if (!linear_bf16_pair_supported(T, N, K)) throw std::runtime_error("linear_bf16_pair: needs more than 128 tokens, N >= 256, N % 8 == 0, K >= 64, K % 8 == 0");
+  if (width < 32 || width > P2_TILE || width % 32) throw std::runtime_error("linear_bf16_pair: tiles of 32 to 256 features, a multiple of 32");
   if ((ldy & 7) || (reinterpret_cast<uintptr_t>(y) & 15)) throw std::runtime_error("linear_bf16_pair: output rows must be 16-byte aligned");
   const int glu = ex ? ex->glu : 0;
   if (glu && ((N & 31) || (ex->glu_pd != 16 && ex->glu_pd != 1))) throw std::runtime_error("linear_bf16_pair: GLU needs N % 32 == 0 and a pair distance of 16 or 1");
   Gemm2Args a{};
   if (glu) { a.glu = glu; a.glu_pd = ex->glu_pd; a.glu_alpha = ex->glu_alpha; a.glu_limit = ex->glu_limit; }
   a.M = T; a.N = N; a.K = K;
-  a.m_tiles = (T + P2_TILE - 1) / P2_TILE; a.n_tiles = (N + P2_TILE - 1) / P2_TILE; a.k_blocks = (K + P2_BK - 1) / P2_BK;
+  a.m_tiles = (T + P2_TILE - 1) / P2_TILE; a.width = width; a.n_tiles = (N + width - 1) / width; a.k_blocks = (K + P2_BK - 1) / P2_BK;
   a.kb_per_split = (a.k_blocks + splits - 1) / splits;
   a.k_splits = (a.k_blocks + a.kb_per_split - 1) / a.kb_per_split;
   a.ws = partials;
   a.ldc = ldy; a.out = reinterpret_cast<__nv_bfloat16*>(y); a.bias = reinterpret_cast<const __nv_bfloat16*>(bias); a.status = status;
   const CUtensorMap tx = make_tmap_2d(x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, T, K, ldx * 2, P2_ROWS, P2_BK, true);
-  const CUtensorMap tw = make_tmap_2d(w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldw * 2, P2_ROWS, P2_BK, true);
+  const CUtensorMap tw = make_tmap_2d(w, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, K, ldw * 2, width / 2, P2_BK, true);
   static bool configured[kMaxDevices] = {};
   if (first_call_on_device(configured))
     cuda_check(cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kP2Smem),

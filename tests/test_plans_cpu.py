@@ -50,6 +50,35 @@ def test_plan_of_pairs_keeps_to_its_limits(plan):
             assert not (gated and not deferred) and 65536 + p * t * n * 4 <= ws and p * 4 <= -(-k // 64)
 
 
+# us on 148 SMs of partial or whole products on CTA pairs by (splits over K, features of a tile)
+WIDTHS = {(200, 24576, 4096): {(1, 256): 57.5, (1, 224): 52.9, (1, 192): 49.4, (1, 128): 54.7, (2, 224): 56.3},
+          (200, 6144, 4096): {(1, 256): 28.2, (1, 96): 20.3, (1, 128): 20.8, (3, 128): 21.3, (2, 192): 21.3, (3, 256): 22.9},
+          (512, 6144, 4096): {(1, 256): 29.4, (1, 224): 26.9, (1, 192): 24.4, (2, 192): 29.6},
+          (768, 4096, 4096): {(1, 256): 27.2, (1, 224): 24.8, (1, 192): 22.6, (1, 96): 30.4},
+          (1024, 6144, 4096): {(1, 256): 48.2, (1, 224): 43.9, (1, 192): 39.9, (1, 128): 45.9},
+          (1024, 4096, 12288): {(1, 256): 73.1, (1, 160): 85.2, (1, 128): 86.1, (1, 192): 97.0},
+          (2048, 2048, 2048): {(1, 256): 18.3, (1, 160): 21.1, (1, 192): 22.2, (1, 128): 22.3}}
+
+
+def test_pairs_take_a_fast_width(plan):
+    """Within a twentieth of the fastest measured width and number of splits (the sums are left to the consumer)."""
+    got = plan([[t, n, k, 148, WORKSPACE, False, True] for t, n, k in WIDTHS], "linear_plan")
+    for (size, times), (splits, width) in zip(WIDTHS.items(), got):
+        assert times[splits, width] <= 1.05 * min(times.values()), (size, splits, width)
+
+
+def test_plan_of_widths_keeps_to_its_limits(plan):
+    sizes = [(t, n, k) for t in (1, 128, 129, 200, 256, 700, 2048) for n in (64, 248, 256, 260, 1000, 4096, 24576) for k in (56, 64, 320, 4096, 12288)]
+    calls = [[t, n, k, sms, ws, gated, deferred] for t, n, k in sizes for sms in (148, 132) for ws in (0, 65536, 8 << 20, WORKSPACE)
+             for gated in (False, True) for deferred in (False, True)]
+    for (t, n, k, sms, ws, gated, deferred), (p, width) in zip(calls, plan(calls, "linear_plan")):
+        assert 0 <= p <= 8 and 96 <= width <= 256 and width % 32 == 0
+        if p:
+            assert t > 128 and n >= 256 and n % 8 == 0 and k >= 64
+        if p > 1:
+            assert not (gated and not deferred) and 65536 + p * t * n * 4 <= ws and p * 4 <= -(-k // 64)
+
+
 # us of packed 4-bit products by [fp16 form][splits over K]
 PACKED = {(64, 24576, 4096): {1: {1: 30.9, 2: 30.2, 3: 30.6, 4: 36.8, 6: 42.5, 8: 52.4}, 0: {1: 38.2, 2: 38.8, 3: 37.6, 8: 53.2}},
           (128, 24576, 4096): {1: {1: 38.0, 2: 41.4, 3: 45.7, 8: 73.9}, 0: {1: 40.9, 2: 43.2, 8: 69.5}},

@@ -50,6 +50,24 @@ def test_pair_kernel_over_each_number_of_splits(ops, T, N, K):
     assert ops.check_status() == 0
 
 
+@pytest.mark.parametrize("T", [129, 256, 300])
+@pytest.mark.parametrize("N,K", [(256, 64), (264, 320), (1000, 1088)])
+@pytest.mark.parametrize("width", [32, 96, 160, 224])
+def test_pair_kernel_of_each_width(ops, T, N, K, width):
+    """Tiles that end in the middle of the features, of a box and of a block of 32: one rounding, and nothing beyond the rows."""
+    x, w, b = _rand((T, K), 1), _rand((N, K), 2, 0.05), _rand((N,), 3)
+    ref = x.double() @ w.double().t()
+    y = torch.full((T + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert ops.k.linear_pair(x, w, b, y[:T], ops.status, 1, None, width) == 1
+    assert _rel(y[:T], ref + b.double()) < 2.5e-3 and (y[T] == 7.0).all()
+    part = torch.full((3, T, N), 7.0, device="cuda")
+    n = ops.k.linear_pair(x, w, None, y[:T], ops.status, 2, part[:2], width)
+    assert (part[n if n > 1 else 0:] == 7.0).all() and (n == 1 or _rel(part[:n].double().sum(0), ref) < 1e-5)
+    with pytest.raises(RuntimeError, match="multiple of 32"):
+        ops.k.linear_pair(x, w, None, y[:T], ops.status, 1, None, width + 8)
+    assert ops.check_status() == 0
+
+
 @pytest.mark.parametrize("T", [129, 200, 300])
 def test_pairs_leave_their_sums_to_the_norm_and_the_activation(ops, T):
     x, w, b, nw = _rand((T, 4096), 1), _rand((4096, 4096), 2, 0.02), _rand((4096,), 3), _rand((4096,), 4)
