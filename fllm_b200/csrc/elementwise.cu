@@ -151,8 +151,11 @@ void rmsnorm_bf16(void* residual, long long ld_res, const void* delta, long long
 // fp32 partial sums [splits][rows][hidden]; one CTA per row with a thread per four columns keeps as many
 // loads in flight as the stand-alone reduction kernel did. Rounding points are those of the two-kernel
 // path (delta -> bf16, updated residual -> bf16), so both paths give the same bits.
-template <int ITERS>
-__global__ void __launch_bounds__(1024)
+// SMALL: CTAs of up to 512 threads have eight planes on their way at a time (one row of 2048, 8 and 16 planes: 4.8 -> 3.9 us). With 1024 threads
+// their registers would fill the SM, and a CTA could not start beside the last ones of the product (64 rows of 4096: 4.9 us as it is, 5.9 with eight planes, 6.5
+// with four under predicates).
+template <int ITERS, bool SMALL>
+__global__ void __launch_bounds__(SMALL ? 512 : 1024)
 rmsnorm_splitk_kernel(__nv_bfloat16* __restrict__ residual, long long ld_res, const float* __restrict__ ws,
                       int splits, int rows, const __nv_bfloat16* __restrict__ bias,
                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, long long ld_y,
@@ -184,11 +187,16 @@ rmsnorm_splitk_kernel(__nv_bfloat16* __restrict__ residual, long long ld_res, co
     const int i = threadIdx.x + it * blockDim.x;
     if (i < nvec) {
       const float* src = ws + (size_t)row * hidden + 4 * i;
-      float4 acc = __ldcg(reinterpret_cast<const float4*>(src));
+      float4 acc;
+      if constexpr (SMALL) {
+        acc = sum_splits4<8>(src, plane, splits);
+      } else {
+        acc = __ldcg(reinterpret_cast<const float4*>(src));
 #pragma unroll 4
-      for (int sp = 1; sp < splits; ++sp) {
-        const float4 v = __ldcg(reinterpret_cast<const float4*>(src + sp * plane));
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        for (int sp = 1; sp < splits; ++sp) {
+          const float4 v = __ldcg(reinterpret_cast<const float4*>(src + sp * plane));
+          acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+        }
       }
       if (bias) {
         const uint2 bb = reinterpret_cast<const uint2*>(bias)[i];
@@ -241,16 +249,19 @@ void rmsnorm_splitk_bf16(void* residual, long long ld_res, const float* partials
   auto* b = (const __nv_bfloat16*)bias;
   auto* ww = (const __nv_bfloat16*)w;
   auto* yy = (__nv_bfloat16*)y;
+#define FLLM_COMMA ,
 #define FLLM_RMS_SK(IT)                                                                                       \
   launch_pdl(rmsnorm_splitk_kernel<IT>, dim3(rows), dim3(threads), 0, s, r, ld_res, partials, splits, rows, b, ww, yy, \
              ld_y, hidden, eps, w_offset)
-  switch (iters) {
-    case 1: FLLM_RMS_SK(1); break;
-    case 2: FLLM_RMS_SK(2); break;
-    case 3: FLLM_RMS_SK(3); break;
-    default: FLLM_RMS_SK(4); break;
+  switch (threads <= 512 ? 0 : iters) {
+    case 0: FLLM_RMS_SK(1 FLLM_COMMA true); break;
+    case 1: FLLM_RMS_SK(1 FLLM_COMMA false); break;
+    case 2: FLLM_RMS_SK(2 FLLM_COMMA false); break;
+    case 3: FLLM_RMS_SK(3 FLLM_COMMA false); break;
+    default: FLLM_RMS_SK(4 FLLM_COMMA false); break;
   }
 #undef FLLM_RMS_SK
+#undef FLLM_COMMA
   cuda_check(cudaGetLastError(), "rmsnorm_splitk_kernel");
 }
 
@@ -289,8 +300,10 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
   // element e of this head as the bf16 value the unfused path would have stored
   auto ld_elem = [&](int e) -> float {
     if (!ws) return __bfloat162float(src[e]);
-    float a = __ldcg(wsrc + e);
-    for (int sp = 1; sp < splits; ++sp) a += __ldcg(wsrc + sp * plane + e);
+    const int at[1] = {e};
+    float sum[1];
+    sum_splits_at<1>(sum, wsrc, plane, splits, at);
+    float a = sum[0];
     if (bias) a += __bfloat162float(bias[h * D + e]);
     return __bfloat162float(__float2bfloat16(a));
   };
@@ -310,14 +323,11 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
       return;
     }
     if (ws) {
-      float a[EPL];            // pairs (2i, 2i+1), i = lane + 32 * (j / 2): every load of a split is independent
+      float a[EPL];            // pairs (2i, 2i+1), i = lane + 32 * (j / 2)
+      int at[EPL];
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) a[j] = __ldcg(wsrc + 2 * (lane + 32 * (j / 2)) + (j & 1));
-#pragma unroll 4
-      for (int sp = 1; sp < splits; ++sp) {
-#pragma unroll
-        for (int j = 0; j < EPL; ++j) a[j] += __ldcg(wsrc + sp * plane + 2 * (lane + 32 * (j / 2)) + (j & 1));
-      }
+      for (int j = 0; j < EPL; ++j) at[j] = 2 * (lane + 32 * (j / 2)) + (j & 1);
+      sum_splits_at<EPL>(a, wsrc, plane, splits, at);
 #pragma unroll
       for (int j = 0; j < EPL; j += 2) {
         const int e = 2 * (lane + 32 * (j / 2));
@@ -344,14 +354,7 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
   for (int j = 0; j < EPL; ++j)
     eidx[j] = rope_style == 0 ? lane + 32 * j : 2 * (lane + 32 * (j / 2)) + (j & 1);
   if (ws) {
-    // all EPL loads of a split are independent; four splits are in flight at a time
-#pragma unroll
-    for (int j = 0; j < EPL; ++j) v[j] = __ldcg(wsrc + eidx[j]);
-#pragma unroll 4
-    for (int sp = 1; sp < splits; ++sp) {
-#pragma unroll
-      for (int j = 0; j < EPL; ++j) v[j] += __ldcg(wsrc + sp * plane + eidx[j]);
-    }
+    sum_splits_at<EPL>(v, wsrc, plane, splits, eidx);
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {
       if (bias) v[j] += __bfloat162float(bias[h * D + eidx[j]]);
@@ -662,25 +665,38 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
       for (int j = 0; j < 8; ++j) g[j] = u[j] = 0.f;
       if (act_kind != 2 || layout == 16) {                    // gate and up values: eight neighbours each
         const float *sg = src + col(0, false), *su = src + col(0, true);
-#pragma unroll 4
-        for (int sp = 0; sp < splits; ++sp) {
+        using Four = Values<float4, 4>;
+        over_splits<4>(splits, [&](int sp) {
+          Four f;
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            f.e[j] = __ldcg(reinterpret_cast<const float4*>(sg + sp * plane + 4 * j));
+            f.e[2 + j] = __ldcg(reinterpret_cast<const float4*>(su + sp * plane + 4 * j));
+          }
+          return f;
+        }, [&](int, const Four& f) {
 #pragma unroll
           for (int j = 0; j < 8; j += 4) {
-            const float4 a = __ldcg(reinterpret_cast<const float4*>(sg + sp * plane + j)), b = __ldcg(reinterpret_cast<const float4*>(su + sp * plane + j));
+            const float4 a = f.e[j / 4], b = f.e[2 + j / 4];
             g[j] += a.x, g[j + 1] += a.y, g[j + 2] += a.z, g[j + 3] += a.w;
             u[j] += b.x, u[j + 1] += b.y, u[j + 2] += b.z, u[j + 3] += b.w;
           }
-        }
+        });
       } else {                                                // pairs
         const float* sp0 = src + 2 * i8;
-#pragma unroll 4
-        for (int sp = 0; sp < splits; ++sp) {
+        using Four = Values<float4, 4>;
+        over_splits<4>(splits, [&](int sp) {
+          Four f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) f.e[j] = __ldcg(reinterpret_cast<const float4*>(sp0 + sp * plane + 4 * j));
+          return f;
+        }, [&](int, const Four& f) {
 #pragma unroll
           for (int j = 0; j < 8; j += 2) {
-            const float4 a = __ldcg(reinterpret_cast<const float4*>(sp0 + sp * plane + 2 * j));
+            const float4 a = f.e[j / 2];
             g[j] += a.x, u[j] += a.y, g[j + 1] += a.z, u[j + 1] += a.w;
           }
-        }
+        });
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {

@@ -656,12 +656,8 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  float4 acc = *reinterpret_cast<const float4*>(ws + i4);
-  for (int s = 1; s < splits; ++s) {
-    const float4 v = *reinterpret_cast<const float4*>(ws + (size_t)s * n + i4);
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-  }
-  const int r = (int)(i4 / cols);
+  float4 acc = sum_splits4(ws + i4, n, splits);
+  const int r = row_of_element(i4, cols);
   const int c = (int)(i4 - (size_t)r * cols);
   if (bias) {
     acc.x += __bfloat162float(bias[c]);
@@ -694,12 +690,8 @@ splitk_reduce_push_kernel(const float* __restrict__ ws, int splits, int rows, in
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 < n) {
-    float4 acc = __ldcg(reinterpret_cast<const float4*>(ws + i4));
-    for (int s = 1; s < splits; ++s) {
-      const float4 v = __ldcg(reinterpret_cast<const float4*>(ws + (size_t)s * n + i4));
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-    }
-    const int r = (int)(i4 / cols);
+    float4 acc = sum_splits4(ws + i4, n, splits);
+    const int r = row_of_element(i4, cols);
     const int c = (int)(i4 - (size_t)r * cols);
     if (bias) {
       acc.x += __bfloat162float(bias[c]);

@@ -338,12 +338,8 @@ __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ ws, int split
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  float4 acc = *reinterpret_cast<const float4*>(ws + i4);
-  for (int s = 1; s < splits; ++s) {
-    const float4 v = *reinterpret_cast<const float4*>(ws + (size_t)s * n + i4);
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-  }
-  const int r = (int)(i4 / cols);
+  const float4 acc = sum_splits4(ws + i4, n, splits);
+  const int r = row_of_element(i4, cols);
   const int c = (int)(i4 - (size_t)r * cols);
   float b[4] = {0.f, 0.f, 0.f, 0.f};
   if (bias) for (int i = 0; i < 4; ++i) b[i] = __bfloat162float(bias[c + i]);
@@ -360,15 +356,11 @@ __global__ void fp8_tail_reduce_kernel(const Fp8GemmArgs p, int bn) {
   const size_t tile = (size_t)F8_BM * bn, n = (size_t)(p.m_tiles * p.n_tiles - p.whole) * tile;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  const int t = p.whole + (int)(i4 / tile), within = (int)(i4 % tile);
+  const int t0 = row_of_element(i4, (int)tile), t = p.whole + t0, within = (int)(i4 - t0 * tile);
   const int n_idx = t / p.m_tiles, m_idx = t - n_idx * p.m_tiles;
   const int r = m_idx * F8_BM + within / bn, c = n_idx * bn + within % bn;
   if (r >= p.M || c >= p.N) return;
-  float4 acc = *reinterpret_cast<const float4*>(p.ws + i4);
-  for (int s = 1; s < p.k_splits; ++s) {
-    const float4 v = *reinterpret_cast<const float4*>(p.ws + (size_t)s * n + i4);
-    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-  }
+  const float4 acc = sum_splits4(p.ws + i4, n, p.k_splits);
   float b[4] = {0.f, 0.f, 0.f, 0.f};
   if (p.bias) for (int i = 0; i < 4; ++i) b[i] = __bfloat162float(p.bias[c + i]);
   uint2 o;

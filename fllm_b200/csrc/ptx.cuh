@@ -375,6 +375,69 @@ __device__ __forceinline__ bool wait_flag_ge(const uint32_t* flag, uint32_t targ
 // ----------------------------------------------------------------------------
 // small numeric helpers
 // ----------------------------------------------------------------------------
+template <typename T, int N>
+struct Values {
+  T e[N];
+};
+// Partial sums of `splits` planes, added in their order with B of them on their way at a time: load(s) -> a value, add(s, value). A loop of one load and
+// one addition, or its remainder when it is unrolled, waits for every plane in turn: some 600 ns each, of kernels that take 4 us.
+template <int B = 8, typename Load, typename Add>
+__device__ __forceinline__ void over_splits(int splits, Load&& load, Add&& add) {
+  for (int s0 = 0; s0 < splits; s0 += B) {
+    decltype(load(0)) v[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+      if (s0 + k < splits) v[k] = load(s0 + k);
+#pragma unroll
+    for (int k = 0; k < B; ++k)
+      if (s0 + k < splits) add(s0 + k, v[k]);
+  }
+}
+// The sums of the N elements at[.]; a: their sums.
+template <int N>
+__device__ __forceinline__ void sum_splits_at(float (&a)[N], const float* src, size_t plane, int splits, const int (&at)[N]) {
+  for (int s0 = 0; s0 < splits; s0 += 8) {
+    float v[8][N];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (s0 + k < splits) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[k][j] = __ldcg(src + (s0 + k) * plane + at[j]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (s0 + k < splits) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) a[j] = s0 + k == 0 ? v[k][j] : a[j] + v[k][j];
+      }
+    }
+  }
+}
+// Row of element i of rows of `cols`: a 64-bit quotient, some hundred instructions, only where it takes one.
+__device__ __forceinline__ int row_of_element(size_t i, int cols) {
+  return (i >> 32) == 0 ? (int)((unsigned)i / (unsigned)cols) : (int)(i / (size_t)cols);
+}
+// The usual sum of four neighbours, B planes at a time.
+template <int B = 4>
+__device__ __forceinline__ float4 sum_splits4(const float* src, size_t plane, int splits) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < splits; s0 += B) {
+    float4 v[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      if (s0 + k < splits) v[k] = __ldcg(reinterpret_cast<const float4*>(src));
+      src += plane;
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      if (s0 + k == 0) acc = v[k];
+      else if (s0 + k < splits) { acc.x += v[k].x; acc.y += v[k].y; acc.z += v[k].z; acc.w += v[k].w; }
+    }
+  }
+  return acc;
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
