@@ -65,6 +65,28 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
+// Two fp32 values an instruction.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // Shared-memory descriptor of an operand stored as 128-byte swizzled rows with 1024 bytes between
 // groups of eight rows, in either major-ness. For the MN-major use (V) every MMA covers one 64-wide
 // swizzle atom along N, so both offset fields describe the same stride: eight K rows = 1024 bytes.
@@ -204,11 +226,15 @@ __device__ __forceinline__ void softmax_row_impl(const FaTmemParams& p, uint32_t
   const int hi = lim - tok0, lo = beg - tok0;
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-  for (int i = 0; i < 128; ++i) {
-    float a = __uint_as_float(s[i >> 5][i & 31]);
-    if (capped) { a = tanhf(a * cap_in); s[i >> 5][i & 31] = __float_as_uint(a); }
-    if (!full && (i >= hi || (windowed && i < lo))) a = -INFINITY;
-    mx[i & 3] = fmaxf(mx[i & 3], a);
+  for (int i = 0; i < 128; i += 2) {
+    float a[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      a[k] = __uint_as_float(s[i >> 5][(i & 31) + k]);
+      if (capped) { a[k] = tanhf(a[k] * cap_in); s[i >> 5][(i & 31) + k] = __float_as_uint(a[k]); }
+      if (!full && (i + k >= hi || (windowed && i + k < lo))) a[k] = -INFINITY;
+    }
+    mx[(i >> 1) & 3] = fmaxf(fmaxf(mx[(i >> 1) & 3], a[0]), a[1]);
   }
   // the scale is positive, so it commutes with the maximum
   const float m = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;
@@ -231,20 +257,23 @@ __device__ __forceinline__ void softmax_row_impl(const FaTmemParams& p, uint32_t
     }
   }
   const float m_ref = m_used == -INFINITY ? 0.f : m_used;
-  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  uint64_t sum[2] = {0, 0};
+  const uint64_t scale2 = pack2(scale, scale), ref2 = pack2(-m_ref, -m_ref);
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     uint32_t w[16];
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {
       const int i = 32 * c + j;
-      float a = ex2(fmaf(__uint_as_float(s[c][j]), scale, -m_ref)), b = ex2(fmaf(__uint_as_float(s[c][j + 1]), scale, -m_ref));
+      const uint64_t x = fma2(pack2(__uint_as_float(s[c][j]), __uint_as_float(s[c][j + 1])), scale2, ref2);
+      float2 e = unpack2(x);
+      e.x = ex2(e.x); e.y = ex2(e.y);
       if (!full) {
-        if (i >= hi || (windowed && i < lo)) a = 0.f;
-        if (i + 1 >= hi || (windowed && i + 1 < lo)) b = 0.f;
+        if (i >= hi || (windowed && i < lo)) e.x = 0.f;
+        if (i + 1 >= hi || (windowed && i + 1 < lo)) e.y = 0.f;
       }
-      sum[j & 2] += a; sum[(j & 2) + 1] += b;
-      w[j >> 1] = pack_bf16x2(a, b);
+      sum[j >> 1 & 1] = add2(sum[j >> 1 & 1], pack2(e.x, e.y));
+      w[j >> 1] = pack_bf16x2(e.x, e.y);
     }
     tmem_st_32x16(t_s + 16 * c, w);
     if (c == 1) {
@@ -254,7 +283,8 @@ __device__ __forceinline__ void softmax_row_impl(const FaTmemParams& p, uint32_t
       if ((threadIdx.x & 31) == 0) mbar_arrive(p_half);
     }
   }
-  l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+  const float2 l0 = unpack2(sum[0]), l1 = unpack2(sum[1]);
+  l += (l0.x + l0.y) + (l1.x + l1.y);
   tmem_st_wait();
 }
 
@@ -274,36 +304,63 @@ __device__ __forceinline__ void softmax_row(const FaTmemParams& p, uint32_t t_s,
   else softmax_row_impl<D, false, false, false>(p, t_s, t_o, tok0, lim, beg, have_o, p_half, m_used, l);
 }
 
-// Final normalisation (with the head's sink, if any) and store of one row of O. The tensor memory loads are
-// warp-wide, so rows past the tile's last query take part and only skip the store.
+// Rows [row0, row0 + 128 TILES) of the CTA's queries to shared memory, in the layout TMA's 128-byte swizzle would have produced, by THREADS threads that
+// leave once their part is there and visible to the tensor cores. Asynchronous copies, all of a thread's under way at once: through registers, a
+// row's index divided out for each, they took 13,000 clocks for 256 rows of 128 and held back everything else.
+template <int D, int TILES, int THREADS>
+__device__ __forceinline__ void load_q(const FaTmemParams& p, uint8_t* sq, int t, int first_token, int kvh, int n_rows) {
+  const int shift = __ffs(p.group) - 1;                 // the group divides 128
+#pragma unroll 4
+  for (int i = t; i < TILES * kRowsT * (D / 8); i += THREADS) {
+    const int r = i / (D / 8), c = i % (D / 8), rr = r & (kRowsT - 1);
+    const int qi = r >> shift, hg = r - (qi << shift);
+    const bool valid = r < n_rows;
+    const __nv_bfloat16* src = p.q + (size_t)(first_token + (valid ? qi : 0)) * p.ldq + (size_t)(kvh * p.group + hg) * D + c * 8;
+    const uint32_t dst = smem_u32(sq + (r >> 7) * tile_bytes<D>() + (c >> 3) * kHalfBytes + rr * 128 + (((c & 7) ^ (rr & 7)) << 4));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  fence_proxy_async_smem();
+}
+
+// Final normalisation (with the head's sink, if any) and store of a warp's 32 rows of O, r0 the first. They pass through 64 D bytes of shared memory of the
+// warp's own, so that a store instruction writes whole rows: with a row to each lane every one of them touched 32 rows, 16 bytes of each (256 rows
+// of 128: 6400 clocks to the end of the CTA, 4400 to 5400 now).
 template <int D>
-__device__ __forceinline__ void store_row(const FaTmemParams& p, uint32_t t_o, bool valid, int token, int head,
-                                          float m_used, float l) {
+__device__ __forceinline__ void store_rows(const FaTmemParams& p, uint32_t t_o, uint8_t* stage, int r0, int n_rows, int first_token, int kvh,
+                                           float m_used, float l) {
+  constexpr int C = D / 8;                              // pieces of 16 bytes in a row
+  const int lane = threadIdx.x & 31, shift = __ffs(p.group) - 1;
   float ll = l, c = 1.f;
-  if (p.sinks && valid) {
-    const float sk2 = p.sinks[head] * kLog2eT;
+  if (p.sinks && r0 + lane < n_rows) {
+    const float sk2 = p.sinks[kvh * p.group + ((r0 + lane) & (p.group - 1))] * kLog2eT;
     const float mn = fmaxf(m_used, sk2);
     c = m_used == -INFINITY ? 0.f : ex2(m_used - mn);
     ll = ll * c + ex2(sk2 - mn);
   }
   const float inv = ll > 0.f ? c / ll : 0.f;
-  __nv_bfloat16* dst = p.out + (size_t)token * p.ldo + (size_t)head * D;
 #pragma unroll 1
   for (int cc = 0; cc < D / 32; ++cc) {
     uint32_t orow[32];
     tmem_ld_32x32(t_o + 32 * cc, orow);
     tmem_ld_wait();
-    if (valid) {
 #pragma unroll
-      for (int i = 0; i < 32; i += 8) {
-        uint4 w;
-        w.x = pack_bf16x2(__uint_as_float(orow[i]) * inv, __uint_as_float(orow[i + 1]) * inv);
-        w.y = pack_bf16x2(__uint_as_float(orow[i + 2]) * inv, __uint_as_float(orow[i + 3]) * inv);
-        w.z = pack_bf16x2(__uint_as_float(orow[i + 4]) * inv, __uint_as_float(orow[i + 5]) * inv);
-        w.w = pack_bf16x2(__uint_as_float(orow[i + 6]) * inv, __uint_as_float(orow[i + 7]) * inv);
-        *reinterpret_cast<uint4*>(dst + 32 * cc + i) = w;
-      }
+    for (int i = 0; i < 32; i += 8) {
+      uint4 w;
+      w.x = pack_bf16x2(__uint_as_float(orow[i]) * inv, __uint_as_float(orow[i + 1]) * inv);
+      w.y = pack_bf16x2(__uint_as_float(orow[i + 2]) * inv, __uint_as_float(orow[i + 3]) * inv);
+      w.z = pack_bf16x2(__uint_as_float(orow[i + 4]) * inv, __uint_as_float(orow[i + 5]) * inv);
+      w.w = pack_bf16x2(__uint_as_float(orow[i + 6]) * inv, __uint_as_float(orow[i + 7]) * inv);
+      *reinterpret_cast<uint4*>(stage + lane * (2 * D) + (((4 * cc + (i >> 3)) ^ (lane & 7)) << 4)) = w;
     }
+  }
+  __syncwarp();
+#pragma unroll 4
+  for (int k = 0; k < C; ++k) {
+    const int r = k * (32 / C) + lane / C, piece = lane % C;
+    const uint4 w = *reinterpret_cast<const uint4*>(stage + r * (2 * D) + ((piece ^ (r & 7)) << 4));
+    const int qi = (r0 + r) >> shift, hg = (r0 + r) - (qi << shift);
+    if (r0 + r < n_rows) *reinterpret_cast<uint4*>(p.out + (size_t)(first_token + qi) * p.ldo + (size_t)(kvh * p.group + hg) * D + piece * 8) = w;
   }
 }
 
@@ -312,9 +369,9 @@ __device__ __forceinline__ void store_row(const FaTmemParams& p, uint32_t t_o, b
 // of 1500, 64 query and 8 key heads of 64, window of 128: 442 -> 77 us with the decode rows.) Called by all THREADS; sums over as many sequences
 // at a time.
 template <int THREADS>
-__device__ bool tile_of_list(const FaTmemParams& p, int rq, int& seq, int& tile) {
+__device__ bool tile_of_list(const FaTmemParams& p, int rq, int want, int& seq, int& tile) {
   __shared__ int warp_sum[THREADS / 32], found[2];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, want = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) found[0] = -1;
   int before = 0;
   for (int s0 = 0; s0 < p.list_seqs; s0 += THREADS) {
@@ -360,15 +417,16 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
   uint64_t* s_full = bars + 4;
   uint64_t* p_ready = bars + 5;
   uint64_t* o_done = bars + 6;
+  uint64_t* q_full = bars + 7;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  int qt = gridDim.x - 1 - blockIdx.x, seq = blockIdx.z;      // the tiles with the longest KV range start first
-  const int kvh = blockIdx.y;
+  const int nth = blockIdx.x / p.hkv, kvh = blockIdx.x - nth * p.hkv;
+  int qt = gridDim.x / p.hkv - 1 - nth, seq = blockIdx.z;      // the tiles with the longest KV range start first
   const int G = p.group;
   const int RQ = kRowsT / G;
-  if (p.list_seqs > 0 && !tile_of_list<kThreadsT>(p, RQ, seq, qt)) return;
+  if (p.list_seqs > 0 && !tile_of_list<kThreadsT>(p, RQ, nth, seq, qt)) return;
   const int q0 = p.q_starts[seq];
   const int qn = p.q_starts[seq + 1] - q0;
   if (qn < p.min_q) return;
@@ -386,23 +444,12 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
 
   if (threadIdx.x == 0) {
     mbar_init(k_full, 1); mbar_init(v_full, 1); mbar_init(k_empty, 1); mbar_init(v_empty, 1);
-    mbar_init(s_full, 1); mbar_init(p_ready, 4); mbar_init(o_done, 1);
+    mbar_init(s_full, 1); mbar_init(p_ready, 4); mbar_init(o_done, 1); mbar_init(q_full, 4);
     *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 0 && lane == 0) { tma_prefetch_desc(&tma_k); tma_prefetch_desc(&tma_v); }
   if (warp == 1) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
-  // Q rows -> shared memory in the layout TMA's 128-byte swizzle would have produced
-  for (int i = threadIdx.x; i < kRowsT * (D / 8); i += kThreadsT) {
-    const int r = i / (D / 8), c = i % (D / 8);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r < n_rows) {
-      const int qi = r / G, hg = r - qi * G;
-      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + qi0 + qi) * p.ldq + (size_t)(kvh * G + hg) * D + c * 8);
-    }
-    *reinterpret_cast<uint4*>(sq + (c >> 3) * kHalfBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = v;
-  }
-  fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -450,7 +497,8 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
     constexpr uint32_t idesc_pv = make_idesc(128, D, 1, 1) | (1u << 16);     // B is MN-major
     const uint64_t dq = make_smem_desc_sw128(smem_u32(sq)), dk = make_smem_desc_sw128(smem_u32(sk));
     const uint64_t dv = smem_desc_sw128_1k(smem_u32(sv), D == 128 ? 2048 : 1024);     // V lands by pages: [page][D / 64][16][64]
-    for (int it = 0; it < n_tiles; ++it) {
+    const bool ok = mbar_wait_warp(q_full, 0, abort_flag);
+    for (int it = 0; ok && it < n_tiles; ++it) {
       const uint32_t ph = it & 1;
       if (!mbar_wait_warp(k_full, ph, abort_flag)) break;
       tc_fence_after_sync();
@@ -480,6 +528,9 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
     const int quarter = warp & 3;                       // the lane quarter this warp may touch
     const int r = quarter * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+    load_q<D, 1, 128>(p, sq, threadIdx.x - 64, q0 + qi0, kvh, n_rows);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(q_full);
     int lim = 0, beg = 0;
     if (r < n_rows) {
       lim = p.bidir ? kv_len : first_pos + r / G + 1;
@@ -500,8 +551,7 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
     }
     if (ok && mbar_wait(o_done, 0, abort_flag)) {
       tc_fence_after_sync();
-      const int qi = r / G, hg = r - qi * G;
-      store_row<D>(p, t_o + lane_off, r < n_rows, q0 + qi0 + qi, kvh * G + hg, m_used, l);
+      store_rows<D>(p, t_o + lane_off, sq + quarter * 64 * D, quarter * 32, n_rows, q0 + qi0, kvh, m_used, l);      // Q has been read
     }
   }
   tc_fence_before_sync();
@@ -516,12 +566,15 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
 // (PV0, next S0, PV1, next S1) so that one group's softmax runs under the other tile's MMAs; K and V are
 // double buffered. Tensor memory: S0 S1 O0 O1 = 512 columns, one CTA per SM.
 //
-// What bounds it: the chain of a group. A tile's softmax took 2620 clocks and its PV and next S 1024, of which the other group's chain
-// hides about half; tensor pipe and exponentials are each busy 47 % of the time. So a row's scores stay in registers (one pass over
-// tensor memory instead of two; the warps that need no registers leave theirs), and PV of the first 64 tokens runs while the others'
-// exponentials are computed: 2017 tokens at 8161, 32 query and 8 key heads of 128: 313 -> 293 us. (Two S buffers of 64 tokens per tile
-// took 355: products of 64 columns read Q twice as often.) Under a window the tiles that every row sees whole take the same unmasked
-// form (2048 tokens, window of 1024, heads as above: 107 -> 65 us).
+// What bounds it: the chain of a group (softmax, PV, next S), 3000 to 3300 clocks per tile where the tensor pipe and the exponentials need 2048
+// each for both groups. A row's scores stay in registers (one pass over tensor memory instead of two; the warps that need no registers leave
+// theirs), two of them to an instruction, and PV of the first 64 tokens runs while the others' exponentials are computed. (Two S buffers of 64 tokens
+// per tile are slower: products of 64 columns read Q twice as often. A share of the exponentials on the multiply-add pipe gave
+// 1 % at best.) One lane walks the issuer's loop: five waits voted on by its warp and five elected regions cost 1850 of a tile's 3570
+// clocks. The grid runs over the key heads first and from a sequence's longest tiles to its shortest, so that the last CTAs to start are short:
+// with a head's tiles next to each other the SMs of 256 CTAs ended up to 40 % apart. K and V are on their way while the queries are
+// loaded. 32 query and 8 key heads of 128, us before and now: 2017 tokens at 8161: 292, 230; 2 x 1024: 56, 37.5; 4096: 190, 144; 64 query and
+// 8 key heads of 64, 2048 tokens: 102, 80. Under a window the tiles that every row sees whole take the unmasked form.
 constexpr int kThreadsT2 = 384;
 template <int D> constexpr int smem_two() { return 6 * tile_bytes<D>() + 256 + 1024; }
 
@@ -546,13 +599,14 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
   uint64_t* p_half = bars + 13;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint64_t* q_full = bars + 16;
 
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
-  int qt = gridDim.x - 1 - blockIdx.x, seq = blockIdx.z;
-  const int kvh = blockIdx.y;
+  const int nth = blockIdx.x / p.hkv, kvh = blockIdx.x - nth * p.hkv;
+  int qt = gridDim.x / p.hkv - 1 - nth, seq = blockIdx.z;
   const int G = p.group;
   const int RQ = 2 * kRowsT / G;
-  if (p.list_seqs > 0 && !tile_of_list<kThreadsT2>(p, RQ, seq, qt)) return;
+  if (p.list_seqs > 0 && !tile_of_list<kThreadsT2>(p, RQ, nth, seq, qt)) return;
   const int q0 = p.q_starts[seq];
   const int qn = p.q_starts[seq + 1] - q0;
   if (qn < p.min_q) return;
@@ -573,23 +627,12 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
       mbar_init(&k_full[i], D / 64); mbar_init(&v_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1); mbar_init(&p_half[i], 4); mbar_init(&p_ready[i], 4);
     }
-    mbar_init(o_done, 1);
+    mbar_init(o_done, 1); mbar_init(q_full, 8);
     *abort_flag = 0;
     fence_barrier_init();
   }
   if (warp == 8 && lane == 0) { tma_prefetch_desc(&tma_k); tma_prefetch_desc(&tma_v); }
   if (warp == 9) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
-  for (int i = threadIdx.x; i < 2 * kRowsT * (D / 8); i += kThreadsT2) {
-    const int r = i / (D / 8), c = i % (D / 8);
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (r < n_rows) {
-      const int qi = r / G, hg = r - qi * G;
-      v = *reinterpret_cast<const uint4*>(p.q + (size_t)(q0 + qi0 + qi) * p.ldq + (size_t)(kvh * G + hg) * D + c * 8);
-    }
-    const int rr = r & (kRowsT - 1);
-    *reinterpret_cast<uint4*>(sq + (r >> 7) * TB + (c >> 3) * kHalfBytes + rr * 128 + (((c & 7) ^ (rr & 7)) << 4)) = v;
-  }
-  fence_proxy_async_smem();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -651,46 +694,42 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
         for (int k = 4 * part; k < 4 * part + 4; ++k)
           tc_mma_bf16_ts(t_o, t_p + 8 * k, dv + (uint64_t)(stage * (TB >> 4)) + k * (D / 64) * (2048 >> 4), idesc_pv, (!first || k > 0) ? 1u : 0u);
       };
-      bool ok = mbar_wait_warp(&k_full[0], 0, abort_flag);
-      if (ok) {
-        tc_fence_after_sync();
-        if (elect_one()) {
+      if (elect_one()) {
+        bool ok = mbar_wait(&k_full[0], 0, abort_flag) && mbar_wait(q_full, 0, abort_flag);
+        if (ok) {
+          tc_fence_after_sync();
           issue_s(0, 0);
           tc_commit(&s_full[0]);
           issue_s(1, 0);
           tc_commit(&s_full[1]);
           tc_commit(&k_empty[0]);
         }
-        __syncwarp();
-      }
-      for (int it = 0; ok && it < n_tiles; ++it) {
-        const int b = it & 1, nb = b ^ 1;
-        const uint32_t ph = (it >> 1) & 1, nph = ((it + 1) >> 1) & 1;
-        const bool more = it + 1 < n_tiles;
-        if (!mbar_wait_warp(&p_half[0], it & 1, abort_flag) || !mbar_wait_warp(&v_full[b], ph, abort_flag)) break;
-        tc_fence_after_sync();
-        if (elect_one()) issue_pv(0, b, it == 0, 0);
-        __syncwarp();
-        if (!mbar_wait_warp(&p_ready[0], it & 1, abort_flag)) break;
-        tc_fence_after_sync();
-        if (elect_one()) issue_pv(0, b, it == 0, 1);
-        __syncwarp();
-        if (more) {
-          if (!mbar_wait_warp(&k_full[nb], nph, abort_flag)) break;
+        for (int it = 0; ok && it < n_tiles; ++it) {
+          const int b = it & 1, nb = b ^ 1;
+          const uint32_t ph = (it >> 1) & 1, nph = ((it + 1) >> 1) & 1;
+          const bool more = it + 1 < n_tiles;
+          ok = mbar_wait(&v_full[b], ph, abort_flag) && mbar_wait(&p_half[0], it & 1, abort_flag);
+          if (!ok) break;
           tc_fence_after_sync();
-          if (elect_one()) {
+          issue_pv(0, b, it == 0, 0);
+          ok = mbar_wait(&p_ready[0], it & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_pv(0, b, it == 0, 1);
+          if (more) {
+            ok = mbar_wait(&k_full[nb], nph, abort_flag);
+            if (!ok) break;
+            tc_fence_after_sync();
             issue_s(0, nb);
             tc_commit(&s_full[0]);
           }
-          __syncwarp();
-        }
-        if (!mbar_wait_warp(&p_half[1], it & 1, abort_flag)) break;
-        tc_fence_after_sync();
-        if (elect_one()) issue_pv(1, b, it == 0, 0);
-        __syncwarp();
-        if (!mbar_wait_warp(&p_ready[1], it & 1, abort_flag)) break;
-        tc_fence_after_sync();
-        if (elect_one()) {
+          ok = mbar_wait(&p_half[1], it & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after_sync();
+          issue_pv(1, b, it == 0, 0);
+          ok = mbar_wait(&p_ready[1], it & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after_sync();
           issue_pv(1, b, it == 0, 1);
           tc_commit(&v_empty[b]);
           if (more) {
@@ -701,8 +740,8 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
             tc_commit(o_done);
           }
         }
-        __syncwarp();
       }
+      __syncwarp();
     }
   } else {                                              // warps 0 - 7
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
@@ -710,6 +749,9 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
     const int quarter = warp & 3;
     const int r = g * kRowsT + quarter * 32 + lane;     // packed row within the CTA
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+    load_q<D, 2, 256>(p, sq, threadIdx.x, q0 + qi0, kvh, n_rows);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(q_full);
     const uint32_t t_s = tmem_base + 128 * g + lane_off, t_o = tmem_base + 256 + 128 * g + lane_off;
     int lim = 0, beg = 0;
     if (r < n_rows) {
@@ -734,8 +776,7 @@ fa_prefill_tmem2_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_
     }
     if (ok && mbar_wait(o_done, 0, abort_flag)) {
       tc_fence_after_sync();
-      const int qi = r / G, hg = r - qi * G;
-      store_row<D>(p, t_o, r < n_rows, q0 + qi0 + qi, kvh * G + hg, m_used, l);
+      store_rows<D>(p, t_o, sq + g * TB + quarter * 64 * D, r - lane, n_rows, q0 + qi0, kvh, m_used, l);      // Q has been read
     }
   }
   tc_fence_before_sync();
@@ -767,16 +808,19 @@ void launch_tmem(const MapPair& maps, FaTmemParams p, int max_q_len, int num_seq
     cuda_check(cudaFuncSetAttribute(fa_prefill_tmem2_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_two<D>()),
                "fa_prefill_tmem2 smem");
   }
-  // Two query tiles per CTA when that still gives every SM a CTA (tile_variant 1 / 2 forces one: tests only).
+  // Two query tiles per CTA when that still gives every SM a CTA (tile_variant 1 / 2 forces one: tests only), but not under windows of
+  // less than two tiles: of three tiles of keys or so the way in and out is the larger part, and two CTAs of one tile on an SM hide each
+  // other's. us with one and two, 2048 tokens, 64 query and 8 key heads of 64: window 128: 48, 54; 256: 61, 62; 512: 83, 67; 32 heads of 128: 35, 37;
+  // 43, 41; 54, 48. (With fewer CTAs than SMs two tiles win beside 4096 cached tokens, 832 tokens: 94, 86, and lose without, 25, 27.)
   const int forced = p.tile_variant;
   const int rq2 = 2 * kRowsT / p.group;
   const long long ctas2 = (long long)((max_q_len + rq2 - 1) / rq2) * p.hkv * num_seqs;
-  const bool two = forced ? forced == 2 : (max_q_len * p.group >= 2 * kRowsT && ctas2 >= sm_count());
+  const bool two = forced ? forced == 2 : (max_q_len * p.group >= 2 * kRowsT && ctas2 >= sm_count() && !(p.window > 0 && p.window < 2 * kTileT));
   const int rq = two ? rq2 : kRowsT / p.group, tiles = (max_q_len + rq - 1) / rq;
-  dim3 grid(tiles, p.hkv, num_seqs);
+  dim3 grid((unsigned)tiles * p.hkv, 1, num_seqs);
   if (mixed_rows > 0) {                // P prompts of q rows each have at most sum(q) / rq + P tiles
     const long long bound = max(1, mixed_rows / rq + min(num_seqs, mixed_rows / max(p.min_q, 1)));    // (max_q_len may be an upper bound)
-    if (bound < (long long)tiles * num_seqs) { grid = dim3((unsigned)bound, p.hkv, 1); p.list_seqs = num_seqs; }
+    if (bound < (long long)tiles * num_seqs) { grid = dim3((unsigned)bound * p.hkv, 1, 1); p.list_seqs = num_seqs; }
   }
   if (two) fa_prefill_tmem2_kernel<D><<<grid, kThreadsT2, smem_two<D>(), s>>>(maps.k, maps.v, p);
   else fa_prefill_tmem_kernel<D><<<grid, kThreadsT, smem_one<D>(), s>>>(maps.k, maps.v, p);

@@ -343,6 +343,16 @@ def test_prompt_attention_under_windows(ops, D, hq, hkv, window, sinks):
     assert _rel(y, ref) < 2 ** -8
 
 
+@pytest.mark.parametrize("D,hq,hkv", [(128, 16, 16), (64, 32, 16), (128, 32, 2), (64, 64, 8)])
+@pytest.mark.parametrize("window", [0, 255, 256])
+@pytest.mark.parametrize("q_lens,kv_lens", [((1291, 1291), (1291, 1500)), ((1301, 40), (1307, 50)), ((129, 3), (260, 3))])
+def test_prompt_attention_over_groups_and_ragged_tiles(ops, D, hq, hkv, window, q_lens, kv_lens):
+    """Groups of 1, 2, 8 and 16 query heads, last tiles of a few rows, and windows on both sides of two tiles of keys, where one or two tiles
+    of queries share a block. Probabilities and results are rounded to bf16 once each: 2^-9 + 2^-9."""
+    y, ref = _attention(ops, q_lens, kv_lens, D, hq, hkv, window)
+    assert _rel(y, ref) < 2 ** -8
+
+
 @pytest.mark.parametrize("D,hq,hkv,window", [(128, 32, 8, 0), (64, 64, 8, 128), (64, 32, 8, 0), (128, 16, 16, 100)])
 @pytest.mark.parametrize("q_lens", [[1] * 40 + [300], [300] + [1] * 40, [1, 2, 700, 1, 64, 1, 1, 129, 1], [1] * 500 + [40], [1] * 3 + [1000, 1000] + [2] * 200])
 def test_decode_rows_beside_prompts(ops, D, hq, hkv, window, q_lens):
