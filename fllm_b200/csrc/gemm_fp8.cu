@@ -439,7 +439,7 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
   // Tile and K splits by the rounds of items over the SMs, in units of 1/100 us. A K block takes the time in which an SM's share of the HBM
   // bandwidth brings its weights (37 per 128 features) when no other tile of the step reads them, too (64-wide tiles spare few tokens the
   // partial sums or some of them, 28: 128 x 1280 x 8192 13.6 -> 12.0 us, 128 x 8192 x 3584 16.9 -> 15.8; 7168 x 8192 needs them and took 27.7
-  // against 24.9); else what L2 takes for its operands with every SM reading (256-wide tiles 60, 128-wide 36). Partial sums are
+  // against 24.9); else its operands from L2 and its promotion with every SM busy (256-wide tiles 60, 128-wide 36, of a round of 1965 x 7168 x 8192). Partial sums are
   // written and read once, and cost a launch. With more tiles than SMs either all are split, or those of the last, partly filled
   // round alone (whole > 0): 1965 x 7168 x 8192 has 448 tiles of 256 for 3 x 148, and the last four took as long
   // as a full round (172 -> 149 us). 16-wide tiles may run as two CTAs per SM with half of the ring each, which share its bandwidth: one's

@@ -55,7 +55,8 @@ __device__ __forceinline__ bool elect_one() {
 // Index of the warp as a value the compiler knows to be the same in all lanes: branches on it stay convergent, and what they compute
 // can live in uniform registers. TMA and tcgen05.mma take their addresses and descriptors from those. Issued by `if (lane == 0)` in divergent
 // code every operand moves there first: 86 clocks per tcgen05.mma measured (a product of 128 x 16 x 16 values needs 8), and more per
-// box of TMA. So the whole warp walks the loop of a producer or MMA role, votes on its waits, and one elected lane issues.
+// box of TMA. Behind elect_one() they stay uniform, around a single issue or around the loop of a whole role. The latter is the faster where
+// a loop is short of time: a vote on a wait and an election for what follows cost some 300 clocks a turn.
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 // ----------------------------------------------------------------------------
