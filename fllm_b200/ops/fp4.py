@@ -157,13 +157,15 @@ class Fp4ExpertStack:
         self.device = codes.device
         self.f16 = fp16_form(self.codes, self.scales, self.fmt)
         # MXFP4 on the block-scaled tensor cores (csrc/gemm_mx4_rows.cu): scales in the order in which they read them, and, where K ends in the
-        # middle of a block of 128, 32 bytes behind the codes that the last row's last box covers
+        # middle of a block of 128, 32 bytes behind the codes that the last row's last box covers. Its boxes of codes start on 32 bytes: a
+        # stack that is a view from between two such boundaries has no atoms and is expanded to fp16, which asks for 16.
         self.atoms = None
         if self.fmt == MXFP4 and self.codes.is_cuda and self.f16 and self.shape[2] % 64 == 0 and self.shape[1] % 8 == 0 and self.codes.numel():
             if self.shape[2] % 128 and self.codes.untyped_storage().nbytes() < self.codes.storage_offset() + self.codes.numel() + 32:
                 room = torch.empty(self.codes.numel() + 32, dtype=torch.uint8, device=self.device)
                 self.codes = room[:self.codes.numel()].view(self.codes.shape).copy_(self.codes.view(torch.uint8))
-            self.atoms = scale_atoms(self.scales.view(torch.uint8))
+            if self.codes.data_ptr() % 32 == 0:
+                self.atoms = scale_atoms(self.scales.view(torch.uint8))
 
     @classmethod
     def from_dense(cls, stack: torch.Tensor, fmt="mxfp4") -> "Fp4ExpertStack":

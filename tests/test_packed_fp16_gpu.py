@@ -121,6 +121,25 @@ def test_routed_experts_end_to_end(ops, counts, k, act, limit, weigh):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("at", [0, 16, 32])
+@pytest.mark.parametrize("act", ["swiglu_oai", "swiglu"])
+def test_stacks_that_start_on_16_bytes(ops, monkeypatch, at, act):
+    """Codes that are a view into a larger buffer: the block-scaled form takes those on 32 bytes, the fp16 form the others. Roundings as in
+    test_routed_experts_end_to_end."""
+    plain, made = Fp4ExpertStack.from_dense, []
+
+    def moved(w):
+        s = plain(w)
+        buf = torch.empty(s.codes.numel() + 64, dtype=torch.uint8, device="cuda")
+        assert buf.data_ptr() % 32 == 0
+        made.append(Fp4ExpertStack(buf[at:at + s.codes.numel()].view(s.codes.shape).copy_(s.codes), s.scales, s.fmt))
+        return made[-1]
+    monkeypatch.setattr(Fp4ExpertStack, "from_dense", staticmethod(moved))
+    assert _experts(ops, [5, 4, 0, 9], 2, act) < 5 * 1.7e-3
+    assert len(made) == 2 and all((s.atoms is None) == (at == 16) and s.codes.data_ptr() % 32 == at % 32 for s in made)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("K", [64, 320, 2880, 28672])
 def test_rows_keep_every_value(ops, K):
     """fp16 rows times their factor are the bf16 rows again, over the whole exponent range and next to values that are not finite. A value
