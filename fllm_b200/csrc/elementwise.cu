@@ -151,7 +151,9 @@ void rmsnorm_bf16(void* residual, long long ld_res, const void* delta, long long
 // fp32 partial sums [splits][rows][hidden]; one CTA per row with a thread per four columns keeps as many
 // loads in flight as the stand-alone reduction kernel did. Rounding points are those of the two-kernel
 // path (delta -> bf16, updated residual -> bf16), so both paths give the same bits.
-// SMALL: CTAs of up to 512 threads have eight planes on their way at a time (one row of 2048, 8 and 16 planes: 4.8 -> 3.9 us). With 1024 threads
+// SMALL: CTAs of up to 512 threads have eight planes on their way at a time (one row of 2048, 8 and 16 planes: 4.8 -> 3.9 us), where there are at least four and
+// all CTAs are on the SMs at once with its 80 registers a thread: beyond that the loop, of which twice as many fit, is the faster (loop and
+// batch, rows of 2048: 148 behind 8 planes 4.7, 3.8; 200 behind 3 3.2, 4.5; 2048 behind 2 16.8, 30.7). With 1024 threads
 // their registers would fill the SM, and a CTA could not start beside the last ones of the product (64 rows of 4096: 4.9 us as it is, 5.9 with eight planes, 6.5
 // with four under predicates).
 template <int ITERS, bool SMALL>
@@ -253,7 +255,8 @@ void rmsnorm_splitk_bf16(void* residual, long long ld_res, const float* partials
 #define FLLM_RMS_SK(IT)                                                                                       \
   launch_pdl(rmsnorm_splitk_kernel<IT>, dim3(rows), dim3(threads), 0, s, r, ld_res, partials, splits, rows, b, ww, yy, \
              ld_y, hidden, eps, w_offset)
-  switch (threads <= 512 ? 0 : iters) {
+  const bool small = threads <= 512 && splits >= 4 && rows <= sm_count() * (65536 / (80 * threads));
+  switch (small ? 0 : iters) {
     case 0: FLLM_RMS_SK(1 FLLM_COMMA true); break;
     case 1: FLLM_RMS_SK(1 FLLM_COMMA false); break;
     case 2: FLLM_RMS_SK(2 FLLM_COMMA false); break;

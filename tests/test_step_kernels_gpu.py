@@ -371,3 +371,27 @@ def test_longest_prompt_given_as_an_upper_bound(ops, q_lens):
     """Fewer rows in all than the shortest prompt has: the prompt kernel finds nothing or one sequence, the decode kernel does the rest."""
     y, ref = _attention(ops, q_lens, [m + 50 for m in q_lens], 128, 32, 8, 0, longest=64)
     assert _rel(y, ref) < 2 ** -7
+
+
+def _planes(S, rows, cols, seed):
+    """Workspace with S planes of partial sums, and their sum in the order of the planes."""
+    p = (torch.randn(S, rows, cols, generator=torch.Generator().manual_seed(seed))).cuda()
+    ws = torch.zeros(65536 + p.numel() * 4, dtype=torch.uint8, device="cuda")
+    ws[65536:].view(torch.float32).copy_(p.view(-1))
+    total = p[0].clone()
+    for s in range(1, S):
+        total += p[s]
+    return ws, total
+
+
+@pytest.mark.parametrize("H", [512, 2048, 4096])
+@pytest.mark.parametrize("S", [2, 4, 9])
+@pytest.mark.parametrize("T", [1, 148, 149, 300])
+def test_norm_adds_planes_in_either_way(ops, H, S, T):
+    """Rows on both sides of what the SMs hold at once: the bits of the norm of the summed product."""
+    ws, total = _planes(S, T, H, S)
+    w, r = _rand((H,), 4), _rand((T, H), 5)
+    r2, y, y2 = r.clone(), torch.empty_like(r), torch.empty_like(r)
+    ops.k.rmsnorm_splitk(r, ws, S, None, w, y, 1e-6, 0.0)
+    ops.k.rmsnorm(r2, total.to(torch.bfloat16), w, y2, 1e-6, 0.0)
+    assert torch.equal(r, r2) and _rel(y, y2.double()) < 1e-3        # (the sum of squares in another order: a last bit here and there)
