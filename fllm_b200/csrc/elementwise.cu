@@ -274,8 +274,12 @@ void rmsnorm_splitk_bf16(void* residual, long long ld_res, const float* partials
 // [hq+hkv, hq+2hkv) value heads (copied to the cache).
 // Cache layout: [block][kv_head][block_size][head_dim] (a head's page is contiguous).
 // rope_style: 0 = rotate-half ("neox": pairs (i, i + rot/2)), 1 = interleaved pairs (2i, 2i+1).
-template <int D>
-__global__ void __launch_bounds__(128)
+// CTAs that an SM is to hold, by the planes on their way. One kernel for all three took 48 / 72 / 119 registers where there are no sums, too, and moved
+// 2048 x 24 heads of 256 in 48.7 us (32 registers: 24.2), 2048 x 48 of 128, interleaved, in 38.7 (27.2).
+template <int D, Sums SUMS>
+constexpr int kRopeCtas = SUMS == Sums::batch ? (D == 64 ? 10 : D == 128 ? 7 : 4) : SUMS == Sums::loop ? (D == 64 ? 16 : D == 128 ? 9 : 7) : 16;
+template <int D, Sums SUMS>
+__global__ void __launch_bounds__(128, kRopeCtas<D, SUMS>)
 rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __restrict__ positions,
                const int* __restrict__ slots, const float* __restrict__ inv_freq,
                const __nv_bfloat16* __restrict__ q_norm_w, const __nv_bfloat16* __restrict__ k_norm_w,
@@ -283,7 +287,7 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
                int hq, int hkv, int block_size, int rot_dim, int rope_style, float eps,
                float attn_factor, int kv_fp8, const float* __restrict__ ws, int splits,
                const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ q_out, long long ld_q) {
-  // ws != null: the projection left fp32 split-K partials [splits][tokens][heads * D] (bias not added);
+  // SUMS other than none: the projection left fp32 split-K partials [splits][tokens][heads * D] (bias not added);
   // this kernel adds them, rounds to bf16 like the reduction kernel would, and writes the rotated query
   // heads to q_out (the key / value heads only go to the cache).
   constexpr int EPL = D / 32;  // elements per lane
@@ -299,13 +303,14 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
   const int slot = slots ? slots[t] : -1;
   const size_t width = (size_t)heads * D;
   const size_t plane = (size_t)tokens * width;
-  const float* wsrc = ws ? ws + (size_t)t * width + (size_t)h * D : nullptr;
+  constexpr bool ADD = SUMS != Sums::none;
+  const float* wsrc = ADD ? ws + (size_t)t * width + (size_t)h * D : nullptr;
   // element e of this head as the bf16 value the unfused path would have stored
   auto ld_elem = [&](int e) -> float {
-    if (!ws) return __bfloat162float(src[e]);
+    if (!ADD) return __bfloat162float(src[e]);
     const int at[1] = {e};
     float sum[1];
-    sum_splits_at<1>(sum, wsrc, plane, splits, at);
+    sum_splits_at<1, SUMS == Sums::batch>(sum, wsrc, plane, splits, at);
     float a = sum[0];
     if (bias) a += __bfloat162float(bias[h * D + e]);
     return __bfloat162float(__float2bfloat16(a));
@@ -319,18 +324,18 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
     if (kv_fp8) {                  // e4m3 cache: one byte per value, same [block][head][slot][dim] order
       uint8_t* d8 = reinterpret_cast<uint8_t*>(v_cache) + (((size_t)blk * hkv + kvh) * block_size + off) * D;
       for (int i = lane; i < D / 2; i += 32) {
-        const float2 f = ws ? make_float2(ld_elem(2 * i), ld_elem(2 * i + 1))
+        const float2 f = ADD ? make_float2(ld_elem(2 * i), ld_elem(2 * i + 1))
                             : unpack_bf16x2(reinterpret_cast<const uint32_t*>(src)[i]);
         reinterpret_cast<uint16_t*>(d8)[i] = (uint16_t)__nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E4M3);
       }
       return;
     }
-    if (ws) {
+    if constexpr (ADD) {
       float a[EPL];            // pairs (2i, 2i+1), i = lane + 32 * (j / 2)
       int at[EPL];
 #pragma unroll
       for (int j = 0; j < EPL; ++j) at[j] = 2 * (lane + 32 * (j / 2)) + (j & 1);
-      sum_splits_at<EPL>(a, wsrc, plane, splits, at);
+      sum_splits_at<EPL, SUMS == Sums::batch>(a, wsrc, plane, splits, at);
 #pragma unroll
       for (int j = 0; j < EPL; j += 2) {
         const int e = 2 * (lane + 32 * (j / 2));
@@ -356,8 +361,8 @@ rope_kv_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int* __r
 #pragma unroll
   for (int j = 0; j < EPL; ++j)
     eidx[j] = rope_style == 0 ? lane + 32 * j : 2 * (lane + 32 * (j / 2)) + (j & 1);
-  if (ws) {
-    sum_splits_at<EPL>(v, wsrc, plane, splits, eidx);
+  if constexpr (ADD) {
+    sum_splits_at<EPL, SUMS == Sums::batch>(v, wsrc, plane, splits, eidx);
 #pragma unroll
     for (int j = 0; j < EPL; ++j) {
       if (bias) v[j] += __bfloat162float(bias[h * D + eidx[j]]);
@@ -554,6 +559,12 @@ rope_kv_rows_kernel(__nv_bfloat16* __restrict__ qkv, long long ld_qkv, const int
   }
 }
 
+// A batch of eight planes holds 48 / 72 / 121 registers for heads of 64 / 128 / 256, a loop 32 / 56 / 72: batches from four planes on, or where a loop
+// adds more than four at a time. us, loop and batch, 32 query and 8 key heads of 128: 16 rows behind 4 planes 3.4, 3.1; 64 behind 8 6.9, 4.9; 200
+// behind 2 6.1, 7.3; 256 behind 4 11.0, 9.6 (but 100 behind 4 4.6, 5.4); 200 behind 8 13.2, 10.4; 2048 behind 2 43.0, 53.6; 16 and 4 of 256: 200 behind
+// 4 8.9, 9.2, 200 behind 8 12.7, 11.7.
+static Sums rope_sums(int splits, int head_dim) { return splits >= (head_dim == 256 ? 6 : 4) ? Sums::batch : Sums::loop; }
+
 void rope_qknorm_kvwrite_bf16(void* qkv, long long ld_qkv, const int* positions, const int* slots,
                               const float* inv_freq, const void* q_norm_w, const void* k_norm_w,
                               void* k_cache, void* v_cache, int tokens, int hq, int hkv,
@@ -582,10 +593,17 @@ void rope_qknorm_kvwrite_bf16(void* qkv, long long ld_qkv, const int* positions,
                  attn_factor);
     return;
   }
-#define FLLM_ROPE(DD)                                                                            \
-  launch_pdl(rope_kv_kernel<DD>, dim3(blocks), dim3(128), 0, s, x, ld_qkv, positions, slots, inv_freq, qn, kn, kc, \
+  const Sums sums = !partials ? Sums::none : rope_sums(splits, head_dim);
+#define FLLM_ROPE_SUMS(DD, SS)                                                                                     \
+  launch_pdl(rope_kv_kernel<DD, SS>, dim3(blocks), dim3(128), 0, s, x, ld_qkv, positions, slots, inv_freq, qn, kn, kc, \
              vc, tokens, hq, hkv, block_size, rot_dim, rope_style, eps, attn_factor, kv_fp8, partials, splits,    \
              (const __nv_bfloat16*)bias, (__nv_bfloat16*)q_out, ld_q)
+#define FLLM_ROPE(DD)                                                   \
+  switch (sums) {                                                       \
+    case Sums::none: FLLM_ROPE_SUMS(DD, Sums::none); break;             \
+    case Sums::loop: FLLM_ROPE_SUMS(DD, Sums::loop); break;             \
+    case Sums::batch: FLLM_ROPE_SUMS(DD, Sums::batch); break;           \
+  }
   switch (head_dim) {
     case 64: FLLM_ROPE(64); break;
     case 128: FLLM_ROPE(128); break;
@@ -593,6 +611,7 @@ void rope_qknorm_kvwrite_bf16(void* qkv, long long ld_qkv, const int* positions,
     default: throw std::runtime_error("rope_qknorm_kvwrite_bf16: head_dim must be 64, 128 or 256");
   }
 #undef FLLM_ROPE
+#undef FLLM_ROPE_SUMS
   cuda_check(cudaGetLastError(), "rope_kv_kernel");
 }
 
@@ -629,8 +648,10 @@ void widen_rows(const void* x, long long ldx, float* out, int rows, int cols, cu
 //             g = min(g, limit); u = clamp(u, -limit, limit); out = g * sigmoid(alpha g) * (u + 1)
 // layout: 0 = the kind's natural one (halves; pairs for kind 2), 16 = blocks of 16 gate columns followed
 // by the 16 up columns of the same features (the order the GEMM's gated epilogue wants its weight rows in).
-// ws != null: x is not read; the columns are the sums of fp32 split-K partials [splits][rows][2 * inter]
+// SUMS other than none: x is not read; the columns are the sums of fp32 split-K partials [splits][rows][2 * inter]
 // (+ bias), kept in fp32 in front of the activation as the epilogue of an unsplit product keeps them.
+// (With the sums in one kernel it took 92 registers where there are none, too: 2048 x 12288 41.8 us, and 26.9 with 32.)
+template <Sums SUMS>
 __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                            __nv_bfloat16* __restrict__ out, long long ldo, int inter, int act_kind,
                            float alpha, float limit, int layout, const float* __restrict__ ws, int splits,
@@ -642,7 +663,8 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
   if (i8 >= inter) return;
   const __nv_bfloat16* xr = x ? x + (size_t)row * ldx : nullptr;
   float g[8], u[8];
-  if (ws || layout == 16) {
+  constexpr bool ADD = SUMS != Sums::none;
+  if (ADD || layout == 16) {
     // column of gate / up value j of this thread's 8 features
     auto col = [&](int j, bool up) -> int {
       const int f = i8 + j;
@@ -650,7 +672,7 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
       if (act_kind == 2) return 2 * f + (up ? 1 : 0);
       return f + (up ? inter : 0);
     };
-    if (!ws && layout == 16) {                               // eight neighbours of one block: 16 bytes each
+    if (!ADD) {                                              // eight neighbours of one block: 16 bytes each
       const uint4 a = *reinterpret_cast<const uint4*>(xr + col(0, false)), b = *reinterpret_cast<const uint4*>(xr + col(0, true));
       const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -658,9 +680,6 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
         const float2 f = unpack_bf16x2(aw[j]), h = unpack_bf16x2(bw[j]);
         g[2 * j] = f.x, g[2 * j + 1] = f.y, u[2 * j] = h.x, u[2 * j + 1] = h.y;
       }
-    } else if (!ws) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { g[j] = __bfloat162float(xr[col(j, false)]); u[j] = __bfloat162float(xr[col(j, true)]); }
     } else {
       const size_t plane = (size_t)rows * 2 * inter;
       const float* src = ws + (size_t)row * 2 * inter;
@@ -669,7 +688,7 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
       if (act_kind != 2 || layout == 16) {                    // gate and up values: eight neighbours each
         const float *sg = src + col(0, false), *su = src + col(0, true);
         using Four = Values<float4, 4>;
-        over_splits<4>(splits, [&](int sp) {
+        over_splits<4, SUMS == Sums::batch>(splits, [&](int sp) {
           Four f;
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
@@ -688,7 +707,7 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
       } else {                                                // pairs
         const float* sp0 = src + 2 * i8;
         using Four = Values<float4, 4>;
-        over_splits<4>(splits, [&](int sp) {
+        over_splits<4, SUMS == Sums::batch>(splits, [&](int sp) {
           Four f;
 #pragma unroll
           for (int j = 0; j < 4; ++j) f.e[j] = __ldcg(reinterpret_cast<const float4*>(sp0 + sp * plane + 4 * j));
@@ -751,6 +770,12 @@ __global__ void glu_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
   *reinterpret_cast<uint4*>(out + (size_t)row * ldo + i8) = r;
 }
 
+// A batch of four planes takes 94 registers, a loop 56, none 32. us, loop and batch: 16 rows of 6144 behind 4 planes 3.0, 2.5; 48 behind 4 3.8, 4.2;
+// 200 behind 2 5.8, 6.0; 200 behind 4 9.7, 8.6; 200 behind 8 17.3, 15.4.
+static Sums glu_sums(long long ctas, int splits) {
+  return ctas <= sm_count() || splits >= 6 || (splits >= 3 && ctas > 3ll * sm_count()) ? Sums::batch : Sums::loop;
+}
+
 void glu_bf16(const void* x, long long ldx, void* out, long long ldo, int rows, int inter,
               int act_kind, float alpha, float limit, cudaStream_t s, int layout, const float* partials, int splits,
               const void* bias) {
@@ -758,8 +783,10 @@ void glu_bf16(const void* x, long long ldx, void* out, long long ldo, int rows, 
   if (inter % 8) throw std::runtime_error("glu_bf16: intermediate size must be a multiple of 8");
   if (layout == 16 && inter % 16) throw std::runtime_error("glu_bf16: the blocked layout needs a multiple of 16 features");
   dim3 grid((inter / 8 + 127) / 128, rows);
-  launch_pdl(glu_kernel, grid, dim3(128), 0, s, (const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)out, ldo, inter,
-             act_kind, alpha, limit, layout, partials, splits, rows, (const __nv_bfloat16*)bias);
+  const Sums sums = !partials ? Sums::none : glu_sums((long long)grid.x * rows, splits);
+  launch_pdl(sums == Sums::none ? glu_kernel<Sums::none> : sums == Sums::loop ? glu_kernel<Sums::loop> : glu_kernel<Sums::batch>, grid, dim3(128), 0, s,
+             (const __nv_bfloat16*)x, ldx, (__nv_bfloat16*)out, ldo, inter, act_kind, alpha, limit, layout, partials, splits, rows,
+             (const __nv_bfloat16*)bias);
   cuda_check(cudaGetLastError(), "glu_kernel");
 }
 

@@ -376,14 +376,22 @@ __device__ __forceinline__ bool wait_flag_ge(const uint32_t* flag, uint32_t targ
 // ----------------------------------------------------------------------------
 // small numeric helpers
 // ----------------------------------------------------------------------------
+// How a kernel takes the partial sums of a split product: it has none, plane after plane (few registers, many CTAs on an SM), or all planes of a batch on
+// their way (few CTAs, whose time is the latency of their loads).
+enum class Sums { none, loop, batch };
 template <typename T, int N>
 struct Values {
   T e[N];
 };
 // Partial sums of `splits` planes, added in their order with B of them on their way at a time: load(s) -> a value, add(s, value). A loop of one load and
-// one addition, or its remainder when it is unrolled, waits for every plane in turn: some 600 ns each, of kernels that take 4 us.
-template <int B = 8, typename Load, typename Add>
+// one addition, or its remainder when it is unrolled, waits for every plane in turn: some 600 ns each, of kernels that take 4 us. BATCH false: such a loop.
+template <int B = 8, bool BATCH = true, typename Load, typename Add>
 __device__ __forceinline__ void over_splits(int splits, Load&& load, Add&& add) {
+  if constexpr (!BATCH) {
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) add(s, load(s));
+    return;
+  }
   for (int s0 = 0; s0 < splits; s0 += B) {
     decltype(load(0)) v[B];
 #pragma unroll
@@ -394,9 +402,19 @@ __device__ __forceinline__ void over_splits(int splits, Load&& load, Add&& add) 
       if (s0 + k < splits) add(s0 + k, v[k]);
   }
 }
-// The sums of the N elements at[.]; a: their sums.
-template <int N>
+// The sums of the N elements at[.]; a: their sums. BATCH: eight planes on their way at a time, in eight times the registers; else plane after plane.
+template <int N, bool BATCH = true>
 __device__ __forceinline__ void sum_splits_at(float (&a)[N], const float* src, size_t plane, int splits, const int (&at)[N]) {
+  if constexpr (!BATCH) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) a[j] = __ldcg(src + at[j]);
+#pragma unroll 4
+    for (int s = 1; s < splits; ++s) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) a[j] += __ldcg(src + s * plane + at[j]);
+    }
+    return;
+  }
   for (int s0 = 0; s0 < splits; s0 += 8) {
     float v[8][N];
 #pragma unroll

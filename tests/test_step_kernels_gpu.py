@@ -384,6 +384,23 @@ def _planes(S, rows, cols, seed):
     return ws, total
 
 
+@pytest.mark.parametrize("D,hq,hkv", [(64, 6, 2), (128, 8, 1), (256, 2, 1)])
+@pytest.mark.parametrize("S", [2, 4, 5, 6, 9])
+@pytest.mark.parametrize("T", [3, 300])
+def test_rotation_adds_planes_in_either_way(ops, D, hq, hkv, S, T):
+    """Few and many rows, planes on both sides of a batch: the bits of the rotation of the summed projection."""
+    ws, total = _planes(S, T, (hq + 2 * hkv) * D, S)
+    bias, w = _rand(((hq + 2 * hkv) * D,), 3), _rand((D,), 4)
+    pos = torch.arange(T, dtype=torch.int32, device="cuda")
+    inv = (1e4 ** (-torch.arange(0, D, 2, device="cuda").float() / D)).contiguous()
+    caches = [torch.zeros(-(-T // 16), hkv, 16, D, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    q = torch.empty(T, hq * D, dtype=torch.bfloat16, device="cuda")
+    ops.k.rope_kv_write_splitk(ws, S, bias, q, pos, pos, inv, w, w, *caches[:2], hq, hkv, D, D, 1, 1e-6, 1.0)
+    qkv = (total + bias.float()).to(torch.bfloat16)
+    ops.k.rope_kv_write(qkv, pos, pos, inv, w, w, *caches[2:], hq, hkv, D, D, 1, 1e-6, 1.0)
+    assert torch.equal(q, qkv[:, :hq * D]) and torch.equal(caches[0], caches[2]) and torch.equal(caches[1], caches[3])
+
+
 @pytest.mark.parametrize("H", [512, 2048, 4096])
 @pytest.mark.parametrize("S", [2, 4, 9])
 @pytest.mark.parametrize("T", [1, 148, 149, 300])
@@ -395,3 +412,25 @@ def test_norm_adds_planes_in_either_way(ops, H, S, T):
     ops.k.rmsnorm_splitk(r, ws, S, None, w, y, 1e-6, 0.0)
     ops.k.rmsnorm(r2, total.to(torch.bfloat16), w, y2, 1e-6, 0.0)
     assert torch.equal(r, r2) and _rel(y, y2.double()) < 1e-3        # (the sum of squares in another order: a last bit here and there)
+
+
+@pytest.mark.parametrize("act,layout", [(0, 16), (1, 0), (2, 0)])
+@pytest.mark.parametrize("T,S", [(1, 2), (50, 2), (50, 6), (200, 2), (200, 3)])
+def test_activation_adds_planes_in_either_way(ops, act, layout, T, S):
+    """Few, some and many blocks: one rounding to bf16 behind fp32 sums."""
+    I = 4096
+    ws, total = _planes(S, T, 2 * I, S)
+    y = torch.empty(T, I, dtype=torch.bfloat16, device="cuda")
+    ops.k.glu_ex(None, y, act, 1.702, 7.0, layout, ws, S, None)
+    x = total.double()
+    if layout == 16:
+        x = x.view(T, I // 16, 2, 16)
+        g, u = x[:, :, 0].reshape(T, I), x[:, :, 1].reshape(T, I)
+    else:
+        g, u = (x[:, 0::2], x[:, 1::2]) if act == 2 else (x[:, :I], x[:, I:])
+    if act == 2:
+        g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
+        ref = g * torch.sigmoid(1.702 * g) * (u + 1)
+    else:
+        ref = (torch.nn.functional.silu(g) if act == 0 else torch.nn.functional.gelu(g, approximate="tanh")) * u
+    assert _rel(y, ref) < 2.5e-3
