@@ -648,6 +648,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a,
 }
 
 // out[i] = bf16(sum_s ws[s][i] + bias), i over a dense [rows][cols] array written with pitch ldc.
+template <int B>
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, int rows, int cols,
                                      long long ldc, const __nv_bfloat16* __restrict__ bias,
                                      __nv_bfloat16* __restrict__ out) {
@@ -656,7 +657,7 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, int splits, i
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  float4 acc = sum_splits4(ws + i4, n, splits);
+  float4 acc = sum_splits4<B>(ws + i4, n, splits);
   const int r = row_of_element(i4, cols);
   const int c = (int)(i4 - (size_t)r * cols);
   if (bias) {
@@ -929,9 +930,9 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
       ex->deferred_splits = splits;
       return 1;
     }
-    const size_t n = (size_t)T * N;
-    launch_pdl(splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float*)partials, splits, T, N, ldy,
-               reinterpret_cast<const __nv_bfloat16*>(bias), reinterpret_cast<__nv_bfloat16*>(y));
+    const unsigned blocks = (unsigned)(((size_t)T * N / 4 + 255) / 256);
+    launch_pdl(eight_planes(blocks, splits) ? splitk_reduce_kernel<8> : splitk_reduce_kernel<4>, dim3(blocks), dim3(256), 0, stream, (const float*)partials,
+               splits, T, N, ldy, reinterpret_cast<const __nv_bfloat16*>(bias), reinterpret_cast<__nv_bfloat16*>(y));
     return 2;
   }
   GemmArgs a{};
@@ -1048,8 +1049,9 @@ int linear_bf16_tp(const void* x, long long ldx, const void* w, long long ldw, c
   }
   if (a.k_splits > 1 && !a.fixup) {
     // dense [token][feature] partials in both orientations
-    const size_t n = (size_t)T * N;
-    launch_pdl(splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float*)a.ws, a.k_splits, T, N, ldy, a.bias, a.out);
+    const unsigned blocks = (unsigned)(((size_t)T * N / 4 + 255) / 256);
+    launch_pdl(eight_planes(blocks, a.k_splits) ? splitk_reduce_kernel<8> : splitk_reduce_kernel<4>, dim3(blocks), dim3(256), 0, stream, (const float*)a.ws,
+               a.k_splits, T, N, ldy, a.bias, a.out);
     return 2;
   }
   return 1;

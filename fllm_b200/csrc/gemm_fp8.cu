@@ -331,6 +331,7 @@ gemm_fp8_block_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
 }
 
 // out[t][n] = bf16(sum_s ws[s][t][n] + bias[n])
+template <int B>
 __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ ws, int splits, int rows, int cols, long long ldc,
                                          const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
@@ -338,7 +339,7 @@ __global__ void fp8_splitk_reduce_kernel(const float* __restrict__ ws, int split
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  const float4 acc = sum_splits4(ws + i4, n, splits);
+  const float4 acc = sum_splits4<B>(ws + i4, n, splits);
   const int r = row_of_element(i4, cols);
   const int c = (int)(i4 - (size_t)r * cols);
   float b[4] = {0.f, 0.f, 0.f, 0.f};
@@ -507,8 +508,9 @@ int linear_fp8_block(const void* xq, const float* sx, const void* wq, const floa
     return 2;
   }
   if (a.k_splits > 1) {
-    const size_t n = (size_t)T * N;
-    launch_pdl(fp8_splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream, (const float*)a.ws, a.k_splits, T, N, ldy, a.bias, a.out);
+    const unsigned blocks = (unsigned)(((size_t)T * N / 4 + 255) / 256);
+    launch_pdl(eight_planes(blocks, a.k_splits) ? fp8_splitk_reduce_kernel<8> : fp8_splitk_reduce_kernel<4>, dim3(blocks), dim3(256), 0, stream, (const float*)a.ws,
+               a.k_splits, T, N, ldy, a.bias, a.out);
     return 2;
   }
   return 1;

@@ -306,6 +306,7 @@ gemm_mx_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant_
 }
 
 // out[n][m] = bf16(alpha * sum_s ws[s][n][m] + bias[m])
+template <int B>
 __global__ void mx_splitk_reduce_kernel(const float* __restrict__ ws, int splits, int rows, int cols, long long ldc,
                                         float alpha, const float* __restrict__ tok_scale,
                                         const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out) {
@@ -314,7 +315,7 @@ __global__ void mx_splitk_reduce_kernel(const float* __restrict__ ws, int splits
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  const float4 acc = sum_splits4(ws + i4, n, splits);
+  const float4 acc = sum_splits4<B>(ws + i4, n, splits);
   const int r = row_of_element(i4, cols);
   const int c = (int)(i4 - (size_t)r * cols);
   float b[4] = {0.f, 0.f, 0.f, 0.f};
@@ -584,8 +585,8 @@ int linear_mx(const void* xq, const void* sfb, const void* wq, const void* sfa, 
   else if (kind == kMxKindRowF8) launch_mx_bn<kMxKindRowF8>(bn, ta, tb, a, stream);
   else launch_mx_bn<kMxKindRowI8>(bn, ta, tb, a, stream);
   if (a.k_splits > 1) {
-    const size_t n = (size_t)T * N;
-    launch_pdl(mx_splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream,
+    const unsigned blocks = (unsigned)(((size_t)T * N / 4 + 255) / 256);
+    launch_pdl(eight_planes(blocks, a.k_splits) ? mx_splitk_reduce_kernel<8> : mx_splitk_reduce_kernel<4>, dim3(blocks), dim3(256), 0, stream,
                (const float*)a.ws, a.k_splits, T, N, ldy, alpha, tok_scale, a.bias, a.out);
     return 2;
   }

@@ -553,6 +553,7 @@ void rows_f16(const void* x, long long ldx, const int* token_of, const float* ro
 }
 
 // out[n][m] = bf16(alpha * sum_s ws[s][n][m] + bias[m])
+template <int B>
 __global__ void w4_splitk_reduce_kernel(const float* __restrict__ ws, int splits, int rows, int cols, long long ldc,
                                         float alpha, const __nv_bfloat16* __restrict__ bias, __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
@@ -560,7 +561,7 @@ __global__ void w4_splitk_reduce_kernel(const float* __restrict__ ws, int splits
   const size_t n = (size_t)rows * cols;
   const size_t i4 = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i4 >= n) return;
-  const float4 acc = sum_splits4(ws + i4, n, splits);
+  const float4 acc = sum_splits4<B>(ws + i4, n, splits);
   const int r = row_of_element(i4, cols);
   const int c = (int)(i4 - (size_t)r * cols);
   float b[4] = {0.f, 0.f, 0.f, 0.f};
@@ -704,8 +705,8 @@ int linear_w4a16(const void* x, long long ldx, const void* codes, const void* sc
   CUtensorMap tb = make_tmap_parts(x, T, K, bn, 4, ldx * 2);
   launch_w4_bn(bn, tr, tb, a, a.m_tiles * a.k_splits, stream);
   if (a.k_splits > 1) {
-    const size_t n = (size_t)T * N;
-    launch_pdl(w4_splitk_reduce_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, stream,
+    const unsigned blocks = (unsigned)(((size_t)T * N / 4 + 255) / 256);
+    launch_pdl(eight_planes(blocks, a.k_splits) ? w4_splitk_reduce_kernel<8> : w4_splitk_reduce_kernel<4>, dim3(blocks), dim3(256), 0, stream,
                (const float*)a.ws, a.k_splits, T, N, ldy, alpha, a.bias, reinterpret_cast<__nv_bfloat16*>(a.out));
     ++launches;
   }

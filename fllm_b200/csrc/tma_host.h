@@ -139,6 +139,13 @@ inline bool first_call_on_device(bool (&done)[kMaxDevices]) {
   return true;
 }
 
+inline int sm_count();
+// Whether a kernel that adds partial sums alone has eight planes on their way in 63 registers (four CTAs of 256 threads on an SM), or four in 48: where there are
+// more of them than four at a time add quickly, and all CTAs are on the SMs at once but not so few that an SM has one. us with four and eight,
+// product included: 100 x 2048 x 2048 behind 8 9.1, 8.3; 64 x 4096 x 4096 behind 8 11.6, 10.8; 100 x 1024 x 4096 behind 12 8.5, 9.2; 160 x 4096 x 4096
+// behind 6 20.8, 21.8.
+inline bool eight_planes(unsigned ctas, int splits) { return splits >= 6 && ctas > (unsigned)sm_count() && ctas <= 4u * sm_count(); }
+
 inline int sm_count() {
   static int n[16] = {0};
   int dev = 0;

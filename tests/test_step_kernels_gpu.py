@@ -434,3 +434,18 @@ def test_activation_adds_planes_in_either_way(ops, act, layout, T, S):
     else:
         ref = (torch.nn.functional.silu(g) if act == 0 else torch.nn.functional.gelu(g, approximate="tanh")) * u
     assert _rel(y, ref) < 2.5e-3
+
+
+@pytest.mark.parametrize("T,S", [(16, 8), (100, 8), (100, 5), (256, 9)])
+def test_product_adds_planes_in_either_way(ops, T, S):
+    """Fewer and more blocks than SMs, planes on both sides of a batch: the bits of the planes added in their order."""
+    x, w, b = _rand((T, 2304), 1), _rand((2048, 2304), 2, 0.05), _rand((2048,), 3)
+    y = torch.empty(T, 2048, dtype=torch.bfloat16, device="cuda")
+    ops.k.linear(x, w, b, y, ops.workspace, ops.status, S)
+    n = T * 2048
+    p = ops.workspace[65536:65536 + S * n * 4].view(torch.float32).view(S, T, 2048)
+    total = p[0].clone()
+    for s in range(1, S):
+        total += p[s]
+    assert torch.equal(y, (total + b.float()).to(torch.bfloat16)) and _rel(y, x.double() @ w.double().t() + b.double()) < 2.5e-3
+    assert ops.check_status() == 0
