@@ -121,6 +121,30 @@ def test_routed_experts_end_to_end(ops, counts, k, act, limit, weigh):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("counts,k,tile", [((65, 97, 106, 0), 1, 96), ((130, 129, 1), 1, 128), ((100, 70, 110), 2, 128), ((1, 0, 299), 1, 128)])
+@pytest.mark.parametrize("act,limit", [("swiglu_oai", 7.0), ("swiglu_oai", 100.0), ("swiglu", 7.0)])
+@pytest.mark.parametrize("weigh", [False, True])
+def test_many_rows_an_expert_end_to_end(ops, counts, k, tile, act, limit, weigh):
+    """More than 64 rows an expert in the mean: MXFP4 stacks are expanded to fp16, on tiles of 96 and 128. Roundings as in
+    test_routed_experts_end_to_end."""
+    from types import SimpleNamespace
+    from fllm_b200.models.moe import _mx_tile, _packed_tile
+    mean = sum(counts) / len(counts)
+    stack = SimpleNamespace(atoms=torch.empty(1))
+    assert _mx_tile(SimpleNamespace(exp_gate_up=stack, exp_down=stack), mean) == 0 and _packed_tile(mean) == tile
+    assert _experts(ops, counts, k, act, limit, weigh=weigh) < 5 * 1.7e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("limit", [7.0, 100.0, 240.0])
+@pytest.mark.parametrize("size", [1.0, 2.0 ** -10, 2.0 ** -18])
+def test_small_activations_of_many_rows(ops, limit, size):
+    """As test_small_activations_of_experts, with more than 64 rows an expert: one factor for all rows of the activation, and rows
+    converted again under the limits that leave it too little."""
+    assert _experts(ops, [90, 70, 50], 2, "swiglu_oai", limit, size) < 4 * 1.7e-3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("at", [0, 16, 32])
 @pytest.mark.parametrize("act", ["swiglu_oai", "swiglu"])
 def test_stacks_that_start_on_16_bytes(ops, monkeypatch, at, act):
