@@ -80,7 +80,8 @@ int64_t moe_grouped_linear_w4_f16(const Tensor& xp, const optional<Tensor>& fact
 }
 
 // x bf16 [tokens, k] -> two pieces of e4m3 per row, xq bytes [rows * 2, k] in groups of 16 rows, and their scale atoms (csrc/gemm_mx4_rows.cu: rows_mx)
-void moe_rows_mx(const Tensor& x, const optional<Tensor>& token_of, Tensor xq, Tensor sf, int64_t bn, const optional<Tensor>& row_weight) {
+void moe_rows_mx(const Tensor& x, const optional<Tensor>& token_of, Tensor xq, Tensor sf, int64_t bn, const optional<Tensor>& row_weight,
+                 bool placed) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1, "x: bf16 rows");
   TORCH_CHECK(xq.is_cuda() && xq.element_size() == 1 && xq.dim() == 2 && xq.is_contiguous() && xq.size(1) == x.size(1) && xq.size(0) % 2 == 0, "xq: contiguous bytes [rows * 2, k]");
   const int64_t rows = xq.size(0) / 2;
@@ -90,16 +91,15 @@ void moe_rows_mx(const Tensor& x, const optional<Tensor>& token_of, Tensor xq, T
   if (token_of.has_value() && token_of->defined()) {
     TORCH_CHECK(token_of->scalar_type() == at::kInt && token_of->is_contiguous() && token_of->numel() >= rows, "token_of: int32 [rows]");
     t = token_of->data_ptr<int>();
-  } else {
-    TORCH_CHECK(rows <= x.size(0), "xq: as many rows as x");
   }
+  TORCH_CHECK((t != nullptr && !placed) || rows <= x.size(0), "xq: as many rows as x");
   const float* w = nullptr;
   if (row_weight.has_value() && row_weight->defined()) {
     TORCH_CHECK(row_weight->scalar_type() == at::kFloat && row_weight->is_contiguous() && row_weight->numel() >= rows, "row_weight: fp32 [rows]");
     w = row_weight->data_ptr<float>();
   }
   c10::cuda::CUDAGuard guard(x.device());
-  fllm::rows_mx(x.data_ptr(), x.stride(0), t, w, xq.data_ptr(), sf.data_ptr(), (int)rows, (int)x.size(1), (int)bn, cur_stream());
+  fllm::rows_mx(x.data_ptr(), x.stride(0), t, placed, w, xq.data_ptr(), sf.data_ptr(), (int)rows, (int)x.size(1), (int)bn, cur_stream());
 }
 
 // Grouped product of such rows (`pieces` each) with a stack of MXFP4 matrices: codes [E, n, k/2] bytes, atoms [E, ceil(n / 128), ceil(k / 128), 512] their
@@ -209,7 +209,7 @@ TORCH_LIBRARY_FRAGMENT(fllm_b200, m) {
   m.def("moe_grouped_linear_w4(Tensor xp, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status) -> int", &moe_grouped_linear_w4);
   m.def("moe_rows_f16(Tensor x, Tensor? token_of, Tensor(a!) xp, Tensor(b!) factor, Tensor? row_weight=None) -> ()", &moe_rows_f16);
   m.def("moe_grouped_linear_w4_f16(Tensor xp, Tensor? factor, Tensor codes, Tensor scales, int fmt, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor tile_expert, Tensor tile_row0, Tensor num_tiles, int bn, Tensor? status, float glu_alpha=1.0, float glu_limit=0.0, float glu_scale=0.0) -> int", &moe_grouped_linear_w4_f16);
-  m.def("moe_rows_mx(Tensor x, Tensor? token_of, Tensor(a!) xq, Tensor(b!) sf, int bn, Tensor? row_weight=None) -> ()", &moe_rows_mx);
+  m.def("moe_rows_mx(Tensor x, Tensor? token_of, Tensor(a!) xq, Tensor(b!) sf, int bn, Tensor? row_weight=None, bool placed=False) -> ()", &moe_rows_mx);
   m.def("moe_grouped_linear_mx4(Tensor xq, Tensor sf, int pieces, Tensor codes, Tensor atoms, float alpha, Tensor? bias_stack, Tensor(a!) y, Tensor(b!)? y_sf, Tensor tile_expert, Tensor tile_row0, Tensor tile_rows, Tensor num_tiles, int bn, Tensor? status, float glu_alpha=1.0, float glu_limit=0.0) -> int", &moe_grouped_linear_mx4);
   m.def("ep_ctx_create(int ranks, int my_rank, int cap, int hidden, int experts_per_rank, int[] recv_x, int[] recv_meta, int[] ctrl, int[] comb_y) -> int", &ep_ctx_create);
   m.def("ep_dispatch(int ctx, Tensor x, Tensor ids, int epoch, Tensor? status, Tensor(a!)? call_ctr=None) -> ()", &ep_dispatch);

@@ -178,7 +178,8 @@ struct Mx4Glu {               // clamped SwiGLU-OAI in the epilogue; its result 
   void *q, *sf;
 };
 size_t mx4_scale_bytes(int rows, int K, int bn, int pieces);
-void rows_mx(const void* x, long long ldx, const int* token_of, const float* row_weight, void* xq, void* sf, int rows, int K, int bn, cudaStream_t s);
+void rows_mx(const void* x, long long ldx, const int* token_of, bool placed, const float* row_weight, void* xq, void* sf, int rows, int K, int bn,
+             cudaStream_t s);
 int moe_grouped_linear_mx4(const Mx4Rows& x, const void* codes, const void* sfa, int experts, int n_out, int K, float alpha, const void* bias, void* y,
                            long long ldy, const Mx4Glu* glu, const Mx4Tiles& tiles, int* status, cudaStream_t stream);
 void w4_dequant_bf16(const void* codes, const void* scales, int fmt, float alpha, void* out, long long rows, int K,

@@ -409,8 +409,9 @@ gemm_mx4_rows_kernel(const __grid_constant__ Mx4Maps maps, const Mx4Args p) {
 
 // Rows of bf16 -> two pieces of e4m3 and their scale atoms, in the order of gemm_mx4_rows_kernel: row r of a tile of bn tokens goes to rows
 // (r / 16) 32 + r % 16 and + 16 of the tile. One CTA per row, half a warp per 128 values. token_of (optional): rows without a token (-1) become
-// zeros, groups of 16 without any are left out. row_weight (optional): routers that weigh an expert's input (rounded to bf16, as there).
-__global__ void __launch_bounds__(192) rows_mx_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ token_of,
+// zeros, groups of 16 without any are left out. placed: x has the rows of the tiles already (an activation between the products). row_weight
+// (optional): routers that weigh an expert's input (rounded to bf16, as there).
+__global__ void __launch_bounds__(192) rows_mx_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ token_of, int placed,
                                                       const float* __restrict__ row_weight, uint8_t* __restrict__ xq, uint8_t* __restrict__ sf, int K, int bn) {
   pdl_launch_dependents();
   pdl_wait();
@@ -419,6 +420,7 @@ __global__ void __launch_bounds__(192) rows_mx_kernel(const __nv_bfloat16* __res
   if (token_of != nullptr) {
     if (token_of[row & ~(M4_G - 1)] < 0) return;              // tokens fill a tile from its start
     t = token_of[row];
+    if (placed && t >= 0) t = row;
   }
   const float rw = row_weight != nullptr && t >= 0 ? row_weight[row] : 1.f;
   const int tile = row / bn, in = row - tile * bn, r0 = (in / M4_G) * (2 * M4_G) + (in % M4_G), atoms = (2 * bn + 127) / 128;
@@ -452,12 +454,13 @@ __global__ void __launch_bounds__(192) rows_mx_kernel(const __nv_bfloat16* __res
   }
 }
 
-void rows_mx(const void* x, long long ldx, const int* token_of, const float* row_weight, void* xq, void* sf, int rows, int K, int bn, cudaStream_t s) {
+void rows_mx(const void* x, long long ldx, const int* token_of, bool placed, const float* row_weight, void* xq, void* sf, int rows, int K, int bn,
+             cudaStream_t s) {
   if (rows <= 0) return;
   if ((K & 63) || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(xq) & 15) || (reinterpret_cast<uintptr_t>(sf) & 15))
     throw std::runtime_error("rows_mx: K % 64 and 16-byte rows required");
   if (bn % M4_G || rows % bn) throw std::runtime_error("rows_mx: whole tiles of a multiple of 16 rows");
-  launch_pdl(rows_mx_kernel, dim3(rows), dim3(192), 0, s, (const __nv_bfloat16*)x, ldx, token_of, row_weight, (uint8_t*)xq, (uint8_t*)sf, K, bn);
+  launch_pdl(rows_mx_kernel, dim3(rows), dim3(192), 0, s, (const __nv_bfloat16*)x, ldx, token_of, placed ? 1 : 0, row_weight, (uint8_t*)xq, (uint8_t*)sf, K, bn);
 }
 
 template <int BN, int P, bool GLU>

@@ -235,7 +235,7 @@ def _mx_ffn(cfg, ops, spec: MoeSpec, lw, x: torch.Tensor, token_of, row_w, tile_
         k_ops.moe_grouped_linear_mx4(xq, xs, 2, gu.codes, gu.atoms, gu.alpha, lw.exp_gate_up_b, u, None, *where)
         u = ops.act_(u, spec.act) if cfg.mlp_kind == "plain" else ops.glu(u, ACT_KIND.get(spec.act, 0), cfg.swiglu_alpha, limit)
         aq, as_ = room(2, u.shape[1])
-        k_ops.moe_rows_mx(u, None, aq, as_, bn)
+        k_ops.moe_rows_mx(u, token_of, aq, as_, bn, None, True)      # (rows of padding are left out: half of them in a tile that is half full)
     y = torch.empty(rows, H, dtype=torch.bfloat16, device=x.device)
     k_ops.moe_grouped_linear_mx4(aq, as_, pieces, dn.codes, dn.atoms, dn.alpha, lw.exp_down_b, y, None, *where)
     return y

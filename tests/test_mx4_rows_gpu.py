@@ -133,3 +133,29 @@ def test_rows_of_a_tile(ops):
     row_of, token_of, te, tr, tn, num = ids.clone(), i32(160), i32(10), i32(10), i32(10), i32(2)
     ops.k.moe_align(ids, 5, 0, 5, 16, row_of, token_of, te, tr, num, None, None, tn)
     assert num.tolist() == [5, 80] and te.tolist()[:5] == [0, 0, 0, 2, 3] and tn.tolist()[:5] == [16, 16, 1, 16, 1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bn", [16, 80])
+def test_rows_that_are_in_place(ops, bn):
+    """An activation between the products lies in the rows of the tiles: those with a token are converted as they are, the others of their group of 16 are zeros,
+    and groups without a token stay as they were."""
+    K, rows = 192, 2 * 80
+    x = _rand((rows, K), 1)
+    token_of = torch.full((rows,), -1, dtype=torch.int32)
+    at = [0, 1, 17, 80, 95, 96] if bn == 80 else [0, 1, 80, 95]
+    at = sorted({*at, *(r // 16 * 16 for r in at)})
+    token_of[at] = torch.arange(len(at) - 1, -1, -1, dtype=torch.int32)          # (which token a row has does not matter here)
+    x[[r for r in range(rows) if token_of[r] < 0]] = float("nan")
+    q, sf = _room(rows, K, bn, 2)
+    ops.k.moe_rows_mx(x.cuda(), token_of.cuda(), q, sf, bn, None, True)
+    got = _values(q, sf, bn, 2)
+    whole, wsf = _room(rows, K, bn, 2)
+    ops.k.moe_rows_mx(x.cuda(), None, whole, wsf, bn)
+    assert torch.equal(got[at], _values(whole, wsf, bn, 2)[at])
+    used = {r // 16 for r in at}
+    assert (got[[r for r in range(rows) if r // 16 in used and token_of[r] < 0]] == 0).all()
+    pieces = q.view(rows // 16, 2 * 16, K)
+    assert all((pieces[g] == 0xFF).all() for g in range(rows // 16) if g not in used)
+    with pytest.raises(RuntimeError, match="as many rows"):
+        ops.k.moe_rows_mx(x[:rows - 16].cuda(), token_of.cuda(), q, sf, bn, None, True)
