@@ -119,6 +119,14 @@ class EpAllToAll:
         return code
 
 
+def release_scale_atoms(layers) -> None:
+    """The experts below multiply expanded codes: their stacks need no second order of the scales (``ops.fp4.Fp4ExpertStack``)."""
+    for lw in layers:
+        for w in (lw.exp_gate_up, lw.exp_down):
+            if hasattr(w, "drop_atoms"):
+                w.drop_atoms()
+
+
 def moe_ffn_a2a_phases(dec, lw, ep: EpAllToAll, h_owned: torch.Tensor):
     """The MoE layer of one rank in all-to-all mode as a generator of phases (route+dispatch |
     expert compute+return | combine), so that a single-GPU test can interleave virtual ranks. The

@@ -101,6 +101,12 @@ class LLMEngine:
                                            kv_tier_host_gb=0.0, kv_tier_disk_gb=0.0)
         self.block_size = self.cfg.block_size
         self.max_blocks_per_seq = -(-self.cfg.max_model_len // self.block_size)
+        alltoall = (self.is_cuda and model_cfg.is_moe and self.par.expert_parallel and self.par.ep_dispatch == "alltoall"
+                    and tp > 1 and getattr(tp_group, "group", None) is not None)
+        if alltoall:
+            from ..comm.ep_a2a import release_scale_atoms
+            release_scale_atoms(self.weights.layers)
+            torch.cuda.empty_cache()                     # the pool is sized by what the device has free
         num_blocks = self.cfg.num_kv_blocks or self._size_kv_pool()
         if self.cfg.kv_cache_dtype not in ("bf16", "fp8", "fp8_e4m3", "fp32"):
             raise ValueError("kv_cache_dtype must be bf16 or fp8_e4m3")
@@ -127,8 +133,7 @@ class LLMEngine:
                                layer_range=self.layer_range, first_stage=self.first_stage,
                                last_stage=self.last_stage, rstate=self.rstate)
         # expert parallel with all-to-all dispatch: peer buffers for the rows each rank owns
-        if (self.is_cuda and model_cfg.is_moe and self.par.expert_parallel and self.par.ep_dispatch == "alltoall"
-                and tp > 1 and getattr(tp_group, "group", None) is not None):
+        if alltoall:
             from ..comm.ep_a2a import EpAllToAll
             rows = -(-self.cfg.max_num_batched_tokens // tp)
             self.decoder.ep_a2a = EpAllToAll(tp, tp_rank, model_cfg.hidden_size, model_cfg.num_experts // tp, rows,

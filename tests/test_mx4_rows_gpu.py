@@ -45,6 +45,31 @@ def test_scale_atoms_hold_every_scale():
     assert a[0, 1, 0, (100 % 32) * 16 + (100 // 32) * 4] == 127 and a[0, 0, 1, 2] == 127
 
 
+def test_bytes_of_a_stack_count_its_atoms():
+    from types import SimpleNamespace
+    from fllm_b200.comm.ep_a2a import release_scale_atoms
+    s = Fp4ExpertStack.from_dense(_rand((2, 128, 192), 3))
+    plain = 2 * 128 * 96 + 2 * 128 * 6
+    assert s.atoms is None and s.nbytes() == plain
+    s.atoms = scale_atoms(s.scales)
+    assert s.nbytes() == plain + 2 * 1 * 2 * 512
+    release_scale_atoms([SimpleNamespace(exp_gate_up=s, exp_down=torch.empty(1)), SimpleNamespace(exp_gate_up=None, exp_down=None)])
+    assert s.atoms is None and s.nbytes() == plain
+
+
+@pytest.mark.gpu
+def test_stacks_reach_the_gpu_in_one_copy():
+    """K ends in the middle of a block: the bytes behind the codes are there from the start. Codes, a sixteenth of them in scales, as much in
+    atoms and in what these are made from; a second copy of the codes would be another whole."""
+    s = Fp4ExpertStack.from_dense(_rand((4, 2048, 1984), 3))
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    g = s.to("cuda")
+    assert torch.cuda.max_memory_allocated() - before < 1.6 * s.codes.numel()
+    assert g.atoms is not None and torch.equal(g.codes.cpu(), s.codes) and g.codes.untyped_storage().nbytes() == s.codes.numel() + 32
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("bn", [16, 32, 80])
 @pytest.mark.parametrize("K", [64, 320, 2880, 8192])
