@@ -364,7 +364,7 @@ __device__ __forceinline__ void store_rows(const FaTmemParams& p, uint32_t t_o, 
   }
 }
 
-// The CTA's sequence and query tile when it is the blockIdx.x-th tile of all prompts; false past the last. (A CTA per tile and sequence
+// The sequence and query tile that are the `want`-th of all prompts; false past the last. (A CTA per tile and sequence
 // leaves the decode rows of a mixed step CTAs that find nothing to do, each of which still takes an SM for its launch: 200 rows beside a prompt
 // of 1500, 64 query and 8 key heads of 64, window of 128: 442 -> 77 us with the decode rows.) Called by all THREADS; sums over as many sequences
 // at a time.
@@ -568,7 +568,7 @@ fa_prefill_tmem_kernel(const __grid_constant__ CUtensorMap tma_k, const __grid_c
 //
 // What bounds it: the chain of a group (softmax, PV, next S), 3000 to 3300 clocks per tile where the tensor pipe and the exponentials need 2048
 // each for both groups. A row's scores stay in registers (one pass over tensor memory instead of two; the warps that need no registers leave
-// theirs), two of them to an instruction, and PV of the first 64 tokens runs while the others' exponentials are computed. (Two S buffers of 64 tokens
+// theirs; compiled for the 168 of the launch, a thread spills 48 bytes and reads 188 back), two of them to an instruction, and PV of the first 64 tokens runs while the others' exponentials are computed. (Two S buffers of 64 tokens
 // per tile are slower: products of 64 columns read Q twice as often. A share of the exponentials on the multiply-add pipe gave
 // 1 % at best.) One lane walks the issuer's loop: five waits voted on by its warp and five elected regions cost 1850 of a tile's 3570
 // clocks. The grid runs over the key heads first and from a sequence's longest tiles to its shortest, so that the last CTAs to start are short:

@@ -98,7 +98,7 @@ void* symm_import(const unsigned char in[64]);
 void symm_close(void* p);
 
 // ---- block-scaled FP8 ------------------------------------------------------------------
-// Large-batch bf16 GEMM on CTA pairs (tcgen05 cta_group::2, 256 x 256 tiles): T > 128, N >= 256, N % 8 == 0, K >= 64, K % 8 == 0.
+// Large-batch bf16 GEMM on CTA pairs (tcgen05 cta_group::2, tiles of 256 tokens x `width` features): T > 128, N >= 256, N % 8 == 0, K >= 64, K % 8 == 0.
 bool linear_bf16_pair_supported(int T, int N, int K);
 int linear_bf16_pair(const void* x, long long ldx, const void* w, long long ldw, const void* bias, void* y, long long ldy,
                      int T, int N, int K, int* status, cudaStream_t stream, const struct LinearExtras* ex = nullptr, int splits = 1,

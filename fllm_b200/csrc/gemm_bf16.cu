@@ -856,12 +856,15 @@ int linear_bf16_plan_pair(int T, int N, int K, int sms, size_t workspace_bytes, 
   return splits;
 }
 
-// What a product takes: one-CTA tiles (splits 0) or pairs, whole or over splits as for square tiles, with the number of splits and the width of a tile (96 .. 256
-// features) that are fastest then. Square tiles leave most clusters without work in their last round, which is the second one for 129 to 256
+// What a product takes. One-CTA tiles (splits 0), pairs, or pairs over splits, is chosen for square tiles by the function above; behind that, the number of
+// splits (from two on, if any) and the width of a tile (96 .. 256 features) that are fastest. So a product that narrow pairs alone would win stays on
+// one-CTA tiles or on splits: 200 x 6144 x 4096 takes two splits of 192, 21.3 us, where whole tiles of 96 take 20.3.
+// Square tiles leave most clusters without work in their last round, which is the second one for 129 to 256
 // tokens of the usual matrices: 200 x 24576 x 4096 has 96 of them for 74 clusters, and 128 of 192 features. In units of 10 ns, fitted to 1100
 // products of 2048 .. 24576 features, K of 2048 .. 12288 and 140 .. 2048 tokens (7 % off in the mean): a K block takes 12.4 and 0.062 a
-// feature, a round 1.9 a feature less 86. Partial sums cost the same whether their consumer adds them or a kernel, so that both give the same bits. us, square
-// tiles over the best number of splits -> this: 200 x 24576 x 4096 57.5 -> 49.4, 200 x 6144 x 4096 22.9 -> 21.3, 200 x 4096 x 4096 17.0 -> 14.9,
+// feature, a round 1.9 a feature less 86. Partial sums cost the same here whether their consumer adds them or a kernel. (The choice for square tiles leaves
+// the launch of that kernel out where a consumer adds them, so a product may have another number of splits then, and other last bits.) us, square
+// tiles over the best number of splits -> this: 200 x 24576 x 4096 57.5 -> 49.4, 200 x 6144 x 4096 22.9 -> 21.3,
 // 512 x 6144 x 4096 29.4 -> 24.4, 768 x 4096 x 4096 27.2 -> 22.6, 1024 x 6144 x 4096 48.2 -> 39.9, 2048 x 24576 x 4096 266.8 -> 264.6.
 PairPlan linear_bf16_plan_width(int T, int N, int K, int sms, size_t workspace_bytes, bool gated, bool deferred) {
   PairPlan plan{linear_bf16_plan_pair(T, N, K, sms, workspace_bytes, gated, deferred), 256};

@@ -1,11 +1,12 @@
 // Dense bf16 GEMM for large token counts on CTA pairs (tcgen05 cta_group::2):  y[T, N] = x[T, K] * w[N, K]^T (+ bias)
 //
-// Two CTAs of a cluster (two SMs) work on one 256 x 256 output tile. Each CTA stages its own 128 token rows
-// of x and only its own half (128 feature rows) of the weight tile; one thread of the even CTA issues
-// tcgen05.mma.cta_group::2 (256 x 256 x 16 per instruction) and the hardware feeds both tensor cores with
-// both halves of the weight tile. Against the one-CTA 128 x 256 tile of gemm_bf16.cu a stage shrinks from
+// Two CTAs of a cluster (two SMs) work on one output tile of 256 tokens x `width` features, 32 to 256 of them. Each CTA
+// stages its own 128 token rows of x and only its own half (width / 2 feature rows) of the weight tile; one thread of the
+// even CTA issues tcgen05.mma.cta_group::2 (256 x width x 16 per instruction) and the hardware feeds both tensor cores with
+// both halves of the weight tile. Against the one-CTA 128 x 256 tile of gemm_bf16.cu a stage of the widest tile shrinks from
 // 48 KB to 32 KB per SM for the same arithmetic, so seven stages instead of four cover the load latency, and
-// every weight byte is read from shared memory by one SM instead of two.
+// every weight byte is read from shared memory by one SM instead of two. Narrower tiles fill rounds over the clusters that
+// 256 features would leave half empty (linear_bf16_plan_width).
 //
 //   TMA (both CTAs, `.cta_group::2` form: the bytes of both land on the even CTA's barrier; no cluster multicast)
 //   -> 128-byte-swizzled ring -> tcgen05.mma.cta_group::2 -> accumulators in both CTAs' tensor memory
@@ -24,9 +25,9 @@
 
 namespace fllm {
 
-constexpr int P2_ROWS = 128;                 // rows of either operand per CTA per stage
+constexpr int P2_ROWS = 128;                 // token rows, and at most as many weight rows, per CTA per stage
 constexpr int P2_BK = 64;                    // 64 bf16 = one 128-byte swizzle row
-constexpr int P2_TILE = 256;                 // tile edge of the pair (tokens and features)
+constexpr int P2_TILE = 256;                 // tokens of a tile, and features of the widest
 constexpr int P2_STAGES = 7;
 constexpr int kP2Threads = 192;
 constexpr int kP2OperandBytes = P2_ROWS * P2_BK * 2;          // 16 KB

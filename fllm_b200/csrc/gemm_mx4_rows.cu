@@ -6,7 +6,10 @@
 // tcgen05.mma kind::mxf8f6f4 multiplies e2m1 codes as they are and applies their scales, but its other operand has 8 bits. So a row is
 // written as a sum of P rows of e4m3 with a scale per 32 values each: the first holds the value rounded to four significant bits, the next what
 // is left of it, and so on. Two pieces hold the 8 bits of a bf16 value (exact down to 2^-12 of its block's largest, off by less than 2^-21 of that
-// below), three 12 bits and a sign of a wider one, one more than fp16. The pieces are further columns of the same product
+// below), three 12 bits and a sign of a wider one, one more than fp16. (What this holds less than rows of fp16 with a factor each, which keep eight
+// bits down to 2^-31 of a row's largest: small values beside a very large one in the same 32. Error of a layer of 2880 x 2880 x 3 against 64 bits, fp16 rows
+// and this: 0.2365 %, 0.2355 % on normal rows; with every 640th value 30 to 3000 times as large the same or less, 3e4 times 0.2359, 0.2391 and 3e5 times 0.236,
+// 0.516 where the weights of those values are zeros, 0.235 in both where they are not.) The pieces are further columns of the same product
 // (accumulators of their own, added up in fp32 by the epilogue), so a tile of codes is read once for all of them, and a
 // piece costs half of a bf16 product.
 //

@@ -126,7 +126,8 @@ def _token_tile(rows_per_expert: float) -> int:
 def _packed_tile(rows_per_expert: float) -> int:
     """Token tile of packed experts, whose weights are expanded once per tile: the smallest that nearly every expert fits into (rows
     spread around their mean by its root). A wider one multiplies padding: 64 rows a mean, 128 experts of 2880 x 2880 x 3: tiles of 96 need
-    three quarters of the products of 128 and half of the expansion of 64."""
+    three quarters of the products of 128 and half of the expansion of 64. (MXFP4 stacks with scale atoms come here above 64 rows, for tiles of 96
+    and 128; the narrow ones are for stacks without: NVFP4, and codes that do not start on 32 bytes.)"""
     most = rows_per_expert + 3 * math.sqrt(rows_per_expert)
     for bn in (16, 32, 64, 96):
         if most <= bn:
@@ -137,8 +138,10 @@ def _packed_tile(rows_per_expert: float) -> int:
 def _mx_tile(lw, rows_per_expert: float) -> int:
     """Token tile of MXFP4 experts on the block-scaled tensor cores (csrc/gemm_mx4_rows.cu), 0: expanded to fp16. A tile's products and reads follow the rows
     that it has, so a wider one costs slots of codes in flight alone. Tiles hold 80 rows, which nearly every expert of 64 in the mean fits into; with 96 in
-    the mean most experts need two, and the fp16 form's tiles of 128 are faster (us per layer of 128 experts of 2880 x 2880 x 3: 624 against 674 at 64 rows
-    per expert, 1065 against 800 at 96)."""
+    the mean most experts need two, and the fp16 form's tiles of 128 are faster (us per layer of 128 experts of 2880 x 2880 x 3: 615 against 668 at 64 rows
+    per expert, 1065 against 800 at 96). Of the fp16 form's time at means of 0.25 to 64, router logits even or with a bias of unit spread: 128 and 32 experts of
+    2880 x 2880 x 3 0.69 to 0.94, 64 of 2048 x 1024 x 3 0.77 to 0.96, 8 of 4096 x 14336 x 3 0.67 to 0.99, all with the clamped activation; with SwiGLU between
+    the products 16 of 5120 x 8192 x 3 0.66 to 0.88, 8 of 4096 x 14336 x 3 0.68 to 0.95, 128 of 2048 x 768 x 3 0.79 to 0.97."""
     if any(getattr(w, "atoms", None) is None for w in (lw.exp_gate_up, lw.exp_down)) or rows_per_expert > 64:
         return 0
     most = rows_per_expert + 3 * math.sqrt(rows_per_expert)

@@ -149,7 +149,8 @@ def scale_atoms(scales: torch.Tensor) -> torch.Tensor:
 class Fp4ExpertStack:
     """The matrices of several experts held packed: codes [E, N, K/2], scales [E, N, K/block] (bytes).
     ``moe_ffn`` hands it to the grouped packed GEMM; gpt-oss checkpoints store their experts this way
-    (MXFP4), so the bytes go from the file to the tensor core unexpanded. As with ``Fp4Weight``, other scales are another stack."""
+    (MXFP4), so the bytes go from the file to the tensor core unexpanded. As with ``Fp4Weight``, other scales are another stack; so are
+    other codes: ``codes`` may be a copy of the caller's, with room behind it."""
 
     def __init__(self, codes: torch.Tensor, scales: torch.Tensor, fmt: int, alpha: float = 1.0):
         self.codes, self.scales, self.fmt, self.alpha = codes.contiguous(), scales.contiguous(), int(fmt), float(alpha)
